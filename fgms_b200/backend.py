@@ -3,7 +3,9 @@
 The reference exports three functions from ``backend/pybind_cuda.cpp:8-10`` (prototypes in
 ``backend/spconv.h:10-49``).  The functions below keep their names, positional signatures,
 in-place accumulate semantics and error behaviour, and forward to the C ABI of
-``libfgms_b200.so`` with raw device pointers — this file is the only torch-aware layer.
+``libfgms_b200.so`` with raw device pointers.  The calls of the operator surface go through the extension module
+``_native`` (``csrc/torch_binding.cpp``), whose checks and launches cost a few microseconds; the rest of this file
+calls the library with ctypes.  These two are the only torch-aware layers.
 
 Differences from the reference, all deliberate:
 
@@ -22,7 +24,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _lib
+from . import _lib, _native
 
 __all__ = ["fgms_fusion_fwd_cuda", "fgms_fwd_cuda", "fgms_bwd_cuda", "fgms_dgrad_cuda", "fgms_wgrad_cuda",
            "wgrad_workspace", "wgrad_finalize", "fgms_wgrad_noalloc_cuda", "kernel_family", "fallback_count",
@@ -105,18 +107,7 @@ def fgms_fusion_fwd_cuda(in_feats, kernel, sum_nnz, out_feats, kpos, qkpos, in_m
 
     ``out_feats[out_map[j]] += in_feats[in_map[j]] @ kernel[k(j)]`` for every pair; with
     ``separate_mid`` the centre offset is applied densely and ``out_feats`` is overwritten."""
-    k_vol = _common(in_feats, kernel, kpos, in_map, out_map)
-    _check_feat("out_feats", out_feats, in_feats.dtype)
-    if qkpos is not None:
-        _check_index("qkpos", qkpos, in_feats.device, k_vol + 1)
-    if out_feats.size(1) != kernel.size(2):
-        raise ValueError("out_feats width differs from the kernel's output channels")
-    dtype, math = _dtype_math(in_feats, arch80)
-    with torch.cuda.device(in_feats.device):
-        _lib.check(_L.fgms_b200_fusion_fwd(
-            _ptr(in_feats), _ptr(kernel), _ptr(out_feats), _ptr(kpos), _ptr(qkpos), _ptr(in_map), _ptr(out_map),
-            in_map.numel(), in_feats.size(0), out_feats.size(0), in_feats.size(1), kernel.size(1), kernel.size(2),
-            k_vol, int(sum_nnz), dtype, math, int(bool(separate_mid)), _stream()))
+    _native.fusion_fwd(in_feats, kernel, sum_nnz, out_feats, kpos, qkpos, in_map, out_map, separate_mid, arch80)
 
 
 def build_neighbor_table(kpos, in_map, out_map, n_in: int, n_out: int):
@@ -141,69 +132,22 @@ def fgms_fwd_os_cuda(in_feats, kernel, out_feats, nbr, arch80, bias=None, relu=F
     the way out; ``accumulate=True`` adds to ``out_feats`` as the reference's forward does
     (``backend/spconv.cu:23-246``) and takes neither.  ``nbr`` comes from :func:`build_neighbor_table`.
     Tensor-core shapes only (``ValueError`` otherwise)."""
-    _check_feat("in_feats", in_feats, None)
-    _check_feat("kernel", kernel, in_feats.dtype, dim=3)
-    _check_feat("out_feats", out_feats, in_feats.dtype)
-    if kernel.size(1) != in_feats.size(1):
-        raise ValueError("Input feature size and kernel size mismatch")
-    if out_feats.size(1) != kernel.size(2):
-        raise ValueError("out_feats width differs from the kernel's output channels")
-    k_vol = kernel.size(0)
-    stride = (out_feats.size(0) + 127) // 128 * 128
-    if nbr.dtype != torch.int32 or not nbr.is_contiguous() or nbr.device != in_feats.device or nbr.numel() != k_vol * stride:
-        raise ValueError("nbr must be the contiguous int32 table build_neighbor_table returns for these sizes")
-    if bias is not None:
-        _check_feat("bias", bias, in_feats.dtype, dim=1)
-        if bias.numel() != kernel.size(2):
-            raise ValueError("bias length differs from the kernel's output channels")
-    dtype, math = _dtype_math(in_feats, arch80)
-    with torch.cuda.device(in_feats.device):
-        _lib.check(_L.fgms_b200_fwd_output_stationary(
-            _ptr(in_feats), _ptr(kernel), _ptr(out_feats), _ptr(nbr), in_feats.size(0), out_feats.size(0),
-            in_feats.size(1), kernel.size(2), k_vol, dtype, math, _ptr(bias), int(bool(relu)), int(bool(accumulate)),
-            _stream()))
+    _native.fwd_os(in_feats, kernel, out_feats, nbr, arch80, bias, relu, accumulate)
 
 
 def fgms_fwd_cuda(in_feats, kernel, sum_nnz, out_feats, kernel_nnz, kernel_pos, in_map, out_map,
                   separate_mid, arch80):
     """Per-offset forward — ``ConvolutionForward`` (``backend/spconv.cu:249-411``).
     ``kernel_nnz`` is a CPU int32 tensor as in the reference (``spconv.cu:308``)."""
-    k_vol = _common(in_feats, kernel, kernel_pos, in_map, out_map)
-    _check_feat("out_feats", out_feats, in_feats.dtype)
-    _check_index("kernel_nnz", kernel_nnz, None, k_vol, cuda=False)
-    if out_feats.size(1) != kernel.size(2):
-        raise ValueError("out_feats width differs from the kernel's output channels")
-    dtype, math = _dtype_math(in_feats, arch80)
-    with torch.cuda.device(in_feats.device):
-        _lib.check(_L.fgms_b200_seq_fwd(
-            _ptr(in_feats), _ptr(kernel), _ptr(out_feats), kernel_nnz.data_ptr(), _ptr(kernel_pos), _ptr(in_map),
-            _ptr(out_map), in_map.numel(), in_feats.size(0), out_feats.size(0), in_feats.size(1), kernel.size(1),
-            kernel.size(2), k_vol, int(sum_nnz), dtype, math, int(bool(separate_mid)), _stream()))
+    _native.seq_fwd(in_feats, kernel, sum_nnz, out_feats, kernel_nnz, kernel_pos, in_map, out_map, separate_mid, arch80)
 
 
 def fgms_bwd_cuda(out_feats_grad, in_feats, kernel, sum_nnz, in_feats_grad, kernel_grad, kpos, qkpos,
                   in_map, out_map, separate_mid, arch80):
     """Backward — ``ConvolutionBackward`` (``backend/spconv.cu:414-571``): accumulates the input
     gradient into ``in_feats_grad`` and the weight gradient into ``kernel_grad``."""
-    k_vol = _common(in_feats, kernel, kpos, in_map, out_map)
-    _check_feat("out_feats_grad", out_feats_grad, in_feats.dtype)
-    _check_feat("in_feats_grad", in_feats_grad, in_feats.dtype)
-    _check_feat("kernel_grad", kernel_grad, in_feats.dtype, dim=3)
-    if in_feats.size(1) == kernel.size(1):
-        if in_feats_grad.shape != in_feats.shape or kernel_grad.shape != kernel.shape:
-            raise ValueError("gradient buffers must have the shapes of in_feats and kernel")
-        if out_feats_grad.size(1) != kernel.size(2):
-            raise ValueError("out_feats_grad width differs from the kernel's output channels")
-    dtype, math = _dtype_math(in_feats, arch80)
-    ws = None
-    if dtype == _lib.DTYPE_F16 and not _single_launch_wgrad(kernel.size(1), kernel.size(2), k_vol, in_feats.dtype, arch80, None):
-        ws = wgrad_workspace(kernel.size(1), kernel.size(2), k_vol, in_feats.device)
-    with torch.cuda.device(in_feats.device):
-        _lib.check(_L.fgms_b200_bwd(
-            _ptr(out_feats_grad), _ptr(in_feats), _ptr(kernel), _ptr(in_feats_grad), _ptr(kernel_grad), _ptr(kpos),
-            _ptr(qkpos), _ptr(in_map), _ptr(out_map), in_map.numel(), in_feats.size(0), out_feats_grad.size(0),
-            in_feats.size(1), kernel.size(1), kernel.size(2), k_vol, int(sum_nnz), dtype, math, int(bool(separate_mid)),
-            _ptr(ws), ws.numel() * 4 if ws is not None else 0, _stream()))
+    _native.bwd(out_feats_grad, in_feats, kernel, sum_nnz, in_feats_grad, kernel_grad, kpos, qkpos, in_map, out_map, separate_mid,
+                arch80, WGRAD_FP32_SUMS)
 
 
 def fgms_dgrad_cuda(out_feats_grad, kernel, in_feats_grad, kpos, in_map, out_map, arch80):

@@ -1,9 +1,9 @@
-"""Build ``libfgms_b200.so`` in-tree with nvcc for sm_100a.
+"""Build ``libfgms_b200.so`` (nvcc, sm_100a) and the PyTorch extension ``_native.so`` (g++) in-tree.
 
     python -m fgms_b200.build [--force] [--verbose]
 
 The library is a plain C-ABI shared object (see ``include/fgms_b200.h``); it links only the CUDA
-runtime, not PyTorch.
+runtime, not PyTorch.  ``_native.so`` is the PyTorch binding on top of it and finds it beside itself.
 """
 from __future__ import annotations
 
@@ -21,6 +21,10 @@ NVCC_FLAGS = [
 ]
 
 
+BINDING = os.path.join(HERE, "_native.so")
+BINDING_SOURCE = os.path.join(CSRC, "torch_binding.cpp")
+
+
 def _deps():
     out = list(SOURCES)
     for d in (CSRC, os.path.join(os.path.dirname(HERE), "include")):
@@ -28,24 +32,43 @@ def _deps():
     return out
 
 
+def _stale(target: str, sources) -> bool:
+    return not os.path.exists(target) or any(os.path.getmtime(f) > os.path.getmtime(target) for f in sources)
+
+
 def needs_build() -> bool:
-    if not os.path.exists(LIB):
-        return True
-    t = os.path.getmtime(LIB)
-    return any(os.path.getmtime(f) > t for f in _deps())
+    return _stale(LIB, _deps()) or _stale(BINDING, [BINDING_SOURCE, os.path.join(os.path.dirname(HERE), "include", "fgms_b200.h")])
+
+
+def _run(cmd, what: str, verbose: bool) -> None:
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+    if res.returncode != 0:
+        raise RuntimeError(f"building {what} failed")
+
+
+def _build_binding(verbose: bool) -> None:
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    lib_dir = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.dirname(os.path.dirname(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")))
+    include = cpp_extension.include_paths() + [os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+    cmd += [f for d in include for f in ("-isystem", d)]
+    cmd += [BINDING_SOURCE, "-o", BINDING, "-L" + HERE, "-lfgms_b200", "-L" + lib_dir, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10",
+            "-lc10_cuda", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + lib_dir]
+    _run(cmd, "_native.so", verbose)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not needs_build():
         return LIB
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    extra = ["-DFGMS_NO_UMMA"] if os.environ.get("FGMS_NO_UMMA") == "1" else []  # bring-up aid only
-    cmd = [nvcc] + NVCC_FLAGS + extra + (["-Xptxas", "-v"] if verbose else []) + SOURCES + ["-o", LIB]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if verbose or res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
-    if res.returncode != 0:
-        raise RuntimeError("nvcc failed building libfgms_b200.so")
+    _run([nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + SOURCES + ["-o", LIB], "libfgms_b200.so", verbose)
+    _build_binding(verbose)
     return LIB
 
 

@@ -171,4 +171,17 @@ __device__ __forceinline__ void scatter_add(__half* p, const float (&v)[N], int 
   }
 }
 
+// Clears [a, a + a_bytes) and [b, b + b_bytes), 16 bytes per store; the buffers start on 16-byte boundaries.  One launch
+// for both gradients of a backward (a fill each through PyTorch is 1.4 us on the device and 3 us on the host).
+__global__ void __launch_bounds__(256) zero2_kernel(uint8_t* a, size_t a_bytes, uint8_t* b, size_t b_bytes) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // kernels before this one may still use the buffers
+  const size_t na = a_bytes >> 4, n = na + (b_bytes >> 4), step = (size_t)gridDim.x * blockDim.x;
+  const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (size_t i = i0; i < n; i += step)
+    *reinterpret_cast<uint4*>(i < na ? a + 16 * i : b + 16 * (i - na)) = make_uint4(0, 0, 0, 0);
+  if (i0 < (a_bytes & 15)) a[(na << 4) + i0] = 0;
+  if (i0 < (b_bytes & 15)) b[(b_bytes & ~(size_t)15) + i0] = 0;
+}
+
 }  // namespace fgms

@@ -247,6 +247,21 @@ int fgms_b200_dgrad(const void* out_grad, const void* kernel, void* in_grad, con
                  dtype, math, 0, 0, static_cast<cudaStream_t>(stream));
 }
 
+int fgms_b200_zero2(void* a, size_t a_bytes, void* b, size_t b_bytes, void* stream) {
+  TraceRange trace_range("fgms_b200_zero2");
+  if ((a_bytes > 0 && !a) || (b_bytes > 0 && !b)) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
+  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) return fail(FGMS_ERR_INVALID_ARG, "buffers must be 16-byte aligned");
+  if (a_bytes + b_bytes == 0) return FGMS_OK;
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  // four 16-byte stores per thread, at most eight blocks of 256 threads per SM
+  const size_t want = (a_bytes + b_bytes) / (256 * 64) + 1, most = (size_t)di.sms * 8;
+  if (fgms::launch_pdl(fgms::zero2_kernel, (int)(want < most ? want : most), 256, 0, static_cast<cudaStream_t>(stream),
+                       static_cast<uint8_t*>(a), a_bytes, static_cast<uint8_t*>(b), b_bytes) != cudaSuccess)
+    return fail(FGMS_ERR_CUDA, "zero2_kernel launch failed");
+  return check_launch("zero2_kernel");
+}
+
 size_t fgms_b200_wgrad_workspace_bytes(int c_in, int c_out, int k_vol, int dtype) {
   if (dtype != FGMS_DTYPE_F16 || c_in < 1 || c_out < 1 || k_vol < 1) return 0;
   return (size_t)k_vol * c_in * c_out * sizeof(float);

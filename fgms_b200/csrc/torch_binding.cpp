@@ -1,0 +1,293 @@
+// PyTorch side of the library: the operator calls and the autograd function as a CPython extension module
+// (fgms_b200._native) over the C ABI of libfgms_b200.so.
+//
+// Argument checks, the choice of the current stream and the kernel launches of a call are a few microseconds of host
+// time here; the same steps in Python took 15-20 us per call (20 us for a forward of a few hundred voxels whose
+// kernel runs 6 us; 56 us per layer and pass through the autograd engine), which is what bounded every layer of up to
+// about a hundred thousand voxels.  Error types are those of the reference's binding: ValueError for what pybind11
+// maps from std::invalid_argument, TypeError for an argument that is no tensor, RuntimeError for a CUDA failure.
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/fgms_b200.h"
+
+namespace {
+
+using at::Tensor;
+
+void check_status(int rc) {
+  if (rc == FGMS_OK) return;
+  const char* msg = fgms_b200_last_error();
+  if (rc == FGMS_ERR_CHANNEL_MISMATCH || rc == FGMS_ERR_INVALID_ARG || rc == FGMS_ERR_UNSUPPORTED || rc == FGMS_ERR_WORKSPACE)
+    TORCH_CHECK_VALUE(false, msg);
+  TORCH_CHECK(false, "fgms_b200 error ", rc, ": ", msg);
+}
+
+void check_feat(const char* name, const Tensor& t, int64_t dim) {
+  TORCH_CHECK_VALUE(t.is_cuda(), name, " must be a CUDA tensor");
+  TORCH_CHECK_VALUE(t.dim() == dim, name, " must have ", dim, " dimensions, got ", t.dim());
+  TORCH_CHECK_VALUE(t.is_contiguous(), name, " must be contiguous");
+}
+void check_feat(const char* name, const Tensor& t, int64_t dim, const Tensor& like) {
+  check_feat(name, t, dim);
+  TORCH_CHECK_VALUE(t.scalar_type() == like.scalar_type(), name, " must have dtype ", like.scalar_type(), ", got ", t.scalar_type());
+}
+void check_index(const char* name, const Tensor& t, const Tensor& like, int64_t min_len) {
+  TORCH_CHECK_VALUE(t.scalar_type() == at::kInt, name, " must be an int32 tensor");
+  TORCH_CHECK_VALUE(t.is_cuda() && t.device() == like.device(), name, " must live on ", like.device());
+  TORCH_CHECK_VALUE(t.is_contiguous(), name, " must be contiguous");
+  TORCH_CHECK_VALUE(t.numel() >= min_len, name, " needs at least ", min_len, " entries, got ", t.numel());
+}
+
+struct Arith { int dtype, math; };
+Arith arith(const Tensor& t, bool arch80) {
+  if (t.scalar_type() == at::kHalf) return {FGMS_DTYPE_F16, FGMS_MATH_F16};
+  TORCH_CHECK_VALUE(t.scalar_type() == at::kFloat, "unsupported feature dtype ", t.scalar_type(), ": the operator takes float16 or float32");
+  return {FGMS_DTYPE_F32, arch80 ? FGMS_MATH_TF32 : FGMS_MATH_FP32};
+}
+
+void* ptr(const Tensor& t) { return t.numel() > 0 ? t.data_ptr() : nullptr; }
+const int32_t* iptr(const Tensor& t) { return static_cast<const int32_t*>(ptr(t)); }
+void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
+
+// checks shared by every pass over a pair list; returns k_vol
+int check_common(const Tensor& feats, const Tensor& kernel, const Tensor& kpos, const Tensor& in_map, const Tensor& out_map) {
+  check_feat("in_feats", feats, 2);
+  check_feat("kernel", kernel, 3, feats);
+  const int64_t k_vol = kernel.size(0);
+  check_index("kpos", kpos, feats, k_vol + 1);
+  check_index("in_map", in_map, feats, 0);
+  check_index("out_map", out_map, feats, 0);
+  TORCH_CHECK_VALUE(in_map.numel() == out_map.numel(), "in_map and out_map differ in length");
+  return (int)k_vol;
+}
+
+void fusion_fwd(const Tensor& in_feats, const Tensor& kernel, int64_t sum_nnz, const Tensor& out, const Tensor& kpos,
+                const Tensor* qkpos, const Tensor& in_map, const Tensor& out_map, bool separate_mid, bool arch80) {
+  const int k_vol = check_common(in_feats, kernel, kpos, in_map, out_map);
+  check_feat("out_feats", out, 2, in_feats);
+  if (qkpos) check_index("qkpos", *qkpos, in_feats, k_vol + 1);
+  TORCH_CHECK_VALUE(out.size(1) == kernel.size(2), "out_feats width differs from the kernel's output channels");
+  const Arith a = arith(in_feats, arch80);
+  c10::cuda::CUDAGuard guard(in_feats.device());
+  check_status(fgms_b200_fusion_fwd(ptr(in_feats), ptr(kernel), ptr(out), iptr(kpos), qkpos ? iptr(*qkpos) : nullptr, iptr(in_map),
+                                    iptr(out_map), in_map.numel(), (int)in_feats.size(0), (int)out.size(0), (int)in_feats.size(1),
+                                    (int)kernel.size(1), (int)kernel.size(2), k_vol, sum_nnz, a.dtype, a.math, separate_mid,
+                                    stream_of(in_feats)));
+}
+
+void seq_fwd(const Tensor& in_feats, const Tensor& kernel, int64_t sum_nnz, const Tensor& out, const Tensor& kernel_nnz,
+             const Tensor& kpos, const Tensor& in_map, const Tensor& out_map, bool separate_mid, bool arch80) {
+  const int k_vol = check_common(in_feats, kernel, kpos, in_map, out_map);
+  check_feat("out_feats", out, 2, in_feats);
+  TORCH_CHECK_VALUE(kernel_nnz.scalar_type() == at::kInt, "kernel_nnz must be an int32 tensor");
+  TORCH_CHECK_VALUE(!kernel_nnz.is_cuda(), "kernel_nnz must be a CPU tensor");
+  TORCH_CHECK_VALUE(kernel_nnz.is_contiguous(), "kernel_nnz must be contiguous");
+  TORCH_CHECK_VALUE(kernel_nnz.numel() >= k_vol, "kernel_nnz needs at least ", k_vol, " entries, got ", kernel_nnz.numel());
+  TORCH_CHECK_VALUE(out.size(1) == kernel.size(2), "out_feats width differs from the kernel's output channels");
+  const Arith a = arith(in_feats, arch80);
+  c10::cuda::CUDAGuard guard(in_feats.device());
+  check_status(fgms_b200_seq_fwd(ptr(in_feats), ptr(kernel), ptr(out), kernel_nnz.data_ptr<int32_t>(), iptr(kpos), iptr(in_map),
+                                 iptr(out_map), in_map.numel(), (int)in_feats.size(0), (int)out.size(0), (int)in_feats.size(1),
+                                 (int)kernel.size(1), (int)kernel.size(2), k_vol, sum_nnz, a.dtype, a.math, separate_mid,
+                                 stream_of(in_feats)));
+}
+
+// fp32 sums of an fp16 weight gradient that has no single-launch form (or was asked for in fp32 sums): from PyTorch's
+// caching allocator, so that calls on different streams or threads never share one
+Tensor wgrad_workspace(const Tensor& kernel_grad, const Arith& a, bool fp32_sums) {
+  if (a.dtype != FGMS_DTYPE_F16) return {};
+  const int c_in = (int)kernel_grad.size(1), c_out = (int)kernel_grad.size(2), k_vol = (int)kernel_grad.size(0);
+  if (!fp32_sums && k_vol >= 1 && fgms_b200_kernel_family(2, c_in, c_out, k_vol, a.dtype, a.math) == 1) return {};
+  const int64_t n = std::max<int64_t>((int64_t)(fgms_b200_wgrad_workspace_bytes(c_in, c_out, k_vol, a.dtype) / 4), 64);
+  return at::empty({n}, kernel_grad.options().dtype(at::kFloat));
+}
+
+void bwd(const Tensor& grad_out, const Tensor& in_feats, const Tensor& kernel, int64_t sum_nnz, const Tensor& in_grad,
+         const Tensor& kernel_grad, const Tensor& kpos, const Tensor* qkpos, const Tensor& in_map, const Tensor& out_map,
+         bool separate_mid, bool arch80, bool fp32_sums) {
+  const int k_vol = check_common(in_feats, kernel, kpos, in_map, out_map);
+  check_feat("out_feats_grad", grad_out, 2, in_feats);
+  check_feat("in_feats_grad", in_grad, 2, in_feats);
+  check_feat("kernel_grad", kernel_grad, 3, in_feats);
+  if (in_feats.size(1) == kernel.size(1)) {  // a channel mismatch is the library's own error below
+    TORCH_CHECK_VALUE(in_grad.sizes() == in_feats.sizes() && kernel_grad.sizes() == kernel.sizes(),
+                      "gradient buffers must have the shapes of in_feats and kernel");
+    TORCH_CHECK_VALUE(grad_out.size(1) == kernel.size(2), "out_feats_grad width differs from the kernel's output channels");
+  }
+  const Arith a = arith(in_feats, arch80);
+  c10::cuda::CUDAGuard guard(in_feats.device());
+  const Tensor ws = in_feats.size(1) == kernel.size(1) ? wgrad_workspace(kernel_grad, a, fp32_sums) : Tensor();
+  check_status(fgms_b200_bwd(ptr(grad_out), ptr(in_feats), ptr(kernel), ptr(in_grad), ptr(kernel_grad), iptr(kpos),
+                             qkpos ? iptr(*qkpos) : nullptr, iptr(in_map), iptr(out_map), in_map.numel(), (int)in_feats.size(0),
+                             (int)grad_out.size(0), (int)in_feats.size(1), (int)kernel.size(1), (int)kernel.size(2), k_vol, sum_nnz,
+                             a.dtype, a.math, separate_mid, ws.defined() ? ws.data_ptr() : nullptr,
+                             ws.defined() ? (size_t)ws.numel() * 4 : 0, stream_of(in_feats)));
+}
+
+// ---------------------------------------------------------------------------------------------
+// autograd
+// ---------------------------------------------------------------------------------------------
+size_t bytes_of(const Tensor& t) { return (size_t)t.numel() * t.element_size(); }
+
+struct SparseConv : torch::autograd::Function<SparseConv> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& feats_, const Tensor& weight_, const Tensor& kpos,
+                        const Tensor& imap, const Tensor& omap, int64_t n_out, bool arch80, bool fp32_sums) {
+    const Tensor feats = feats_.contiguous(), weight = weight_.contiguous();
+    TORCH_CHECK_VALUE(feats.is_cuda(), "in_feats must be a CUDA tensor");
+    TORCH_CHECK_VALUE(weight.dim() == 3, "kernel must have 3 dimensions, got ", weight.dim());
+    c10::cuda::CUDAGuard guard(feats.device());
+    Tensor out = at::empty({n_out, weight.size(2)}, feats.options().requires_grad(false));
+    check_status(fgms_b200_zero2(ptr(out), bytes_of(out), nullptr, 0, stream_of(feats)));
+    fusion_fwd(feats, weight, 0, out, kpos, nullptr, imap, omap, false, arch80);
+    ctx->save_for_backward({feats, weight, kpos, imap, omap});
+    ctx->saved_data["arch80"] = arch80;
+    ctx->saved_data["fp32_sums"] = fp32_sums;
+    return out;
+  }
+
+  // Only the gradients that something needs are computed: the first layer of a network has no input gradient, a
+  // frozen layer no weight gradient.
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &feats = saved[0], &weight = saved[1], &kpos = saved[2], &imap = saved[3], &omap = saved[4];
+    const bool arch80 = ctx->saved_data["arch80"].toBool();
+    const Tensor grad_out = grads[0].contiguous();
+    const bool need_in = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
+    c10::cuda::CUDAGuard guard(feats.device());
+    void* st = stream_of(feats);
+    Tensor in_grad, w_grad;
+    if (need_in) in_grad = at::empty_like(feats);
+    if (need_w) w_grad = at::empty_like(weight);
+    check_feat("out_feats_grad", grad_out, 2, feats);
+    TORCH_CHECK_VALUE(grad_out.size(1) == weight.size(2), "out_feats_grad width differs from the kernel's output channels");
+    const Arith a = arith(feats, arch80);
+    const int n_in = (int)feats.size(0), n_out = (int)grad_out.size(0), c_in = (int)weight.size(1), c_out = (int)weight.size(2),
+              k_vol = (int)weight.size(0);
+    check_status(fgms_b200_zero2(need_in ? ptr(in_grad) : nullptr, need_in ? bytes_of(in_grad) : 0, need_w ? ptr(w_grad) : nullptr,
+                                 need_w ? bytes_of(w_grad) : 0, st));
+    if (need_in)
+      check_status(fgms_b200_dgrad(ptr(grad_out), ptr(weight), ptr(in_grad), iptr(kpos), iptr(imap), iptr(omap), imap.numel(), n_in,
+                                   n_out, c_in, c_out, k_vol, a.dtype, a.math, st));
+    if (need_w) {
+      const Tensor ws = wgrad_workspace(w_grad, a, ctx->saved_data["fp32_sums"].toBool());
+      check_status(fgms_b200_wgrad(ptr(feats), ptr(grad_out), ptr(w_grad), iptr(kpos), iptr(imap), iptr(omap), imap.numel(), n_in,
+                                   n_out, c_in, c_out, k_vol, a.dtype, a.math, ws.defined() ? ws.data_ptr() : nullptr,
+                                   ws.defined() ? (size_t)ws.numel() * 4 : 0, 1, st));
+    }
+    return {in_grad, w_grad, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// output-stationary forward into `out`; nbr is the table fgms_b200_build_neighbor_table fills
+void fwd_os(const Tensor& in_feats, const Tensor& kernel, const Tensor& out, const Tensor& nbr, bool arch80, const Tensor* bias,
+            bool relu, bool accumulate) {
+  check_feat("in_feats", in_feats, 2);
+  check_feat("kernel", kernel, 3, in_feats);
+  check_feat("out_feats", out, 2, in_feats);
+  TORCH_CHECK_VALUE(kernel.size(1) == in_feats.size(1), "Input feature size and kernel size mismatch");
+  TORCH_CHECK_VALUE(out.size(1) == kernel.size(2), "out_feats width differs from the kernel's output channels");
+  const int64_t k_vol = kernel.size(0), stride = (out.size(0) + 127) / 128 * 128;
+  TORCH_CHECK_VALUE(nbr.scalar_type() == at::kInt && nbr.is_contiguous() && nbr.device() == in_feats.device() && nbr.numel() == k_vol * stride,
+                    "nbr must be the contiguous int32 table build_neighbor_table returns for these sizes");
+  if (bias) {
+    check_feat("bias", *bias, 1, in_feats);
+    TORCH_CHECK_VALUE(bias->numel() == kernel.size(2), "bias length differs from the kernel's output channels");
+  }
+  const Arith a = arith(in_feats, arch80);
+  c10::cuda::CUDAGuard guard(in_feats.device());
+  check_status(fgms_b200_fwd_output_stationary(ptr(in_feats), ptr(kernel), ptr(out), iptr(nbr), (int)in_feats.size(0), (int)out.size(0),
+                                               (int)in_feats.size(1), (int)kernel.size(2), (int)k_vol, a.dtype, a.math,
+                                               bias ? ptr(*bias) : nullptr, relu, accumulate, stream_of(in_feats)));
+}
+
+// ---------------------------------------------------------------------------------------------
+// Python entry points (positional arguments only; the functions of backend.py / nn.py give them their names)
+// ---------------------------------------------------------------------------------------------
+const Tensor& feat_arg(PyObject* o, const char* name) {
+  TORCH_CHECK_TYPE(THPVariable_Check(o), name, " must be a torch.Tensor");
+  return THPVariable_Unpack(o);
+}
+const Tensor& index_arg(PyObject* o, const char* name) {
+  TORCH_CHECK_VALUE(THPVariable_Check(o), name, " must be an int32 tensor");
+  return THPVariable_Unpack(o);
+}
+const Tensor* optional_arg(PyObject* o, const char* name) { return o == Py_None ? nullptr : &index_arg(o, name); }
+int64_t int_arg(PyObject* o) {  // like int(o): a Python or NumPy integer, or a tensor of one element
+  PyObject* n = PyLong_CheckExact(o) ? Py_NewRef(o) : PyNumber_Long(o);
+  if (!n) throw python_error();
+  const long long v = PyLong_AsLongLong(n);
+  Py_DECREF(n);
+  if (v == -1 && PyErr_Occurred()) throw python_error();
+  return v;
+}
+bool bool_arg(PyObject* o) {
+  const int v = PyObject_IsTrue(o);
+  if (v < 0) throw python_error();
+  return v != 0;
+}
+void expect(Py_ssize_t got, Py_ssize_t want) { TORCH_CHECK_TYPE(got == want, "expected ", want, " arguments, got ", got); }
+
+PyObject* py_fusion_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 10);
+  const Tensor &in_feats = feat_arg(a[0], "in_feats"), &kernel = feat_arg(a[1], "kernel"), &out = feat_arg(a[3], "out_feats");
+  const Tensor &kpos = index_arg(a[4], "kpos"), *qkpos = optional_arg(a[5], "qkpos");
+  const Tensor &in_map = index_arg(a[6], "in_map"), &out_map = index_arg(a[7], "out_map");
+  fusion_fwd(in_feats, kernel, int_arg(a[2]), out, kpos, qkpos, in_map, out_map, bool_arg(a[8]), bool_arg(a[9]));
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+PyObject* py_seq_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 10);
+  const Tensor &in_feats = feat_arg(a[0], "in_feats"), &kernel = feat_arg(a[1], "kernel"), &out = feat_arg(a[3], "out_feats");
+  const Tensor &nnz = index_arg(a[4], "kernel_nnz"), &kpos = index_arg(a[5], "kpos");
+  const Tensor &in_map = index_arg(a[6], "in_map"), &out_map = index_arg(a[7], "out_map");
+  seq_fwd(in_feats, kernel, int_arg(a[2]), out, nnz, kpos, in_map, out_map, bool_arg(a[8]), bool_arg(a[9]));
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+PyObject* py_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 13);
+  const Tensor &grad_out = feat_arg(a[0], "out_feats_grad"), &in_feats = feat_arg(a[1], "in_feats"), &kernel = feat_arg(a[2], "kernel");
+  const Tensor &in_grad = feat_arg(a[4], "in_feats_grad"), &kernel_grad = feat_arg(a[5], "kernel_grad");
+  const Tensor &kpos = index_arg(a[6], "kpos"), *qkpos = optional_arg(a[7], "qkpos");
+  const Tensor &in_map = index_arg(a[8], "in_map"), &out_map = index_arg(a[9], "out_map");
+  bwd(grad_out, in_feats, kernel, int_arg(a[3]), in_grad, kernel_grad, kpos, qkpos, in_map, out_map, bool_arg(a[10]), bool_arg(a[11]),
+      bool_arg(a[12]));
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+PyObject* py_sparse_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 8);
+  const Tensor &feats = feat_arg(a[0], "in_feats"), &weight = feat_arg(a[1], "kernel");
+  const Tensor &kpos = index_arg(a[2], "kpos"), &imap = index_arg(a[3], "in_map"), &omap = index_arg(a[4], "out_map");
+  return THPVariable_Wrap(SparseConv::apply(feats, weight, kpos, imap, omap, int_arg(a[5]), bool_arg(a[6]), bool_arg(a[7])));
+  END_HANDLE_TH_ERRORS
+}
+PyObject* py_fwd_os(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 8);
+  const Tensor &in_feats = feat_arg(a[0], "in_feats"), &kernel = feat_arg(a[1], "kernel"), &out = feat_arg(a[2], "out_feats");
+  const Tensor &nbr = index_arg(a[3], "nbr"), *bias = a[5] == Py_None ? nullptr : &feat_arg(a[5], "bias");
+  fwd_os(in_feats, kernel, out, nbr, bool_arg(a[4]), bias, bool_arg(a[6]), bool_arg(a[7]));
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+#define FGMS_METHOD(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(fn)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {
+    FGMS_METHOD("fusion_fwd", py_fusion_fwd), FGMS_METHOD("seq_fwd", py_seq_fwd),         FGMS_METHOD("bwd", py_bwd),
+    FGMS_METHOD("fwd_os", py_fwd_os),         FGMS_METHOD("sparse_conv", py_sparse_conv), {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&module_def); }

@@ -14,30 +14,9 @@ import math
 
 import torch
 
-from . import backend
+from . import _native, backend
 
 __all__ = ["sparse_conv", "sparse_conv_inference", "SparseConv3d", "SparseUNet"]
-
-
-class _SparseConvFunction(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, feats, weight, kpos, imap, omap, n_out, arch80):
-        feats = feats.contiguous()
-        weight = weight.contiguous()
-        out = torch.zeros((n_out, weight.size(2)), dtype=feats.dtype, device=feats.device)
-        backend.fgms_fusion_fwd_cuda(feats, weight, 0, out, kpos, None, imap, omap, False, arch80)
-        ctx.save_for_backward(feats, weight, kpos, imap, omap)
-        ctx.arch80 = arch80
-        return out
-
-    @staticmethod
-    def backward(ctx, grad_out):
-        feats, weight, kpos, imap, omap = ctx.saved_tensors
-        grad_out = grad_out.contiguous()
-        in_grad = torch.zeros_like(feats)
-        w_grad = torch.zeros_like(weight)
-        backend.fgms_bwd_cuda(grad_out, feats, weight, 0, in_grad, w_grad, kpos, None, imap, omap, False, ctx.arch80)
-        return in_grad, w_grad, None, None, None, None, None
 
 
 def sparse_conv(feats: torch.Tensor, weight: torch.Tensor, kmap, arch80: bool = True) -> torch.Tensor:
@@ -46,7 +25,8 @@ def sparse_conv(feats: torch.Tensor, weight: torch.Tensor, kmap, arch80: bool = 
         raise ValueError(f"feats has {feats.size(0)} rows, the kernel map expects {kmap.n_in}")
     if weight.size(0) != kmap.kpos.numel() - 1:
         raise ValueError("weight and kernel map disagree on the number of offsets")
-    return _SparseConvFunction.apply(feats, weight, kmap.kpos, kmap.imap, kmap.omap, kmap.n_out, arch80)
+    return _native.sparse_conv(feats, weight, kmap.kpos, kmap.imap, kmap.omap, kmap.n_out, arch80,
+                               backend.WGRAD_FP32_SUMS)
 
 
 def sparse_conv_inference(feats: torch.Tensor, weight: torch.Tensor, kmap, bias: torch.Tensor | None = None,

@@ -94,6 +94,11 @@ int fgms_b200_dgrad(const void* out_grad, const void* kernel, void* in_grad, con
                     const int32_t* in_map, const int32_t* out_map, int64_t map_len, int n_in, int n_out,
                     int c_in, int c_out, int k_vol, int dtype, int math, void* stream);
 
+/* Clear two buffers (either may be empty: NULL and 0) in one launch: the outputs the entry points above add into.
+ * The pointers must be 16-byte aligned.  Launched like the library's other kernels, so that the next one may start
+ * its preamble while this one runs. */
+int fgms_b200_zero2(void* a, size_t a_bytes, void* b, size_t b_bytes, void* stream);
+
 /* Weight gradient:  kernel_grad[k] += sum over the pairs of offset k of in[in_map[j]]^T (x) out_grad[out_map[j]].
  * Second launch of ConvolutionBackward (backend/spconv.cu:495-548 fp16, 562-569 tf32).
  * Partial sums are accumulated in fp32.  For fp16 storage they live in `workspace`
