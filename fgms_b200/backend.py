@@ -245,7 +245,8 @@ def wgrad_finalize(kernel_grad: torch.Tensor, partial_f32: torch.Tensor) -> None
 
 
 def kernel_family(pass_: str, c_in: int, c_out: int, dtype: torch.dtype, arch80: bool = True, k_vol: int = 27) -> str:
-    """``"tcgen05"`` or ``"simt"``: which kernel family the dispatch uses for a shape (channel counts that are
+    """``"tcgen05"`` or ``"simt"``: which kernel family the dispatch uses for a shape: tensor cores (tcgen05, or warp-level
+    MMA for rows of up to 64 channels) or CUDA cores (channel counts that are
     multiples of 16 up to 256 whose operands fit shared memory run on tcgen05 unless ``arch80`` is false for
     fp32 storage)."""
     d = _lib.DTYPE_F16 if dtype == torch.float16 else _lib.DTYPE_F32

@@ -62,26 +62,22 @@ struct WgradParams {
 __device__ __forceinline__ void build_tile_table(int TILE, const int32_t* __restrict__ kpos, int pairs, int k_vol,
                                                  int dense_rows, int* kpos_s /* [k_vol+1] */,
                                                  int* tile_start /* [k_vol+2] */) {
-  for (int s = threadIdx.x; s <= k_vol; s += blockDim.x) {
-    const int v = __ldg(kpos + s);
-    const int c = min(max(v, 0), pairs);
-    if (v != c && blockIdx.x == 0) report_problem();
-    kpos_s[s] = c;
-  }
-  __syncthreads();
-  // counts first (parallel), then the first warp turns them into running sums, 32 segments at a time
-  for (int s = threadIdx.x; s <= k_vol; s += blockDim.x) {
-    int cnt = (s < k_vol) ? (kpos_s[s + 1] - kpos_s[s]) : dense_rows;
-    if (cnt < 0) cnt = 0;
-    tile_start[s + 1] = (cnt + TILE - 1) / TILE;
-  }
-  __syncthreads();
+  // The first warp does it alone, 32 segments at a time: both ends of a segment are loaded side by side, so the table
+  // costs one trip to memory, one scan by shuffles and one barrier (three barriers and a second pass before).
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     int carry = 0;
     for (int s0 = 0; s0 <= k_vol; s0 += 32) {
       const int s = s0 + lane;
-      int v = s <= k_vol ? tile_start[s + 1] : 0;
+      int v = 0;
+      if (s <= k_vol) {
+        const int first = __ldg(kpos + s), next = s < k_vol ? __ldg(kpos + s + 1) : 0;
+        const int c = min(max(first, 0), pairs);
+        if (first != c && blockIdx.x == 0) report_problem();
+        kpos_s[s] = c;
+        const int cnt = s < k_vol ? min(max(next, 0), pairs) - c : dense_rows;
+        v = cnt > 0 ? (cnt + TILE - 1) / TILE : 0;
+      }
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int n = __shfl_up_sync(0xffffffffu, v, o);
@@ -111,6 +107,37 @@ __device__ __forceinline__ void cta_tile_range(int total, int* t0, int* t1) {
   *t0 = (int)((long long)total * b / g);
   *t1 = (int)((long long)total * (b + 1) / g);
 }
+
+// Tiles handed out by turns.  All tiles' turns, offset after offset, are cut into shares of F consecutive ones; worker w
+// (a warp or a block) has turns [w F, w F + F).  Without `spread` turns and tiles are the same thing: a worker takes a
+// consecutive part of an offset's list.  With it the workers that share an offset step through its list side by side: at
+// turn i (counted from the start of a worker's share) the offset's next tiles go to the `full` workers between its first
+// and its last, from turn first_i on also to the first one, and until turn last_r also to the last one.  In a canonical
+// map (ascending output rows inside an offset) all offsets are then at about the same rows at the same time, and a row is
+// read from memory once and found in L2 by the other offsets.
+struct Turns {
+  int i0, full, first_i, last_r, me;
+  // [s0, s1): the offset's turns; t: this worker's first turn inside it
+  __device__ __forceinline__ Turns(int s0, int s1, int share, int worker, int t, bool spread) {
+    const int first = s0 / share, last = (s1 - 1) / share;
+    full = spread ? last - first - 1 : -1;
+    first_i = s0 - first * share;
+    last_r = s1 - last * share;
+    me = worker - first;
+    i0 = full < 0 ? t - s0 : t - worker * share;
+  }
+  // the offset's tile for this worker's n-th turn inside it
+  __device__ __forceinline__ int tile(int n) const {
+    const int i = i0 + n;
+    if (full < 0) return i;  // consecutive parts, or the offset lies inside one share
+    const int rank = me == 0 ? full : (me <= full ? me - 1 : full + (i >= first_i ? 1 : 0));
+    return i * full + max(0, i - first_i) + min(i, last_r) + rank;
+  }
+};
+// Spread when gathered and scattered rows together exceed half of L2 (a row read from both dies is held twice):
+// 122 MB of 64-byte rows forward 163 -> 154 us, weight gradient 289 -> 200 us; rows that stay in L2 prefer consecutive
+// parts (41 MB of tf32 rows 16.6 against 18.2 us).
+inline bool spread_tiles(size_t row_bytes) { return row_bytes > ((size_t)64 << 20); }
 
 // ---------------------------------------------------------------------------------------------
 // element helpers

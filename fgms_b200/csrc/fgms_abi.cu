@@ -16,8 +16,10 @@
 #include "common.cuh"
 #include "simt_kernels.cuh"
 #include "map_builder.cuh"
+#include "rows_gms.cuh"
 #include "umma_gms3.cuh"
 #include "umma_wgrad3.cuh"
+#include "rows_wgrad.cuh"
 #include "peer_exchange.cuh"
 #include "umma_osfwd.cuh"
 
@@ -138,7 +140,10 @@ int run_gms(bool trans, const void* src, const void* kernel, void* dst, const in
   p.c_in = c_in; p.c_out = c_out; p.k_vol = k_vol;
   p.dense_rows = dense_rows; p.dense_weight = dense_weight;
   if (plan_gms(trans, c_in, c_out, k_vol, dtype, math, di.max_smem_optin)) {
-    int rc = fgms::launch_umma_gms3(p, trans, dtype == FGMS_DTYPE_F16, st, di.sms, di.max_smem_optin);
+    int rc = fgms::launch_rows_gms(p, trans, dtype == FGMS_DTYPE_F16, st, di.sms);
+    if (rc == 0) return check_launch("rows_gms_kernel");
+    if (rc < 0) return fail(FGMS_ERR_CUDA, "rows_gms_kernel setup failed (%d)", rc);
+    rc = fgms::launch_umma_gms3(p, trans, dtype == FGMS_DTYPE_F16, st, di.sms, di.max_smem_optin);
     if (rc == 0) return check_launch("umma_gms3_kernel");
     if (rc < 0) return fail(FGMS_ERR_CUDA, "umma_gms3_kernel setup failed (%d)", rc);
     g_fallbacks.fetch_add(1, std::memory_order_relaxed);  // pointers not 16-byte aligned: CUDA-core path, counted
@@ -327,12 +332,14 @@ int fgms_b200_wgrad(const void* in_feats, const void* out_grad, void* kernel_gra
 
   bool launched = false;
   if (umma) {
-    int rc = fgms::launch_umma_wgrad3(p, dtype == FGMS_DTYPE_F16, st, di.sms, di.max_smem_optin);
+    const bool f16 = dtype == FGMS_DTYPE_F16;
+    int rc = fgms::launch_rows_wgrad(p, f16, st, di.sms, di.max_smem_optin);
+    if (rc == 1) rc = fgms::launch_umma_wgrad3(p, f16, st, di.sms, di.max_smem_optin);
     if (rc == 0) {
-      if (int rc2 = check_launch("umma_wgrad3_kernel")) return rc2;
+      if (int rc2 = check_launch("weight-gradient kernel")) return rc2;
       launched = true;
     } else if (rc < 0) {
-      return fail(FGMS_ERR_CUDA, "umma_wgrad3_kernel setup failed (%d)", rc);
+      return fail(FGMS_ERR_CUDA, "weight-gradient kernel setup failed (%d)", rc);
     } else if (direct_f16) {
       return fail(FGMS_ERR_WORKSPACE, "the single-launch fp16 weight gradient needs 16-byte aligned tensors: pass a workspace");
     } else {

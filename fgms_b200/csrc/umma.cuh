@@ -4,6 +4,8 @@
 // operand layouts.  All waits are bounded: a wait that runs out returns false and the caller
 // reports it instead of spinning forever.
 #pragma once
+#include <atomic>
+
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -73,9 +75,14 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool v
 __device__ __forceinline__ void cp_async16_n(uint32_t dst, const void* src, uint32_t n) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
-// 4-byte copy (goes through L1): used to prefetch map entries into shared memory without tying up a register
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+// 4- and 8-byte copies (these go through L1)
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, bool valid = true) {
+  const uint32_t n = valid ? 4u : 0u;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src, bool valid) {
+  const uint32_t n = valid ? 8u : 0u;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 __device__ __forceinline__ void st_shared_i32(uint32_t dst, int v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst), "r"(v) : "memory"); }
 __device__ __forceinline__ int ld_shared_i32(uint32_t src) {
@@ -212,5 +219,16 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, siz
   lc.attrs = at;
   lc.numAttrs = 1;
   return cudaLaunchKernelEx(&lc, kernel, static_cast<KArgs>(args)...);
+}
+
+// cudaFuncSetAttribute is needed once per kernel and device; `granted` remembers it (any thread may call)
+template <typename K>
+inline int ensure_smem(K kernel, int bytes, std::atomic<int>* granted /* [64], by device */) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
+  if (granted[dev].load(std::memory_order_acquire) >= bytes) return 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return -1;
+  granted[dev].store(bytes, std::memory_order_release);
+  return 0;
 }
 }  // namespace fgms

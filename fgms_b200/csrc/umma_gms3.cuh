@@ -505,17 +505,6 @@ inline bool g3_plan(int c_in, int c_out, int es, int k_vol, int max_smem, bool t
   return true;
 }
 
-// cudaFuncSetAttribute is needed once per kernel and device; `granted` remembers it (any thread may call)
-template <typename K>
-inline int ensure_smem(K kernel, int bytes, std::atomic<int>* granted /* [64], by device */) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
-  if (granted[dev].load(std::memory_order_acquire) >= bytes) return 0;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return -1;
-  granted[dev].store(bytes, std::memory_order_release);
-  return 0;
-}
-
 template <bool TF32, bool TRANS_W, bool FULL>
 inline int g3_launch_as(const GmsParams& p, const G3Config& cfg, cudaStream_t st, int sms, int max_smem) {
   static std::atomic<int> granted[64];

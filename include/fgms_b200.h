@@ -252,7 +252,8 @@ int fgms_b200_peer_exchange(const float* const* sums, float* const* reduced, uin
  * whose grids follow the problem size (backend/spconv.cu:111-245). */
 int fgms_b200_set_reserved_sms(int n);
 
-/* Which kernel family the dispatch picks for a shape: 0 = CUDA-core (SIMT), 1 = tcgen05.
+/* Which kernel family the dispatch picks for a shape: 0 = CUDA-core (SIMT), 1 = tensor cores
+ * (tcgen05, or for rows of up to 64 channels, which the hand-offs of a tcgen05 tile would bound, warp-level MMA).
  * pass: 0 forward, 1 dgrad, 2 wgrad.  The answer comes from the same plan the launch uses (channel
  * counts multiples of 16 and at most 256, and the operands of this k_vol fitting the current device's
  * shared memory), so it is what a call with 16-byte aligned tensors will run.  The reference makes the
