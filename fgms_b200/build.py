@@ -17,7 +17,8 @@ LIB = os.path.join(HERE, "libfgms_b200.so")
 SOURCES = [os.path.join(CSRC, "fgms_abi.cu")]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-"-Xcompiler", "-fPIC", "-shared", "-cudart", "shared", "-ldl",
+# no GNU-unique symbols: two builds of the library in one process keep their launch state apart
+    "-Xcompiler", "-fPIC,-fno-gnu-unique", "-shared", "-cudart", "shared", "-ldl",
 ]
 
 

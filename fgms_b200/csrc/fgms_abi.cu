@@ -16,6 +16,7 @@
 #include "common.cuh"
 #include "simt_kernels.cuh"
 #include "map_builder.cuh"
+#include "map_pyramid.cuh"
 #include "rows_gms.cuh"
 #include "umma_gms3.cuh"
 #include "umma_wgrad3.cuh"
@@ -570,6 +571,69 @@ int fgms_b200_transpose_map(const int32_t* kpos, const int32_t* in_map, const in
   if (!fgms::maps::finish(w.dense(), k_vol, n_in, w.tile_sums(), kpos_t, in_map_t, out_map_t, st)) return cuda_fail("map builder launch");
   g_launches += 5;
   return FGMS_OK;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Kernel maps of a pyramid of resolutions (csrc/map_pyramid.cuh)
+// ---------------------------------------------------------------------------------------------
+size_t fgms_b200_pyramid_workspace_bytes(int n, int levels, int what) {
+  fgms::pyramid::Plan p;
+  return fgms::pyramid::plan(n, levels, what, &p) ? p.total : 0;
+}
+
+namespace {
+int pyramid_args(const int32_t* coords, int n, int levels, int what, int32_t* kpos, int32_t* const* out_coords, void* workspace,
+                 size_t workspace_bytes, fgms::pyramid::Plan* p, fgms::pyramid::Args* a) {
+  if (!fgms::pyramid::plan(n, levels, what, p))
+    return fail(FGMS_ERR_INVALID_ARG, "a pyramid needs n >= 1, 1..%d levels and at least one map", fgms::pyramid::MAX_LEVELS);
+  if (!coords || !kpos || (levels > 1 && !out_coords)) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
+  for (int l = 1; l < levels; ++l)
+    if (!out_coords[l - 1]) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
+  if (27ll * n > 0x7fffffffll) return fail(FGMS_ERR_INVALID_ARG, "27 * n exceeds the int32 range of the maps");
+  if (!workspace || workspace_bytes < p->total || (reinterpret_cast<uintptr_t>(workspace) & 255))
+    return fail(FGMS_ERR_WORKSPACE, "the pyramid needs a 256-byte aligned workspace of %zu bytes", p->total);
+  *a = fgms::pyramid::arguments(*p, coords, n, levels, kpos, out_coords, static_cast<uint8_t*>(workspace));
+  return FGMS_OK;
+}
+}  // namespace
+
+int fgms_b200_pyramid_plan(const int32_t* coords, int n, int levels, int what, int32_t* kpos, int32_t* const* out_coords,
+                           void* workspace, size_t workspace_bytes, int32_t* sizes_host, void* stream) {
+  TraceRange trace_range("fgms_b200_pyramid_plan");
+  fgms::pyramid::Plan p;
+  fgms::pyramid::Args a;
+  if (int rc = pyramid_args(coords, n, levels, what, kpos, out_coords, workspace, workspace_bytes, &p, &a)) return rc;
+  if (!sizes_host) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  auto* ws = static_cast<uint8_t*>(workspace);
+  if (!fgms::pyramid::launch_plan(p, a, ws, di.sms, st)) return cuda_fail("pyramid launch");
+  g_launches += 8;
+  if (cudaMemcpyAsync(sizes_host, ws + p.sizes, (size_t)(1 + levels + p.n_jobs) * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+      cudaStreamSynchronize(st) != cudaSuccess)
+    return cuda_fail("reading the sizes of the maps");
+  return FGMS_OK;
+}
+
+int fgms_b200_pyramid_emit(const int32_t* coords, int n, int levels, int what, int32_t* kpos, int32_t* const* out_coords,
+                           int32_t* const* in_maps, int32_t* const* out_maps, void* workspace, size_t workspace_bytes, void* stream) {
+  TraceRange trace_range("fgms_b200_pyramid_emit");
+  fgms::pyramid::Plan p;
+  fgms::pyramid::Args a;
+  if (int rc = pyramid_args(coords, n, levels, what, kpos, out_coords, workspace, workspace_bytes, &p, &a)) return rc;
+  if (!in_maps || !out_maps) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
+  for (int j = 0; j < p.n_jobs; ++j) {
+    if (!in_maps[j] || !out_maps[j]) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
+    a.in_map[j] = in_maps[j];
+    a.out_map[j] = out_maps[j];
+  }
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  if (fgms::launch_pdl(fgms::pyramid::emit_kernel, fgms::pyramid::map_blocks(p, n, di.sms), fgms::pyramid::THREADS, 0,
+                       static_cast<cudaStream_t>(stream), a) != cudaSuccess)
+    return cuda_fail("pyramid launch");
+  return check_launch("pyramid emit_kernel");
 }
 
 // ---------------------------------------------------------------------------------------------

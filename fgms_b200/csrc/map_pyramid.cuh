@@ -1,0 +1,574 @@
+// Kernel maps of a whole pyramid of resolutions at once: for every level the 3x3x3 submanifold map, and between two levels
+// the 2x2x2 stride-2 map and its transpose.  Same canonical form, bit for bit, as map_builder.cuh.
+//
+// One map after the other (hash table, dense table of k_vol x voxels, scan, sort of the parents, and the host waiting for
+// a count after each) took 1.1 ms for the 13 maps of a 120 k-voxel scene: 170 launches, nine waits, 580 us of kernels.
+// A scene's voxels fill a box of a few hundred cells a side, so here every level is a BITMAP of that box:
+//
+//   * setting a bit inserts a voxel and all its ancestors, and removes duplicates among the ancestors;
+//   * the number of set bits before a cell is the voxel's rank in lexicographic order: what the sort was for;
+//   * the neighbours of a voxel along z are three bits side by side, so the 27 hash probes are 9 words.
+//
+// A row's neighbours become one mask of k_vol bits; counting the bits per (offset, block of rows), scanning those counts
+// and writing the pairs needs no dense table.  The host waits once, for the sizes of the maps.
+//
+// The box is limited by the workspace (cells / 8 bytes): a cloud with a larger box, a voxel met twice or a coordinate
+// beyond the packable range is left to map_builder.cuh (the plan says so).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "common.cuh"
+#include "map_builder.cuh"  // COORD_BIAS, align256
+#include "umma.cuh"         // launch_pdl, griddep_*
+
+namespace fgms {
+namespace pyramid {
+
+constexpr int MAX_LEVELS = 8;             // resolutions
+constexpr int MAX_JOBS = 3 * MAX_LEVELS;  // maps
+constexpr int THREADS = 256, ROWS = 256;  // rows of a map a block works on
+constexpr int SCAN_BLOCKS = 592;
+constexpr int WARPS = THREADS / 32;
+enum { SUBM = 1, DOWN = 2, UP = 4 };      // which maps
+enum { TOO_LARGE = 1, DUPLICATE = 2, OUT_OF_RANGE = 4 };
+
+struct Level {
+  int ox, oy, oz;  // coordinate of cell 0: one below the smallest, so that a neighbour of a voxel is always a cell
+  int dy, dzw;     // rows of z per x, words per row of z
+  int word0;       // first word of the level (a multiple of 4)
+};
+// Lives in the workspace.  lo / neg_hi / ticket start as 0x7f7f7f7f (one memset).
+struct Header {
+  int lo[3], neg_hi[3];
+  unsigned ticket;
+  int flags;       // what makes the cloud unfit
+  int groups;      // groups of 4 words, all levels
+  int first_group[MAX_LEVELS + 1];
+  Level level[MAX_LEVELS];
+};
+struct Job { int kind, level, k_vol; };  // DOWN / UP: between level and level + 1
+// Where the blocks of the jobs begin, and the levels' sizes and ranks.
+struct Jobs {
+  int base[MAX_LEVELS + 1];       // rank before the level
+  int first_block[MAX_JOBS + 1];  // blocks of ROWS rows, job after job
+  int rows[MAX_JOBS];
+  int first_count[MAX_JOBS];      // of the job's [k_vol][blocks] in counts
+};
+struct Args {
+  const int32_t* coords;       // [n, 3]
+  int n, levels, n_jobs;
+  Job job[MAX_JOBS];
+  Header* head;
+  uint32_t* bits;
+  int* prefix;                 // [groups + 1] set bits before a group
+  int* block_sums;             // [SCAN_BLOCKS]
+  Jobs* jobs;                  // written with the positions, read by the last kernel
+  int* row_of;                 // [n] input row of the voxel of a rank
+  uint32_t* mask;              // [n_jobs][n]
+  int* counts;                 // per job [k_vol][blocks], job after job, sized for n rows each
+  int32_t* kpos;               // [n_jobs][28]
+  int32_t* out_coords[MAX_LEVELS];  // level 1 ..: [n, 3]
+  int32_t *in_map[MAX_JOBS], *out_map[MAX_JOBS];
+  int cap_words;
+};
+constexpr int KPOS_STRIDE = 28;
+
+__device__ __forceinline__ const int32_t* coords_of(const Args& a, int level) { return level == 0 ? a.coords : a.out_coords[level]; }
+
+// Three bits from cell z on (a cell of the padded row): bit d is cell z + d.
+__device__ __forceinline__ uint32_t window(const uint32_t* __restrict__ row, int z) {
+  const int w = z >> 5, b = z & 31;
+  uint32_t v = __ldg(row + w) >> b;
+  if (b > 29) v |= __ldg(row + w + 1) << (32 - b);  // cell z + 2 is inside the padded row
+  return v & 7u;
+}
+// set bits of the level before bit b of word w
+__device__ __forceinline__ int rank_before(const Args& a, int w, int b, int level_base) {
+  const uint4 v = __ldg(reinterpret_cast<const uint4*>(a.bits) + (w >> 2));
+  const int i = w & 3;
+  const uint32_t mine = i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w));
+  int r = __ldg(a.prefix + (w >> 2)) - level_base + __popc(mine & ((1u << b) - 1u));
+  if (i > 0) r += __popc(v.x);
+  if (i > 1) r += __popc(v.y);
+  if (i > 2) r += __popc(v.z);
+  return r;
+}
+__device__ __forceinline__ int row_word(const Level& L, int x, int y) { return L.word0 + ((x - L.ox) * L.dy + (y - L.oy)) * L.dzw; }
+__device__ __forceinline__ int rank_of(const Args& a, const Level& L, int base, int x, int y, int z) {
+  const int zz = z - L.oz;
+  return rank_before(a, row_word(L, x, y) + (zz >> 5), zz & 31, base);
+}
+
+// ---- 1: bounding box; the last block lays out the levels -----------------------------------------------------------
+__global__ void __launch_bounds__(THREADS) box_kernel(Args a) {
+  umma::griddep_wait();
+  umma::griddep_launch_dependents();
+  int m[6] = {0x7f7f7f7f, 0x7f7f7f7f, 0x7f7f7f7f, 0x7f7f7f7f, 0x7f7f7f7f, 0x7f7f7f7f};
+  bool wide = false;
+  for (int i = blockIdx.x * THREADS + threadIdx.x; i < a.n; i += gridDim.x * THREADS) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const int v = __ldg(a.coords + 3 * i + d);
+      if (v < -maps::COORD_BIAS || v >= maps::COORD_BIAS) wide = true;
+      else { m[d] = min(m[d], v); m[3 + d] = min(m[3 + d], -v); }
+    }
+  }
+#pragma unroll
+  for (int d = 0; d < 6; ++d) m[d] = __reduce_min_sync(0xffffffffu, m[d]);
+  wide = __any_sync(0xffffffffu, wide);
+  __shared__ int part[WARPS][6];
+  __shared__ bool wide_any, last;
+  if (threadIdx.x == 0) wide_any = false;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int d = 0; d < 6; ++d) part[threadIdx.x >> 5][d] = m[d];
+    if (wide) wide_any = true;
+  }
+  __syncthreads();
+  Header* h = a.head;
+  if (threadIdx.x < 6) {
+    int v = part[0][threadIdx.x];
+    for (int w = 1; w < WARPS; ++w) v = min(v, part[w][threadIdx.x]);
+    atomicMin((threadIdx.x < 3 ? h->lo : h->neg_hi) + threadIdx.x % 3, v);
+  }
+  if (threadIdx.x == 6 && wide_any) atomicMin(&h->flags, 0x7f7f7f7f - OUT_OF_RANGE);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&h->ticket, 1u) == 0x7f7f7f7fu + gridDim.x - 1;
+  __syncthreads();
+  if (!last || threadIdx.x != 0) return;
+  __threadfence();
+  volatile Header* hv = h;
+  int flags = hv->flags == 0x7f7f7f7f ? 0 : OUT_OF_RANGE;
+  long long word = 0;
+  for (int l = 0; l < a.levels; ++l) {
+    Level L;
+    const int lx = hv->lo[0] >> l, ly = hv->lo[1] >> l, lz = hv->lo[2] >> l;
+    const int hx = -hv->neg_hi[0] >> l, hy = -hv->neg_hi[1] >> l, hz = -hv->neg_hi[2] >> l;
+    L.ox = lx - 1; L.oy = ly - 1; L.oz = lz - 1;
+    L.dy = hy - ly + 3;
+    L.dzw = (hz - lz + 3 + 31) / 32;
+    L.word0 = (int)word;
+    word = (word + (long long)(hx - lx + 3) * L.dy * L.dzw + 3) & ~3ll;
+    if (flags || word > a.cap_words) { flags |= TOO_LARGE; word = 0; }
+    h->level[l] = L;
+    h->first_group[l + 1] = (int)(word >> 2);
+  }
+  h->first_group[0] = 0;
+  h->groups = (int)(word >> 2);
+  h->flags = flags;
+}
+
+// ---- 2: clear ----------------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(THREADS) clear_kernel(Args a) {
+  umma::griddep_wait();
+  umma::griddep_launch_dependents();
+  const int n = a.head->groups;
+  uint4* p = reinterpret_cast<uint4*>(a.bits);
+  for (int i = blockIdx.x * THREADS + threadIdx.x; i < n; i += gridDim.x * THREADS) p[i] = make_uint4(0, 0, 0, 0);
+}
+
+// ---- 3: voxels and their ancestors -------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(THREADS) insert_kernel(Args a) {
+  umma::griddep_wait();
+  umma::griddep_launch_dependents();
+  if (a.head->flags & ~DUPLICATE) return;
+  const int i = blockIdx.x * THREADS + threadIdx.x, lane = threadIdx.x & 31;
+  const uint32_t active = __ballot_sync(0xffffffffu, i < a.n);
+  if (i >= a.n) return;
+  const int x = a.coords[3 * i], y = a.coords[3 * i + 1], z = a.coords[3 * i + 2];
+  for (int l = 0; l < a.levels; ++l) {
+    const Level L = a.head->level[l];
+    const int zz = (z >> l) - L.oz, w = row_word(L, x >> l, y >> l) + (zz >> 5);
+    const uint32_t bit = 1u << (zz & 31);
+    if (l == 0) {
+      if (atomicOr(a.bits + w, bit) & bit) atomicOr(&a.head->flags, DUPLICATE);
+    } else {
+      // neighbouring rows mostly share an ancestor's word: one atomic for those of a warp (the few hundred words of a
+      // coarse level took one per voxel before, 37 us on 120 k voxels)
+      const uint32_t same = __match_any_sync(active, w);
+      const uint32_t all = __reduce_or_sync(same, bit);
+      if (lane == __ffs(same) - 1 && (*(volatile uint32_t*)(a.bits + w) & all) != all) atomicOr(a.bits + w, all);
+    }
+  }
+}
+
+// ---- 4: set bits before every group of 4 words ---------------------------------------------------------------------------
+__device__ __forceinline__ int group_count(const Args& a, int g) {
+  const uint4 x = reinterpret_cast<const uint4*>(a.bits)[g];
+  return __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+}
+__device__ __forceinline__ int block_sum(int v, int* part) {  // every thread gets the sum
+  v = __reduce_add_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  int s = 0;
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w) s += part[w];
+  __syncthreads();
+  return s;
+}
+__global__ void __launch_bounds__(THREADS) sum_kernel(Args a) {
+  umma::griddep_wait();
+  umma::griddep_launch_dependents();
+  if (a.head->flags) return;
+  __shared__ int part[WARPS];
+  const int groups = a.head->groups, per = (groups + SCAN_BLOCKS - 1) / SCAN_BLOCKS;
+  const int g0 = min(groups, (int)blockIdx.x * per), g1 = min(groups, g0 + per);
+  int c = 0;
+  for (int g = g0 + threadIdx.x; g < g1; g += THREADS) c += group_count(a, g);
+  const int s = block_sum(c, part);
+  if (threadIdx.x == 0) a.block_sums[blockIdx.x] = s;
+}
+__global__ void __launch_bounds__(THREADS) prefix_kernel(Args a) {
+  umma::griddep_wait();
+  umma::griddep_launch_dependents();
+  if (a.head->flags) return;
+  __shared__ int part[WARPS];
+  const int groups = a.head->groups, per = (groups + SCAN_BLOCKS - 1) / SCAN_BLOCKS;
+  const int g0 = min(groups, (int)blockIdx.x * per), g1 = min(groups, g0 + per);
+  int before = 0;
+  for (int b = threadIdx.x; b < (int)blockIdx.x; b += THREADS) before += a.block_sums[b];
+  before = block_sum(before, part);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int g = g0; g < g1; g += THREADS) {
+    const int c = g + (int)threadIdx.x < g1 ? group_count(a, g + threadIdx.x) : 0;
+    int incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) part[warp] = incl;
+    __syncthreads();
+    int ahead = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+      if (w < warp) ahead += part[w];
+      all += part[w];
+    }
+    if (g + (int)threadIdx.x < g1) a.prefix[g + threadIdx.x] = before + ahead + incl - c;
+    before += all;
+    __syncthreads();
+  }
+  if (g1 == groups && g0 < g1 && threadIdx.x == 0) a.prefix[groups] = before;
+}
+
+// ---- 5: rows of every level ------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(THREADS) rows_kernel(Args a) {
+  umma::griddep_wait();
+  umma::griddep_launch_dependents();
+  if (a.head->flags) return;
+  const int i = blockIdx.x * THREADS + threadIdx.x;
+  if (i >= a.n) return;
+  const int x = a.coords[3 * i], y = a.coords[3 * i + 1], z = a.coords[3 * i + 2];
+  a.row_of[rank_of(a, a.head->level[0], 0, x, y, z)] = i;
+  for (int l = 1; l < a.levels; ++l) {
+    const int px = x >> l, py = y >> l, pz = z >> l;
+    const int r = rank_of(a, a.head->level[l], a.prefix[a.head->first_group[l]], px, py, pz);
+    int32_t* o = a.out_coords[l] + 3 * (size_t)r;  // the same value from every voxel below this one
+    o[0] = px; o[1] = py; o[2] = pz;
+  }
+}
+
+__device__ __forceinline__ void find_jobs(const Args& a, Jobs& s) {
+  if ((int)threadIdx.x <= a.levels) s.base[threadIdx.x] = a.prefix[a.head->first_group[threadIdx.x]];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int b = 0, c = 0;
+    for (int j = 0; j < a.n_jobs; ++j) {
+      const int l = a.job[j].level + (a.job[j].kind == DOWN ? 1 : 0);  // the level of the map's output rows
+      s.first_block[j] = b;
+      s.first_count[j] = c;
+      s.rows[j] = s.base[l + 1] - s.base[l];
+      const int blocks = (s.rows[j] + ROWS - 1) / ROWS;
+      b += blocks;
+      c += blocks * a.job[j].k_vol;
+    }
+    s.first_block[a.n_jobs] = b;
+  }
+  __syncthreads();
+}
+
+// ---- 6: which offsets a row has, and how many rows of a block have each -----------------------------------------------------
+__device__ __forceinline__ uint32_t row_mask(const Args& a, const Job& job, int row) {
+  uint32_t m = 0;
+  if (job.kind == SUBM) {
+    const Level L = a.head->level[job.level];
+    const int32_t* c = coords_of(a, job.level) + 3 * (size_t)row;
+    const int x = c[0], y = c[1], z = c[2] - L.oz - 1;
+#pragma unroll
+    for (int d = 0; d < 9; ++d) m |= window(a.bits + row_word(L, x + d / 3 - 1, y + d % 3 - 1), z) << (3 * d);
+  } else if (job.kind == DOWN) {
+    const Level L = a.head->level[job.level];
+    const int32_t* c = coords_of(a, job.level + 1) + 3 * (size_t)row;
+    // a parent's children may lie outside the box of the finer level by one cell, the padding
+    const int x = 2 * c[0], y = 2 * c[1], z = 2 * c[2] - L.oz;
+#pragma unroll
+    for (int d = 0; d < 4; ++d) m |= (window(a.bits + row_word(L, x + d / 2, y + d % 2), z) & 3u) << (2 * d);
+  } else {
+    const int32_t* c = coords_of(a, job.level) + 3 * (size_t)row;
+    m = 1u << (((c[0] & 1) * 2 + (c[1] & 1)) * 2 + (c[2] & 1));
+  }
+  return m;
+}
+__global__ void __launch_bounds__(THREADS) count_kernel(Args a) {
+  umma::griddep_wait();
+  umma::griddep_launch_dependents();
+  if (a.head->flags) return;
+  __shared__ Jobs s;
+  __shared__ int part[WARPS][32];
+  find_jobs(a, s);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int blk = blockIdx.x; blk < s.first_block[a.n_jobs]; blk += gridDim.x) {
+    int j = 0;
+    while (blk >= s.first_block[j + 1]) ++j;
+    const int b = blk - s.first_block[j], row = b * ROWS + (int)threadIdx.x, k_vol = a.job[j].k_vol;
+    uint32_t m = 0;
+    if (row < s.rows[j]) {
+      m = row_mask(a, a.job[j], row);
+      a.mask[(size_t)j * a.n + row] = m;
+    }
+    int mine = 0;  // lane k: rows of the warp with offset k
+    for (int k = 0; k < k_vol; ++k) {
+      const int c = __popc(__ballot_sync(0xffffffffu, m >> k & 1u));
+      if (lane == k) mine = c;
+    }
+    part[warp][lane] = mine;
+    __syncthreads();
+    if ((int)threadIdx.x < k_vol) {
+      int c = 0;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) c += part[w][threadIdx.x];
+      a.counts[s.first_count[j] + (int)threadIdx.x * (s.first_block[j + 1] - s.first_block[j]) + b] = c;
+    }
+    __syncthreads();
+  }
+}
+
+// ---- 7: position of every (offset, block) in its map; one block per job -------------------------------------------------------
+constexpr int SCAN_THREADS = 1024;
+__global__ void __launch_bounds__(SCAN_THREADS) position_kernel(Args a, int* sizes /* [1 + levels + jobs]: flags, voxels, pairs */) {
+  umma::griddep_wait();
+  umma::griddep_launch_dependents();
+  const int j = blockIdx.x, flags = a.head->flags;
+  if (j == 0 && threadIdx.x == 0) sizes[0] = flags;
+  if (flags) return;
+  __shared__ Jobs s;
+  __shared__ int part[SCAN_THREADS / 32];
+  find_jobs(a, s);
+  if (j == 0 && (int)threadIdx.x < a.levels) sizes[1 + threadIdx.x] = s.base[threadIdx.x + 1] - s.base[threadIdx.x];
+  const int blocks = s.first_block[j + 1] - s.first_block[j], k_vol = a.job[j].k_vol, total = blocks * k_vol;
+  int* c = a.counts + s.first_count[j];
+  int32_t* kpos = a.kpos + j * KPOS_STRIDE;
+  if (j == 0)
+    for (int i = threadIdx.x; i < (int)(sizeof(Jobs) / 4); i += SCAN_THREADS) reinterpret_cast<int*>(a.jobs)[i] = reinterpret_cast<const int*>(&s)[i];
+  // every warp sums a consecutive part, then scans it from the sum of the parts before
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int per = (total + SCAN_THREADS - 1) / SCAN_THREADS * 32, i0 = min(total, warp * per), i1 = min(total, i0 + per);
+  int sum = 0;
+#pragma unroll 4
+  for (int i = i0 + lane; i < i1; i += 32) sum += c[i];
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if (lane == 0) part[warp] = sum;
+  __syncthreads();
+  int at = __reduce_add_sync(0xffffffffu, lane < warp ? part[lane] : 0);
+  const int before = __reduce_add_sync(0xffffffffu, part[lane]);
+#pragma unroll 4
+  for (int i = i0; i < i1; i += 32) {
+    const int v = i + lane < i1 ? c[i + lane] : 0;
+    int incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += n;
+    }
+    if (i + lane < i1) c[i + lane] = at + incl - v;
+    at += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < k_vol) kpos[threadIdx.x] = c[(int)threadIdx.x * blocks];
+  if (threadIdx.x == 0) {
+    kpos[k_vol] = before;
+    sizes[1 + a.levels + j] = before;
+  }
+}
+
+// ---- 8: the pairs ---------------------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(THREADS, 4) emit_kernel(Args a) {
+  umma::griddep_wait();
+  umma::griddep_launch_dependents();
+  __shared__ Jobs s;
+  __shared__ int part[WARPS][32];  // pairs of the warp per offset, then where they go
+  for (int i = threadIdx.x; i < (int)(sizeof(Jobs) / 4); i += THREADS) reinterpret_cast<int*>(&s)[i] = reinterpret_cast<const int*>(a.jobs)[i];
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int blk = blockIdx.x; blk < s.first_block[a.n_jobs]; blk += gridDim.x) {
+    int j = 0;
+    while (blk >= s.first_block[j + 1]) ++j;
+    const Job job = a.job[j];
+    const int b = blk - s.first_block[j], row = b * ROWS + (int)threadIdx.x, k_vol = job.k_vol;
+    const bool there = row < s.rows[j];
+    const uint32_t m = there ? a.mask[(size_t)j * a.n + row] : 0u;
+    int mine = 0;
+    for (int k = 0; k < k_vol; ++k) {
+      const int c = __popc(__ballot_sync(0xffffffffu, m >> k & 1u));
+      if (lane == k) mine = c;
+    }
+    part[warp][lane] = mine;
+    // input rows: the rank before the first of a column's cells; the cells after it follow in rank
+    int first[9];
+    if (there) {
+      const int32_t* c = coords_of(a, job.level + (job.kind == DOWN ? 1 : 0)) + 3 * (size_t)row;
+      if (job.kind == SUBM) {
+        const Level L = a.head->level[job.level];
+        const int z = c[2] - L.oz - 1;
+#pragma unroll
+        for (int d = 0; d < 9; ++d)
+          if (m >> (3 * d) & 7u) first[d] = rank_before(a, row_word(L, c[0] + d / 3 - 1, c[1] + d % 3 - 1) + (z >> 5), z & 31, s.base[job.level]);
+      } else if (job.kind == DOWN) {
+        const Level L = a.head->level[job.level];
+        const int z = 2 * c[2] - L.oz;
+#pragma unroll
+        for (int d = 0; d < 4; ++d)
+          if (m >> (2 * d) & 3u) first[d] = rank_before(a, row_word(L, 2 * c[0] + d / 2, 2 * c[1] + d % 2) + (z >> 5), z & 31, s.base[job.level]);
+      } else {
+        first[0] = rank_of(a, a.head->level[job.level + 1], s.base[job.level + 1], c[0] >> 1, c[1] >> 1, c[2] >> 1);
+      }
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < k_vol) {
+      int at = a.counts[s.first_count[j] + (int)threadIdx.x * (s.first_block[j + 1] - s.first_block[j]) + b];
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) {
+        const int c = part[w][threadIdx.x];
+        part[w][threadIdx.x] = at;
+        at += c;
+      }
+    }
+    __syncthreads();
+    int32_t *in_map = a.in_map[j], *out_map = a.out_map[j];
+    const uint32_t below = (1u << lane) - 1u;
+    auto put = [&](int k, int src) {  // the whole warp calls it
+      const uint32_t who = __ballot_sync(0xffffffffu, m >> k & 1u);
+      if (m >> k & 1u) {
+        const int at = part[warp][k] + __popc(who & below);
+        in_map[at] = src;
+        out_map[at] = row;
+      }
+    };
+    // all of a row's input rows are asked for before the first pair is written: one trip to memory instead of one per offset
+    if (job.kind == SUBM) {
+      int src[27];
+#pragma unroll
+      for (int d = 0; d < 9; ++d) {
+        int r = first[d];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+          const bool on = m >> (3 * d + u) & 1u;
+          src[3 * d + u] = on && job.level == 0 ? __ldg(a.row_of + r) : r;
+          r += on ? 1 : 0;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 27; ++k) put(k, src[k]);
+    } else if (job.kind == DOWN) {
+      int src[8];
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {
+        int r = first[d];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const bool on = m >> (2 * d + u) & 1u;
+          src[2 * d + u] = on && job.level == 0 ? __ldg(a.row_of + r) : r;
+          r += on ? 1 : 0;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) put(k, src[k]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) put(k, first[0]);
+    }
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------------------
+struct Plan {
+  size_t sizes, jobs, bits, prefix, block_sums, row_of, mask, counts, total;  // offsets into the workspace (the header is at 0)
+  int n_jobs, cap_words;
+  Job job[MAX_JOBS];
+};
+// Cells of all levels' boxes the workspace has room for: 64 MB of bits (a 2000 x 2000 x 80 scan and its coarser levels
+// take 55 MB), more for clouds of more than 200 k voxels, at most 400 MB.
+inline int capacity_words(int n) {
+  const long long want = 80ll * n, least = 16ll << 20, most = 100ll << 20;
+  return (int)(want < least ? least : (want > most ? most : want));
+}
+inline bool plan(int n, int levels, int what, Plan* p) {
+  if (n < 1 || levels < 1 || levels > MAX_LEVELS || (what & ~(SUBM | DOWN | UP)) || !what) return false;
+  p->n_jobs = 0;
+  for (int kind : {SUBM, DOWN, UP})
+    if (what & kind)
+      for (int l = 0; l < levels - (kind == SUBM ? 0 : 1); ++l) p->job[p->n_jobs++] = Job{kind, l, kind == SUBM ? 27 : 8};
+  if (p->n_jobs == 0) return false;
+  p->cap_words = capacity_words(n);
+  size_t off = maps::align256(sizeof(Header));
+  auto take = [&](size_t bytes) { const size_t at = off; off += maps::align256(bytes); return at; };
+  p->sizes = take((1 + MAX_LEVELS + MAX_JOBS) * 4);
+  p->jobs = take(sizeof(Jobs));
+  p->bits = take(((size_t)p->cap_words + 64) * 4);
+  p->prefix = take(((size_t)p->cap_words / 4 + 1) * 4);
+  p->block_sums = take(SCAN_BLOCKS * 4);
+  p->row_of = take((size_t)n * 4);
+  p->mask = take((size_t)p->n_jobs * n * 4);
+  size_t counts = 0;
+  for (int j = 0; j < p->n_jobs; ++j) counts += (size_t)p->job[j].k_vol * (((size_t)n + ROWS - 1) / ROWS);
+  p->counts = take(counts * 4);
+  p->total = off;
+  return true;
+}
+inline Args arguments(const Plan& p, const int32_t* coords, int n, int levels, int32_t* kpos, int32_t* const* out_coords, uint8_t* ws) {
+  Args a = {};
+  a.coords = coords; a.n = n; a.levels = levels; a.n_jobs = p.n_jobs;
+  for (int j = 0; j < p.n_jobs; ++j) a.job[j] = p.job[j];
+  a.head = reinterpret_cast<Header*>(ws);
+  a.bits = reinterpret_cast<uint32_t*>(ws + p.bits);
+  a.prefix = reinterpret_cast<int*>(ws + p.prefix);
+  a.block_sums = reinterpret_cast<int*>(ws + p.block_sums);
+  a.jobs = reinterpret_cast<Jobs*>(ws + p.jobs);
+  a.row_of = reinterpret_cast<int*>(ws + p.row_of);
+  a.mask = reinterpret_cast<uint32_t*>(ws + p.mask);
+  a.counts = reinterpret_cast<int*>(ws + p.counts);
+  a.kpos = kpos;
+  for (int l = 1; l < levels; ++l) a.out_coords[l] = out_coords[l - 1];
+  a.cap_words = p.cap_words;
+  return a;
+}
+inline int map_blocks(const Plan& p, int n, int sms) {
+  const long long most = (long long)p.n_jobs * ((n + ROWS - 1) / ROWS);
+  return (int)(most < 4ll * sms ? most : 4ll * sms);
+}
+// everything up to the sizes of the maps; false on a launch error
+inline bool launch_plan(const Plan& p, const Args& a, uint8_t* ws, int sms, cudaStream_t st) {
+  const int per_voxel = (a.n + THREADS - 1) / THREADS;
+  const int few = per_voxel < 2 * sms ? per_voxel : 2 * sms;
+  bool ok = cudaMemsetAsync(ws, 0x7f, 32, st) == cudaSuccess;  // lo, neg_hi, ticket, flags
+  ok = ok && launch_pdl(box_kernel, few, THREADS, 0, st, a) == cudaSuccess;
+  ok = ok && launch_pdl(clear_kernel, 8 * sms, THREADS, 0, st, a) == cudaSuccess;
+  ok = ok && launch_pdl(insert_kernel, per_voxel, THREADS, 0, st, a) == cudaSuccess;
+  ok = ok && launch_pdl(sum_kernel, SCAN_BLOCKS, THREADS, 0, st, a) == cudaSuccess;
+  ok = ok && launch_pdl(prefix_kernel, SCAN_BLOCKS, THREADS, 0, st, a) == cudaSuccess;
+  ok = ok && launch_pdl(rows_kernel, per_voxel, THREADS, 0, st, a) == cudaSuccess;
+  ok = ok && launch_pdl(count_kernel, map_blocks(p, a.n, sms), THREADS, 0, st, a) == cudaSuccess;
+  ok = ok && launch_pdl(position_kernel, p.n_jobs, SCAN_THREADS, 0, st, a, reinterpret_cast<int*>(ws + p.sizes)) == cudaSuccess;
+  return ok;
+}
+
+}  // namespace pyramid
+}  // namespace fgms

@@ -6,12 +6,16 @@
 // kernel runs 6 us; 56 us per layer and pass through the autograd engine), which is what bounded every layer of up to
 // about a hundred thousand voxels.  Error types are those of the reference's binding: ValueError for what pybind11
 // maps from std::invalid_argument, TypeError for an argument that is no tensor, RuntimeError for a CUDA failure.
+#include <array>
+#include <vector>
+
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <pybind11/pybind11.h>
 
 #include "../../include/fgms_b200.h"
 
@@ -206,6 +210,68 @@ void fwd_os(const Tensor& in_feats, const Tensor& kernel, const Tensor& out, con
 }
 
 // ---------------------------------------------------------------------------------------------
+// kernel maps
+// ---------------------------------------------------------------------------------------------
+struct Pyramid {
+  bool fits = false;
+  std::vector<int64_t> voxels;                  // per level
+  std::vector<std::array<Tensor, 3>> maps;      // kpos, imap, omap
+  std::vector<Tensor> out_coords;               // level 1 ..
+};
+
+// The maps of `what` (see fgms_b200_pyramid_plan) of the cloud and its coarser levels.  One wait, for the sizes; the
+// Python objects around the maps are made while the last kernel runs.
+Pyramid build_pyramid(const Tensor& coords, int levels, int what) {
+  TORCH_CHECK_VALUE(coords.is_cuda() && coords.scalar_type() == at::kInt && coords.dim() == 2 && coords.size(1) == 3 && coords.is_contiguous(),
+                    "coords must be a contiguous CUDA int32 tensor of shape [n, 3]");
+  Pyramid r;
+  const int64_t n64 = coords.size(0);
+  if (n64 < 1 || n64 > 0x7fffffffll / 27) return r;
+  const int n = (int)n64;
+  const size_t bytes = fgms_b200_pyramid_workspace_bytes(n, levels, what);
+  if (bytes == 0) return r;
+  c10::cuda::CUDAGuard guard(coords.device());
+  void* st = stream_of(coords);
+  const auto ints = coords.options();
+  const int n_maps = ((what & 1) ? levels : 0) + ((what & 2) ? levels - 1 : 0) + ((what & 4) ? levels - 1 : 0);
+  const Tensor ws = at::empty({(int64_t)bytes}, ints.dtype(at::kByte)), kpos = at::empty({n_maps * 28}, ints);
+  std::vector<int32_t*> coord_ptrs;
+  for (int l = 1; l < levels; ++l) {
+    r.out_coords.push_back(at::empty({n64, 3}, ints));
+    coord_ptrs.push_back(r.out_coords.back().data_ptr<int32_t>());
+  }
+  const Tensor host = at::empty({64}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+  const int32_t* sizes = host.data_ptr<int32_t>();
+  int rc;
+  {
+    pybind11::gil_scoped_release unlock;  // this waits for the device
+    rc = fgms_b200_pyramid_plan(iptr(coords), n, levels, what, kpos.data_ptr<int32_t>(), coord_ptrs.data(), ws.data_ptr(), bytes,
+                                host.data_ptr<int32_t>(), st);
+  }
+  check_status(rc);
+  if (sizes[0] != 0) return r;
+  r.fits = true;
+  for (int l = 0; l < levels; ++l) r.voxels.push_back(sizes[1 + l]);
+  std::vector<Tensor> flat;
+  std::vector<int32_t*> in_maps, out_maps;
+  for (int j = 0; j < n_maps; ++j) {  // both maps of a layer in one allocation, each on a 256-byte boundary
+    const int64_t pad = (sizes[1 + levels + j] + 64) / 64 * 64;
+    flat.push_back(at::empty({2 * pad}, ints));
+    in_maps.push_back(flat[j].data_ptr<int32_t>());
+    out_maps.push_back(in_maps[j] + pad);
+  }
+  check_status(fgms_b200_pyramid_emit(iptr(coords), n, levels, what, kpos.data_ptr<int32_t>(), coord_ptrs.data(), in_maps.data(),
+                                      out_maps.data(), ws.data_ptr(), bytes, st));
+  for (int j = 0; j < n_maps; ++j) {
+    const int64_t pairs = sizes[1 + levels + j], pad = flat[j].numel() / 2;
+    const bool subm = (what & 1) && j < levels;
+    r.maps.push_back({kpos.narrow(0, j * 28, subm ? 28 : 9), flat[j].narrow(0, 0, pairs), flat[j].narrow(0, pad, pairs)});
+  }
+  for (int l = 1; l < levels; ++l) r.out_coords[l - 1] = r.out_coords[l - 1].narrow(0, 0, r.voxels[l]);
+  return r;
+}
+
+// ---------------------------------------------------------------------------------------------
 // Python entry points (positional arguments only; the functions of backend.py / nn.py give them their names)
 // ---------------------------------------------------------------------------------------------
 const Tensor& feat_arg(PyObject* o, const char* name) {
@@ -282,10 +348,29 @@ PyObject* py_fwd_os(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// (voxels per level, [(kpos, imap, omap) ...], [coords of level 1 ...]), or None for a cloud that does not suit
+PyObject* py_build_pyramid(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 3);
+  const Pyramid r = build_pyramid(index_arg(a[0], "coords"), (int)int_arg(a[1]), (int)int_arg(a[2]));
+  if (!r.fits) Py_RETURN_NONE;
+  PyObject *voxels = PyList_New(r.voxels.size()), *maps = PyList_New(r.maps.size()), *coords = PyList_New(r.out_coords.size());
+  for (size_t i = 0; i < r.voxels.size(); ++i) PyList_SET_ITEM(voxels, i, PyLong_FromLongLong(r.voxels[i]));
+  for (size_t i = 0; i < r.maps.size(); ++i) {
+    PyObject* t = PyTuple_New(3);
+    for (int k = 0; k < 3; ++k) PyTuple_SET_ITEM(t, k, THPVariable_Wrap(r.maps[i][k]));
+    PyList_SET_ITEM(maps, i, t);
+  }
+  for (size_t i = 0; i < r.out_coords.size(); ++i) PyList_SET_ITEM(coords, i, THPVariable_Wrap(r.out_coords[i]));
+  return Py_BuildValue("(NNN)", voxels, maps, coords);
+  END_HANDLE_TH_ERRORS
+}
+
 #define FGMS_METHOD(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(fn)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     FGMS_METHOD("fusion_fwd", py_fusion_fwd), FGMS_METHOD("seq_fwd", py_seq_fwd),         FGMS_METHOD("bwd", py_bwd),
-    FGMS_METHOD("fwd_os", py_fwd_os),         FGMS_METHOD("sparse_conv", py_sparse_conv), {nullptr, nullptr, 0, nullptr}};
+    FGMS_METHOD("fwd_os", py_fwd_os),         FGMS_METHOD("sparse_conv", py_sparse_conv),
+    FGMS_METHOD("build_pyramid", py_build_pyramid), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

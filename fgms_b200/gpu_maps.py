@@ -1,4 +1,4 @@
-"""Kernel maps built on the GPU (``csrc/map_builder.cuh`` through the C ABI).
+"""Kernel maps built on the GPU (``csrc/map_pyramid.cuh`` and ``csrc/map_builder.cuh`` through the C ABI).
 
 Same canonical form, bit for bit, as the host builders in :mod:`fgms_b200.maps`; the results stay on
 the device as int32 tensors, ready for ``fgms_fusion_fwd_cuda`` / ``fgms_bwd_cuda``.  The reference has
@@ -11,11 +11,14 @@ from dataclasses import dataclass
 
 import torch
 
-from . import _lib
+from . import _lib, _native
 
 _L = _lib.lib
 
-__all__ = ["DeviceKernelMap", "build_submanifold_map", "build_strided_map", "transpose_map"]
+__all__ = ["DeviceKernelMap", "build_submanifold_map", "build_strided_map", "transpose_map", "build_pyramid"]
+
+
+_SUBM, _DOWN, _UP = 1, 2, 4  # what of fgms_b200_pyramid_plan
 
 
 @dataclass
@@ -54,9 +57,38 @@ def _workspace(n: int, n_cols: int, k_vol: int, device) -> torch.Tensor:
     return torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
 
 
+def build_pyramid(coords: torch.Tensor, levels: int):
+    """The maps of ``levels`` + 1 resolutions of a cloud in one go: ``(subm, down, up)``, lists of
+    :class:`DeviceKernelMap` as :func:`build_submanifold_map` (3x3x3), :func:`build_strided_map` (stride 2) and
+    :func:`transpose_map` would give them one by one."""
+    coords = _check_coords(coords)
+    got = _native.build_pyramid(coords, levels + 1, _SUBM | _DOWN | _UP) if levels > 0 else None
+    subm, down, up = [], [], []
+    if got is None:  # no such pyramid, or a cloud that does not suit its builder
+        for r in range(levels + 1):
+            subm.append(build_submanifold_map(coords, 3))
+            if r < levels:
+                down.append(build_strided_map(coords, 2))
+                up.append(transpose_map(down[-1], coords))
+                coords = down[-1].out_coords
+        return subm, down, up
+    voxels, maps, coarser = got
+    c = [coords] + coarser
+    for r in range(levels + 1):
+        subm.append(DeviceKernelMap(voxels[r], voxels[r], 27, *maps[r], c[r]))
+    for r in range(levels):
+        down.append(DeviceKernelMap(voxels[r], voxels[r + 1], 8, *maps[levels + 1 + r], c[r + 1]))
+        up.append(DeviceKernelMap(voxels[r + 1], voxels[r], 8, *maps[2 * levels + 1 + r], c[r]))
+    return subm, down, up
+
+
 def build_submanifold_map(coords: torch.Tensor, kernel_size: int = 3) -> DeviceKernelMap:
     """Stride-1 map: pair ``(i, o)`` in offset ``d`` iff ``coords[i] == coords[o] + d``."""
     coords = _check_coords(coords)
+    got = _native.build_pyramid(coords, 1, _SUBM) if kernel_size == 3 else None
+    if got is not None:
+        n = coords.size(0)
+        return DeviceKernelMap(n, n, 27, *got[1][0], coords)
     n, k_vol, dev = coords.size(0), kernel_size ** 3, coords.device
     kpos = torch.empty(k_vol + 1, dtype=torch.int32, device=dev)
     imap = torch.empty(n * k_vol, dtype=torch.int32, device=dev)
@@ -73,6 +105,10 @@ def build_submanifold_map(coords: torch.Tensor, kernel_size: int = 3) -> DeviceK
 def build_strided_map(coords: torch.Tensor, stride: int = 2) -> DeviceKernelMap:
     """Downsampling map with ``kernel_size == stride``; output voxels are the distinct ``coords // stride``."""
     coords = _check_coords(coords)
+    got = _native.build_pyramid(coords, 2, _DOWN) if stride == 2 else None
+    if got is not None:
+        (n, n_out), (maps,), (out_coords,) = got
+        return DeviceKernelMap(n, n_out, 8, *maps, out_coords)
     n, k_vol, dev = coords.size(0), stride ** 3, coords.device
     kpos = torch.empty(k_vol + 1, dtype=torch.int32, device=dev)
     imap = torch.empty(n, dtype=torch.int32, device=dev)

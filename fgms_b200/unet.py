@@ -94,16 +94,7 @@ class UNetMaps:
 def build_unet_maps(coords, levels: int = 4) -> UNetMaps:
     """All maps of the stack on the device (``coords``: CUDA int32 ``[n, 3]``, no voxel twice)."""
     from . import gpu_maps
-    subm, down, up = [], [], []
-    c = coords
-    for r in range(levels + 1):
-        subm.append(gpu_maps.build_submanifold_map(c, 3))
-        if r < levels:
-            d = gpu_maps.build_strided_map(c, 2)
-            down.append(d)
-            up.append(gpu_maps.transpose_map(d, c))
-            c = d.out_coords
-    return UNetMaps(subm, down, up)
+    return UNetMaps(*gpu_maps.build_pyramid(coords, levels))
 
 
 def build_unet_maps_host(coords: np.ndarray, levels: int = 4) -> UNetMaps:

@@ -194,6 +194,23 @@ int fgms_b200_transpose_map(const int32_t* kpos, const int32_t* in_map, const in
                             int n_in, int k_vol, int64_t pairs, int32_t* kpos_t, int32_t* in_map_t,
                             int32_t* out_map_t, void* workspace, size_t workspace_bytes, void* stream);
 
+/* Kernel maps of a pyramid of `levels` resolutions (1..8) in one go: level 0 is the cloud `coords` (int32 [n, 3], any
+ * order), level l + 1 its distinct coords >> (l + 1) in lexicographic order.  `what` selects maps: 1 = the 3x3x3
+ * submanifold map of every level, 2 = the 2x2x2 stride-2 map from every level to the next, 4 = their transposes; they are
+ * numbered in this order, levels ascending.  Same canonical form as the builders above, bit for bit.
+ *
+ * pyramid_plan fills kpos (int32 [maps][28], 9 or 28 entries used), out_coords[l - 1] (device int32 [n, 3], the first
+ * voxels-of-level-l rows) and, after waiting for the stream, sizes_host[1 + levels + maps]: a flag, the voxels of every
+ * level, the pairs of every map.  flag != 0: the cloud does not suit this builder (a box of too many cells for the
+ * workspace, a voxel met twice, a coordinate outside [-2^20, 2^20)); the results are then undefined and the builders
+ * above are the way to go.  pyramid_emit, with the same arguments and the untouched workspace, writes the maps into
+ * buffers of those sizes (host arrays of device pointers, one per map). */
+size_t fgms_b200_pyramid_workspace_bytes(int n, int levels, int what);
+int fgms_b200_pyramid_plan(const int32_t* coords, int n, int levels, int what, int32_t* kpos, int32_t* const* out_coords,
+                           void* workspace, size_t workspace_bytes, int32_t* sizes_host, void* stream);
+int fgms_b200_pyramid_emit(const int32_t* coords, int n, int levels, int what, int32_t* kpos, int32_t* const* out_coords,
+                           int32_t* const* in_maps, int32_t* const* out_maps, void* workspace, size_t workspace_bytes, void* stream);
+
 /* ---------------------------------------------------------------------------------------------
  * Output-stationary forward.  The reference's forward (backend/spconv.cu:23-246, epilogue
  * backend/fwd_kernels.cuh:130-141) and fgms_b200_fusion_fwd add every pair's product to its output row with an
