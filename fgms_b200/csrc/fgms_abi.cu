@@ -15,6 +15,7 @@
 
 #include "common.cuh"
 #include "simt_kernels.cuh"
+#include "ffma_rows.cuh"
 #include "map_builder.cuh"
 #include "map_pyramid.cuh"
 #include "rows_gms.cuh"
@@ -151,6 +152,9 @@ int run_gms(bool trans, const void* src, const void* kernel, void* dst, const in
   }
   if (dtype == FGMS_DTYPE_F16)
     return trans ? launch_simt_gms<__half, true>(p, st, di.sms) : launch_simt_gms<__half, false>(p, st, di.sms);
+  const int rc = fgms::launch_ffma_gms(p, trans, st, di.sms);
+  if (rc == 0) return check_launch("ffma_gms_kernel");
+  if (rc < 0) return fail(FGMS_ERR_CUDA, "ffma_gms_kernel setup failed (%d)", rc);
   return trans ? launch_simt_gms<float, true>(p, st, di.sms) : launch_simt_gms<float, false>(p, st, di.sms);
 }
 
@@ -348,17 +352,15 @@ int fgms_b200_wgrad(const void* in_feats, const void* out_grad, void* kernel_gra
     }
   }
   if (!launched) {
-    const size_t dyn = (size_t)(2 * k_vol + 3) * sizeof(int);
-    const int grid = simt_grid(map_len, 0, k_vol, fgms::SIMT_WG_TILE, di.sms);
-    const bool small = c_in <= 16 && c_out <= 16;
     if (dtype == FGMS_DTYPE_F16) {
-      if (small) fgms::simt_wgrad_kernel<__half, 1><<<grid, fgms::SIMT_THREADS, dyn, st>>>(p);
+      const size_t dyn = (size_t)(2 * k_vol + 3) * sizeof(int);
+      const int grid = simt_grid(map_len, 0, k_vol, fgms::SIMT_WG_TILE, di.sms);
+      if (c_in <= 16 && c_out <= 16) fgms::simt_wgrad_kernel<__half, 1><<<grid, fgms::SIMT_THREADS, dyn, st>>>(p);
       else fgms::simt_wgrad_kernel<__half, 4><<<grid, fgms::SIMT_THREADS, dyn, st>>>(p);
-    } else {
-      if (small) fgms::simt_wgrad_kernel<float, 1><<<grid, fgms::SIMT_THREADS, dyn, st>>>(p);
-      else fgms::simt_wgrad_kernel<float, 4><<<grid, fgms::SIMT_THREADS, dyn, st>>>(p);
+    } else if (fgms::launch_ffma_wgrad(p, st, di.sms) != 0) {
+      return fail(FGMS_ERR_CUDA, "ffma_wgrad_kernel setup failed");
     }
-    if (int rc = check_launch("simt_wgrad_kernel")) return rc;
+    if (int rc = check_launch("CUDA-core weight-gradient kernel")) return rc;
   }
   if (dtype == FGMS_DTYPE_F16 && accumulate_into_kernel_grad && !direct_f16)
     return fgms_b200_wgrad_finalize(kernel_grad, workspace, (int64_t)count, stream);
