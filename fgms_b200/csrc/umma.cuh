@@ -5,6 +5,7 @@
 // reports it instead of spinning forever.
 #pragma once
 #include <atomic>
+#include <mutex>
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -221,12 +222,18 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, siz
   return cudaLaunchKernelEx(&lc, kernel, static_cast<KArgs>(args)...);
 }
 
-// cudaFuncSetAttribute is needed once per kernel and device; `granted` remembers it (any thread may call)
+// The dynamic shared memory a kernel may be launched with, raised when a launch needs more than any before it on its
+// device; `granted` remembers it (any thread may call).  Looking, setting and writing down are one step: of two threads
+// that ask for different sizes the smaller would otherwise be set last and the larger written down, and every later
+// launch of the larger size would fail.
 template <typename K>
 inline int ensure_smem(K kernel, int bytes, std::atomic<int>* granted /* [64], by device */) {
+  static std::mutex raising;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
   if (granted[dev].load(std::memory_order_acquire) >= bytes) return 0;
+  std::lock_guard<std::mutex> lock(raising);
+  if (granted[dev].load(std::memory_order_relaxed) >= bytes) return 0;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return -1;
   granted[dev].store(bytes, std::memory_order_release);
   return 0;
