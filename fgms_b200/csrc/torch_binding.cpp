@@ -162,16 +162,18 @@ struct SparseConv : torch::autograd::Function<SparseConv> {
     const bool arch80 = ctx->saved_data["arch80"].toBool();
     const Tensor grad_out = grads[0].contiguous();
     const bool need_in = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
+    // saved tensors come back through whatever hooks were installed when they were saved: as good as new arguments
+    const int k_vol = check_common(feats, weight, kpos, imap, omap);
+    check_feat("out_feats_grad", grad_out, 2, feats);
+    TORCH_CHECK_VALUE(feats.size(1) == weight.size(1), "Input feature size and kernel size mismatch");
+    TORCH_CHECK_VALUE(grad_out.size(1) == weight.size(2), "out_feats_grad width differs from the kernel's output channels");
     c10::cuda::CUDAGuard guard(feats.device());
     void* st = stream_of(feats);
     Tensor in_grad, w_grad;
     if (need_in) in_grad = at::empty_like(feats);
     if (need_w) w_grad = at::empty_like(weight);
-    check_feat("out_feats_grad", grad_out, 2, feats);
-    TORCH_CHECK_VALUE(grad_out.size(1) == weight.size(2), "out_feats_grad width differs from the kernel's output channels");
     const Arith a = arith(feats, arch80);
-    const int n_in = (int)feats.size(0), n_out = (int)grad_out.size(0), c_in = (int)weight.size(1), c_out = (int)weight.size(2),
-              k_vol = (int)weight.size(0);
+    const int n_in = (int)feats.size(0), n_out = (int)grad_out.size(0), c_in = (int)weight.size(1), c_out = (int)weight.size(2);
     check_status(fgms_b200_zero2(need_in ? ptr(in_grad) : nullptr, need_in ? bytes_of(in_grad) : 0, need_w ? ptr(w_grad) : nullptr,
                                  need_w ? bytes_of(w_grad) : 0, st));
     if (need_in)
