@@ -15,6 +15,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 #include <pybind11/pybind11.h>
 
 #include "../../include/fgms_b200.h"
@@ -136,11 +137,26 @@ void bwd(const Tensor& grad_out, const Tensor& in_feats, const Tensor& kernel, i
 // ---------------------------------------------------------------------------------------------
 // autograd
 // ---------------------------------------------------------------------------------------------
+// backend.WGRAD_FP32_SUMS as it is now.  A backward follows the switch of its own time, not of the forward's; it runs on a
+// thread of the autograd engine, without the GIL.
+bool fp32_sums_wanted() {
+  pybind11::gil_scoped_acquire gil;
+  THPObjectPtr backend(PyImport_ImportModule("fgms_b200.backend"));
+  THPObjectPtr value(backend ? PyObject_GetAttrString(backend, "WGRAD_FP32_SUMS") : nullptr);
+  const int v = value ? PyObject_IsTrue(value) : -1;
+  if (v < 0) {
+    python_error error;
+    error.persist();
+    throw std::move(error);
+  }
+  return v != 0;
+}
+
 size_t bytes_of(const Tensor& t) { return (size_t)t.numel() * t.element_size(); }
 
 struct SparseConv : torch::autograd::Function<SparseConv> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& feats_, const Tensor& weight_, const Tensor& kpos,
-                        const Tensor& imap, const Tensor& omap, int64_t n_out, bool arch80, bool fp32_sums) {
+                        const Tensor& imap, const Tensor& omap, int64_t n_out, bool arch80) {
     const Tensor feats = feats_.contiguous(), weight = weight_.contiguous();
     TORCH_CHECK_VALUE(feats.is_cuda(), "in_feats must be a CUDA tensor");
     TORCH_CHECK_VALUE(weight.dim() == 3, "kernel must have 3 dimensions, got ", weight.dim());
@@ -150,7 +166,6 @@ struct SparseConv : torch::autograd::Function<SparseConv> {
     fusion_fwd(feats, weight, 0, out, kpos, nullptr, imap, omap, false, arch80);
     ctx->save_for_backward({feats, weight, kpos, imap, omap});
     ctx->saved_data["arch80"] = arch80;
-    ctx->saved_data["fp32_sums"] = fp32_sums;
     return out;
   }
 
@@ -180,12 +195,12 @@ struct SparseConv : torch::autograd::Function<SparseConv> {
       check_status(fgms_b200_dgrad(ptr(grad_out), ptr(weight), ptr(in_grad), iptr(kpos), iptr(imap), iptr(omap), imap.numel(), n_in,
                                    n_out, c_in, c_out, k_vol, a.dtype, a.math, st));
     if (need_w) {
-      const Tensor ws = wgrad_workspace(w_grad, a, ctx->saved_data["fp32_sums"].toBool());
+      const Tensor ws = wgrad_workspace(w_grad, a, a.dtype == FGMS_DTYPE_F16 && fp32_sums_wanted());
       check_status(fgms_b200_wgrad(ptr(feats), ptr(grad_out), ptr(w_grad), iptr(kpos), iptr(imap), iptr(omap), imap.numel(), n_in,
                                    n_out, c_in, c_out, k_vol, a.dtype, a.math, ws.defined() ? ws.data_ptr() : nullptr,
                                    ws.defined() ? (size_t)ws.numel() * 4 : 0, 1, st));
     }
-    return {in_grad, w_grad, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    return {in_grad, w_grad, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 
@@ -334,10 +349,10 @@ PyObject* py_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 PyObject* py_sparse_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  expect(n, 8);
+  expect(n, 7);
   const Tensor &feats = feat_arg(a[0], "in_feats"), &weight = feat_arg(a[1], "kernel");
   const Tensor &kpos = index_arg(a[2], "kpos"), &imap = index_arg(a[3], "in_map"), &omap = index_arg(a[4], "out_map");
-  return THPVariable_Wrap(SparseConv::apply(feats, weight, kpos, imap, omap, int_arg(a[5]), bool_arg(a[6]), bool_arg(a[7])));
+  return THPVariable_Wrap(SparseConv::apply(feats, weight, kpos, imap, omap, int_arg(a[5]), bool_arg(a[6])));
   END_HANDLE_TH_ERRORS
 }
 PyObject* py_fwd_os(PyObject*, PyObject* const* a, Py_ssize_t n) {

@@ -25,8 +25,7 @@ def sparse_conv(feats: torch.Tensor, weight: torch.Tensor, kmap, arch80: bool = 
         raise ValueError(f"feats has {feats.size(0)} rows, the kernel map expects {kmap.n_in}")
     if weight.size(0) != kmap.kpos.numel() - 1:
         raise ValueError("weight and kernel map disagree on the number of offsets")
-    return _native.sparse_conv(feats, weight, kmap.kpos, kmap.imap, kmap.omap, kmap.n_out, arch80,
-                               backend.WGRAD_FP32_SUMS)
+    return _native.sparse_conv(feats, weight, kmap.kpos, kmap.imap, kmap.omap, kmap.n_out, arch80)
 
 
 def sparse_conv_inference(feats: torch.Tensor, weight: torch.Tensor, kmap, bias: torch.Tensor | None = None,
