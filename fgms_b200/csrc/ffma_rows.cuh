@@ -136,14 +136,16 @@ __global__ void __launch_bounds__(FF_THREADS, ff_gms_blocks(PT)) ffma_gms_kernel
       const int n0 = block * 4 * cg;
       // map entries of tile lt, two per lane; looked at only when its rows are fetched, a tile later
       int eg[2], es[2];
+      auto has_pair = [&](int lt, int i) {
+        return lt < lt1 && i < tile_pairs && (uint32_t)lt * (uint32_t)tile_pairs + (uint32_t)i < (uint32_t)j_count;
+      };
       auto load_rows = [&](int lt) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int i = lane + 32 * h;
-          const uint32_t in_seg = (uint32_t)lt * (uint32_t)tile_pairs + (uint32_t)i;
           eg[h] = es[h] = -1;
-          if (lt < lt1 && i < tile_pairs && in_seg < (uint32_t)j_count) {
-            const int j = j_base + (int)in_seg;
+          if (has_pair(lt, i)) {
+            const int j = j_base + lt * tile_pairs + i;
             eg[h] = dense ? j : __ldg(p.gather_map + j);
             es[h] = dense ? j : __ldg(p.scatter_map + j);
           }
@@ -153,7 +155,7 @@ __global__ void __launch_bounds__(FF_THREADS, ff_gms_blocks(PT)) ffma_gms_kernel
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           if ((unsigned)eg[h] >= (unsigned)p.n_gather || (unsigned)es[h] >= (unsigned)p.n_scatter) {
-            if (block == 0 && (eg[h] != -1 || es[h] != -1)) report_problem();  // pair skipped, counted once
+            if (block == 0 && has_pair(lt, lane + 32 * h)) report_problem();  // pair skipped, counted once
             eg[h] = es[h] = -1;
           }
           rows_g[lane + 32 * h] = eg[h];
@@ -284,11 +286,13 @@ __global__ void __launch_bounds__(FF_THREADS, FF_WGRAD_BLOCKS) ffma_wgrad_kernel
         const int cols_a = min(bm, p.c_in - m0), cols_g = min(bn, p.c_out - n0);
         const Walk walk_a(tid, FF_THREADS, vec_a ? cols_a / 4 : cols_a), walk_g(tid, FF_THREADS, vec_g ? cols_g / 4 : cols_g);
         int ei = -1, eo = -1;
+        auto has_pair = [&](int chunk) {
+          return tid < FW_PAIRS && chunk < chunks && (uint32_t)chunk * FW_PAIRS + (uint32_t)tid < (uint32_t)j_count;
+        };
         auto load_rows = [&](int chunk) {
-          const uint32_t in_run = (uint32_t)chunk * FW_PAIRS + (uint32_t)tid;
           ei = eo = -1;
-          if (tid < FW_PAIRS && chunk < chunks && in_run < (uint32_t)j_count) {
-            const int j = j0 + (int)in_run;
+          if (has_pair(chunk)) {
+            const int j = j0 + chunk * FW_PAIRS + tid;
             ei = __ldg(p.in_map + j);
             eo = __ldg(p.out_map + j);
           }
@@ -296,7 +300,7 @@ __global__ void __launch_bounds__(FF_THREADS, FF_WGRAD_BLOCKS) ffma_wgrad_kernel
         auto store_rows = [&](int chunk) {
           if (tid < FW_PAIRS) {
             if ((unsigned)ei >= (unsigned)p.n_in || (unsigned)eo >= (unsigned)p.n_out) {
-              if (m0 == 0 && n0 == 0 && (ei != -1 || eo != -1)) report_problem();  // counted once per skipped pair
+              if (m0 == 0 && n0 == 0 && has_pair(chunk)) report_problem();  // counted once per skipped pair
               ei = eo = -1;
             }
             rows[(chunk & 1) * 2 * FW_PAIRS + tid] = ei;
