@@ -12,9 +12,12 @@
 // memory and was bound by the copy instructions (334 us on 9.1 M pairs of 32 -> 32 fp16, where two gathers of the same
 // rows alone take about 110 us).
 //
-// One block per SM takes a contiguous share of the pairs, its warps take the share's tiles in turn, and the block adds
-// up its warps' fp32 sums when the offset changes: as many partial sums reach the gradient as in the tcgen05 form, so
-// the rounding of an fp16 gradient is the same.
+// One block per SM takes a share of the pairs, its warps take the share's tiles of 16 in turn, and the block adds up its
+// warps' fp32 sums when the offset changes.  Where those sums go straight into an fp16 gradient every block's is rounded,
+// and the pairs are shared out in units of 256 of one offset, the stages of the tcgen05 form, so that an offset of up to
+// 256 pairs is rounded once.  Shares cut by single tiles split such an offset among up to six blocks: relative error of
+// the gradient (32 -> 32, 27 offsets) 4.3e-4 against 2.1e-4 now for 80 pairs each, 4.7e-4 against 3.6e-4 for 1300,
+// 4.7e-4 both for 35 000; the block's warps share a unit's tiles, so that costs little: 3.0 against 3.4 us, 5.4 / 4.7, 19.4 / 19.6.
 #pragma once
 #include "common.cuh"
 #include "rows_gms.cuh"  // rw_mma
@@ -46,8 +49,11 @@ struct WgRow {
   }
 };
 
+constexpr int WG_F16_UNIT = 4;  // log2 of a unit's tiles where block sums are rounded to fp16; single tiles elsewhere
+
 template <bool TF32, int MU, int NU, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 1) rows_wgrad_kernel(WgradParams p, bool spread) {
+  static_assert(WARPS <= 1 << WG_F16_UNIT, "a full unit has a tile for every warp");
   using A = WgRow<TF32, MU>;
   using B = WgRow<TF32, NU>;
   constexpr int NT = 2 * NU, SUMS = MU * 4 * NT;  // n-tiles of 8 columns; accumulators per lane
@@ -59,8 +65,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1) rows_wgrad_kernel(WgradParams p
 
   umma::griddep_wait();
   umma::griddep_launch_dependents();
-  build_tile_table(16, p.kpos, p.pairs, p.k_vol, 0, kpos_s, tile_start);
-  // Tiles by turns; spread (see Turns) when the rows exceed what L2 holds: with consecutive parts 61 MB of rows on either
+  const int unit = !TF32 && p.dw_f16 != nullptr ? WG_F16_UNIT : 0;
+  build_tile_table(16 << unit, p.kpos, p.pairs, p.k_vol, 0, kpos_s, tile_start);
+  // Units by turns; spread (see Turns) when the rows exceed what L2 holds: with consecutive parts 61 MB of rows on either
   // side were read 5.6 times over (683 MB).
   const int total = tile_start[n_seg], share = (total + gridDim.x - 1) / gridDim.x;
   int t0 = min(total, (int)blockIdx.x * share);
@@ -69,12 +76,14 @@ __global__ void __launch_bounds__(WARPS * 32, 1) rows_wgrad_kernel(WgradParams p
   const uint8_t* og = static_cast<const uint8_t*>(p.out_grad);
 
   while (t0 < t1) {
-    // this block's turns inside one offset; warp w takes turns w, w + WARPS, ...
+    // this block's turns inside one offset; warp w takes tiles w, w + WARPS, ... of their units
     const int seg = find_segment(tile_start, n_seg, t0);
-    const int run = min(t1, tile_start[seg + 1]) - t0;
+    const int units = min(t1, tile_start[seg + 1]) - t0;
     const Turns turns(tile_start[seg], tile_start[seg + 1], share, (int)blockIdx.x, t0, spread);
     const int j_begin = kpos_s[seg], j_end = kpos_s[seg + 1];
-    t0 += run;
+    // a single unit may be the offset's last, partly filled one; of several at least one is full
+    const int run = units > 1 ? units << unit : min(1 << unit, (j_end - j_begin + 15) / 16 - (turns.tile(0) << unit));
+    t0 += units;
     float acc[MU][NT][4];
 #pragma unroll
     for (int u = 0; u < MU; ++u)
@@ -87,7 +96,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) rows_wgrad_kernel(WgradParams p
     // read the same words: four broadcast loads, where handing the entries round by shuffles was 15 % slower.
     struct Entries { int i[4], o[4]; };
     auto load_entries = [&](int n, Entries& e) {
-      const int j = (n < run ? j_begin + 16 * turns.tile(n) : j_end) + t4;
+      const int j = (n < run ? j_begin + 16 * ((turns.tile(n >> unit) << unit) + (n & ((1 << unit) - 1))) : j_end) + t4;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         e.i[q] = e.o[q] = -1;
@@ -165,11 +174,11 @@ __global__ void __launch_bounds__(WARPS * 32, 1) rows_wgrad_kernel(WgradParams p
 #pragma unroll
           for (int j = 0; j < NT; ++j) mine[((u * 4 + e) * NT + j) * 32] = acc[u][j][e];
     }
+    const int used = min(run, WARPS);
     __syncthreads();
     // element e = 2 h + c of n-tile j = 2 v + w: gradient row channel(u, g) + h, column channel(v, 2 t + c) + w.  The two
     // units of an even pair hold four consecutive columns, an odd last unit two: one vector red each.
     constexpr int GROUPS = (NU + 1) / 2;
-    const int used = min(run, WARPS);
     for (int item = threadIdx.x; item < MU * 4 * GROUPS * 32; item += WARPS * 32) {
       const int grp = (item >> 5) % GROUPS, ue = (item >> 5) / GROUPS, u = ue >> 2, e = ue & 3;
       const float* from = wg_smem + (ue * NT + grp * 4) * 32 + lane;
@@ -220,9 +229,9 @@ inline int rw_wgrad_launch_as(const WgradParams& p, cudaStream_t st, int sms, in
     if (smem > (size_t)max_smem) return 1;
     static std::atomic<int> granted[64];
     if (int rc = ensure_smem(kernel, max_smem, granted)) return rc;
-    const long long tiles = (long long)p.pairs / 16 + p.k_vol + 1;
+    const long long units = (long long)p.pairs / (p.dw_f16 != nullptr ? 16 << WG_F16_UNIT : 16) + p.k_vol + 1;
     const bool spread = spread_tiles((size_t)p.n_in * MU * 16 * (TF32 ? 4 : 2) + (size_t)p.n_out * NU * 16 * (TF32 ? 4 : 2));
-    return launch_pdl(kernel, (int)(tiles < sms ? tiles : sms), WARPS * 32, smem, st, p, spread) == cudaSuccess ? 0 : -1;
+    return launch_pdl(kernel, (int)(units < sms ? units : sms), WARPS * 32, smem, st, p, spread) == cudaSuccess ? 0 : -1;
   }
 }
 template <bool TF32, int MU>
