@@ -22,6 +22,9 @@ Differences from the reference, all deliberate:
 """
 from __future__ import annotations
 
+import sys
+import types
+
 import torch
 
 from . import _lib, _native
@@ -147,7 +150,7 @@ def fgms_bwd_cuda(out_feats_grad, in_feats, kernel, sum_nnz, in_feats_grad, kern
     """Backward — ``ConvolutionBackward`` (``backend/spconv.cu:414-571``): accumulates the input
     gradient into ``in_feats_grad`` and the weight gradient into ``kernel_grad``."""
     _native.bwd(out_feats_grad, in_feats, kernel, sum_nnz, in_feats_grad, kernel_grad, kpos, qkpos, in_map, out_map, separate_mid,
-                arch80, WGRAD_FP32_SUMS)
+                arch80, _native.wgrad_fp32_sums())
 
 
 def fgms_dgrad_cuda(out_feats_grad, kernel, in_feats_grad, kpos, in_map, out_map, arch80):
@@ -162,14 +165,28 @@ def fgms_dgrad_cuda(out_feats_grad, kernel, in_feats_grad, kpos, in_map, out_map
             dtype, math, _stream()))
 
 
-# fp16 weight gradients: False = single launch, every CTA adds its fp32 partial sums (rounded to fp16) into
-# ``kernel_grad`` with fp16 atomics; True = fp32 sums in a workspace, added to ``kernel_grad`` once at the
-# end (three launches).  ``fgms_bwd_cuda`` keeps the reference's signature and follows this switch.
-WGRAD_FP32_SUMS = False
+class _Module(types.ModuleType):
+    """This module, with ``WGRAD_FP32_SUMS`` kept where a backward pass on a thread of the autograd engine sees it.
+
+    fp16 weight gradients: False (the default) = single launch, every CTA adds its fp32 partial sums (rounded to fp16)
+    into ``kernel_grad`` with fp16 atomics; True = fp32 sums in a workspace, added to ``kernel_grad`` once at the end
+    (three launches).  ``fgms_bwd_cuda`` keeps the reference's signature and follows this switch, as does the backward
+    pass of ``nn.sparse_conv``."""
+
+    @property
+    def WGRAD_FP32_SUMS(self) -> bool:
+        return _native.wgrad_fp32_sums()
+
+    @WGRAD_FP32_SUMS.setter
+    def WGRAD_FP32_SUMS(self, on) -> None:
+        _native.wgrad_fp32_sums(on)
+
+
+sys.modules[__name__].__class__ = _Module
 
 
 def _single_launch_wgrad(c_in, c_out, k_vol, dtype, arch80, fp32_sums) -> bool:
-    want_fp32 = WGRAD_FP32_SUMS if fp32_sums is None else fp32_sums
+    want_fp32 = _native.wgrad_fp32_sums() if fp32_sums is None else fp32_sums
     return dtype == torch.float16 and not want_fp32 and kernel_family("wgrad", c_in, c_out, dtype, arch80, k_vol) == "tcgen05"
 
 

@@ -7,6 +7,7 @@
 // about a hundred thousand voxels.  Error types are those of the reference's binding: ValueError for what pybind11
 // maps from std::invalid_argument, TypeError for an argument that is no tensor, RuntimeError for a CUDA failure.
 #include <array>
+#include <atomic>
 #include <vector>
 
 #include <ATen/ATen.h>
@@ -15,7 +16,6 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
-#include <torch/csrc/utils/object_ptr.h>
 #include <pybind11/pybind11.h>
 
 #include "../../include/fgms_b200.h"
@@ -137,20 +137,9 @@ void bwd(const Tensor& grad_out, const Tensor& in_feats, const Tensor& kernel, i
 // ---------------------------------------------------------------------------------------------
 // autograd
 // ---------------------------------------------------------------------------------------------
-// backend.WGRAD_FP32_SUMS as it is now.  A backward follows the switch of its own time, not of the forward's; it runs on a
-// thread of the autograd engine, without the GIL.
-bool fp32_sums_wanted() {
-  pybind11::gil_scoped_acquire gil;
-  THPObjectPtr backend(PyImport_ImportModule("fgms_b200.backend"));
-  THPObjectPtr value(backend ? PyObject_GetAttrString(backend, "WGRAD_FP32_SUMS") : nullptr);
-  const int v = value ? PyObject_IsTrue(value) : -1;
-  if (v < 0) {
-    python_error error;
-    error.persist();
-    throw std::move(error);
-  }
-  return v != 0;
-}
+// backend.WGRAD_FP32_SUMS.  A backward follows the switch of its own time, not of the forward's; it runs on a thread of the
+// autograd engine without the GIL, so the switch is kept here and the module's attribute reads and sets it.
+std::atomic<bool> g_fp32_sums{false};
 
 size_t bytes_of(const Tensor& t) { return (size_t)t.numel() * t.element_size(); }
 
@@ -195,7 +184,7 @@ struct SparseConv : torch::autograd::Function<SparseConv> {
       check_status(fgms_b200_dgrad(ptr(grad_out), ptr(weight), ptr(in_grad), iptr(kpos), iptr(imap), iptr(omap), imap.numel(), n_in,
                                    n_out, c_in, c_out, k_vol, a.dtype, a.math, st));
     if (need_w) {
-      const Tensor ws = wgrad_workspace(w_grad, a, a.dtype == FGMS_DTYPE_F16 && fp32_sums_wanted());
+      const Tensor ws = wgrad_workspace(w_grad, a, g_fp32_sums.load(std::memory_order_relaxed));
       check_status(fgms_b200_wgrad(ptr(feats), ptr(grad_out), ptr(w_grad), iptr(kpos), iptr(imap), iptr(omap), imap.numel(), n_in,
                                    n_out, c_in, c_out, k_vol, a.dtype, a.math, ws.defined() ? ws.data_ptr() : nullptr,
                                    ws.defined() ? (size_t)ws.numel() * 4 : 0, 1, st));
@@ -355,6 +344,13 @@ PyObject* py_sparse_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return THPVariable_Wrap(SparseConv::apply(feats, weight, kpos, imap, omap, int_arg(a[5]), bool_arg(a[6])));
   END_HANDLE_TH_ERRORS
 }
+PyObject* py_wgrad_fp32_sums(PyObject*, PyObject* const* a, Py_ssize_t n) {  // () -> the switch; (value) sets it
+  HANDLE_TH_ERRORS
+  TORCH_CHECK_TYPE(n <= 1, "expected at most 1 argument, got ", n);
+  if (n == 1) g_fp32_sums.store(bool_arg(a[0]), std::memory_order_relaxed);
+  return PyBool_FromLong(g_fp32_sums.load(std::memory_order_relaxed));
+  END_HANDLE_TH_ERRORS
+}
 PyObject* py_fwd_os(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   expect(n, 8);
@@ -387,6 +383,7 @@ PyObject* py_build_pyramid(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyMethodDef methods[] = {
     FGMS_METHOD("fusion_fwd", py_fusion_fwd), FGMS_METHOD("seq_fwd", py_seq_fwd),         FGMS_METHOD("bwd", py_bwd),
     FGMS_METHOD("fwd_os", py_fwd_os),         FGMS_METHOD("sparse_conv", py_sparse_conv),
+    FGMS_METHOD("wgrad_fp32_sums", py_wgrad_fp32_sums),
     FGMS_METHOD("build_pyramid", py_build_pyramid), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
