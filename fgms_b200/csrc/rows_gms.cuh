@@ -29,6 +29,18 @@ namespace fgms {
 constexpr int RW_WARPS = 4;
 constexpr int RW_THREADS = RW_WARPS * 32;
 
+// The kernels of a backward leave every SM room for one block of the exchange kernel (peer_exchange.cuh: 128 threads of 32
+// registers, a little shared memory), which is meant to run beside them: registers per thread of `threads` resident ones,
+// and the percentage of the SM's shared memory that is not cache.  With all registers taken (128 per thread at 32 -> 32) or
+// with the 8 KB of shared memory the driver chooses by itself, the exchange waits for the input gradient to end (8.1 M
+// pairs: 285 us); with both it is done after 90 us, and the input gradient takes the same 136 us (64 -> 64: 282).  From 20 %
+// on the smaller cache shows: 64 -> 64 303 us.
+constexpr int rw_max_regs(int threads, bool backward) {
+  const int regs = (backward ? 65536 - 4096 : 65536) / threads / 8 * 8;
+  return regs < 248 ? regs : 248;
+}
+constexpr int RW_SMEM_PERCENT = 8;
+
 __device__ __forceinline__ void rw_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, bool tf32) {
   if (tf32)
     asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -129,7 +141,7 @@ __device__ __forceinline__ void rw_load_b(const uint8_t* w, int c_out, int lane,
 
 // MT: m-tiles of 16 pairs a warp works on at a time.
 template <bool TF32, bool TRANS, int KU, int NU, int MT, int MIN_BLOCKS>
-__global__ void __launch_bounds__(RW_THREADS, MIN_BLOCKS) rows_gms_kernel(GmsParams p, bool spread) {
+__global__ void __maxnreg__(rw_max_regs(RW_THREADS * MIN_BLOCKS, TRANS)) rows_gms_kernel(GmsParams p, bool spread) {
   using S = RowShape<TF32, KU, NU>;
   constexpr int TILE = 16 * MT;
   constexpr uint32_t K_BYTES = KU * 16 * S::ES, N_BYTES = NU * 16 * S::ES;
@@ -288,6 +300,7 @@ inline int rw_launch_as(const GmsParams& p, cudaStream_t st, int sms) {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
   int occ = resident[dev].load(std::memory_order_acquire);
   if (occ == 0) {
+    if (TRANS && cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, RW_SMEM_PERCENT) != cudaSuccess) return -1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, RW_THREADS, 0) != cudaSuccess || occ < 1) return -1;
     resident[dev].store(occ, std::memory_order_release);
   }

@@ -20,7 +20,7 @@
 // 4.7e-4 both for 35 000; the block's warps share a unit's tiles, so that costs little: 3.0 against 3.4 us, 5.4 / 4.7, 19.4 / 19.6.
 #pragma once
 #include "common.cuh"
-#include "rows_gms.cuh"  // rw_mma
+#include "rows_gms.cuh"  // rw_mma, rw_max_regs
 #include "umma.cuh"
 
 namespace fgms {
@@ -52,7 +52,7 @@ struct WgRow {
 constexpr int WG_F16_UNIT = 4;  // log2 of a unit's tiles where block sums are rounded to fp16; single tiles elsewhere
 
 template <bool TF32, int MU, int NU, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, 1) rows_wgrad_kernel(WgradParams p, bool spread) {
+__global__ void __maxnreg__(rw_max_regs(WARPS * 32, true)) rows_wgrad_kernel(WgradParams p, bool spread) {
   static_assert(WARPS <= 1 << WG_F16_UNIT, "a full unit has a tile for every warp");
   using A = WgRow<TF32, MU>;
   using B = WgRow<TF32, NU>;

@@ -1,0 +1,63 @@
+"""What runs beside the short-row kernels: the exchange of the ranks' sums beside the backward it is meant to hide
+behind."""
+import pytest
+import torch
+
+from fgms_b200 import backend
+from fgms_b200.dist import PeerExchange
+
+pytestmark = pytest.mark.gpu
+
+
+class _Layer:
+    """A layer whose passes take some hundred microseconds: 27 offsets of 300 k pairs each, of more where rows are short."""
+
+    def __init__(self, c_in, c_out, dtype):
+        n = max(400_000, 25_600_000 // (c_in + c_out))
+        per = n * 3 // 4
+        gen = torch.Generator(device="cuda").manual_seed(4)
+        rows = lambda c: torch.randn((n, c), generator=gen, device="cuda").to(dtype)
+        self.feats, self.grad_out, self.in_grad = rows(c_in), rows(c_out), torch.zeros((n, c_in), dtype=dtype, device="cuda")
+        self.weight = torch.randn((27, c_in, c_out), generator=gen, device="cuda").to(dtype) * 0.05
+        pick = lambda: torch.randperm(n, generator=gen, device="cuda")[:per].sort().values.int()
+        self.imap = torch.cat([pick() for _ in range(27)])
+        self.omap = torch.cat([pick() for _ in range(27)])
+        self.kpos = torch.arange(28, device="cuda", dtype=torch.int32) * per
+
+    def wgrad(self):
+        backend.fgms_wgrad_cuda(self.feats, self.grad_out, torch.zeros_like(self.weight), self.kpos, self.imap, self.omap, True)
+
+    def dgrad(self):
+        backend.fgms_dgrad_cuda(self.grad_out, self.weight, self.in_grad, self.kpos, self.imap, self.omap, True)
+
+
+def _side_and_main_ms(call, side, beside):
+    """Times from the start of ``call()`` to the end of ``beside()`` on ``side`` and of the call itself."""
+    main = torch.cuda.current_stream()
+    start, end_side, end_main = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+    torch.cuda.synchronize()
+    start.record()
+    side.wait_event(start)
+    call()
+    with torch.cuda.stream(side):
+        # the call fills the chip before the other kernel is let go
+        torch.cuda._sleep(60_000)
+        beside()
+        end_side.record(side)
+    end_main.record(main)
+    torch.cuda.synchronize()
+    return start.elapsed_time(end_side), start.elapsed_time(end_main)
+
+
+@pytest.mark.parametrize("pass_", ["dgrad", "wgrad"])
+@pytest.mark.parametrize("c_in,c_out,dtype", [(32, 32, torch.float16), (64, 64, torch.float16), (16, 16, torch.float16),
+                                              (32, 32, torch.float32), (48, 16, torch.float16), (64, 32, torch.float32)])
+def test_the_exchange_runs_beside_the_backward(pass_, c_in, c_out, dtype):
+    layer = _Layer(c_in, c_out, dtype)
+    call = getattr(layer, pass_)
+    side = torch.cuda.Stream(priority=-1)
+    px = PeerExchange(27 * c_in * c_out, "cuda")
+    px.run(side)
+    call()
+    best = min((_side_and_main_ms(call, side, lambda: px.run(side)) for _ in range(5)), key=lambda t: t[0] / t[1])
+    assert best[0] < 0.85 * best[1], f"the exchange ended after {best[0]:.3f} ms, the {pass_} after {best[1]:.3f} ms"
