@@ -51,7 +51,8 @@ int check_launch(const char* what) {
 }
 
 struct DeviceInfo {
-  int sms = 0;
+  int sms = 0;       // to launch on
+  int reserved = 0;  // to leave free
   int max_smem_optin = 0;
 };
 
@@ -71,6 +72,7 @@ int device_info(DeviceInfo* out) {
   }
   *out = cached;
   const int keep = g_reserved_sms.load(std::memory_order_relaxed);
+  out->reserved = keep;
   if (keep > 0) out->sms = cached.sms - keep > 1 ? cached.sms - keep : 1;
   return FGMS_OK;
 }
@@ -142,7 +144,9 @@ int run_gms(bool trans, const void* src, const void* kernel, void* dst, const in
   p.c_in = c_in; p.c_out = c_out; p.k_vol = k_vol;
   p.dense_rows = dense_rows; p.dense_weight = dense_weight;
   if (plan_gms(trans, c_in, c_out, k_vol, dtype, math, di.max_smem_optin)) {
-    int rc = fgms::launch_rows_gms(p, trans, dtype == FGMS_DTYPE_F16, st, di.sms);
+    // Several small blocks to an SM are spread over all SMs however few there are, so with SMs to leave free the
+    // short-row kernel stands back for the one with one block per SM.
+    int rc = di.reserved > 0 ? 1 : fgms::launch_rows_gms(p, trans, dtype == FGMS_DTYPE_F16, st, di.sms);
     if (rc == 0) return check_launch("rows_gms_kernel");
     if (rc < 0) return fail(FGMS_ERR_CUDA, "rows_gms_kernel setup failed (%d)", rc);
     rc = fgms::launch_umma_gms3(p, trans, dtype == FGMS_DTYPE_F16, st, di.sms, di.max_smem_optin);

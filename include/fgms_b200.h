@@ -261,11 +261,13 @@ int fgms_b200_peer_exchange(const float* const* sums, float* const* reduced, uin
                             int world, int64_t count, uint32_t epoch, int64_t wait_limit_cycles, int ctas,
                             void* stream);
 
-/* The tensor-core kernels are persistent: one CTA per SM that holds nearly all of the SM's shared memory and
- * registers, so a kernel of another stream does not start on that SM before they finish.  A caller that wants
- * such a kernel to run BESIDE them (fgms_b200_peer_exchange beside the input gradient, a collective) tells the
+/* The tensor-core kernels are persistent and hold nearly all of an SM's shared memory or registers, so a kernel of
+ * another stream does not start on that SM before they finish (fgms_b200_peer_exchange, whose blocks are small enough
+ * for what they leave, does).  A caller that wants such a kernel to run BESIDE them (a collective) tells the
  * library to launch on `n` fewer SMs; the setting is process-wide and applies to the launches that follow
- * (set it around the one call it is meant for).  0 restores the full grid.  No counterpart in the reference,
+ * (set it around the one call it is meant for).  While it is not 0, forward and input gradient of layers of up to 64
+ * channels run on the tcgen05 kernel, which has one CTA per SM, instead of the faster one for short rows.  The
+ * CUDA-core kernels follow the number only roughly.  0 restores the full grid.  No counterpart in the reference,
  * whose grids follow the problem size (backend/spconv.cu:111-245). */
 int fgms_b200_set_reserved_sms(int n);
 

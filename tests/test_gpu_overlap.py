@@ -1,9 +1,9 @@
 """What runs beside the short-row kernels: the exchange of the ranks' sums beside the backward it is meant to hide
-behind."""
+behind, and kernels of other streams on the SMs ``fgms_b200_set_reserved_sms`` keeps free."""
 import pytest
 import torch
 
-from fgms_b200 import backend
+from fgms_b200 import _lib, backend
 from fgms_b200.dist import PeerExchange
 
 pytestmark = pytest.mark.gpu
@@ -61,3 +61,19 @@ def test_the_exchange_runs_beside_the_backward(pass_, c_in, c_out, dtype):
     call()
     best = min((_side_and_main_ms(call, side, lambda: px.run(side)) for _ in range(5)), key=lambda t: t[0] / t[1])
     assert best[0] < 0.85 * best[1], f"the exchange ended after {best[0]:.3f} ms, the {pass_} after {best[1]:.3f} ms"
+
+
+@pytest.mark.parametrize("c_in,c_out", [(32, 32), (64, 64)])
+def test_reserved_sms_are_free_for_another_stream(c_in, c_out):
+    """A kernel whose blocks need most of an SM's registers (softmax over long rows: 1024 threads each) finds room."""
+    layer = _Layer(c_in, c_out, torch.float16)
+    side = torch.cuda.Stream(priority=-1)
+    x = torch.randn((8, 16384), device="cuda")
+    torch.softmax(x, 1)
+    try:
+        assert _lib.lib.fgms_b200_set_reserved_sms(16) == 0
+        layer.dgrad()
+        best = min((_side_and_main_ms(layer.dgrad, side, lambda: torch.softmax(x, 1)) for _ in range(5)), key=lambda t: t[0] / t[1])
+    finally:
+        _lib.lib.fgms_b200_set_reserved_sms(0)
+    assert best[0] < 0.75 * best[1], f"the other kernel ended after {best[0]:.3f} ms, the input gradient after {best[1]:.3f} ms"
