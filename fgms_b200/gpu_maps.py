@@ -64,11 +64,11 @@ def build_pyramid(coords: torch.Tensor, levels: int):
     coords = _check_coords(coords)
     got = _native.build_pyramid(coords, levels + 1, _SUBM | _DOWN | _UP) if levels > 0 else None
     subm, down, up = [], [], []
-    if got is None:  # no such pyramid, or a cloud that does not suit its builder
+    if got is None:  # no such pyramid, or a cloud that does not suit its builder: not asked again for each map
         for r in range(levels + 1):
-            subm.append(build_submanifold_map(coords, 3))
+            subm.append(_hashed_submanifold_map(coords, 3))
             if r < levels:
-                down.append(build_strided_map(coords, 2))
+                down.append(_hashed_strided_map(coords, 2))
                 up.append(transpose_map(down[-1], coords))
                 coords = down[-1].out_coords
         return subm, down, up
@@ -89,6 +89,11 @@ def build_submanifold_map(coords: torch.Tensor, kernel_size: int = 3) -> DeviceK
     if got is not None:
         n = coords.size(0)
         return DeviceKernelMap(n, n, 27, *got[1][0], coords)
+    return _hashed_submanifold_map(coords, kernel_size)
+
+
+def _hashed_submanifold_map(coords: torch.Tensor, kernel_size: int) -> DeviceKernelMap:
+    """The hash-table builder, for what the bitmap builder does not take."""
     n, k_vol, dev = coords.size(0), kernel_size ** 3, coords.device
     kpos = torch.empty(k_vol + 1, dtype=torch.int32, device=dev)
     imap = torch.empty(n * k_vol, dtype=torch.int32, device=dev)
@@ -109,6 +114,10 @@ def build_strided_map(coords: torch.Tensor, stride: int = 2) -> DeviceKernelMap:
     if got is not None:
         (n, n_out), (maps,), (out_coords,) = got
         return DeviceKernelMap(n, n_out, 8, *maps, out_coords)
+    return _hashed_strided_map(coords, stride)
+
+
+def _hashed_strided_map(coords: torch.Tensor, stride: int) -> DeviceKernelMap:
     n, k_vol, dev = coords.size(0), stride ** 3, coords.device
     kpos = torch.empty(k_vol + 1, dtype=torch.int32, device=dev)
     imap = torch.empty(n, dtype=torch.int32, device=dev)
