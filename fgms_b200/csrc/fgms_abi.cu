@@ -583,21 +583,21 @@ int fgms_b200_transpose_map(const int32_t* kpos, const int32_t* in_map, const in
 // Kernel maps of a pyramid of resolutions (csrc/map_pyramid.cuh)
 // ---------------------------------------------------------------------------------------------
 size_t fgms_b200_pyramid_workspace_bytes(int n, int levels, int what) {
-  fgms::pyramid::Plan p;
-  return fgms::pyramid::plan(n, levels, what, &p) ? p.total : 0;
+  return n < 1 ? 0 : fgms::pyramid::bytes_for(n, levels, what, fgms::pyramid::first_words(n));
 }
 
 namespace {
 int pyramid_args(const int32_t* coords, int n, int levels, int what, int32_t* kpos, int32_t* const* out_coords, void* workspace,
                  size_t workspace_bytes, fgms::pyramid::Plan* p, fgms::pyramid::Args* a) {
-  if (!fgms::pyramid::plan(n, levels, what, p))
+  if (fgms_b200_pyramid_workspace_bytes(n, levels, what) == 0)
     return fail(FGMS_ERR_INVALID_ARG, "a pyramid needs n >= 1, 1..%d levels and at least one map", fgms::pyramid::MAX_LEVELS);
   if (!coords || !kpos || (levels > 1 && !out_coords)) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
   for (int l = 1; l < levels; ++l)
     if (!out_coords[l - 1]) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
   if (27ll * n > 0x7fffffffll) return fail(FGMS_ERR_INVALID_ARG, "27 * n exceeds the int32 range of the maps");
-  if (!workspace || workspace_bytes < p->total || (reinterpret_cast<uintptr_t>(workspace) & 255))
-    return fail(FGMS_ERR_WORKSPACE, "the pyramid needs a 256-byte aligned workspace of %zu bytes", p->total);
+  if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) || !fgms::pyramid::plan_in(n, levels, what, workspace_bytes, p))
+    return fail(FGMS_ERR_WORKSPACE, "the pyramid needs a 256-byte aligned workspace of %zu bytes",
+                fgms_b200_pyramid_workspace_bytes(n, levels, what));
   *a = fgms::pyramid::arguments(*p, coords, n, levels, kpos, out_coords, static_cast<uint8_t*>(workspace));
   return FGMS_OK;
 }
@@ -619,6 +619,11 @@ int fgms_b200_pyramid_plan(const int32_t* coords, int n, int levels, int what, i
   if (cudaMemcpyAsync(sizes_host, ws + p.sizes, (size_t)(1 + levels + p.n_jobs) * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
     return cuda_fail("reading the sizes of the maps");
+  if (sizes_host[0] != 0) {
+    const int need = sizes_host[1];
+    const bool roomier = sizes_host[0] == fgms::pyramid::TOO_LARGE && need <= fgms::pyramid::most_words(n);
+    sizes_host[1] = roomier ? (int)((fgms::pyramid::bytes_for(n, levels, what, need) + 255) / 256) : 0;
+  }
   return FGMS_OK;
 }
 

@@ -12,8 +12,8 @@
 // A row's neighbours become one mask of k_vol bits; counting the bits per (offset, block of rows), scanning those counts
 // and writing the pairs needs no dense table.  The host waits once, for the sizes of the maps.
 //
-// The box is limited by the workspace (cells / 8 bytes): a cloud with a larger box, a voxel met twice or a coordinate
-// beyond the packable range is left to map_builder.cuh (the plan says so).
+// The box is limited by the workspace (cells / 8 bytes; the plan says what a larger box needs): a cloud whose box exceeds
+// the builder's own limit, a voxel met twice or a coordinate beyond the packable range is left to map_builder.cuh.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -44,6 +44,7 @@ struct Header {
   unsigned ticket;
   int flags;       // what makes the cloud unfit
   int groups;      // groups of 4 words, all levels
+  int need;        // words the levels' boxes take, 0x7fffffff where it is more
   int first_group[MAX_LEVELS + 1];
   Level level[MAX_LEVELS];
 };
@@ -142,7 +143,7 @@ __global__ void __launch_bounds__(THREADS) box_kernel(Args a) {
   __threadfence();
   volatile Header* hv = h;
   int flags = hv->flags == 0x7f7f7f7f ? 0 : OUT_OF_RANGE;
-  long long word = 0;
+  long long word = 0, need = 0;
   for (int l = 0; l < a.levels; ++l) {
     Level L;
     const int lx = hv->lo[0] >> l, ly = hv->lo[1] >> l, lz = hv->lo[2] >> l;
@@ -151,13 +152,16 @@ __global__ void __launch_bounds__(THREADS) box_kernel(Args a) {
     L.dy = hy - ly + 3;
     L.dzw = (hz - lz + 3 + 31) / 32;
     L.word0 = (int)word;
-    word = (word + (long long)(hx - lx + 3) * L.dy * L.dzw + 3) & ~3ll;
+    const long long words = ((long long)(hx - lx + 3) * L.dy * L.dzw + 3) & ~3ll;
+    need += words;
+    word += words;
     if (flags || word > a.cap_words) { flags |= TOO_LARGE; word = 0; }
     h->level[l] = L;
     h->first_group[l + 1] = (int)(word >> 2);
   }
   h->first_group[0] = 0;
   h->groups = (int)(word >> 2);
+  h->need = (int)min(need, 0x7fffffffll);
   h->flags = flags;
 }
 
@@ -354,7 +358,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) position_kernel(Args a, int* siz
   umma::griddep_wait();
   umma::griddep_launch_dependents();
   const int j = blockIdx.x, flags = a.head->flags;
-  if (j == 0 && threadIdx.x == 0) sizes[0] = flags;
+  if (j == 0 && threadIdx.x == 0) {
+    sizes[0] = flags;
+    if (flags) sizes[1] = a.head->need;
+  }
   if (flags) return;
   __shared__ Jobs s;
   __shared__ int part[SCAN_THREADS / 32];
@@ -504,34 +511,50 @@ struct Plan {
   int n_jobs, cap_words;
   Job job[MAX_JOBS];
 };
-// Cells of all levels' boxes the workspace has room for: 64 MB of bits (a 2000 x 2000 x 80 scan and its coarser levels
-// take 55 MB), more for clouds of more than 200 k voxels, at most 400 MB.
-inline int capacity_words(int n) {
+// Words of bitmaps a cloud may have: 64 MB (a 2000 x 2000 x 80 scan and its coarser levels take 55 MB), more for clouds of
+// more than 200 k voxels, at most 400 MB.
+inline int most_words(int n) {
   const long long want = 80ll * n, least = 16ll << 20, most = 100ll << 20;
   return (int)(want < least ? least : (want > most ? most : want));
 }
-inline bool plan(int n, int levels, int what, Plan* p) {
+// What a first attempt makes room for: all of that from 16 k voxels on, in proportion below (300 voxels: 1.2 MB).
+inline int first_words(int n) { return (int)(1024ll * n < most_words(n) ? 1024ll * n : most_words(n)); }
+// Layout of a workspace with room for `words` words of bitmaps.
+inline bool plan(int n, int levels, int what, int words, Plan* p) {
   if (n < 1 || levels < 1 || levels > MAX_LEVELS || (what & ~(SUBM | DOWN | UP)) || !what) return false;
   p->n_jobs = 0;
   for (int kind : {SUBM, DOWN, UP})
     if (what & kind)
       for (int l = 0; l < levels - (kind == SUBM ? 0 : 1); ++l) p->job[p->n_jobs++] = Job{kind, l, kind == SUBM ? 27 : 8};
   if (p->n_jobs == 0) return false;
-  p->cap_words = capacity_words(n);
+  p->cap_words = words;
   size_t off = maps::align256(sizeof(Header));
   auto take = [&](size_t bytes) { const size_t at = off; off += maps::align256(bytes); return at; };
   p->sizes = take((1 + MAX_LEVELS + MAX_JOBS) * 4);
   p->jobs = take(sizeof(Jobs));
-  p->bits = take(((size_t)p->cap_words + 64) * 4);
-  p->prefix = take(((size_t)p->cap_words / 4 + 1) * 4);
   p->block_sums = take(SCAN_BLOCKS * 4);
   p->row_of = take((size_t)n * 4);
   p->mask = take((size_t)p->n_jobs * n * 4);
   size_t counts = 0;
   for (int j = 0; j < p->n_jobs; ++j) counts += (size_t)p->job[j].k_vol * (((size_t)n + ROWS - 1) / ROWS);
   p->counts = take(counts * 4);
+  p->bits = take(((size_t)words + 64) * 4);
+  p->prefix = take(((size_t)words / 4 + 1) * 4);
   p->total = off;
   return true;
+}
+// The layout of a workspace of `bytes`: as many words as fit (each takes 5 bytes, its share of the prefix included).
+// False if that is less than the first attempt's.
+inline bool plan_in(int n, int levels, int what, size_t bytes, Plan* p) {
+  if (!plan(n, levels, what, 0, p) || bytes < p->total) return false;
+  const size_t room = (bytes - p->total) / 5;
+  const int words = room < (size_t)most_words(n) ? (int)room & ~63 : most_words(n);
+  return words >= (first_words(n) & ~63) && plan(n, levels, what, words, p);
+}
+// Bytes with which plan_in has room for `words` words: 2 x 256 for the alignment of both arrays, 64 words for the rounding.
+inline size_t bytes_for(int n, int levels, int what, int words) {
+  Plan p;
+  return plan(n, levels, what, 0, &p) ? p.total + ((size_t)words + 64) * 5 + 512 : 0;
 }
 inline Args arguments(const Plan& p, const int32_t* coords, int n, int levels, int32_t* kpos, int32_t* const* out_coords, uint8_t* ws) {
   Args a = {};

@@ -225,37 +225,47 @@ struct Pyramid {
   std::vector<Tensor> out_coords;               // level 1 ..
 };
 
-// The maps of `what` (see fgms_b200_pyramid_plan) of the cloud and its coarser levels.  One wait, for the sizes; the
-// Python objects around the maps are made while the last kernel runs.
-Pyramid build_pyramid(const Tensor& coords, int levels, int what) {
+// The maps of `what` (see fgms_b200_pyramid_plan) of the cloud and its coarser levels.  One wait, for the sizes (two if the
+// box turns out larger than the first workspace has room for); the Python objects around the maps are made while the last
+// kernel runs.
+Pyramid try_pyramid(const Tensor& coords, int levels, int what) {
   TORCH_CHECK_VALUE(coords.is_cuda() && coords.scalar_type() == at::kInt && coords.dim() == 2 && coords.size(1) == 3 && coords.is_contiguous(),
                     "coords must be a contiguous CUDA int32 tensor of shape [n, 3]");
   Pyramid r;
   const int64_t n64 = coords.size(0);
   if (n64 < 1 || n64 > 0x7fffffffll / 27) return r;
   const int n = (int)n64;
-  const size_t bytes = fgms_b200_pyramid_workspace_bytes(n, levels, what);
+  size_t bytes = fgms_b200_pyramid_workspace_bytes(n, levels, what);
   if (bytes == 0) return r;
   c10::cuda::CUDAGuard guard(coords.device());
   void* st = stream_of(coords);
   const auto ints = coords.options();
   const int n_maps = ((what & 1) ? levels : 0) + ((what & 2) ? levels - 1 : 0) + ((what & 4) ? levels - 1 : 0);
-  const Tensor ws = at::empty({(int64_t)bytes}, ints.dtype(at::kByte)), kpos = at::empty({n_maps * 28}, ints);
-  std::vector<int32_t*> coord_ptrs;
-  for (int l = 1; l < levels; ++l) {
-    r.out_coords.push_back(at::empty({n64, 3}, ints));
-    coord_ptrs.push_back(r.out_coords.back().data_ptr<int32_t>());
-  }
   const Tensor host = at::empty({64}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
   const int32_t* sizes = host.data_ptr<int32_t>();
-  int rc;
-  {
-    pybind11::gil_scoped_release unlock;  // this waits for the device
-    rc = fgms_b200_pyramid_plan(iptr(coords), n, levels, what, kpos.data_ptr<int32_t>(), coord_ptrs.data(), ws.data_ptr(), bytes,
-                                host.data_ptr<int32_t>(), st);
+  Tensor ws, kpos;
+  std::vector<int32_t*> coord_ptrs;
+  for (int attempt = 0;; ++attempt) {
+    ws = Tensor();  // before the larger one
+    ws = at::empty({(int64_t)bytes}, ints.dtype(at::kByte));
+    if (attempt == 0) {
+      kpos = at::empty({n_maps * 28}, ints);
+      for (int l = 1; l < levels; ++l) {
+        r.out_coords.push_back(at::empty({n64, 3}, ints));
+        coord_ptrs.push_back(r.out_coords.back().data_ptr<int32_t>());
+      }
+    }
+    int rc;
+    {
+      pybind11::gil_scoped_release unlock;  // this waits for the device
+      rc = fgms_b200_pyramid_plan(iptr(coords), n, levels, what, kpos.data_ptr<int32_t>(), coord_ptrs.data(), ws.data_ptr(), bytes,
+                                  host.data_ptr<int32_t>(), st);
+    }
+    check_status(rc);
+    if (sizes[0] == 0) break;
+    if (sizes[1] == 0 || attempt > 0) return Pyramid();
+    bytes = (size_t)sizes[1] * 256;
   }
-  check_status(rc);
-  if (sizes[0] != 0) return r;
   r.fits = true;
   for (int l = 0; l < levels; ++l) r.voxels.push_back(sizes[1 + l]);
   std::vector<Tensor> flat;
@@ -275,6 +285,15 @@ Pyramid build_pyramid(const Tensor& coords, int levels, int what) {
   }
   for (int l = 1; l < levels; ++l) r.out_coords[l - 1] = r.out_coords[l - 1].narrow(0, 0, r.voxels[l]);
   return r;
+}
+
+// A cloud for whose bitmaps there is no memory does not fit either: the other builders need less.
+Pyramid build_pyramid(const Tensor& coords, int levels, int what) {
+  try {
+    return try_pyramid(coords, levels, what);
+  } catch (const c10::OutOfMemoryError&) {
+    return Pyramid();
+  }
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -202,9 +202,12 @@ int fgms_b200_transpose_map(const int32_t* kpos, const int32_t* in_map, const in
  * pyramid_plan fills kpos (int32 [maps][28], 9 or 28 entries used), out_coords[l - 1] (device int32 [n, 3], the first
  * voxels-of-level-l rows) and, after waiting for the stream, sizes_host[1 + levels + maps]: a flag, the voxels of every
  * level, the pairs of every map.  flag != 0: the cloud does not suit this builder (a box of too many cells for the
- * workspace, a voxel met twice, a coordinate outside [-2^20, 2^20)); the results are then undefined and the builders
- * above are the way to go.  pyramid_emit, with the same arguments and the untouched workspace, writes the maps into
- * buffers of those sizes (host arrays of device pointers, one per map). */
+ * workspace, a voxel met twice, a coordinate outside [-2^20, 2^20)); the results are then undefined.  If
+ * sizes_host[1] is not 0 then, a workspace of sizes_host[1] * 256 bytes has room for the box and plan may be called
+ * again with it; otherwise the builders above are the way to go.  pyramid_workspace_bytes is the least a workspace
+ * may have: room for boxes of 1024 words of 32 cells per voxel, from 16 k voxels on for the largest this builder takes.
+ * pyramid_emit, with the same arguments and the untouched workspace, writes the maps into buffers of those sizes (host
+ * arrays of device pointers, one per map). */
 size_t fgms_b200_pyramid_workspace_bytes(int n, int levels, int what);
 int fgms_b200_pyramid_plan(const int32_t* coords, int n, int levels, int what, int32_t* kpos, int32_t* const* out_coords,
                            void* workspace, size_t workspace_bytes, int32_t* sizes_host, void* stream);

@@ -1,4 +1,5 @@
-"""Clouds the bitmap builder leaves to the hash-table builders: it is asked once, not once per map."""
+"""Clouds the bitmap builder leaves to the hash-table builders: it is asked once, not once per map, and neither its
+scratch nor the lack of it stands in the way of a cloud that the hash-table builders can do."""
 import numpy as np
 import pytest
 import torch
@@ -61,3 +62,28 @@ def test_a_voxel_met_twice_is_refused_once(monkeypatch):
     monkeypatch.setattr(gpu_maps, "_native", counting)
     unet.build_unet_maps(_dev(coords), 3)
     assert counting.calls == 1
+
+
+def test_a_small_cloud_takes_little_memory():
+    coords = _dev(clouds.surface_cloud(300, 20, 5))
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    gpu_maps.build_submanifold_map(coords, 3)
+    gpu_maps.build_strided_map(coords, 2)
+    assert torch.cuda.max_memory_allocated() - before < 2 << 20
+
+
+def test_a_wide_box_without_room_for_its_bitmaps_is_still_built():
+    """2000 x 2000 x 80 cells take 64 MB of bits; with 40 MB left the hash-table builders do it."""
+    coords = np.unique(np.random.default_rng(3).integers(0, [2000, 2000, 80], (3000, 3)).astype(np.int32), axis=0)
+    dev = _dev(coords)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (40 << 20)) / total)
+        got = unet.build_unet_maps(dev, 2)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    _check(got, unet.build_unet_maps_host(coords, 2))
