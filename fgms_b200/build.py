@@ -10,6 +10,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import tempfile
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -17,7 +18,7 @@ LIB = os.path.join(HERE, "libfgms_b200.so")
 SOURCES = [os.path.join(CSRC, "fgms_abi.cu")]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-# no GNU-unique symbols: two builds of the library in one process keep their launch state apart
+    # no GNU-unique symbols: two builds of the library in one process keep their launch state apart
     "-Xcompiler", "-fPIC,-fno-gnu-unique", "-shared", "-cudart", "shared", "-ldl",
 ]
 
@@ -59,9 +60,14 @@ def _build_binding(verbose: bool) -> None:
     include = cpp_extension.include_paths() + [os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
     cmd += [f for d in include for f in ("-isystem", d)]
-    cmd += [BINDING_SOURCE, "-o", BINDING, "-L" + HERE, "-lfgms_b200", "-L" + lib_dir, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10",
-            "-lc10_cuda", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + lib_dir]
-    _run(cmd, "_native.so", verbose)
+    # The extension names the library by its place beside itself, through a stand-in of that name at link time: under a
+    # bare name the loader would hand it the library of another copy that the process has loaded already.
+    with tempfile.TemporaryDirectory() as tmp:
+        beside = os.path.join(tmp, "beside.so")
+        _run(["g++", "-shared", "-fPIC", "-x", "c++", os.devnull, "-o", beside, "-Wl,-soname,$ORIGIN/libfgms_b200.so"], "a stand-in", verbose)
+        cmd += [BINDING_SOURCE, "-o", BINDING, "-Wl,--no-as-needed", beside, "-L" + lib_dir, "-ltorch_python", "-ltorch", "-ltorch_cpu",
+                "-lc10", "-lc10_cuda", "-Wl,-rpath," + lib_dir]
+        _run(cmd, "_native.so", verbose)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
