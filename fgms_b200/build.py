@@ -3,14 +3,17 @@
     python -m fgms_b200.build [--force] [--verbose]
 
 The library is a plain C-ABI shared object (see ``include/fgms_b200.h``); it links only the CUDA
-runtime, not PyTorch.  ``_native.so`` is the PyTorch binding on top of it and finds it beside itself.
+runtime, not PyTorch.  ``_native.so`` is the PyTorch binding on top of it and finds it beside itself; without PyTorch
+the library alone is built.
 """
 from __future__ import annotations
 
 import os
 import subprocess
 import sys
+import sysconfig
 import tempfile
+from importlib import metadata
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -25,6 +28,7 @@ NVCC_FLAGS = [
 
 BINDING = os.path.join(HERE, "_native.so")
 BINDING_SOURCE = os.path.join(CSRC, "torch_binding.cpp")
+BUILT_FOR = os.path.join(HERE, "_native.built_for")  # the PyTorch and Python that _native.so was built for
 
 
 def _deps():
@@ -38,8 +42,27 @@ def _stale(target: str, sources) -> bool:
     return not os.path.exists(target) or any(os.path.getmtime(f) > os.path.getmtime(target) for f in sources)
 
 
+def _host() -> str | None:
+    """The PyTorch and Python of this environment; None without PyTorch."""
+    try:
+        return f"torch {metadata.version('torch')}, {sysconfig.get_config_var('SOABI')}"
+    except metadata.PackageNotFoundError:
+        return None
+
+
+def _built_for() -> str | None:
+    if not os.path.exists(BUILT_FOR):
+        return None
+    with open(BUILT_FOR) as f:
+        return f.read()
+
+
 def needs_build() -> bool:
-    return _stale(LIB, _deps()) or _stale(BINDING, [BINDING_SOURCE, os.path.join(os.path.dirname(HERE), "include", "fgms_b200.h")])
+    if _stale(LIB, _deps()):
+        return True
+    host = _host()
+    return host is not None and (_built_for() != host or
+                                 _stale(BINDING, [BINDING_SOURCE, os.path.join(os.path.dirname(HERE), "include", "fgms_b200.h")]))
 
 
 def _run(cmd, what: str, verbose: bool) -> None:
@@ -51,8 +74,6 @@ def _run(cmd, what: str, verbose: bool) -> None:
 
 
 def _build_binding(verbose: bool) -> None:
-    import sysconfig
-
     import torch
     from torch.utils import cpp_extension
     lib_dir = os.path.join(os.path.dirname(torch.__file__), "lib")
@@ -68,6 +89,8 @@ def _build_binding(verbose: bool) -> None:
         cmd += [BINDING_SOURCE, "-o", BINDING, "-Wl,--no-as-needed", beside, "-L" + lib_dir, "-ltorch_python", "-ltorch", "-ltorch_cpu",
                 "-lc10", "-lc10_cuda", "-Wl,-rpath," + lib_dir]
         _run(cmd, "_native.so", verbose)
+    with open(BUILT_FOR, "w") as f:
+        f.write(_host())
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -75,7 +98,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return LIB
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
     _run([nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + SOURCES + ["-o", LIB], "libfgms_b200.so", verbose)
-    _build_binding(verbose)
+    if _host() is None:
+        sys.stderr.write("PyTorch is not installed: _native.so is not built\n")
+    else:
+        _build_binding(verbose)
     return LIB
 
 
