@@ -118,7 +118,7 @@ __device__ __forceinline__ void cta_tile_range(int total, int* t0, int* t1) {
 struct Turns {
   int i0, full, first_i, last_r, me;
   // [s0, s1): the offset's turns; t: this worker's first turn inside it
-  __device__ __forceinline__ Turns(int s0, int s1, int share, int worker, int t, bool spread) {
+  __host__ __device__ __forceinline__ Turns(int s0, int s1, int share, int worker, int t, bool spread) {
     const int first = s0 / share, last = (s1 - 1) / share;
     full = spread ? last - first - 1 : -1;
     first_i = s0 - first * share;
@@ -127,7 +127,7 @@ struct Turns {
     i0 = full < 0 ? t - s0 : t - worker * share;
   }
   // the offset's tile for this worker's n-th turn inside it
-  __device__ __forceinline__ int tile(int n) const {
+  __host__ __device__ __forceinline__ int tile(int n) const {
     const int i = i0 + n;
     if (full < 0) return i;  // consecutive parts, or the offset lies inside one share
     const int rank = me == 0 ? full : (me <= full ? me - 1 : full + (i >= first_i ? 1 : 0));

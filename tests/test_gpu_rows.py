@@ -51,3 +51,14 @@ def test_tiles_side_by_side_when_rows_exceed_l2(mode, c_in, c_out):
 def test_dense_centre():
     p = Problem(_map(333, [50, 0, 60], 4), 48, 32, seed=1, mode="fp16")
     assert err(p.run_fwd(separate_mid=True), p.ref_fwd(precompute=True)) <= TOL["fp16"]
+
+
+@pytest.mark.parametrize("separate_mid", [False, True])
+def test_many_tiles_a_warp_side_by_side(separate_mid):
+    """Shares of a dozen tiles and more over offsets of very different lengths, with the centre as a dense segment too."""
+    n = (72 << 20) // (64 * 2)
+    p = Problem(_map(n, [300000, 0, 300000, 5, 300000, 70, 300000], 7), 32, 32, seed=2, mode="fp16")
+    if separate_mid:
+        assert err(p.run_fwd(separate_mid=True), p.ref_fwd(precompute=True)) <= TOL["fp16"]
+    else:
+        _check(p)
