@@ -15,8 +15,8 @@
 //     consecutive bytes of the output row, which go out as one vector red.
 //   * B (the weight matrix) stays in registers while consecutive tiles belong to one offset: up to 64 registers.
 //
-// No shared memory beyond the tile table, no barrier, no shuffle in the loop; 14-24 warps per SM each with the rows of
-// one tile in flight while they multiply the one before.
+// No shared memory beyond the tile table, no barrier, no shuffle in the loop; 8 (tf32 64 -> 32) to 24 (fp16 16 -> 16) warps per
+// SM, each with the rows of one tile in flight while it multiplies the one before.
 #pragma once
 #include <atomic>
 #include <type_traits>
@@ -336,9 +336,12 @@ inline int rw_launch(const GmsParams& p, cudaStream_t st, int sms) {
 // 0 launched, 1 not a shape of this kernel or a pointer is not 16-byte aligned, < 0 CUDA error
 inline int launch_rows_gms(const GmsParams& p, bool trans, bool f16, cudaStream_t st, int sms) {
   if (!rw_supported(p.k_dim, p.n_dim, f16)) return 1;
-  // tf32 32 -> 64: 64 weight registers and a 256-byte red per pair leave nothing over the tcgen05 form once a warp has more
-  // than a few tiles (200 k pairs: 17.9 against 16.3 us); with fewer the shorter start decides
-  if (!f16 && p.n_dim > p.k_dim && p.k_dim * p.n_dim == 8 * 256 && p.pairs >= (1 << 17)) return 1;
+  // tf32 32 -> 64, the one pair of widths whose weights fill the 64 registers and whose scattered rows are the longer ones:
+  // from 32 k pairs on the tcgen05 form is the faster (this kernel / that one, 27 offsets: 8 k pairs 3.7 / 5.6 us, 16 k
+  // 5.5 / 5.8, 32 k 7.5 / 6.8, 131 k 12.5 / 11.8, 200 k 17.7 / 15.8, 1 M 65 / 59); 64 -> 32 is faster here at every size
+  // (32 k 6.1 / 6.8, 200 k 13.7 / 18.1, 1 M 45 / 69), and so are 32 -> 48 (200 k 14.5 / 15.5) and, but for 5 % at 262 k
+  // pairs, 16 -> 64
+  if (!f16 && p.k_dim == 32 && p.n_dim == 64 && p.pairs >= (1 << 15)) return 1;
   if ((long long)p.pairs + p.dense_rows > 0x7fffffffll - 4096) return 1;  // positions two tiles past the end stay in an int
   if ((reinterpret_cast<uintptr_t>(p.src) | reinterpret_cast<uintptr_t>(p.weights) | reinterpret_cast<uintptr_t>(p.dst)) & 15) return 1;
   if (f16) return trans ? rw_launch<false, true>(p, st, sms) : rw_launch<false, false>(p, st, sms);

@@ -48,6 +48,11 @@ def test_tiles_side_by_side_when_rows_exceed_l2(mode, c_in, c_out):
     _check(Problem(_map(n, [40, 3000, 0, 17, 60000, 1, 9000], 7), c_in, c_out, seed=2, mode=mode))
 
 
+@pytest.mark.parametrize("counts", [[16384, 16383], [16384, 16384]])
+def test_both_sides_of_the_line_of_tf32_32_to_64(counts):
+    _check(Problem(_map(20000, counts, 3), 32, 64, seed=1, mode="tf32"))
+
+
 def test_dense_centre():
     p = Problem(_map(333, [50, 0, 60], 4), 48, 32, seed=1, mode="fp16")
     assert err(p.run_fwd(separate_mid=True), p.ref_fwd(precompute=True)) <= TOL["fp16"]
