@@ -48,6 +48,8 @@ import time
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
+# what the families of backend.kernel_family run on (short rows: mma.sync, the others: tcgen05)
+FAMILY = {"tcgen05": "tensor cores", "simt": "CUDA cores"}
 METRIC = "spconv fwd+bwd effective TFLOPS (6*pairs*c_in*c_out / time), one layer"
 UNIT = "TFLOPS"
 
@@ -357,7 +359,7 @@ def run_cfg5(args, dev, rank, world, flush):
             b = workloads.layer_bytes(pairs, l.c_in, l.c_out, l.k_vol, 2, r["pass"])
             fl = 2.0 * pairs * l.c_in * l.c_out
             t_roof = max(b / (hbm * 1e9), fl / (f16_peak * 1e12)) * 1e3
-            fam = backend.kernel_family(r["pass"], run_l.c_in, run_l.c_out, torch.float16, True, l.k_vol)
+            fam = FAMILY[backend.kernel_family(r["pass"], run_l.c_in, run_l.c_out, torch.float16, True, l.k_vol)]
             row = {"layer": l.name, "pass": r["pass"], "shape": f"{l.c_in}->{l.c_out} k{l.k_vol}", "pairs": pairs,
                    "ms": round(r["ms"], 5), "frac": round(t_roof / r["ms"], 4), "family": fam}
             table.append(row)
@@ -949,7 +951,7 @@ def run_ours(args):
         achieved = dom_bytes / (dom_ms * 1e-3) / 1e9
         all_bytes = workloads.algorithmic_bytes(wl, "all")
         t_roof_step = max(all_bytes / (hbm * 1e9), 3 * pass_flops / (t_peak * 1e12)) * 1e3
-        family = backend.kernel_family(dom, wl.c_in, wl.c_out, p.dtype, p.arch80, km.k_vol)
+        family = FAMILY[backend.kernel_family(dom, wl.c_in, wl.c_out, p.dtype, p.arch80, km.k_vol)]
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": k, "warmup": args.warmup,
             "ms_per_step": total_ms / k, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,

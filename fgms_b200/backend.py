@@ -262,10 +262,11 @@ def wgrad_finalize(kernel_grad: torch.Tensor, partial_f32: torch.Tensor) -> None
 
 
 def kernel_family(pass_: str, c_in: int, c_out: int, dtype: torch.dtype, arch80: bool = True, k_vol: int = 27) -> str:
-    """``"tcgen05"`` or ``"simt"``: which kernel family the dispatch uses for a shape: tensor cores (tcgen05, or warp-level
-    MMA for rows of up to 64 channels) or CUDA cores (channel counts that are
-    multiples of 16 up to 256 whose operands fit shared memory run on tcgen05 unless ``arch80`` is false for
-    fp32 storage)."""
+    """Which kernel family the dispatch uses for a shape: ``"tcgen05"`` for the tensor cores, ``"simt"`` for the CUDA cores.
+
+    Channel counts that are multiples of 16 up to 256 whose operands fit shared memory run on the tensor cores unless
+    ``arch80`` is false for fp32 storage.  ``"tcgen05"`` names the whole family: within it, rows of up to 64 channels
+    run on warp-level MMA (``mma.sync``: ``csrc/rows_gms.cuh``, ``csrc/rows_wgrad.cuh``), the others on tcgen05."""
     d = _lib.DTYPE_F16 if dtype == torch.float16 else _lib.DTYPE_F32
     m = _lib.MATH_F16 if dtype == torch.float16 else (_lib.MATH_TF32 if arch80 else _lib.MATH_FP32)
     fam = _L.fgms_b200_kernel_family({"fwd": 0, "dgrad": 1, "wgrad": 2}[pass_], c_in, c_out, k_vol, d, m)
@@ -275,7 +276,7 @@ def kernel_family(pass_: str, c_in: int, c_out: int, dtype: torch.dtype, arch80:
 
 
 def fallback_count() -> int:
-    """Launches that should have run on tcgen05 by their shape but ran on the CUDA-core kernels because a
+    """Launches that should have run on the tensor cores by their shape but ran on the CUDA-core kernels because a
     tensor was not 16-byte aligned (0 in a healthy run)."""
     return int(_L.fgms_b200_fallback_count())
 

@@ -1,4 +1,5 @@
-// Exact fp32 on the CUDA cores, fp32 storage: forward / dgrad up to 128 contraction channels, and the weight gradient.
+// Exact fp32 on the CUDA cores, fp32 storage: forward / dgrad up to 128 contraction channels (about 108 where there are at most
+// four output channels: one lane a pair, and the rows of 32 of them exceed shared memory), and the weight gradient.
 //
 // The products of a ragged layer (20 -> 36 channels, 390 k pairs) are 7.5 us of FMA a pass, moving its rows 11-15 us;
 // the tiles of simt_kernels.cuh, 64 x 64 whatever the width, read shared memory a word at a time and keep no row in

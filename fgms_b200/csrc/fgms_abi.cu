@@ -674,8 +674,8 @@ int fgms_b200_peer_exchange(const float* const* sums, float* const* reduced, uin
   }
   p.count = count; p.epoch = epoch; p.rank = rank; p.world = world;
   p.wait_limit = wait_limit_cycles > 0 ? wait_limit_cycles : fgms::PX_WAIT_LIMIT_CYCLES;
-  // Same shared-memory carve-out as the tensor-core kernels (the largest): an SM keeps ONE carve-out for all the
-  // CTAs it holds, so a kernel that prefers another one would wait for the persistent kernel's CTAs to leave.
+  // A block's little shared memory has to fit the share that the kernels on the SM have set.  Preferring the largest one,
+  // it runs beside all of the backward's kernels; preferring none, it waits for the tcgen05 kernels to leave.
   static std::atomic<int> carveout_set[64];
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !carveout_set[dev].load(std::memory_order_acquire)) {

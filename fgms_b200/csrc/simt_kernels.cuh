@@ -1,6 +1,6 @@
 // CUDA-core (FFMA) kernels for the shapes no other kernel takes: fp16 storage with channel counts the tensor-core
 // kernels do not cover (not a multiple of 16, or more than 256), and fp32 storage with a contraction too wide for
-// ffma_rows.cuh (more than 128 channels).  Products are formed and accumulated in fp32.  Every global access is guarded, so any
+// ffma_rows.cuh (more than 128 channels; more than about 108 into at most four).  Products are formed and accumulated in fp32.  Every global access is guarded, so any
 // c_in / c_out >= 1 and any k_vol is accepted.  Rows are gathered with 16-byte loads whenever the row
 // length and the base address allow it (scalar loads otherwise), results leave with 16- or 8-byte
 // vector reds.

@@ -76,14 +76,9 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool v
 __device__ __forceinline__ void cp_async16_n(uint32_t dst, const void* src, uint32_t n) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
-// 4- and 8-byte copies (these go through L1)
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, bool valid = true) {
-  const uint32_t n = valid ? 4u : 0u;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src, bool valid) {
-  const uint32_t n = valid ? 8u : 0u;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+// 4-byte copy (goes through L1): used to prefetch map entries into shared memory without tying up a register
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void st_shared_i32(uint32_t dst, int v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst), "r"(v) : "memory"); }
 __device__ __forceinline__ int ld_shared_i32(uint32_t src) {

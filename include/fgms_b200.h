@@ -282,7 +282,7 @@ int fgms_b200_set_reserved_sms(int n);
  * same choice inside its dispatch and does not expose it (backend/spconv.cu:108-245). */
 int fgms_b200_kernel_family(int pass, int c_in, int c_out, int k_vol, int dtype, int math);
 
-/* Number of launches of this process that the plan above put on tcgen05 but that ran on the CUDA-core
+/* Number of launches of this process that the plan above put on the tensor cores but that ran on the CUDA-core
  * kernels instead because a tensor's base address was not 16-byte aligned.  Such a call is correct but
  * many times slower; a caller that cares asserts that this stays 0. */
 int64_t fgms_b200_fallback_count(void);
