@@ -115,6 +115,16 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// True in one lane of the (converged) warp.  tcgen05 instructions are issued by the lane that elect.sync names: the compiler
+// then knows that one thread runs the code.  Behind a plain `lane == 0` it does not, and every tcgen05.mma and commit costs
+// more issue slots: 128 x 64 x 16 back to back 56.8 cycles each against 48 (N = 32: 56.8 / 40, the tensor pipe's own time),
+// with a commit after every four 87 against 49; in a kernel whose other warps compete for those slots it was 144 an MMA.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+  return ok != 0;
+}
+
 // D[tmem] (+)= A[smem] * B[smem]; one thread issues
 template <bool TF32>
 __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,

@@ -317,9 +317,10 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
     int s = 0;
     uint32_t ph = 0;
     int cur_w = -1, n_load = -1, wb = 0, tile_i = 0;
-    // One lane runs the whole loop — waits, issue, commits — so that no warp-wide hand-shake sits between a
-    // stage landing and its MMAs; the other lanes wait at the end.
-    if (lane == 0)
+    // One lane, named by elect.sync (see elect_one), runs the whole loop — waits, issue, commits — so that no warp-wide
+    // hand-shake sits between a stage landing and its MMAs; the other lanes wait at the end.
+    // 128 -> 128 on 303 k pairs, forward + dgrad + weight gradient: 92 -> 86 us; 96 -> 160 on 321 k pairs 39.2 -> 36.6.
+    if (elect_one())
     for (int t = t0; t < t1 && ok; ++t, ++tile_i) {
       const int buf = tile_i & (cfg.n_tbuf - 1);
       const uint32_t use = (uint32_t)tile_i >> cfg.tbuf_shift;
@@ -362,7 +363,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
       }
     }
     __syncwarp();
-    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+    ok = __all_sync(0xffffffffu, ok) != 0;
   } else {
     // ------------------------------------------------------------------ epilogue (warps 0-7)
     // Two groups of four warps take alternate tiles, so that one group's TMEM reads and conversions run

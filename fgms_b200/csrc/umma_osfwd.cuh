@@ -256,8 +256,9 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, G
     cur.init(t0, gsz, t1);
     int s = 0, n_load = -1, wb = 0, grp_i = 0, last_tb = t0;
     uint32_t ph = 0;
-    // one lane runs the whole loop (waits, issue, commits); the other lanes wait at the end
-    if (lane == 0)
+    // One lane, named by elect.sync (see elect_one), runs the whole loop (waits, issue, commits); the other lanes wait at the
+    // end.  64 -> 64 on a full block of 48^3: 141 -> 128 us.
+    if (elect_one())
     while (cur.tb < t1 && ok) {
       if (cur.tb != last_tb) { last_tb = cur.tb; ++grp_i; }
       if (cur.g == 0) {
@@ -296,7 +297,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, G
       cur.next(gsz, t1, p.k_vol);
     }
     __syncwarp();
-    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+    ok = __all_sync(0xffffffffu, ok) != 0;
   } else {
     // ------------------------------------------------------------------ epilogue (warps 0-3)
     // Warp q owns TMEM lanes 32 q .. 32 q + 31 = tile rows 32 q + lane.  16 accumulator columns at a time:

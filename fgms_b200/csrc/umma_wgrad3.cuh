@@ -269,9 +269,9 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
     int s = 0, sg = 0, run_i = 0, cur_seg = -1;
     uint32_t ph = 0;
     bool first = true;
-    // One lane runs the whole loop — waits, issue, commits — so that no warp-wide hand-shake sits between a
-    // stage landing and its MMAs; the other lanes wait at the end.
-    if (lane == 0) {
+    // One lane, named by elect.sync (see elect_one), runs the whole loop — waits, issue, commits — so that no warp-wide
+    // hand-shake sits between a stage landing and its MMAs; the other lanes wait at the end.
+    if (elect_one()) {
     for (int t = t0; t < t1 && ok; ++t) {
       if (cur.seg != cur_seg) {
         if (cur_seg >= 0) {
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
     if (ok && cur_seg >= 0) mma_commit(smem_u32(&sh->tmem_full[run_i & (cfg.n_buf - 1)]));
     }
     __syncwarp();
-    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+    ok = __all_sync(0xffffffffu, ok) != 0;
   } else if (warp < W3_EPI_WARPS) {
     // ------------------------------------------------------------------ epilogue (warps 0-3)
     // Thread (warp, lane) holds accumulator row m in its TMEM lane.  32 columns of the warp's 32 rows
