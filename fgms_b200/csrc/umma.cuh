@@ -7,6 +7,7 @@
 #include <atomic>
 #include <mutex>
 
+#include <cuda.h>  // CUtensorMap; its encoder is looked up at run time
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -27,6 +28,16 @@ __device__ __forceinline__ void mbar_fence_init() {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// one arrival, and `bytes` more for TMA copies to report
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// box of a 2-D tensor map at (x, y), into shared memory; reports its bytes to `bar`
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+               "l"(map), "r"(bar), "r"(x), "r"(y)
+               : "memory");
+}
 // One non-blocking probe of the barrier.  (mbarrier.try_wait may park the thread for an
 // implementation-defined time slice and was measured to wake up late; hand-offs between the roles of
 // these kernels are latency-critical, so the waiting lane probes with test_wait instead.)
@@ -35,6 +46,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// The same, but the thread may be parked until the phase completes or a time limit of the hardware's own runs out.
+__device__ __forceinline__ bool mbar_park(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
       : "r"(bar), "r"(parity)
@@ -56,6 +79,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
   if (abort_flag) *abort_flag = 1;
   return false;
+}
+
+// The bounded wait of a warp that is ahead of the others: it leaves them its issue slots.
+__device__ __forceinline__ bool mbar_parked_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long start = clock64();
+  while (!mbar_park(bar, parity)) {
+    if (abort_flag && *abort_flag) return false;
+    if (clock64() - start > WAIT_LIMIT_CYCLES) {
+      if (abort_flag) *abort_flag = 1;
+      return false;
+    }
+  }
+  return true;
 }
 
 // ------------------------------------------------------------------ programmatic dependent launch
@@ -144,6 +181,24 @@ __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_
         : "memory");
   }
 }
+// accumulating, except into the accumulator rows whose bit of off0 .. off3 is set (row = tensor-memory lane)
+template <bool TF32>
+__device__ __forceinline__ void mma_ss_masked(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t off0, uint32_t off1,
+                                              uint32_t off2, uint32_t off3) {
+  if (TF32) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%4, %5, %6, %7}, p;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(off0), "r"(off1), "r"(off2), "r"(off3)
+        : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%4, %5, %6, %7}, p;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(off0), "r"(off1), "r"(off2), "r"(off3)
+        : "memory");
+  }
+}
 // arrive on an mbarrier once every tcgen05.mma issued so far by this thread has finished
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -157,6 +212,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
       : "r"(taddr)
       : "memory");
 }
+// zeros to 16 consecutive columns of the warp's 32 lanes
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr), "r"(0u) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // ------------------------------------------------------------------ descriptors
@@ -210,6 +270,27 @@ __host__ __device__ constexpr uint32_t mnmajor32_offset(uint32_t k, uint32_t byt
 }
 
 }  // namespace umma
+
+// Tensor map over weights [k_vol, c_in, c_out] whose box is one 128-byte column block of one matrix: what tma_load_2d writes is
+// the MN-major 128-byte-swizzled operand (rows = contraction index), block after block.  Columns beyond c_out come as zeros.
+// Made for every call (42 ns): nothing is kept by an address.
+inline bool weight_tensor_map(CUtensorMap* map, const void* weights, int k_vol, int c_in, int c_out, bool f16) {
+  using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                              const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Encode encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) fn = nullptr;
+    return reinterpret_cast<Encode>(fn);
+  }();
+  if (encode == nullptr) return false;
+  const int es = f16 ? 2 : 4;
+  const cuuint64_t dims[2] = {(cuuint64_t)c_out, (cuuint64_t)k_vol * c_in}, pitch[1] = {(cuuint64_t)c_out * es};
+  const cuuint32_t box[2] = {(cuuint32_t)(128 / es), (cuuint32_t)c_in}, steps[2] = {1, 1};
+  return encode(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(weights), dims, pitch, box, steps,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, f16 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 // Launch with the programmatic-stream-serialization attribute.
 template <typename... KArgs, typename... Args>

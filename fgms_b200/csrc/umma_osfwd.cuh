@@ -28,12 +28,23 @@ namespace fgms {
 
 constexpr int OS_EPI_WARPS = 4;
 constexpr int OS_MMA_WARP = 4;
-constexpr int OS_PROD_WARP0 = 5;
-constexpr int OS_PROD_WARPS = 8;
-constexpr int OS_PROD_THREADS = OS_PROD_WARPS * 32;
-constexpr int OS_THREADS = (OS_PROD_WARP0 + OS_PROD_WARPS) * 32;  // 416
-constexpr int OS_PREFETCH = 4;  // neighbour entries are fetched this many stages ahead
+constexpr int OS_W_WARP = 8;
+constexpr int OS_PROD_WARPS = 12;
+constexpr int OS_THREADS = 640;
+// producer of a warp (< 0: none): the warps from 5 on that do not share a scheduler with the MMA warp
+__device__ __forceinline__ int os_producer(int warp) { return (warp & 3) && warp > OS_MMA_WARP ? ((warp >> 2) - 1) * 3 + (warp & 3) - 1 : -1; }
 constexpr int OS_TILE = 128;
+constexpr int OS_MAX_STAGES = 12;
+constexpr int OS_MAX_GROUP = 8;  // tiles walked together, an accumulator each
+
+struct OsConfig {
+  int n_stage, n_wbuf, w_bytes;
+  int n_prod;  // producer warps that work: no more than there are stages (see the producers)
+  int kch;     // 128-byte chunks of an input row (= stages of a tile and offset)
+  int n_acc;   // tensor-memory columns of an accumulator: whole 128-byte blocks of the output row
+  int group;   // tiles walked together
+  int smem;
+};
 
 struct OsParams {
   const void* src;       // [n_in , c_in ]
@@ -49,37 +60,22 @@ struct OsParams {
 };
 
 struct OsShared {
-  uint64_t full[G3_MAX_STAGES];
-  uint64_t empty[G3_MAX_STAGES];
-  uint64_t tmem_full[4];
-  uint64_t tmem_empty[4];
+  uint64_t full[OS_MAX_STAGES];   // stage landed: 32 hardware arrivals and one after the mask was written
+  uint64_t empty[OS_MAX_STAGES];  // stage consumed (tcgen05.commit)
+  uint64_t tmem_full[OS_MAX_GROUP];
+  uint64_t tmem_empty[OS_MAX_GROUP];  // accumulator read and cleared (one arrival per epilogue warp)
+  uint64_t w_full[2];
   uint64_t w_free[2];
+  uint4 on[OS_MAX_STAGES];  // rows a stage holds, a bit each
   uint32_t tmem_base;
   int abort_flag;
 };
 constexpr int OS_SHARED_BYTES = (sizeof(OsShared) + 15) & ~15;
 
-// The walk every role makes over the CTA's tiles [.., t1): groups of up to `gsz` consecutive tiles; within a group
-// offset by offset, within an offset tile by tile.  A CTA's tile range is cut to the tile (not to the group), so the
-// CTAs' loads differ by one tile at most; the last group of a CTA may be smaller.
-struct OsWalk {
-  int tb, k, g, gv;  // first tile of the group, offset, tile of the group, tiles this group has (<= 0: past the end)
-  __device__ __forceinline__ void init(int t0, int gsz, int t1) {
-    tb = t0; k = 0; g = 0;
-    gv = min(gsz, t1 - tb);
-  }
-  __device__ __forceinline__ void next(int gsz, int t1, int k_vol) {
-    if (++g >= gv) {
-      g = 0;
-      if (++k == k_vol) {
-        k = 0;
-        tb += gsz;
-        gv = min(gsz, t1 - tb);
-      }
-    }
-  }
-  __device__ __forceinline__ int tile() const { return tb + g; }
-};
+__device__ __forceinline__ bool os_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  const bool ok = umma::mbar_parked_wait(umma::smem_u32(bar), parity, abort_flag);
+  return __all_sync(0xffffffffu, ok) != 0;
+}
 
 // nbr[k][out_map[j]] = in_map[j] for every pair j of offset k (the table is filled with -1 beforehand).  Every kpos
 // entry is clamped to [0, map_len]; a pair with an entry outside the tensors is skipped and counted.
@@ -106,7 +102,7 @@ __global__ void os_fill_nbr_kernel(const int32_t* __restrict__ kpos, const int32
 }
 
 template <bool TF32>
-__global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, G3Config cfg) {
+__global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, OsConfig cfg, const __grid_constant__ CUtensorMap w_map) {
   using namespace umma;
   constexpr int ES = TF32 ? 4 : 2;
   constexpr int EPR = 128 / ES;
@@ -115,24 +111,26 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, G
   uint8_t* sW = smem;
   uint8_t* sStage = sW + (size_t)cfg.n_wbuf * cfg.w_bytes;
   uint8_t* sPatch = sStage + (size_t)cfg.n_stage * G3_STAGE_BYTES;
-  OsShared* sh = reinterpret_cast<OsShared*>(sPatch + G3_PATCH_BYTES);
+  OsShared* sh = reinterpret_cast<OsShared*>(sPatch + OS_EPI_WARPS * 4096);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int kch = cfg.kch, n_stage = cfg.n_stage, gsz = cfg.n_tbuf;
+  const int kch = cfg.kch, n_stage = cfg.n_stage, gsz = cfg.group;
   const int k_bytes = p.c_in * ES;
   volatile int* abort_flag = &sh->abort_flag;
 
   if (tid == 0) {
     for (int s = 0; s < n_stage; ++s) {
-      mbar_init(smem_u32(&sh->full[s]), OS_PROD_THREADS);
+      mbar_init(smem_u32(&sh->full[s]), 33);
       mbar_init(smem_u32(&sh->empty[s]), 1);
     }
-    for (int b = 0; b < 4; ++b) {
+    for (int b = 0; b < OS_MAX_GROUP; ++b) {
       mbar_init(smem_u32(&sh->tmem_full[b]), 1);
       mbar_init(smem_u32(&sh->tmem_empty[b]), OS_EPI_WARPS);
     }
-    mbar_init(smem_u32(&sh->w_free[0]), 1);
-    mbar_init(smem_u32(&sh->w_free[1]), 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&sh->w_full[b]), 1);
+      mbar_init(smem_u32(&sh->w_free[b]), 1);
+    }
     sh->abort_flag = 0;
     mbar_fence_init();
   }
@@ -156,149 +154,145 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, G
 
   if (t0 >= t1) {
     // nothing for this CTA
-  } else if (warp >= OS_PROD_WARP0) {
+  } else if (os_producer(warp) >= cfg.n_prod) {
+    // more warps than stages
+  } else if (os_producer(warp) >= 0) {
     // ------------------------------------------------------------------ producers
-    // Warp pw owns tile rows [16 pw, 16 pw + 16); lane (rs, pc) = (lane / 8, lane % 8) copies 16-byte chunk pc of
-    // every 128-byte K chunk of the rows rs, rs + 4, rs + 8, rs + 12 of that block.
-    const int pw = warp - OS_PROD_WARP0;
-    const int tp = tid - OS_PROD_WARP0 * 32;
+    // Warp w fills stages w, w + nw, ...  With nw <= n_stage a wait for a ring slot by parity is safe: the warp's stage
+    // before, q - nw, was let in after stage q - nw - n_stage had been consumed, stages are consumed in order, and so the slot's
+    // barrier is at most one phase behind the one that stage q waits for.  (With more warps than slots it may be two behind,
+    // which looks the same, and two warps fill one slot.)  Lane l holds the neighbour entries of the tile's rows l, l + 32,
+    // l + 64, l + 96, and copies 16-byte chunk l % 8 of the rows l / 8, l / 8 + 4, ...
+    const int w = os_producer(warp), nw = cfg.n_prod;
     const int rs = lane >> 3, pc = lane & 7;
-    const uint8_t* src = static_cast<const uint8_t*>(p.src);
-    const uint8_t* wts = static_cast<const uint8_t*>(p.weights);
-    uint32_t a_dst[4];
+    const uint8_t* src = static_cast<const uint8_t*>(p.src) + pc * 16;
+    uint32_t a_dst[2];  // rows rs, rs + 4 of a group of eight
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t r = (uint32_t)(16 * pw + rs + 4 * j);
-      a_dst[j] = (r >> 3) * 1024u + (r & 7u) * 128u + (((uint32_t)pc ^ (r & 7u)) << 4);
+    for (int j = 0; j < 2; ++j) {
+      const uint32_t r = (uint32_t)(rs + 4 * j);
+      a_dst[j] = r * 128u + (((uint32_t)pc ^ r) << 4);
     }
-    // lane r < 16 fetches the neighbour entry of the warp's row r
-    auto load_entry = [&](const OsWalk& w) -> int {
-      if (lane >= 16) return -1;
-      return __ldg(p.nbr + (long long)w.k * p.nbr_stride + (long long)w.tile() * OS_TILE + 16 * pw + lane);
-    };
-    // weight matrix W_k -> MN-major operand (rows = contraction index), as in the scatter-form forward
-    const int cpr = p.c_out * ES / 16;  // 16-byte chunks per row of W_k
-    const uint32_t w_row_bytes = (uint32_t)p.c_out * ES;
-    const uint32_t w_lbo = (uint32_t)p.c_in * 128u;
-    auto load_weights = [&](int k, int wb) {
-      const uint8_t* wk = wts + (size_t)k * p.c_in * p.c_out * ES;
-      const uint32_t sw = smem_u32(sW + (size_t)wb * cfg.w_bytes);
-      const int total = p.c_in * cpr;
-      for (int e = tp; e < total; e += OS_PROD_THREADS) {
-        const uint32_t row = e / cpr, c = e % cpr;
-        const uint32_t off = TF32 ? mnmajor32_offset(row, c * 16u, w_lbo, 512u) : mnmajor_offset(row, c * 16u, w_lbo, 1024u);
-        cp_async16(sw + off, wk + (size_t)row * w_row_bytes + c * 16u, true);
-      }
-    };
-
-    OsWalk cur, pf;
-    cur.init(t0, gsz, t1);
-    pf = cur;
-    int e[OS_PREFETCH];
-#pragma unroll
-    for (int d = 0; d < OS_PREFETCH; ++d) {
-      e[d] = pf.tb < t1 ? load_entry(pf) : -1;
-      pf.next(gsz, t1, p.k_vol);
-    }
-    int s = 0, n_load = -1, wb = 0;
+    const uint32_t kch_recip = (65536u + (uint32_t)kch - 1u) / (uint32_t)kch;  // x / kch = x * kch_recip >> 16 for x < 64, kch <= 8
+    int s = w, base = 0;  // the warp's next ring slot, stages of the groups before
     uint32_t ph = 0;
-    while (cur.tb < t1 && ok) {
-      int ent = e[0];
+    for (int tb = t0; tb < t1 && ok; tb += gsz) {
+      // the group's stages: offset k, then r = tile of the group * kch + chunk
+      const int per_k = min(gsz, t1 - tb) * kch, n = per_k * p.k_vol;
+      const int first = (w + nw - base % nw) % nw;
+      const int step_k = nw / per_k, step_r = nw % per_k;
+      int k = first / per_k, r = first % per_k;
+      auto load_entries = [&](int (&e)[4]) {
+        const int g = (int)((uint32_t)r * kch_recip >> 16);
+        const int32_t* at = p.nbr + (long long)k * p.nbr_stride + (long long)(tb + g) * OS_TILE + lane;
 #pragma unroll
-      for (int d = 0; d + 1 < OS_PREFETCH; ++d) e[d] = e[d + 1];
-      e[OS_PREFETCH - 1] = pf.tb < t1 ? load_entry(pf) : -1;
-      pf.next(gsz, t1, p.k_vol);
-      if ((unsigned)ent >= (unsigned)p.n_in) {
-        if (ent != -1) report_problem();  // an entry outside the tensor: treated as no neighbour, counted
-        ent = -1;
-      }
-      if (cur.g == 0) {
-        // a new offset: weight load number n_load goes to buffer n_load % n_wbuf, whose previous tenant was load
-        // n_load - n_wbuf — wait until the MMA warp has reported that tenant's last MMA finished
-        ++n_load;
-        wb = (cfg.n_wbuf == 2) ? (n_load & 1) : 0;
-        if (n_load >= cfg.n_wbuf) {
-          const uint32_t use = (uint32_t)(cfg.n_wbuf == 2 ? (n_load >> 1) : n_load) - 1u;
-          ok = g3_wait(&sh->w_free[wb], use & 1u, abort_flag);
-          if (!ok) break;
-        }
-        load_weights(cur.k, wb);  // the first stage's barrier below also covers these copies
-      }
-      const uint8_t* rsrc[4];
-      bool valid[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int g = __shfl_sync(0xffffffffu, ent, rs + 4 * j);
-        valid[j] = g >= 0;
-        rsrc[j] = src + (size_t)max(g, 0) * k_bytes + (size_t)pc * 16;
-      }
-      for (int kc = 0; kc < kch && ok; ++kc) {
-        ok = g3_wait(&sh->empty[s], ph ^ 1u, abort_flag);
+        for (int x = 0; x < 4; ++x) e[x] = __ldg(at + 32 * x);
+      };
+      int e[4];
+      if (first < n) load_entries(e);
+      for (int i = first; i < n; i += nw) {
+        const int kc = r - (int)((uint32_t)r * kch_recip >> 16) * kch;
+        ok = os_wait(&sh->empty[s], ph ^ 1u, abort_flag);
         if (!ok) break;
-        const uint32_t st = smem_u32(sStage + (size_t)s * G3_STAGE_BYTES);
-        if (kc * 128 + pc * 16 < k_bytes) {
+        int ent[4];
+        uint32_t on[4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) cp_async16(st + a_dst[j], rsrc[j] + (size_t)kc * 128, valid[j]);
+        for (int x = 0; x < 4; ++x) {
+          const bool good = (unsigned)e[x] < (unsigned)p.n_in;
+          if (!good && e[x] != -1 && kc == 0) report_problem();  // outside the tensor: treated as no neighbour, counted
+          on[x] = __ballot_sync(0xffffffffu, good);
+          ent[x] = good ? e[x] : -1;
+        }
+        k += step_k; r += step_r;
+        if (r >= per_k) { r -= per_k; ++k; }
+        if (i + nw < n) load_entries(e);
+        const uint32_t st = smem_u32(sStage) + (uint32_t)s * G3_STAGE_BYTES;
+        const uint8_t* from = src + kc * 128;
+        // a place whose row has no neighbour keeps what it held: the MMA leaves that accumulator row alone
+        const bool pc_ok = kc * 128 + pc * 16 < k_bytes;
+#pragma unroll
+        for (int x = 0; x < 32; ++x) {
+          const int g = __shfl_sync(0xffffffffu, ent[x / 8], (4 * x & 31) + rs);
+          if (g >= 0 && pc_ok) cp_async16(st + a_dst[x & 1] + (uint32_t)(x >> 1) * 1024u, from + (size_t)(unsigned)g * (uint32_t)k_bytes, true);
+        }
+        if (lane == 0) {
+          sh->on[s] = make_uint4(on[0], on[1], on[2], on[3]);
+          mbar_arrive(smem_u32(&sh->full[s]));
         }
         cp_async_arrive_noinc(smem_u32(&sh->full[s]));
-        if (++s == n_stage) { s = 0; ph ^= 1u; }
+        s += nw;
+        if (s >= n_stage) { s -= n_stage; ph ^= 1u; }
       }
-      cur.next(gsz, t1, p.k_vol);
+      base += n;
     }
-  } else if (warp == OS_MMA_WARP) {
-    // ------------------------------------------------------------------ MMA issuer
-    const uint32_t idesc = make_idesc(TF32, false, true, OS_TILE, cfg.n_mma);
-    const uint64_t a_desc0 = make_sdesc(smem_u32(sStage), 16u, 1024u);
-    const uint64_t b_desc0 = make_sdesc(smem_u32(sW), (uint32_t)p.c_in * 128u, TF32 ? 512u : 1024u, TF32 ? 1u : 2u);
-    const uint32_t b_kc_step = (uint32_t)EPR * 8u;        // one 128-byte K chunk further, in 16-byte units
-    const uint32_t b_ks_step = (32u / ES) * 8u;           // one 32-byte MMA step further
-    OsWalk cur;
-    cur.init(t0, gsz, t1);
-    int s = 0, n_load = -1, wb = 0, grp_i = 0, last_tb = t0;
-    uint32_t ph = 0;
-    // One lane, named by elect.sync (see elect_one), runs the whole loop (waits, issue, commits); the other lanes wait at the
-    // end.  64 -> 64 on a full block of 48^3: 141 -> 128 us.
-    if (elect_one())
-    while (cur.tb < t1 && ok) {
-      if (cur.tb != last_tb) { last_tb = cur.tb; ++grp_i; }
-      if (cur.g == 0) {
-        ++n_load;
-        wb = (cfg.n_wbuf == 2) ? (n_load & 1) : 0;
-      }
-      if (cur.k == 0) {
-        // first offset of the group: the accumulator must have been drained by the epilogue of the previous group
-        ok = mbar_wait(smem_u32(&sh->tmem_empty[cur.g]), ((uint32_t)grp_i & 1u) ^ 1u, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-      }
-      const uint32_t d_tmem = tmem_base + (uint32_t)(cur.g * cfg.n_acc);
-      const uint64_t b_desc_w = b_desc0 + (uint64_t)((uint32_t)wb * ((uint32_t)cfg.w_bytes >> 4));
-      const bool last_k = cur.k == p.k_vol - 1, last_of_w = cur.g == cur.gv - 1;
-      for (int kc = 0; kc < kch && ok; ++kc) {
-        ok = mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag);
-        if (!ok) break;
-        {
-          fence_proxy_async();
-          tc_fence_after();
-          const uint64_t a_desc_s = a_desc0 + (uint64_t)((uint32_t)s * (G3_STAGE_BYTES >> 4));
-          const uint64_t b_desc_kc = b_desc_w + (uint64_t)((uint32_t)kc * b_kc_step);
-          const int n_ks = min(4, (k_bytes - kc * 128) >> 5);
-          for (int ks = 0; ks < n_ks; ++ks)
-            mma_ss<TF32>(d_tmem, a_desc_s + (uint64_t)(ks * 2), b_desc_kc + (uint64_t)((uint32_t)ks * b_ks_step), idesc,
-                         (cur.k | kc | ks) != 0);
-          mma_commit(smem_u32(&sh->empty[s]));
-          if (kc == kch - 1) {
-            if (last_k) mma_commit(smem_u32(&sh->tmem_full[cur.g]));
-            if (last_of_w) mma_commit(smem_u32(&sh->w_free[wb]));
-          }
+  } else if (warp == OS_W_WARP) {
+    // ------------------------------------------------------------------ weights: W_k, once per group and offset, a TMA box per
+    // 128-byte column block (by one warp with cp.async it bounded wide layers: 128 -> 128 on a full block of 48^3 270 us)
+    if (elect_one()) {
+      int n_load = 0;
+      for (int tb = t0; tb < t1 && ok; tb += gsz)
+        for (int k = 0; k < p.k_vol; ++k, ++n_load) {
+          const int wb = cfg.n_wbuf == 2 ? n_load & 1 : 0;
+          const uint32_t use = (uint32_t)(cfg.n_wbuf == 2 ? n_load >> 1 : n_load);
+          ok = mbar_parked_wait(smem_u32(&sh->w_free[wb]), (use & 1u) ^ 1u, abort_flag);
+          if (!ok) break;
+          const uint32_t bar = smem_u32(&sh->w_full[wb]), sw = smem_u32(sW + (size_t)wb * cfg.w_bytes);
+          mbar_expect_tx(bar, (uint32_t)cfg.w_bytes);
+          for (int b = 0; b * EPR < cfg.n_acc; ++b) tma_load_2d(sw + (uint32_t)(b * p.c_in) * 128u, &w_map, bar, b * EPR, k * p.c_in);
         }
-        if (++s == n_stage) { s = 0; ph ^= 1u; }
-      }
-      cur.next(gsz, t1, p.k_vol);
     }
     __syncwarp();
     ok = __all_sync(0xffffffffu, ok) != 0;
-  } else {
+  } else if (warp == OS_MMA_WARP) {
+    // ------------------------------------------------------------------ MMA issuer
+    const uint32_t idesc = make_idesc(TF32, false, true, OS_TILE, cfg.n_acc);
+    const uint64_t a_desc0 = make_sdesc(smem_u32(sStage), 16u, 1024u);
+    const uint64_t b_desc0 = make_sdesc(smem_u32(sW), (uint32_t)p.c_in * 128u, TF32 ? 512u : 1024u, TF32 ? 1u : 2u);
+    constexpr uint32_t B_KC = (uint32_t)EPR * 8u, B_KS = (32u / ES) * 8u;  // one 128-byte K chunk / 32-byte MMA step further, in 16-byte units
+    // One lane, named by elect.sync (see elect_one), runs the whole loop (waits, issue, commits); the other lanes wait at the
+    // end.
+    if (elect_one()) {
+      int s = 0, n_load = 0, grp = 0;
+      uint32_t ph = 0;
+      for (int tb = t0; tb < t1 && ok; tb += gsz, ++grp) {
+        const int gv = min(gsz, t1 - tb);
+        for (int k = 0; k < p.k_vol && ok; ++k, ++n_load) {
+          const int wb = cfg.n_wbuf == 2 ? n_load & 1 : 0;
+          ok = mbar_wait(smem_u32(&sh->w_full[wb]), (uint32_t)(cfg.n_wbuf == 2 ? n_load >> 1 : n_load) & 1u, abort_flag);
+          const uint64_t b_desc_w = b_desc0 + (uint64_t)((uint32_t)wb * ((uint32_t)cfg.w_bytes >> 4));
+          for (int g = 0; g < gv && ok; ++g) {
+            if (k == 0) {
+              // first offset of the group: the accumulator must have been read and cleared
+              ok = mbar_wait(smem_u32(&sh->tmem_empty[g]), (uint32_t)grp & 1u, abort_flag);
+              if (!ok) break;
+              tc_fence_after();
+            }
+            const uint32_t d_tmem = tmem_base + (uint32_t)(g * cfg.n_acc);
+            for (int kc = 0; kc < kch; ++kc) {
+              ok = mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag);
+              if (!ok) break;
+              const uint4 on = sh->on[s];
+              fence_proxy_async();  // the stage was written through cp.async; the MMA reads it through the async proxy
+              tc_fence_after();
+              if (on.x | on.y | on.z | on.w) {
+                const uint64_t a_desc = a_desc0 + (uint64_t)((uint32_t)s * (G3_STAGE_BYTES >> 4)), b_desc = b_desc_w + (uint64_t)((uint32_t)kc * B_KC);
+                const int n_ks = min(4, (k_bytes - kc * 128) >> 5);
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks)
+                  if (ks < n_ks)
+                    mma_ss_masked<TF32>(d_tmem, a_desc + (uint64_t)(ks * 2), b_desc + (uint64_t)((uint32_t)ks * B_KS), idesc, ~on.x, ~on.y, ~on.z, ~on.w);
+              }
+              mma_commit(smem_u32(&sh->empty[s]));
+              if (++s == n_stage) { s = 0; ph ^= 1u; }
+            }
+            if (ok && k + 1 == p.k_vol) mma_commit(smem_u32(&sh->tmem_full[g]));
+          }
+          if (ok) mma_commit(smem_u32(&sh->w_free[wb]));
+        }
+      }
+    }
+    __syncwarp();
+    ok = __all_sync(0xffffffffu, ok) != 0;
+  } else if (warp < OS_EPI_WARPS) {
     // ------------------------------------------------------------------ epilogue (warps 0-3)
     // Warp q owns TMEM lanes 32 q .. 32 q + 31 = tile rows 32 q + lane.  16 accumulator columns at a time:
     // tcgen05.ld -> bias, ReLU, conversion -> the warp's patch -> eight consecutive lanes write 128 consecutive
@@ -309,11 +303,17 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, G
     uint8_t* patch = sPatch + warp * 4096;
     const uint32_t sw7 = (uint32_t)(lane & 7);
     const uint32_t ch = (uint32_t)(lane & 7), rsub = (uint32_t)(lane >> 3);
+    for (int g = 0; g < min(gsz, t1 - t0); ++g)
+      for (int c = 0; c < cfg.n_acc; c += 16) tmem_zero16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(g * cfg.n_acc + c));
+    tmem_st_wait();
+    tc_fence_before();
+    __syncwarp();
+    if (lane < OS_MAX_GROUP) mbar_arrive(smem_u32(&sh->tmem_empty[lane]));
     int grp_i = 0;
     for (int tb = t0; tb < t1 && ok; tb += gsz, ++grp_i) {
       const int gv = min(gsz, t1 - tb);
       for (int g = 0; g < gv && ok; ++g) {
-        ok = g3_wait(&sh->tmem_full[g], (uint32_t)grp_i & 1u, abort_flag);
+        ok = os_wait(&sh->tmem_full[g], (uint32_t)grp_i & 1u, abort_flag);
         if (!ok) break;
         tc_fence_after();
         const int row0 = (tb + g) * OS_TILE + 32 * warp;  // output row of this warp's lane 0
@@ -327,6 +327,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, G
             uint32_t v[16];
             tmem_ld16(taddr + col0 + c0, v);
             tmem_ld_wait();
+            tmem_zero16(taddr + col0 + c0);
             float f[16];
 #pragma unroll
             for (int k = 0; k < 16; ++k) f[k] = __uint_as_float(v[k]);
@@ -370,7 +371,8 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, G
             }
           }
           if (cb + 128 >= row_bytes) {
-            // accumulator fully read: hand it back before the last rows go out
+            // accumulator read and cleared: hand it back before the last rows go out
+            tmem_st_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&sh->tmem_empty[g]));
@@ -402,24 +404,46 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, G
   if (warp == OS_MMA_WARP) tmem_dealloc(tmem_base, tmem_cols);
 }
 
+// Shared memory and accumulators of a launch; false: not a shape of this kernel.
+inline bool os_plan(int c_in, int c_out, int es, int max_smem, OsConfig* cfg) {
+  if (!umma_supported(c_in, c_out, es)) return false;
+  const int epr = 128 / es;
+  cfg->kch = (c_in * es + 127) / 128;
+  cfg->n_acc = (c_out + epr - 1) / epr * epr;
+  cfg->w_bytes = c_in * 128 * (cfg->n_acc / epr);
+  cfg->group = 512 / cfg->n_acc < OS_MAX_GROUP ? 512 / cfg->n_acc : OS_MAX_GROUP;
+  const int fixed = 1024 + OS_EPI_WARPS * 4096 + OS_SHARED_BYTES;
+  // two weight buffers if at least four stages still fit beside them
+  cfg->n_wbuf = fixed + 2 * cfg->w_bytes + 4 * G3_STAGE_BYTES <= max_smem ? 2 : 1;
+  cfg->n_stage = (max_smem - fixed - cfg->n_wbuf * cfg->w_bytes) / G3_STAGE_BYTES;
+  if (cfg->n_stage > OS_MAX_STAGES) cfg->n_stage = OS_MAX_STAGES;
+  if (cfg->n_stage < 2) return false;
+  cfg->n_prod = cfg->n_stage < OS_PROD_WARPS ? cfg->n_stage : OS_PROD_WARPS;
+  cfg->smem = fixed + cfg->n_wbuf * cfg->w_bytes + cfg->n_stage * G3_STAGE_BYTES;
+  return true;
+}
+
 // 0 launched, 1 the shape has no plan or a pointer is not 16-byte aligned (there is no CUDA-core form of this
 // kernel: the caller reports it), < 0 CUDA error
 inline int launch_umma_osfwd(const OsParams& p, bool f16, cudaStream_t st, int sms, int max_smem) {
   if ((reinterpret_cast<uintptr_t>(p.src) | reinterpret_cast<uintptr_t>(p.weights) | reinterpret_cast<uintptr_t>(p.dst) |
        reinterpret_cast<uintptr_t>(p.bias)) & 15)
     return 1;
-  G3Config cfg;
-  if (!g3_plan(p.c_in, p.c_out, f16 ? 2 : 4, p.k_vol, max_smem, false, &cfg)) return 1;
+  OsConfig cfg;
+  G3Config scatter;  // the shapes of the scatter form, no more
+  if (!g3_plan(p.c_in, p.c_out, f16 ? 2 : 4, p.k_vol, max_smem, false, &scatter) || !os_plan(p.c_in, p.c_out, f16 ? 2 : 4, max_smem, &cfg)) return 1;
   const int grid = p.n_tiles < sms ? p.n_tiles : sms;
   if (grid <= 0) return 0;
+  CUtensorMap w_map;
+  if (!weight_tensor_map(&w_map, p.weights, p.k_vol, p.c_in, p.c_out, f16)) return -1;
   if (f16) {
     static std::atomic<int> granted[64];
     if (int rc = ensure_smem(umma_osfwd_kernel<false>, max_smem, granted)) return rc;
-    return launch_pdl(umma_osfwd_kernel<false>, grid, OS_THREADS, (size_t)cfg.smem, st, p, cfg) == cudaSuccess ? 0 : -1;
+    return launch_pdl(umma_osfwd_kernel<false>, grid, OS_THREADS, (size_t)cfg.smem, st, p, cfg, w_map) == cudaSuccess ? 0 : -1;
   }
   static std::atomic<int> granted[64];
   if (int rc = ensure_smem(umma_osfwd_kernel<true>, max_smem, granted)) return rc;
-  return launch_pdl(umma_osfwd_kernel<true>, grid, OS_THREADS, (size_t)cfg.smem, st, p, cfg) == cudaSuccess ? 0 : -1;
+  return launch_pdl(umma_osfwd_kernel<true>, grid, OS_THREADS, (size_t)cfg.smem, st, p, cfg, w_map) == cudaSuccess ? 0 : -1;
 }
 
 }  // namespace fgms
