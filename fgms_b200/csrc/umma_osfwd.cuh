@@ -7,18 +7,21 @@
 // to k_vol atomics in an order that changes from run to run, and nothing can be applied to the finished row
 // inside the kernel.  Here the map is a neighbour table nbr[k][r] (input row of output row r under offset k, -1
 // for none; built from the pair list by os_fill_nbr_kernel): a tile is 128 consecutive output rows, its
-// accumulator stays in tensor memory while the CTA walks all k_vol offsets (rows without a neighbour are
-// zero-filled), and the epilogue adds the bias, applies ReLU and stores the rows — plain stores, the same bits on
-// every run.  Up to four tiles (as many accumulators as the 512 TMEM columns hold) are walked together, offset
-// by offset, so that a weight matrix is staged once per group of tiles and offset.
+// accumulator stays in tensor memory while the CTA walks all k_vol offsets, and the epilogue adds the bias, applies ReLU
+// and stores the rows — plain stores, the same bits on every run.  Up to eight tiles (as many accumulators as the 512
+// tensor-memory columns hold) are walked together, offset by offset, so that a weight matrix is staged once per group of
+// tiles and offset.
 //
-// The price is one 128-row stage per (tile, offset) however few of the tile's rows have a neighbour there:
-// k_vol stages per 128 output rows against pairs / 128 stages in the scatter form — measured 0.9-1.1 times the
-// scatter form's time on fully occupied grids, 2.6 times at 9.5 pairs per voxel, 8 times at 2.1.  It is the form
-// for callers to whom reproducible bits or the fused epilogue are worth the extra stages.
+// The price is one 128-row stage per (tile, offset) however few of the tile's rows have a neighbour there: k_vol stages per
+// 128 output rows against pairs / 128 stages in the scatter form.  Rows without a neighbour are not copied, and
+// tcgen05.mma's output-lane mask leaves their accumulator rows alone: whatever their place in shared memory holds does not
+// matter (the accumulators are cleared by the epilogue before the first MMA).
 //
-// Roles (13 warps): 8 producers (16-byte cp.async gathers into the K-major 128-byte-swizzled stage ring, weight
-// matrices into one of two buffers), one MMA warp, 4 epilogue warps.  All waits are bounded.
+// Roles (20 warps): 12 producers, each filling whole stages (16-byte cp.async gathers into the K-major 128-byte-swizzled
+// ring), one MMA warp, one warp that loads weights by TMA, 4 epilogue warps.  All waits are bounded; all but the MMA lane's
+// are parked (85 -> 79 us on the layer below).  64 -> 64 on a full block of 48^3 (2.9 M pairs, 27 stages for each of 864 tiles):
+// 141 us with eight warps that each filled 16 rows of every stage and copied zeros, 56 us now: 650 cycles a stage, of which
+// 400-580 are the stage's 32 warp-wide copies; 128 -> 128 246 -> 97 us, 1000 voxels 64 -> 64 32 -> 17 us.
 #pragma once
 #include "common.cuh"
 #include "umma.cuh"
@@ -33,6 +36,7 @@ constexpr int OS_PROD_WARPS = 12;
 constexpr int OS_THREADS = 640;
 // producer of a warp (< 0: none): the warps from 5 on that do not share a scheduler with the MMA warp
 __device__ __forceinline__ int os_producer(int warp) { return (warp & 3) && warp > OS_MMA_WARP ? ((warp >> 2) - 1) * 3 + (warp & 3) - 1 : -1; }
+constexpr int OS_UNROLL = 4;
 constexpr int OS_TILE = 128;
 constexpr int OS_MAX_STAGES = 12;
 constexpr int OS_MAX_GROUP = 8;  // tiles walked together, an accumulator each
@@ -239,6 +243,9 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
           mbar_expect_tx(bar, (uint32_t)cfg.w_bytes);
           for (int b = 0; b * EPR < cfg.n_acc; ++b) tma_load_2d(sw + (uint32_t)(b * p.c_in) * 128u, &w_map, bar, b * EPR, k * p.c_in);
         }
+      // the CTA's shared memory outlives its copies, also after a wait that ran out
+      for (int i = max(0, n_load - cfg.n_wbuf); i < n_load; ++i)
+        mbar_parked_wait(smem_u32(&sh->w_full[cfg.n_wbuf == 2 ? i & 1 : 0]), (uint32_t)(cfg.n_wbuf == 2 ? i >> 1 : i) & 1u, nullptr);
     }
     __syncwarp();
     ok = __all_sync(0xffffffffu, ok) != 0;
@@ -249,44 +256,45 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
     const uint64_t b_desc0 = make_sdesc(smem_u32(sW), (uint32_t)p.c_in * 128u, TF32 ? 512u : 1024u, TF32 ? 1u : 2u);
     constexpr uint32_t B_KC = (uint32_t)EPR * 8u, B_KS = (32u / ES) * 8u;  // one 128-byte K chunk / 32-byte MMA step further, in 16-byte units
     // One lane, named by elect.sync (see elect_one), runs the whole loop (waits, issue, commits); the other lanes wait at the
-    // end.
+    // end.  The loop is flat and leaves no stage early: with a loop over tiles around one over chunks and a break behind every
+    // wait, 64 -> 64 on a full block of 48^3 took 77 us, flat 58, four stages unrolled 56.  After a wait that ran out the abort
+    // flag lets every other one return, and the MMAs issued meanwhile read shared memory only.
     if (elect_one()) {
       int s = 0, n_load = 0, grp = 0;
       uint32_t ph = 0;
-      for (int tb = t0; tb < t1 && ok; tb += gsz, ++grp) {
-        const int gv = min(gsz, t1 - tb);
-        for (int k = 0; k < p.k_vol && ok; ++k, ++n_load) {
+      for (int tb = t0; tb < t1; tb += gsz, ++grp) {
+        const int per_k = min(gsz, t1 - tb) * kch;
+        for (int k = 0; k < p.k_vol; ++k, ++n_load) {
           const int wb = cfg.n_wbuf == 2 ? n_load & 1 : 0;
-          ok = mbar_wait(smem_u32(&sh->w_full[wb]), (uint32_t)(cfg.n_wbuf == 2 ? n_load >> 1 : n_load) & 1u, abort_flag);
+          ok = mbar_wait(smem_u32(&sh->w_full[wb]), (uint32_t)(cfg.n_wbuf == 2 ? n_load >> 1 : n_load) & 1u, abort_flag) && ok;
           const uint64_t b_desc_w = b_desc0 + (uint64_t)((uint32_t)wb * ((uint32_t)cfg.w_bytes >> 4));
-          for (int g = 0; g < gv && ok; ++g) {
-            if (k == 0) {
+          int g = 0, kc = 0;
+          for (int r0 = 0; r0 < per_k; r0 += OS_UNROLL) {
+#pragma unroll
+            for (int u = 0; u < OS_UNROLL; ++u) {
+              if (r0 + u >= per_k) break;
               // first offset of the group: the accumulator must have been read and cleared
-              ok = mbar_wait(smem_u32(&sh->tmem_empty[g]), (uint32_t)grp & 1u, abort_flag);
-              if (!ok) break;
-              tc_fence_after();
-            }
-            const uint32_t d_tmem = tmem_base + (uint32_t)(g * cfg.n_acc);
-            for (int kc = 0; kc < kch; ++kc) {
-              ok = mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag);
-              if (!ok) break;
+              if (k == 0 && kc == 0) ok = mbar_wait(smem_u32(&sh->tmem_empty[g]), (uint32_t)grp & 1u, abort_flag) && ok;
+              ok = mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag) && ok;
               const uint4 on = sh->on[s];
               fence_proxy_async();  // the stage was written through cp.async; the MMA reads it through the async proxy
               tc_fence_after();
-              if (on.x | on.y | on.z | on.w) {
-                const uint64_t a_desc = a_desc0 + (uint64_t)((uint32_t)s * (G3_STAGE_BYTES >> 4)), b_desc = b_desc_w + (uint64_t)((uint32_t)kc * B_KC);
-                const int n_ks = min(4, (k_bytes - kc * 128) >> 5);
+              const uint32_t d_tmem = tmem_base + (uint32_t)(g * cfg.n_acc);
+              const uint64_t a_desc = a_desc0 + (uint64_t)((uint32_t)s * (G3_STAGE_BYTES >> 4)), b_desc = b_desc_w + (uint64_t)((uint32_t)kc * B_KC);
+              const int n_ks = min(4, (k_bytes - kc * 128) >> 5);
 #pragma unroll
-                for (int ks = 0; ks < 4; ++ks)
-                  if (ks < n_ks)
-                    mma_ss_masked<TF32>(d_tmem, a_desc + (uint64_t)(ks * 2), b_desc + (uint64_t)((uint32_t)ks * B_KS), idesc, ~on.x, ~on.y, ~on.z, ~on.w);
-              }
+              for (int ks = 0; ks < 4; ++ks)
+                if (ks < n_ks)
+                  mma_ss_masked<TF32>(d_tmem, a_desc + (uint64_t)(ks * 2), b_desc + (uint64_t)((uint32_t)ks * B_KS), idesc, ~on.x, ~on.y, ~on.z, ~on.w);
               mma_commit(smem_u32(&sh->empty[s]));
               if (++s == n_stage) { s = 0; ph ^= 1u; }
+              if (++kc == kch) {
+                if (k + 1 == p.k_vol) mma_commit(smem_u32(&sh->tmem_full[g]));
+                kc = 0; ++g;
+              }
             }
-            if (ok && k + 1 == p.k_vol) mma_commit(smem_u32(&sh->tmem_full[g]));
           }
-          if (ok) mma_commit(smem_u32(&sh->w_free[wb]));
+          mma_commit(smem_u32(&sh->w_free[wb]));
         }
       }
     }
