@@ -2,19 +2,24 @@
 //
 //   out[scatter[j]] += src[gather[j]] . W_k        for the pairs j of every offset k
 //
-// One persistent CTA per SM walks a contiguous range of 128-pair tiles.  Seventeen warps, three roles,
+// One persistent CTA per SM walks a contiguous range of 128-pair tiles.  Eighteen warps, four roles,
 // and the only things that cross between roles are mbarrier phases:
 //
-//   producers (8 warps)  fetch their rows' map entries straight from global memory two tiles ahead,
+//   producers (8 warps)  fetch their rows' map entries straight from global memory two tiles ahead and
 //                        gather feature rows with 16-byte cp.async into a ring of 16 KB stages (one
-//                        128-byte K chunk of 128 rows each, K-major SWIZZLE_128B) and, when the offset
-//                        changes, the next weight matrix into the other of two weight buffers;
+//                        128-byte K chunk of 128 rows each, K-major SWIZZLE_128B);
+//   weights (1 warp)     one lane loads the next offset's matrix by TMA, a box per 128-byte column block,
+//                        into the other of two buffers (one, where two do not fit);
 //   MMA warp             one lane issues tcgen05.mma per stage, commits the stage back to the producers
 //                        and the finished accumulator (two TMEM buffers) to the epilogue;
-//   epilogue (8 warps)   two warps per TMEM lane quarter, each owning half of every 256-byte block of the
-//                        output row: tcgen05.ld -> convert -> a 4 KB patch private to the warp -> 16-byte
+//   epilogue (8 warps)   tcgen05.ld -> convert -> a 4 KB patch private to the warp -> 16-byte
 //                        vector reds with consecutive lanes on consecutive addresses of one row.  The map
 //                        entries of its 32 rows come from global memory two tiles ahead as well.
+//
+// What bounds it: at many tiles a CTA what L2 gives, 5.4 TB/s of reds beside 12 TB/s of gathers (128 -> 128 on 303 k pairs
+// 23.0 us, 77 MB each way); at few the chain from kpos to the last red.  Weights by the producers' own cp.async, a nested MMA
+// loop, waits that keep issuing and one red per patch read took 24.5 us there, 256 -> 256 on 3000 / 600 voxels 14.6 / 8.9 us
+// (now 12.9 / 7.6), 96 -> 256 on 50 k pairs 12.2 (10.5), 96 -> 160 on 358 k pairs 35.4 (32.5).
 //
 // Every role recomputes the (cheap) tile bookkeeping from the tile table in shared memory, so there is
 // no index ring and no patch hand-off.  All waits are bounded; a wait that runs out sets the CTA's
@@ -42,7 +47,8 @@ constexpr int G3_MMA_WARP = 8;
 constexpr int G3_PROD_WARP0 = 9;
 constexpr int G3_PROD_WARPS = 8;
 constexpr int G3_PROD_THREADS = G3_PROD_WARPS * 32;
-constexpr int G3_THREADS = (G3_PROD_WARP0 + G3_PROD_WARPS) * 32;  // 544
+constexpr int G3_W_WARP = G3_PROD_WARP0 + G3_PROD_WARPS;
+constexpr int G3_THREADS = (G3_W_WARP + 1) * 32;  // 576
 constexpr int G3_STAGE_BYTES = 16384;
 constexpr int G3_MAX_STAGES = 8;
 constexpr int G3_PATCH_BYTES = G3_EPI_WARPS * 4096;
@@ -57,6 +63,7 @@ struct G3Shared {
   uint64_t empty[G3_MAX_STAGES];  // stage consumed (tcgen05.commit)
   uint64_t tmem_full[4];          // accumulator finished (tcgen05.commit)
   uint64_t tmem_empty[4];         // accumulator drained (one arrival per warp of the group that owns it)
+  uint64_t w_full[2];             // weight matrix landed (TMA)
   uint64_t w_free[2];             // every MMA that reads this weight buffer has finished (tcgen05.commit)
   uint32_t tmem_base;
   int abort_flag;
@@ -75,10 +82,11 @@ struct G3Config {
   int smem;     // dynamic shared memory of the launch
 };
 
-// Every lane probes the barrier itself (one broadcast read per probe, and each lane's own acquire orders its later
-// reads); one vote makes the outcome the warp's, so that a wait that ran out takes the whole warp out of its loop.
+// Every lane waits for the barrier itself (each lane's own acquire orders its later reads), parked so that it leaves the
+// other roles its issue slots (weight gradient 128 -> 128 on 303 k pairs 28.2 -> 27.0 us); one vote makes the outcome the warp's,
+// so that a wait that ran out takes the whole warp out of its loop.
 __device__ __forceinline__ bool g3_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  const bool ok = umma::mbar_wait(umma::smem_u32(bar), parity, abort_flag);
+  const bool ok = umma::mbar_parked_wait(umma::smem_u32(bar), parity, abort_flag);
   return __all_sync(0xffffffffu, ok) != 0;
 }
 
@@ -119,7 +127,7 @@ __device__ __forceinline__ int g3_widx(const G3Walk& w, const GmsParams& p) { re
 // FULL: both row lengths are whole 128-byte spans (the large-channel layers).  Every per-chunk guard below is
 // then a compile-time constant; the hot loops of that instantiation carry no test the short-row shapes need.
 template <bool TF32, bool TRANS_W, bool FULL>
-__global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G3Config cfg) {
+__global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G3Config cfg, const __grid_constant__ CUtensorMap w_map) {
   using namespace umma;
   constexpr int ES = TF32 ? 4 : 2;
   constexpr int EPR = 128 / ES;  // elements per 128-byte span
@@ -149,8 +157,10 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
       mbar_init(smem_u32(&sh->tmem_full[b]), 1);
       mbar_init(smem_u32(&sh->tmem_empty[b]), G3_EPI_WARPS / 2);
     }
-    mbar_init(smem_u32(&sh->w_free[0]), 1);
-    mbar_init(smem_u32(&sh->w_free[1]), 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&sh->w_full[b]), 1);
+      mbar_init(smem_u32(&sh->w_free[b]), 1);
+    }
     sh->abort_flag = 0;
     mbar_fence_init();
   }
@@ -178,12 +188,37 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
 
   if (t0 >= t1) {
     // nothing for this CTA
+  } else if (warp == G3_W_WARP) {
+    // ------------------------------------------------------------------ weights: a TMA box per 128-byte column block, as soon as
+    // the buffer is free (load number n goes to buffer n % n_wbuf)
+    if (elect_one()) {
+      int wb = 0, loads = 0, cur_w = -1;
+      uint32_t ph = 0;
+      for (int seg = find_segment(tile_start, n_seg, t0); seg < n_seg && tile_start[seg] < t1; ++seg) {
+        const int widx = seg == p.k_vol ? p.dense_weight : seg;
+        if (tile_start[seg + 1] <= max(tile_start[seg], t0) || widx == cur_w) continue;
+        cur_w = widx;
+        ok = mbar_parked_wait(smem_u32(&sh->w_free[wb]), ph ^ 1u, abort_flag);
+        if (!ok) break;
+        const uint32_t bar = smem_u32(&sh->w_full[wb]), sw = smem_u32(sW + (size_t)wb * cfg.w_bytes);
+        mbar_expect_tx(bar, (uint32_t)cfg.w_bytes);
+        for (int b = 0; b * p.c_in * 128 < cfg.w_bytes; ++b) tma_load_2d(sw + (uint32_t)(b * p.c_in) * 128u, &w_map, bar, b * EPR, widx * p.c_in);
+        if (loads < cfg.n_wbuf) ++loads;
+        if (++wb == cfg.n_wbuf) { wb = 0; ph ^= 1u; }
+      }
+      // the CTA's shared memory outlives its copies, also after a wait that ran out: the last load of every buffer
+      for (; loads > 0; --loads) {
+        if (--wb < 0) { wb = cfg.n_wbuf - 1; ph ^= 1u; }
+        mbar_parked_wait(smem_u32(&sh->w_full[wb]), ph, nullptr);
+      }
+    }
+    __syncwarp();
+    ok = __all_sync(0xffffffffu, ok) != 0;
   } else if (warp >= G3_PROD_WARP0) {
     // ------------------------------------------------------------------ producers
     // Warp pw owns tile rows [16 pw, 16 pw + 16).  Lanes 0-15 fetch those rows' gather entries, lanes
     // 16-31 their scatter entries (needed to skip pairs whose destination is outside the tensor).
     const int pw = warp - G3_PROD_WARP0;
-    const int tp = tid - G3_PROD_WARP0 * 32;
     // `lpr` lanes share a row, one 16-byte chunk each: 8 for rows of a whole span or more, 4 / 2 for 64- /
     // 32-byte rows, so that short rows still keep every lane busy.  This thread copies chunk pc of the rows
     // 16 pw + rsub + rpp j, j < n_pass.
@@ -191,9 +226,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
     const int rpp = 32 / lpr, n_pass = FULL ? 4 : 16 / rpp;  // rows per warp-wide copy: 4 / 8 / 16; copies per tile: 4 / 2 / 1
     const int pc = lane % lpr, rsub = lane / lpr;
     const uint8_t* src = static_cast<const uint8_t*>(p.src);
-    const uint8_t* wts = static_cast<const uint8_t*>(p.weights);
     const size_t src_row_bytes = (size_t)k_bytes;
-    const uint32_t w_row_bytes = (uint32_t)p.c_out * ES;
     uint32_t a_dst[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -208,37 +241,8 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
       if (row < ti.cnt && !ti.dense) cp_async4(dst, (lane < 16 ? p.gather_map : p.scatter_map) + ti.base + row);
       else st_shared_i32(dst, row < ti.cnt ? ti.base + row : -1);
     };
-    // Weight matrix -> operand layout.  The matrix is `w_rows` rows of `cpr` 16-byte chunks; when cpr divides the
-    // number of producer threads every thread keeps one chunk column and strides over rows (no division in the loop).
-    const int w_rows = p.c_in;             // rows of W_k in global memory: n_dim of them for dgrad, k_dim for forward
-    const int cpr = p.c_out * ES / 16;     // 16-byte chunks per row
-    const bool cpr_divides = (G3_PROD_THREADS % cpr) == 0;
-    const uint32_t w_c = cpr_divides ? (uint32_t)(tp % cpr) : 0u;
-    const int w_r0 = cpr_divides ? tp / cpr : 0, w_rstep = cpr_divides ? G3_PROD_THREADS / cpr : 0;
-    const uint32_t w_lbo = (uint32_t)p.k_dim * 128u;
-    auto w_offset = [&](uint32_t row, uint32_t c) -> uint32_t {
-      if (TRANS_W) return kmajor_offset(row, c * 16u, p.n_dim);  // rows = output index: K-major operand
-      return TF32 ? mnmajor32_offset(row, c * 16u, w_lbo, 512u) : mnmajor_offset(row, c * 16u, w_lbo, 1024u);  // rows = contraction index: MN-major
-    };
-    auto load_weights = [&](int widx, int wb) {
-      const uint8_t* wk = wts + (size_t)widx * p.c_in * p.c_out * ES;
-      const uint32_t sw = smem_u32(sW + (size_t)wb * cfg.w_bytes);
-      if (cpr_divides) {
-        const uint8_t* col = wk + w_c * 16u;
-        for (int row = w_r0; row < w_rows; row += w_rstep)
-          cp_async16(sw + w_offset((uint32_t)row, w_c), col + (size_t)row * w_row_bytes, true);
-      } else {
-        const int total = w_rows * cpr;
-        for (int e = tp; e < total; e += G3_PROD_THREADS) {
-          const uint32_t row = e / cpr, c = e % cpr;
-          cp_async16(sw + w_offset(row, c), wk + (size_t)row * w_row_bytes + c * 16u, true);
-        }
-      }
-    };
-
-    G3Walk cur, pf;
-    cur.init(tile_start, n_seg, t0);
-    pf = cur;
+    G3Walk pf;
+    pf.init(tile_start, n_seg, t0);
     fetch_entry(pf, 0);
     cp_async_commit();
     pf.next(tile_start, n_seg);
@@ -247,27 +251,11 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
     pf.next(tile_start, n_seg);
     int s = 0;
     uint32_t ph = 0;          // stage and its phase
-    int cur_w = -1, n_load = -1, wb = 0;
 
     for (int t = t0; t < t1 && ok; ++t) {
       if (pf.t < t1) fetch_entry(pf, (t - t0 + 2) & (G3_RING_SLOTS - 1));
       cp_async_commit();  // also closes the group of the previous tile's gathers
       pf.next(tile_start, n_seg);
-      const G3Tile ti = g3_tile(cur, p, kpos_s);
-      if (ti.widx != cur_w) {
-        // weight load number n_load goes to buffer n_load % n_wbuf, whose previous tenant was load
-        // n_load - n_wbuf: wait until the MMA warp has reported that tenant's last MMA finished
-        ++n_load;
-        wb = (cfg.n_wbuf == 2) ? (n_load & 1) : 0;
-        if (n_load >= cfg.n_wbuf) {
-          const uint32_t use = (uint32_t)(cfg.n_wbuf == 2 ? (n_load >> 1) : n_load) - 1u;
-          ok = g3_wait(&sh->w_free[wb], use & 1u, abort_flag);
-          if (!ok) break;
-        }
-        cur_w = ti.widx;
-        // issued before the wait for this tile's map entries; the first stage's barrier below also covers these copies
-        load_weights(ti.widx, wb);
-      }
       cp_async_wait<2>();  // everything older than the last two groups has landed: this tile's entries have
       const int e0 = ld_shared_i32(ring + (uint32_t)((t - t0) & (G3_RING_SLOTS - 1)) * 128u);
       // lanes 0-15 hold gather entries, lanes 16-31 the scatter entries of the same rows: settle once per
@@ -298,7 +286,6 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
         cp_async_arrive_noinc(smem_u32(&sh->full[s]));
         if (++s == n_stage) { s = 0; ph ^= 1u; }
       }
-      cur.next(tile_start, n_seg);
     }
   } else if (warp == G3_MMA_WARP) {
     // ------------------------------------------------------------------ MMA issuer
@@ -314,52 +301,51 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
     const uint32_t b_ks_step = TRANS_W ? 2u : (32u / ES) * 8u;                          // one 32-byte MMA step further
     G3Walk cur;
     cur.init(tile_start, n_seg, t0);
-    int s = 0;
-    uint32_t ph = 0;
-    int cur_w = -1, n_load = -1, wb = 0, tile_i = 0;
     // One lane, named by elect.sync (see elect_one), runs the whole loop — waits, issue, commits — so that no warp-wide
-    // hand-shake sits between a stage landing and its MMAs; the other lanes wait at the end.
-    // 128 -> 128 on 303 k pairs, forward + dgrad + weight gradient: 92 -> 86 us; 96 -> 160 on 321 k pairs 39.2 -> 36.6.
-    if (elect_one())
-    for (int t = t0; t < t1 && ok; ++t, ++tile_i) {
-      const int buf = tile_i & (cfg.n_tbuf - 1);
-      const uint32_t use = (uint32_t)tile_i >> cfg.tbuf_shift;
-      const int widx = g3_widx(cur, p);
-      if (widx != cur_w) {  // same numbering of weight loads as in the producers
-        ++n_load;
-        wb = (cfg.n_wbuf == 2) ? (n_load & 1) : 0;
-        cur_w = widx;
-      }
-      cur.next(tile_start, n_seg);
-      const bool last_of_w = (t + 1 == t1) || g3_widx(cur, p) != cur_w;
-      ok = mbar_wait(smem_u32(&sh->tmem_empty[buf]), (use & 1u) ^ 1u, abort_flag);
-      if (!ok) break;
-      tc_fence_after();
-      const uint32_t d_tmem = tmem_base + (uint32_t)(buf * cfg.n_acc);
-      const uint64_t b_desc_w = b_desc0 + (uint64_t)((uint32_t)wb * ((uint32_t)cfg.w_bytes >> 4));
-      for (int kc = 0; kc < kch && ok; ++kc) {
-        ok = mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag);
-        if (!ok) break;
-        {
-          fence_proxy_async();  // the stage was written through cp.async; the MMA reads it through the async proxy
-          tc_fence_after();
-          const uint64_t a_desc_s = a_desc0 + (uint64_t)((uint32_t)s * (G3_STAGE_BYTES >> 4));
-          const uint64_t b_desc_kc = b_desc_w + (uint64_t)((uint32_t)kc * b_kc_step);
-          const int n_ks = FULL ? 4 : min(4, (k_bytes - kc * 128) >> 5);  // 32-byte MMA steps this chunk holds
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks) {
-            if (!FULL && ks >= n_ks) break;
-            // A (K-major): 32 bytes further along the row per step.  B: MN-major (forward) steps 32 / ES rows of
-            // 128 bytes, K-major (dgrad) 32 bytes along the row.
-            mma_ss<TF32>(d_tmem, a_desc_s + (uint64_t)(ks * 2), b_desc_kc + (uint64_t)((uint32_t)ks * b_ks_step), idesc, (kc | ks) != 0);
+    // hand-shake sits between a stage landing and its MMAs; the other lanes wait at the end.  The loop goes over stages and is
+    // not left early: branches are what it spends its time on (see umma_osfwd.cuh).  After a wait that ran out the abort
+    // flag lets every other one return, and the MMAs issued meanwhile read shared memory only.
+    if (elect_one()) {
+      int s = 0, kc = 0, cur_w = -1, wb = cfg.n_wbuf - 1, buf = 0;
+      uint32_t ph = 0, w_ph = 1, use = 0, d_tmem = 0;
+      bool last_of_w = false;
+      uint64_t b_desc_w = 0;
+      const int n = (t1 - t0) * kch;
+      for (int i = 0; i < n; ++i) {
+        if (kc == 0) {
+          const int widx = g3_widx(cur, p);
+          if (widx != cur_w) {
+            cur_w = widx;
+            if (++wb == cfg.n_wbuf) { wb = 0; w_ph ^= 1u; }
+            ok = mbar_wait(smem_u32(&sh->w_full[wb]), w_ph, abort_flag) && ok;
+            b_desc_w = b_desc0 + (uint64_t)((uint32_t)wb * ((uint32_t)cfg.w_bytes >> 4));
           }
-          mma_commit(smem_u32(&sh->empty[s]));
-          if (kc == kch - 1) {
-            mma_commit(smem_u32(&sh->tmem_full[buf]));
-            if (last_of_w) mma_commit(smem_u32(&sh->w_free[wb]));
-          }
+          cur.next(tile_start, n_seg);
+          last_of_w = i + kch >= n || g3_widx(cur, p) != cur_w;
+          ok = mbar_wait(smem_u32(&sh->tmem_empty[buf]), use ^ 1u, abort_flag) && ok;
+          d_tmem = tmem_base + (uint32_t)(buf * cfg.n_acc);
         }
+        ok = mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag) && ok;
+        fence_proxy_async();  // the stage was written through cp.async; the MMA reads it through the async proxy
+        tc_fence_after();
+        const uint64_t a_desc_s = a_desc0 + (uint64_t)((uint32_t)s * (G3_STAGE_BYTES >> 4));
+        const uint64_t b_desc_kc = b_desc_w + (uint64_t)((uint32_t)kc * b_kc_step);
+        const int n_ks = FULL ? 4 : min(4, (k_bytes - kc * 128) >> 5);  // 32-byte MMA steps this chunk holds
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          // A (K-major): 32 bytes further along the row per step.  B: MN-major (forward) steps 32 / ES rows of
+          // 128 bytes, K-major (dgrad) 32 bytes along the row.
+          if (FULL || ks < n_ks)
+            mma_ss<TF32>(d_tmem, a_desc_s + (uint64_t)(ks * 2), b_desc_kc + (uint64_t)((uint32_t)ks * b_ks_step), idesc, (kc | ks) != 0);
+        }
+        mma_commit(smem_u32(&sh->empty[s]));
         if (++s == n_stage) { s = 0; ph ^= 1u; }
+        if (++kc == kch) {
+          mma_commit(smem_u32(&sh->tmem_full[buf]));
+          if (last_of_w) mma_commit(smem_u32(&sh->w_free[wb]));
+          kc = 0;
+          if (++buf == cfg.n_tbuf) { buf = 0; use ^= 1u; }
+        }
       }
     }
     __syncwarp();
@@ -367,7 +353,8 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
   } else {
     // ------------------------------------------------------------------ epilogue (warps 0-7)
     // Two groups of four warps take alternate tiles, so that one group's TMEM reads and conversions run
-    // while the other group's reds drain.  Warp q of a group owns TMEM lanes 32 q .. 32 q + 31 (a warp
+    // while the other group's reds drain.  (Blocks of columns instead of tiles: 256 -> 256 on 3000 voxels 12.4 us against
+    // 12.9, but 128 -> 128 on 303 k pairs 25.7 against 23.0.)  Warp q of a group owns TMEM lanes 32 q .. 32 q + 31 (a warp
     // may only read the lane quarter given by its index mod 4), i.e. tile rows 32 q .. 32 q + 31, and
     // walks the output row in 128-byte blocks: tcgen05.ld -> convert -> private patch -> reds.
     const int grp = warp >> 2, q4 = warp & 3;
@@ -454,16 +441,24 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
           __syncwarp();
           uint8_t* dcol = dst + cb + (ch << 4);
           const bool ch_ok = FULL || (ch << 4) < vb;
+          // 32 rows = lpe passes of rpe rows, four passes' pieces read before the first of their reds
 #pragma unroll
-          for (uint32_t u = 0; u < 8; ++u) {
-            if (!FULL && u >= lpe) break;  // 32 rows = lpe passes of rpe rows
-            const uint32_t r = rsub + rpe * u;
-            const int sr = __shfl_sync(0xffffffffu, srow, r);
-            const uint4 v = *reinterpret_cast<const uint4*>(patch + r * 128 + ((ch ^ (r & 7)) << 4));
-            if (sr >= 0 && ch_ok) {
-              uint8_t* o = dcol + (size_t)sr * row_bytes;
-              if (TF32) red_add_v4(reinterpret_cast<float*>(o), __uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
-              else red_add_h8(reinterpret_cast<__half*>(o), v.x, v.y, v.z, v.w);
+          for (uint32_t u0 = 0; u0 < 8; u0 += 4) {
+            if (!FULL && u0 >= lpe) break;
+            uint4 v[4];
+            int sr[4];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) {
+              const uint32_t r = (rsub + rpe * (u0 + u)) & 31u;
+              sr[u] = __shfl_sync(0xffffffffu, srow, r);
+              v[u] = *reinterpret_cast<const uint4*>(patch + r * 128 + ((ch ^ (r & 7)) << 4));
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) {
+              if (sr[u] < 0 || !ch_ok || (!FULL && u0 + u >= lpe)) continue;
+              uint8_t* o = dcol + (size_t)sr[u] * row_bytes;
+              if (TF32) red_add_v4(reinterpret_cast<float*>(o), __uint_as_float(v[u].x), __uint_as_float(v[u].y), __uint_as_float(v[u].z), __uint_as_float(v[u].w));
+              else red_add_h8(reinterpret_cast<__half*>(o), v[u].x, v[u].y, v[u].z, v[u].w);
             }
           }
           __syncwarp();
@@ -510,7 +505,9 @@ template <bool TF32, bool TRANS_W, bool FULL>
 inline int g3_launch_as(const GmsParams& p, const G3Config& cfg, cudaStream_t st, int sms, int max_smem) {
   static std::atomic<int> granted[64];
   if (int rc = ensure_smem(umma_gms3_kernel<TF32, TRANS_W, FULL>, max_smem, granted)) return rc;
-  return launch_pdl(umma_gms3_kernel<TF32, TRANS_W, FULL>, sms, G3_THREADS, (size_t)cfg.smem, st, p, cfg) == cudaSuccess ? 0 : -1;
+  CUtensorMap w_map;
+  if (!weight_tensor_map(&w_map, p.weights, p.k_vol, p.c_in, p.c_out, !TF32, !TRANS_W)) return -1;
+  return launch_pdl(umma_gms3_kernel<TF32, TRANS_W, FULL>, sms, G3_THREADS, (size_t)cfg.smem, st, p, cfg, w_map) == cudaSuccess ? 0 : -1;
 }
 template <bool TF32, bool TRANS_W>
 inline int g3_launch(const GmsParams& p, const G3Config& cfg, cudaStream_t st, int sms, int max_smem) {

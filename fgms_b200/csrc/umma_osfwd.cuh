@@ -76,11 +76,6 @@ struct OsShared {
 };
 constexpr int OS_SHARED_BYTES = (sizeof(OsShared) + 15) & ~15;
 
-__device__ __forceinline__ bool os_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  const bool ok = umma::mbar_parked_wait(umma::smem_u32(bar), parity, abort_flag);
-  return __all_sync(0xffffffffu, ok) != 0;
-}
-
 // nbr[k][out_map[j]] = in_map[j] for every pair j of offset k (the table is filled with -1 beforehand).  Every kpos
 // entry is clamped to [0, map_len]; a pair with an entry outside the tensors is skipped and counted.
 __global__ void os_fill_nbr_kernel(const int32_t* __restrict__ kpos, const int32_t* __restrict__ in_map,
@@ -195,7 +190,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
       if (first < n) load_entries(e);
       for (int i = first; i < n; i += nw) {
         const int kc = r - (int)((uint32_t)r * kch_recip >> 16) * kch;
-        ok = os_wait(&sh->empty[s], ph ^ 1u, abort_flag);
+        ok = g3_wait(&sh->empty[s], ph ^ 1u, abort_flag);
         if (!ok) break;
         int ent[4];
         uint32_t on[4];
@@ -321,7 +316,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
     for (int tb = t0; tb < t1 && ok; tb += gsz, ++grp_i) {
       const int gv = min(gsz, t1 - tb);
       for (int g = 0; g < gv && ok; ++g) {
-        ok = os_wait(&sh->tmem_full[g], (uint32_t)grp_i & 1u, abort_flag);
+        ok = g3_wait(&sh->tmem_full[g], (uint32_t)grp_i & 1u, abort_flag);
         if (!ok) break;
         tc_fence_after();
         const int row0 = (tb + g) * OS_TILE + 32 * warp;  // output row of this warp's lane 0
@@ -443,7 +438,7 @@ inline int launch_umma_osfwd(const OsParams& p, bool f16, cudaStream_t st, int s
   const int grid = p.n_tiles < sms ? p.n_tiles : sms;
   if (grid <= 0) return 0;
   CUtensorMap w_map;
-  if (!weight_tensor_map(&w_map, p.weights, p.k_vol, p.c_in, p.c_out, f16)) return -1;
+  if (!weight_tensor_map(&w_map, p.weights, p.k_vol, p.c_in, p.c_out, f16, true)) return -1;
   if (f16) {
     static std::atomic<int> granted[64];
     if (int rc = ensure_smem(umma_osfwd_kernel<false>, max_smem, granted)) return rc;
