@@ -255,41 +255,61 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
     // wait, 64 -> 64 on a full block of 48^3 took 77 us, flat 58, four stages unrolled 56.  After a wait that ran out the abort
     // flag lets every other one return, and the MMAs issued meanwhile read shared memory only.
     if (elect_one()) {
-      int s = 0, n_load = 0, grp = 0;
-      uint32_t ph = 0;
+      int s = 0, wb = 0, grp = 0, g = 0, kc = 0;  // ring slot, weight buffer, group; tile of the group, chunk of its row
+      uint32_t ph = 0, w_ph = 0;
+      auto take_weights = [&]() { ok = mbar_wait(smem_u32(&sh->w_full[wb]), w_ph, abort_flag) && ok; };
+      auto free_weights = [&]() {
+        mma_commit(smem_u32(&sh->w_free[wb]));
+        if (++wb == cfg.n_wbuf) { wb = 0; w_ph ^= 1u; }
+        g = 0;
+      };
+      auto stage = [&](bool first_k, bool last_k) {
+        // first offset of the group: the accumulator must have been read and cleared
+        if (first_k && kc == 0) ok = mbar_wait(smem_u32(&sh->tmem_empty[g]), (uint32_t)grp & 1u, abort_flag) && ok;
+        ok = mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag) && ok;
+        const uint4 on = sh->on[s];
+        fence_proxy_async();  // the stage was written through cp.async; the MMA reads it through the async proxy
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + (uint32_t)(g * cfg.n_acc);
+        const uint64_t a_desc = a_desc0 + (uint64_t)((uint32_t)s * (G3_STAGE_BYTES >> 4));
+        const uint64_t b_desc = b_desc0 + (uint64_t)((uint32_t)wb * ((uint32_t)cfg.w_bytes >> 4) + (uint32_t)kc * B_KC);
+        const int n_ks = min(4, (k_bytes - kc * 128) >> 5);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+          if (ks < n_ks)
+            mma_ss_masked<TF32>(d_tmem, a_desc + (uint64_t)(ks * 2), b_desc + (uint64_t)((uint32_t)ks * B_KS), idesc, ~on.x, ~on.y, ~on.z, ~on.w);
+        mma_commit(smem_u32(&sh->empty[s]));
+        if (++s == n_stage) { s = 0; ph ^= 1u; }
+        if (++kc == kch) {
+          if (last_k) mma_commit(smem_u32(&sh->tmem_full[g]));
+          kc = 0; ++g;
+        }
+      };
       for (int tb = t0; tb < t1; tb += gsz, ++grp) {
         const int per_k = min(gsz, t1 - tb) * kch;
-        for (int k = 0; k < p.k_vol; ++k, ++n_load) {
-          const int wb = cfg.n_wbuf == 2 ? n_load & 1 : 0;
-          ok = mbar_wait(smem_u32(&sh->w_full[wb]), (uint32_t)(cfg.n_wbuf == 2 ? n_load >> 1 : n_load) & 1u, abort_flag) && ok;
-          const uint64_t b_desc_w = b_desc0 + (uint64_t)((uint32_t)wb * ((uint32_t)cfg.w_bytes >> 4));
-          int g = 0, kc = 0;
-          for (int r0 = 0; r0 < per_k; r0 += OS_UNROLL) {
+        if (per_k == 1) {
+          // a single stage per offset: one loop over the offsets (1000 voxels 64 -> 64 15.3 us, 17.7 with a loop inside it)
+          for (int k0 = 0; k0 < p.k_vol; k0 += OS_UNROLL) {
 #pragma unroll
             for (int u = 0; u < OS_UNROLL; ++u) {
-              if (r0 + u >= per_k) break;
-              // first offset of the group: the accumulator must have been read and cleared
-              if (k == 0 && kc == 0) ok = mbar_wait(smem_u32(&sh->tmem_empty[g]), (uint32_t)grp & 1u, abort_flag) && ok;
-              ok = mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag) && ok;
-              const uint4 on = sh->on[s];
-              fence_proxy_async();  // the stage was written through cp.async; the MMA reads it through the async proxy
-              tc_fence_after();
-              const uint32_t d_tmem = tmem_base + (uint32_t)(g * cfg.n_acc);
-              const uint64_t a_desc = a_desc0 + (uint64_t)((uint32_t)s * (G3_STAGE_BYTES >> 4)), b_desc = b_desc_w + (uint64_t)((uint32_t)kc * B_KC);
-              const int n_ks = min(4, (k_bytes - kc * 128) >> 5);
-#pragma unroll
-              for (int ks = 0; ks < 4; ++ks)
-                if (ks < n_ks)
-                  mma_ss_masked<TF32>(d_tmem, a_desc + (uint64_t)(ks * 2), b_desc + (uint64_t)((uint32_t)ks * B_KS), idesc, ~on.x, ~on.y, ~on.z, ~on.w);
-              mma_commit(smem_u32(&sh->empty[s]));
-              if (++s == n_stage) { s = 0; ph ^= 1u; }
-              if (++kc == kch) {
-                if (k + 1 == p.k_vol) mma_commit(smem_u32(&sh->tmem_full[g]));
-                kc = 0; ++g;
-              }
+              if (k0 + u >= p.k_vol) break;
+              take_weights();
+              stage(k0 + u == 0, k0 + u + 1 == p.k_vol);
+              free_weights();
             }
           }
-          mma_commit(smem_u32(&sh->w_free[wb]));
+        } else {
+          for (int k = 0; k < p.k_vol; ++k) {
+            take_weights();
+            for (int r0 = 0; r0 < per_k; r0 += OS_UNROLL) {
+#pragma unroll
+              for (int u = 0; u < OS_UNROLL; ++u) {
+                if (r0 + u >= per_k) break;
+                stage(k == 0, k + 1 == p.k_vol);
+              }
+            }
+            free_weights();
+          }
         }
       }
     }
