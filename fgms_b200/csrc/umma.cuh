@@ -274,7 +274,8 @@ __host__ __device__ constexpr uint32_t mnmajor32_offset(uint32_t k, uint32_t byt
 // Tensor map over weights [k_vol, c_in, c_out] whose box is one 128-byte column block of one matrix: what tma_load_2d writes,
 // block after block c_in * 128 bytes apart, is the 128-byte-swizzled operand: MN-major (forward: rows = contraction index) or
 // K-major (input gradient: rows = output index), which differ only for 32-bit elements.  Columns beyond c_out come as zeros.
-// Made for every call (42 ns): nothing is kept by an address.
+// Made for every call (42 ns): nothing is kept by an address.  The encoder wants a context, which a host thread has after its first
+// launch and not after cudaGetDevice: where it finds none, the current device's is made the thread's and the encoder asked again.
 inline bool weight_tensor_map(CUtensorMap* map, const void* weights, int k_vol, int c_in, int c_out, bool f16, bool mn_major) {
   using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                               const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -288,9 +289,17 @@ inline bool weight_tensor_map(CUtensorMap* map, const void* weights, int k_vol, 
   const int es = f16 ? 2 : 4;
   const cuuint64_t dims[2] = {(cuuint64_t)c_out, (cuuint64_t)k_vol * c_in}, pitch[1] = {(cuuint64_t)c_out * es};
   const cuuint32_t box[2] = {(cuuint32_t)(128 / es), (cuuint32_t)c_in}, steps[2] = {1, 1};
-  return encode(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(weights), dims, pitch, box, steps,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, f16 || !mn_major ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B,
-                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  auto made = [&] {
+    return encode(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(weights), dims, pitch, box, steps,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, f16 || !mn_major ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult rc = made();
+  if (rc == CUDA_ERROR_INVALID_CONTEXT) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) rc = made();
+  }
+  return rc == CUDA_SUCCESS;
 }
 
 // Launch with the programmatic-stream-serialization attribute.
