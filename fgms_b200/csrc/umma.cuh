@@ -276,16 +276,20 @@ __host__ __device__ constexpr uint32_t mnmajor32_offset(uint32_t k, uint32_t byt
 // K-major (input gradient: rows = output index), which differ only for 32-bit elements.  Columns beyond c_out come as zeros.
 // Made for every call (42 ns): nothing is kept by an address.  The encoder wants a context, which a host thread has after its first
 // launch and not after cudaGetDevice: where it finds none, the current device's is made the thread's and the encoder asked again.
-inline bool weight_tensor_map(CUtensorMap* map, const void* weights, int k_vol, int c_in, int c_out, bool f16, bool mn_major) {
+// Returns 0, or -1000 less the driver's status.  An encoder that was not found is looked up again by the next call.
+inline int weight_tensor_map(CUtensorMap* map, const void* weights, int k_vol, int c_in, int c_out, bool f16, bool mn_major) {
   using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                               const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static const Encode encode = [] {
+  static std::atomic<Encode> known{nullptr};
+  Encode encode = known.load(std::memory_order_acquire);
+  if (encode == nullptr) {
     void* fn = nullptr;
-    cudaDriverEntryPointQueryResult found;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) fn = nullptr;
-    return reinterpret_cast<Encode>(fn);
-  }();
-  if (encode == nullptr) return false;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    const cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found);
+    if (e != cudaSuccess || found != cudaDriverEntryPointSuccess || fn == nullptr) return -1000 - (int)CUDA_ERROR_NOT_FOUND;
+    encode = reinterpret_cast<Encode>(fn);
+    known.store(encode, std::memory_order_release);
+  }
   const int es = f16 ? 2 : 4;
   const cuuint64_t dims[2] = {(cuuint64_t)c_out, (cuuint64_t)k_vol * c_in}, pitch[1] = {(cuuint64_t)c_out * es};
   const cuuint32_t box[2] = {(cuuint32_t)(128 / es), (cuuint32_t)c_in}, steps[2] = {1, 1};
@@ -299,7 +303,7 @@ inline bool weight_tensor_map(CUtensorMap* map, const void* weights, int k_vol, 
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) rc = made();
   }
-  return rc == CUDA_SUCCESS;
+  return rc == CUDA_SUCCESS ? 0 : -1000 - (int)rc;
 }
 
 // Launch with the programmatic-stream-serialization attribute.

@@ -506,7 +506,7 @@ inline int g3_launch_as(const GmsParams& p, const G3Config& cfg, cudaStream_t st
   static std::atomic<int> granted[64];
   if (int rc = ensure_smem(umma_gms3_kernel<TF32, TRANS_W, FULL>, max_smem, granted)) return rc;
   CUtensorMap w_map;
-  if (!weight_tensor_map(&w_map, p.weights, p.k_vol, p.c_in, p.c_out, !TF32, !TRANS_W)) return -1;
+  if (int rc = weight_tensor_map(&w_map, p.weights, p.k_vol, p.c_in, p.c_out, !TF32, !TRANS_W)) return rc;
   return launch_pdl(umma_gms3_kernel<TF32, TRANS_W, FULL>, sms, G3_THREADS, (size_t)cfg.smem, st, p, cfg, w_map) == cudaSuccess ? 0 : -1;
 }
 template <bool TF32, bool TRANS_W>

@@ -458,7 +458,7 @@ inline int launch_umma_osfwd(const OsParams& p, bool f16, cudaStream_t st, int s
   const int grid = p.n_tiles < sms ? p.n_tiles : sms;
   if (grid <= 0) return 0;
   CUtensorMap w_map;
-  if (!weight_tensor_map(&w_map, p.weights, p.k_vol, p.c_in, p.c_out, f16, true)) return -1;
+  if (int rc = weight_tensor_map(&w_map, p.weights, p.k_vol, p.c_in, p.c_out, f16, true)) return rc;
   if (f16) {
     static std::atomic<int> granted[64];
     if (int rc = ensure_smem(umma_osfwd_kernel<false>, max_smem, granted)) return rc;
