@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
   using namespace umma;
   constexpr int ES = TF32 ? 4 : 2;
   constexpr int EPR = 128 / ES;  // elements per 128-byte span
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(16) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* sW = smem;                                      // n_wbuf weight operands
   uint8_t* sStage = sW + (size_t)cfg.n_wbuf * cfg.w_bytes;  // gather ring
@@ -491,7 +491,8 @@ inline bool g3_plan(int c_in, int c_out, int es, int k_vol, int max_smem, bool t
   cfg->n_tbuf = (4 * cfg->n_acc <= 512) ? 4 : 2;
   cfg->tbuf_shift = cfg->n_tbuf == 4 ? 2 : 1;
   const int table = ((2 * k_vol + 3) * 4 + 15) & ~15;
-  const int fixed = 1024 + G3_PATCH_BYTES + G3_RING_BYTES + G3_SHARED_BYTES + table;
+  // 1008: what rounding a 16-byte-aligned base up to a multiple of 1024 can take
+  const int fixed = 1008 + G3_PATCH_BYTES + G3_RING_BYTES + G3_SHARED_BYTES + table;
   // two weight buffers if at least four gather stages still fit beside them
   cfg->n_wbuf = (fixed + 2 * cfg->w_bytes + 4 * G3_STAGE_BYTES <= max_smem) ? 2 : 1;
   cfg->n_stage = (max_smem - fixed - cfg->n_wbuf * cfg->w_bytes) / G3_STAGE_BYTES;
