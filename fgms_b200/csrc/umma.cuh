@@ -64,17 +64,17 @@ __device__ __forceinline__ bool mbar_park(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait: gives up after about one second of SM clock.  `abort_flag` (shared memory) lets one
+// Bounded wait: gives up after about one second of SM clock, or `limit` cycles of it.  `abort_flag` (shared memory) lets one
 // role tell the others to stop waiting once something has gone wrong.
 constexpr long long WAIT_LIMIT_CYCLES = 2000000000ll;
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, long long limit = WAIT_LIMIT_CYCLES) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long start = clock64();
   for (uint32_t it = 1;; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 255u) == 0) {
       if (abort_flag && *abort_flag) return false;
-      if (clock64() - start > WAIT_LIMIT_CYCLES) break;
+      if (clock64() - start > limit) break;
     }
   }
   if (abort_flag) *abort_flag = 1;
@@ -218,6 +218,13 @@ __device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// the issuing lane, behind its last MMA: returns when the tensor cores are done with shared and tensor memory, whatever became
+// of the roles that would have waited for it (a barrier of its own, in its first phase)
+__device__ __forceinline__ void mma_drain(uint32_t bar) {
+  mma_commit(bar);
+  mbar_wait(bar, 0u, nullptr);
+}
 
 // ------------------------------------------------------------------ descriptors
 // Instruction descriptor of tcgen05.mma kind::f16 / kind::tf32 with fp32 accumulation:

@@ -23,7 +23,8 @@
 //
 // Every role recomputes the (cheap) tile bookkeeping from the tile table in shared memory, so there is
 // no index ring and no patch hand-off.  All waits are bounded; a wait that runs out sets the CTA's
-// abort flag, every role leaves its loop, in-flight copies are awaited and TMEM is freed.
+// abort flag, every role leaves its loop without handing on what it has not got, in-flight copies and MMAs are awaited and
+// TMEM is freed: a tile whose rows did not land is missing from the output, not wrong in it.
 #pragma once
 #include <atomic>
 
@@ -65,6 +66,7 @@ struct G3Shared {
   uint64_t tmem_empty[4];         // accumulator drained (one arrival per warp of the group that owns it)
   uint64_t w_full[2];             // weight matrix landed (TMA)
   uint64_t w_free[2];             // every MMA that reads this weight buffer has finished (tcgen05.commit)
+  uint64_t drained;               // every MMA has finished (tcgen05.commit)
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -80,6 +82,7 @@ struct G3Config {
   int n_acc;    // TMEM columns per accumulator: n_dim rounded up to whole 128-byte blocks of the output row
   int n_mma;    // N of the MMA: n_acc for the MN-major weight operand (forward), n_dim for the K-major one (dgrad)
   int smem;     // dynamic shared memory of the launch
+  long long w_limit;  // cycles the MMA lane waits for a weight matrix before it gives up (for anything else: about a second)
 };
 
 // Every lane waits for the barrier itself (each lane's own acquire orders its later reads), parked so that it leaves the
@@ -161,6 +164,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
       mbar_init(smem_u32(&sh->w_full[b]), 1);
       mbar_init(smem_u32(&sh->w_free[b]), 1);
     }
+    mbar_init(smem_u32(&sh->drained), 1);
     sh->abort_flag = 0;
     mbar_fence_init();
   }
@@ -302,9 +306,10 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
     G3Walk cur;
     cur.init(tile_start, n_seg, t0);
     // One lane, named by elect.sync (see elect_one), runs the whole loop — waits, issue, commits — so that no warp-wide
-    // hand-shake sits between a stage landing and its MMAs; the other lanes wait at the end.  The loop goes over stages and is
-    // not left early: branches are what it spends its time on (see umma_osfwd.cuh).  After a wait that ran out the abort
-    // flag lets every other one return, and the MMAs issued meanwhile read shared memory only.
+    // hand-shake sits between a stage landing and its MMAs; the other lanes wait at the end.  The loop goes over stages and has
+    // one way out, behind a stage's last wait: branches are what it spends its time on (see umma_osfwd.cuh).  Once a wait has run
+    // out nothing is issued or committed: no accumulator whose rows or weights did not land reaches the epilogue, and no stage or
+    // buffer is handed back that is still being filled.
     if (elect_one()) {
       int s = 0, kc = 0, cur_w = -1, wb = cfg.n_wbuf - 1, buf = 0;
       uint32_t ph = 0, w_ph = 1, use = 0, d_tmem = 0;
@@ -317,7 +322,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
           if (widx != cur_w) {
             cur_w = widx;
             if (++wb == cfg.n_wbuf) { wb = 0; w_ph ^= 1u; }
-            ok = mbar_wait(smem_u32(&sh->w_full[wb]), w_ph, abort_flag) && ok;
+            ok = mbar_wait(smem_u32(&sh->w_full[wb]), w_ph, abort_flag, cfg.w_limit) && ok;
             b_desc_w = b_desc0 + (uint64_t)((uint32_t)wb * ((uint32_t)cfg.w_bytes >> 4));
           }
           cur.next(tile_start, n_seg);
@@ -326,6 +331,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
           d_tmem = tmem_base + (uint32_t)(buf * cfg.n_acc);
         }
         ok = mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag) && ok;
+        if (!ok) break;
         fence_proxy_async();  // the stage was written through cp.async; the MMA reads it through the async proxy
         tc_fence_after();
         const uint64_t a_desc_s = a_desc0 + (uint64_t)((uint32_t)s * (G3_STAGE_BYTES >> 4));
@@ -347,6 +353,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
           if (++buf == cfg.n_tbuf) { buf = 0; use ^= 1u; }
         }
       }
+      mma_drain(smem_u32(&sh->drained));
     }
     __syncwarp();
     ok = __all_sync(0xffffffffu, ok) != 0;
@@ -499,6 +506,7 @@ inline bool g3_plan(int c_in, int c_out, int es, int k_vol, int max_smem, bool t
   if (cfg->n_stage > G3_MAX_STAGES) cfg->n_stage = G3_MAX_STAGES;
   if (cfg->n_stage < 2) return false;
   cfg->smem = fixed + cfg->n_wbuf * cfg->w_bytes + cfg->n_stage * G3_STAGE_BYTES;
+  cfg->w_limit = umma::WAIT_LIMIT_CYCLES;
   return true;
 }
 

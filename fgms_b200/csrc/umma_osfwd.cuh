@@ -48,6 +48,7 @@ struct OsConfig {
   int n_acc;   // tensor-memory columns of an accumulator: whole 128-byte blocks of the output row
   int group;   // tiles walked together
   int smem;
+  long long w_limit;  // cycles the MMA lane waits for a weight matrix before it gives up (for anything else: about a second)
 };
 
 struct OsParams {
@@ -71,6 +72,7 @@ struct OsShared {
   uint64_t w_full[2];
   uint64_t w_free[2];
   uint4 on[OS_MAX_STAGES];  // rows a stage holds, a bit each
+  uint64_t drained;  // every MMA has finished
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -130,6 +132,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
       mbar_init(smem_u32(&sh->w_full[b]), 1);
       mbar_init(smem_u32(&sh->w_free[b]), 1);
     }
+    mbar_init(smem_u32(&sh->drained), 1);
     sh->abort_flag = 0;
     mbar_fence_init();
   }
@@ -251,22 +254,24 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
     const uint64_t b_desc0 = make_sdesc(smem_u32(sW), (uint32_t)p.c_in * 128u, TF32 ? 512u : 1024u, TF32 ? 1u : 2u);
     constexpr uint32_t B_KC = (uint32_t)EPR * 8u, B_KS = (32u / ES) * 8u;  // one 128-byte K chunk / 32-byte MMA step further, in 16-byte units
     // One lane, named by elect.sync (see elect_one), runs the whole loop (waits, issue, commits); the other lanes wait at the
-    // end.  The loop is flat and leaves no stage early: with a loop over tiles around one over chunks and a break behind every
-    // wait, 64 -> 64 on a full block of 48^3 took 77 us, flat 58, four stages unrolled 56.  After a wait that ran out the abort
-    // flag lets every other one return, and the MMAs issued meanwhile read shared memory only.
+    // end.  The loop is flat and has one way out, behind a stage's last wait: with a loop over tiles around one over chunks and a
+    // break behind every wait, 64 -> 64 on a full block of 48^3 took 77 us, flat and never left 58, four stages unrolled 56, with
+    // the way out 57.  Once a wait has run out nothing is issued or committed: no accumulator whose rows or weights did not land reaches the epilogue, none that it
+    // may still be reading is written, and no stage or buffer is handed back that is still being filled.
     if (elect_one()) {
       int s = 0, wb = 0, grp = 0, g = 0, kc = 0;  // ring slot, weight buffer, group; tile of the group, chunk of its row
       uint32_t ph = 0, w_ph = 0;
-      auto take_weights = [&]() { ok = mbar_wait(smem_u32(&sh->w_full[wb]), w_ph, abort_flag) && ok; };
+      auto take_weights = [&]() { ok = mbar_wait(smem_u32(&sh->w_full[wb]), w_ph, abort_flag, cfg.w_limit) && ok; };
       auto free_weights = [&]() {
         mma_commit(smem_u32(&sh->w_free[wb]));
         if (++wb == cfg.n_wbuf) { wb = 0; w_ph ^= 1u; }
         g = 0;
       };
-      auto stage = [&](bool first_k, bool last_k) {
+      auto stage = [&](bool first_k, bool last_k) -> bool {
         // first offset of the group: the accumulator must have been read and cleared
         if (first_k && kc == 0) ok = mbar_wait(smem_u32(&sh->tmem_empty[g]), (uint32_t)grp & 1u, abort_flag) && ok;
         ok = mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag) && ok;
+        if (!ok) return false;
         const uint4 on = sh->on[s];
         fence_proxy_async();  // the stage was written through cp.async; the MMA reads it through the async proxy
         tc_fence_after();
@@ -284,6 +289,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
           if (last_k) mma_commit(smem_u32(&sh->tmem_full[g]));
           kc = 0; ++g;
         }
+        return true;
       };
       for (int tb = t0; tb < t1; tb += gsz, ++grp) {
         const int per_k = min(gsz, t1 - tb) * kch;
@@ -294,7 +300,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
             for (int u = 0; u < OS_UNROLL; ++u) {
               if (k0 + u >= p.k_vol) break;
               take_weights();
-              stage(k0 + u == 0, k0 + u + 1 == p.k_vol);
+              if (!stage(k0 + u == 0, k0 + u + 1 == p.k_vol)) goto done;
               free_weights();
             }
           }
@@ -305,13 +311,15 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
 #pragma unroll
               for (int u = 0; u < OS_UNROLL; ++u) {
                 if (r0 + u >= per_k) break;
-                stage(k == 0, k + 1 == p.k_vol);
+                if (!stage(k == 0, k + 1 == p.k_vol)) goto done;
               }
             }
             free_weights();
           }
         }
       }
+    done:
+      mma_drain(smem_u32(&sh->drained));
     }
     __syncwarp();
     ok = __all_sync(0xffffffffu, ok) != 0;
@@ -443,6 +451,7 @@ inline bool os_plan(int c_in, int c_out, int es, int max_smem, OsConfig* cfg) {
   if (cfg->n_stage < 2) return false;
   cfg->n_prod = cfg->n_stage < OS_PROD_WARPS ? cfg->n_stage : OS_PROD_WARPS;
   cfg->smem = fixed + cfg->n_wbuf * cfg->w_bytes + cfg->n_stage * G3_STAGE_BYTES;
+  cfg->w_limit = umma::WAIT_LIMIT_CYCLES;
   return true;
 }
 
