@@ -19,7 +19,8 @@
 //                        on a change of offset it commits the accumulator to the epilogue;
 //   epilogue (4 warps)   tcgen05.ld -> private 4 KB patch -> reds with consecutive lanes on consecutive
 //                        addresses of one gradient row.
-// All waits are bounded; a wait that runs out sets the CTA's abort flag and every role leaves its loop.
+// All waits are bounded; a wait that runs out sets the CTA's abort flag and every role leaves its loop; in-flight copies and MMAs
+// are awaited before tensor memory is freed.
 #pragma once
 #include "common.cuh"
 #include "umma.cuh"
@@ -44,6 +45,7 @@ struct W3Shared {
   uint64_t empty[W3_MAX_STAGES];  // used at the first stage of every group: the group's stages have been consumed
   uint64_t tmem_full[4];
   uint64_t tmem_empty[4];
+  uint64_t drained;  // every MMA has finished
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -109,6 +111,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
       mbar_init(smem_u32(&sh->tmem_full[b]), 1);
       mbar_init(smem_u32(&sh->tmem_empty[b]), W3_EPI_WARPS);
     }
+    mbar_init(smem_u32(&sh->drained), 1);
     sh->abort_flag = 0;
     mbar_fence_init();
   }
@@ -308,6 +311,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
       cur.next(tile_start, n_seg);
     }
     if (ok && cur_seg >= 0) mma_commit(smem_u32(&sh->tmem_full[run_i & (cfg.n_buf - 1)]));
+    mma_drain(smem_u32(&sh->drained));
     }
     __syncwarp();
     ok = __all_sync(0xffffffffu, ok) != 0;
