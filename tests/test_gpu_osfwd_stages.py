@@ -21,12 +21,12 @@ def _map(n, seed):
                           np.concatenate(o).astype(np.int32))
 
 
-def _run(p):
+def _run(p, accumulate=False, start=7.0):
     from fgms_b200 import backend
     nbr = backend.build_neighbor_table(p.kpos, p.imap, p.omap, p.km.n_in, p.km.n_out)
-    out = torch.full((p.km.n_out, p.c_out), 7.0, dtype=p.dtype, device="cuda")
+    out = torch.full((p.km.n_out, p.c_out), start, dtype=p.dtype, device="cuda")
     backend.device_status(reset=True)
-    backend.fgms_fwd_os_cuda(p.feats, p.weights, out, nbr, p.arch80)
+    backend.fgms_fwd_os_cuda(p.feats, p.weights, out, nbr, p.arch80, accumulate=accumulate)
     assert backend.device_status() == 0
     return out
 
@@ -40,10 +40,23 @@ def test_parity(mode, c_in, c_out, n):
     assert err(_run(p), p.ref_fwd()) <= TOL[mode]
 
 
+def _sms():
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
 def test_many_groups_of_tiles():
-    n = 148 * 128 * 9 + 77  # ten tiles of 32 channels in a CTA: two groups
+    n = _sms() * 128 * 9 + 77  # nine and ten tiles of 32 channels in a CTA: two groups
     p = Problem(_map(n, 3), 16, 32, seed=5, mode="fp16")
     assert err(_run(p), p.ref_fwd()) <= TOL["fp16"]
+
+
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_a_single_tile_behind_a_full_group(accumulate):
+    n = _sms() * 128 * 9 - 40  # nine tiles in every CTA: eight at a time, then one, a single stage per offset
+    p = Problem(_map(n, 4), 64, 32, seed=6, mode="fp16")
+    start = 0.25 if accumulate else 0.0
+    out = _run(p, accumulate=accumulate, start=0.25 if accumulate else 7.0)
+    assert err(out, p.ref_fwd() + start) <= TOL["fp16"]
 
 
 def test_rows_without_a_neighbour_see_nothing_of_the_others():
@@ -54,4 +67,5 @@ def test_rows_without_a_neighbour_see_nothing_of_the_others():
     out = _run(p)
     touched = np.unique(p.km.omap[p.km.imap == last])
     rest = np.setdiff1d(np.arange(700), touched)
-    assert torch.equal(out[rest], clean[rest]) and not torch.isfinite(out[touched]).all()
+    assert torch.equal(out[rest], clean[rest])
+    assert (~torch.isfinite(out[touched])).any(dim=1).all()  # every row that has the pair
