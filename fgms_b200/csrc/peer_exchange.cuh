@@ -97,8 +97,8 @@ __device__ __forceinline__ void px_reduce_slice(const PeerExchangeParams& p, lon
 }
 
 // At most 32 registers per thread (16 CTAs of 128 threads per SM by the bounds): the kernel is meant to run
-// BESIDE the persistent forward / dgrad kernel, whose 17 warps leave the warp scheduler that holds five of them
-// only 1024 free registers — room for exactly one warp of 32 registers per thread.  With more registers its CTAs
+// BESIDE the persistent forward / dgrad kernel, whose 18 warps leave the two warp schedulers that hold five of them
+// only 1024 free registers each — room for exactly one warp of 32 registers per thread.  With more registers its CTAs
 // are not scheduled until that kernel ends (measured: the exchange then starts when dgrad finishes).
 __global__ void __launch_bounds__(PX_THREADS, 16) peer_exchange_kernel(PeerExchangeParams p) {
   const int world = p.world, rank = p.rank;

@@ -4,9 +4,9 @@
 //
 // What bounds a layer of short rows is how many row pieces the SMs can ask L2 for, not arithmetic: a kernel that only
 // copies (gather a row, red it to its destination; no product) takes 143 us on 9.1 M pairs of 64-byte rows, 28 us on
-// 0.93 M pairs of 128-byte rows, while the tcgen05 form (umma_gms3.cuh) takes 374 us and 46 us there: its tiles pass
-// through shared memory, tensor memory and a patch, and each of those hand-offs costs a fixed few hundred cycles per
-// 128 rows whatever their length.  A product of 32 x 32 is 2 % of the warp-level matrix rate, so this kernel gives up
+// 0.93 M pairs of 128-byte rows, while the tcgen05 form (umma_gms3.cuh) takes 318 us and 35 us there (this kernel 141 and
+// 37): its tiles pass through shared memory, tensor memory and a patch, and each of those hand-offs costs a fixed few hundred
+// cycles per 128 rows whatever their length.  A product of 32 x 32 is 2 % of the warp-level matrix rate, so this kernel gives up
 // the faster tensor path and keeps nothing between the gather and the red but registers:
 //
 //   * mma.sync takes A with four lanes per row.  The contraction index may be enumerated in any order as long as A and B
@@ -336,11 +336,13 @@ inline int rw_launch(const GmsParams& p, cudaStream_t st, int sms) {
 // 0 launched, 1 not a shape of this kernel or a pointer is not 16-byte aligned, < 0 CUDA error
 inline int launch_rows_gms(const GmsParams& p, bool trans, bool f16, cudaStream_t st, int sms) {
   if (!rw_supported(p.k_dim, p.n_dim, f16)) return 1;
-  // tf32 32 -> 64, the one pair of widths whose weights fill the 64 registers and whose scattered rows are the longer ones:
-  // from 32 k pairs on the tcgen05 form is the faster (this kernel / that one, 27 offsets: 8 k pairs 3.7 / 5.6 us, 16 k
-  // 5.5 / 5.8, 32 k 7.5 / 6.8, 131 k 12.5 / 11.8, 200 k 17.7 / 15.8, 1 M 65 / 59); 64 -> 32 is faster here at every size
-  // (32 k 6.1 / 6.8, 200 k 13.7 / 18.1, 1 M 45 / 69), and so are 32 -> 48 (200 k 14.5 / 15.5) and, but for 5 % at 262 k
-  // pairs, 16 -> 64
+  // tf32 32 -> 64, a pair of widths whose weights fill the 64 registers and whose scattered rows are the longer ones: from
+  // about 32 k pairs on the tcgen05 form is the faster (this kernel / that one, 27 offsets: 4 k pairs 3.7 / 5.0 us, 11 k
+  // 4.6 / 5.1, 21 k 5.6 / 5.9; with the weights of this kernel 32 k 7.5, 131 k 12.5, 200 k 17.7, 1 M 65 against 39 k 7.0, 137 k
+  // 11.7, 208 k 15.4, 0.93 M 51.7).  The other widths stay here whatever their size.  Most are faster here throughout (32 -> 48
+  // 208 k 14.6 / 14.9; fp16 32 -> 32 0.93 M 18.8 / 35.8); where weights fill the registers the two forms cross as well, and
+  // the line is not drawn for them: tf32 64 -> 32 39 k 7.2 / 6.4, 208 k 13.9 / 13.6, 0.93 M 42.1 / 43.2; tf32 16 -> 64 21 k 5.1 / 5.9, 39 k
+  // 7.5 / 7.0, 0.93 M 59.0 / 52.4; fp16 64 -> 64 11 k 4.3 / 4.6, 39 k 6.9 / 5.8, 208 k 12.6 / 11.4, 0.93 M 37.4 / 34.8
   if (!f16 && p.k_dim == 32 && p.n_dim == 64 && p.pairs >= (1 << 15)) return 1;
   if ((long long)p.pairs + p.dense_rows > 0x7fffffffll - 4096) return 1;  // positions two tiles past the end stay in an int
   if ((reinterpret_cast<uintptr_t>(p.src) | reinterpret_cast<uintptr_t>(p.weights) | reinterpret_cast<uintptr_t>(p.dst)) & 15) return 1;

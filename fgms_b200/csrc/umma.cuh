@@ -38,10 +38,9 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
                "l"(map), "r"(bar), "r"(x), "r"(y)
                : "memory");
 }
-// One non-blocking probe of the barrier.  (mbarrier.try_wait may park the thread for an
-// implementation-defined time slice and was measured to wake up late; hand-offs between the roles of
-// these kernels are latency-critical, so the waiting lane probes with test_wait instead.)
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+// One non-blocking probe of the barrier.  The MMA lanes poll with it: every stage passes through them, and a thread that
+// mbarrier.try_wait has parked wakes up late.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
@@ -52,7 +51,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// The same, but the thread may be parked until the phase completes or a time limit of the hardware's own runs out.
+// The same, but the thread may be parked until the phase completes or a time limit of the hardware's own runs out.  All other
+// roles wait with it: they are ahead of the MMA lane or wide, and parked they leave it its issue slots.
 __device__ __forceinline__ bool mbar_park(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -68,10 +68,10 @@ __device__ __forceinline__ bool mbar_park(uint32_t bar, uint32_t parity) {
 // role tell the others to stop waiting once something has gone wrong.
 constexpr long long WAIT_LIMIT_CYCLES = 2000000000ll;
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, long long limit = WAIT_LIMIT_CYCLES) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_test(bar, parity)) return true;
   const long long start = clock64();
   for (uint32_t it = 1;; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_test(bar, parity)) return true;
     if ((it & 255u) == 0) {
       if (abort_flag && *abort_flag) return false;
       if (clock64() - start > limit) break;
@@ -81,9 +81,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return false;
 }
 
-// The bounded wait of a warp that is ahead of the others: it leaves them its issue slots.
+// The bounded wait that parks.
 __device__ __forceinline__ bool mbar_parked_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_test(bar, parity)) return true;
   const long long start = clock64();
   while (!mbar_park(bar, parity)) {
     if (abort_flag && *abort_flag) return false;
@@ -255,10 +255,7 @@ __device__ __forceinline__ uint64_t make_sdesc(uint32_t smem_addr, uint32_t lbo_
 // [R rows x 128 bytes]; inside a sub-tile rows are 128 bytes apart, groups of 8 rows 1024 bytes apart
 // (the stride byte offset), and the 16-byte chunk c of row r sits at chunk position c ^ (r % 8).
 // One MMA consumes 32 bytes of every row: advancing the start address by 32 selects the next K step.
-__host__ __device__ constexpr uint32_t kmajor_offset(uint32_t row, uint32_t byte_in_row, uint32_t rows) {
-  return (byte_in_row >> 7) * (rows * 128u) + (row >> 3) * 1024u + (row & 7u) * 128u +
-         ((((byte_in_row >> 4) & 7u) ^ (row & 7u)) << 4) + (byte_in_row & 15u);
-}
+//
 // MN-major (the M or N index is contiguous in a row, one row per contraction index k): rows of
 // [128 bytes] are grouped in atoms of 8 consecutive k (1024 bytes); atoms that follow each other in k
 // are `sbo` bytes apart, atoms that follow each other along M/N (the next 128 bytes of every row) are

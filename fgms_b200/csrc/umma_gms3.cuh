@@ -448,7 +448,9 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
           __syncwarp();
           uint8_t* dcol = dst + cb + (ch << 4);
           const bool ch_ok = FULL || (ch << 4) < vb;
-          // 32 rows = lpe passes of rpe rows, four passes' pieces read before the first of their reds
+          // 32 rows = lpe passes of rpe rows, four passes' pieces read before the first of their reds (the whole-span
+          // instantiations spill two registers for it; with the rows' numbers shuffled at the red, without a spill, 128 -> 128
+          // on 303 k pairs 23.3 -> 24.3 us, with the loop not unrolled 23.8)
 #pragma unroll
           for (uint32_t u0 = 0; u0 < 8; u0 += 4) {
             if (!FULL && u0 >= lpe) break;

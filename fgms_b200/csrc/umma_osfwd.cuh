@@ -20,8 +20,8 @@
 // Roles (20 warps): 12 producers, each filling whole stages (16-byte cp.async gathers into the K-major 128-byte-swizzled
 // ring), one MMA warp, one warp that loads weights by TMA, 4 epilogue warps.  All waits are bounded; all but the MMA lane's
 // are parked (85 -> 79 us on the layer below).  64 -> 64 on a full block of 48^3 (2.9 M pairs, 27 stages for each of 864 tiles):
-// 141 us with eight warps that each filled 16 rows of every stage and copied zeros, 56 us now: 650 cycles a stage, of which
-// 400-580 are the stage's 32 warp-wide copies; 128 -> 128 246 -> 97 us, 1000 voxels 64 -> 64 32 -> 17 us.
+// 141 us with eight warps that each filled 16 rows of every stage and copied zeros, 57 us now: 660 cycles a stage, of which
+// 400-580 are the stage's 32 warp-wide copies; 128 -> 128 246 -> 96 us, 1000 voxels 64 -> 64 32 -> 15 us.
 #pragma once
 #include "common.cuh"
 #include "umma.cuh"
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
       for (int tb = t0; tb < t1; tb += gsz, ++grp) {
         const int per_k = min(gsz, t1 - tb) * kch;
         if (per_k == 1) {
-          // a single stage per offset: one loop over the offsets (1000 voxels 64 -> 64 15.3 us, 17.7 with a loop inside it)
+          // a single stage per offset: one loop over the offsets (1000 voxels 64 -> 64 15.0 us, 17.7 with a loop inside it)
           for (int k0 = 0; k0 < p.k_vol; k0 += OS_UNROLL) {
 #pragma unroll
             for (int u = 0; u < OS_UNROLL; ++u) {
