@@ -20,8 +20,8 @@
 // Roles (20 warps): 12 producers, each filling whole stages (16-byte cp.async gathers into the K-major 128-byte-swizzled
 // ring), one MMA warp, one warp that loads weights by TMA, 4 epilogue warps.  All waits are bounded; all but the MMA lane's
 // are parked (85 -> 79 us on the layer below).  64 -> 64 on a full block of 48^3 (2.9 M pairs, 27 stages for each of 864 tiles):
-// 141 us with eight warps that each filled 16 rows of every stage and copied zeros, 57 us now: 660 cycles a stage, of which
-// 400-580 are the stage's 32 warp-wide copies; 128 -> 128 246 -> 96 us, 1000 voxels 64 -> 64 32 -> 15 us.
+// 141 us with eight warps that each filled 16 rows of every stage and copied zeros, 56 us now: 650 cycles a stage, of which
+// 400-580 are the stage's 32 warp-wide copies; 128 -> 128 246 -> 93 us, 1000 voxels 64 -> 64 32 -> 15 us.
 #pragma once
 #include "common.cuh"
 #include "umma.cuh"
@@ -254,14 +254,14 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
     const uint64_t b_desc0 = make_sdesc(smem_u32(sW), (uint32_t)p.c_in * 128u, TF32 ? 512u : 1024u, TF32 ? 1u : 2u);
     constexpr uint32_t B_KC = (uint32_t)EPR * 8u, B_KS = (32u / ES) * 8u;  // one 128-byte K chunk / 32-byte MMA step further, in 16-byte units
     // One lane, named by elect.sync (see elect_one), runs the whole loop (waits, issue, commits); the other lanes wait at the
-    // end.  The loop is flat and has one way out, behind a stage's last wait: with a loop over tiles around one over chunks and a
-    // break behind every wait, 64 -> 64 on a full block of 48^3 took 77 us, flat and never left 58, four stages unrolled 56, with
-    // the way out 57.  Once a wait has run out nothing is issued or committed: no accumulator whose rows or weights did not land reaches the epilogue, none that it
-    // may still be reading is written, and no stage or buffer is handed back that is still being filled.
+    // end.  A loop over tiles around one over chunks takes 77 us for 64 -> 64 on a full block of 48^3, a flat one 58, with four
+    // stages unrolled 56.  A wait that runs out leaves at once and by itself: nothing is issued or committed behind it, so no
+    // accumulator whose rows or weights did not land reaches the epilogue, none that it may still be reading is written, and no
+    // stage or buffer is handed back that is still being filled (one test of all waits behind a stage's last: 57.5 us).
     if (elect_one()) {
       int s = 0, wb = 0, grp = 0, g = 0, kc = 0;  // ring slot, weight buffer, group; tile of the group, chunk of its row
       uint32_t ph = 0, w_ph = 0;
-      auto take_weights = [&]() { ok = mbar_wait(smem_u32(&sh->w_full[wb]), w_ph, abort_flag, cfg.w_limit) && ok; };
+      auto take_weights = [&]() { return mbar_wait(smem_u32(&sh->w_full[wb]), w_ph, abort_flag, cfg.w_limit); };
       auto free_weights = [&]() {
         mma_commit(smem_u32(&sh->w_free[wb]));
         if (++wb == cfg.n_wbuf) { wb = 0; w_ph ^= 1u; }
@@ -269,9 +269,8 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
       };
       auto stage = [&](bool first_k, bool last_k) -> bool {
         // first offset of the group: the accumulator must have been read and cleared
-        if (first_k && kc == 0) ok = mbar_wait(smem_u32(&sh->tmem_empty[g]), (uint32_t)grp & 1u, abort_flag) && ok;
-        ok = mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag) && ok;
-        if (!ok) return false;
+        if (first_k && kc == 0 && !mbar_wait(smem_u32(&sh->tmem_empty[g]), (uint32_t)grp & 1u, abort_flag)) return false;
+        if (!mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag)) return false;
         const uint4 on = sh->on[s];
         fence_proxy_async();  // the stage was written through cp.async; the MMA reads it through the async proxy
         tc_fence_after();
@@ -291,34 +290,37 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
         }
         return true;
       };
-      for (int tb = t0; tb < t1; tb += gsz, ++grp) {
-        const int per_k = min(gsz, t1 - tb) * kch;
-        if (per_k == 1) {
-          // a single stage per offset: one loop over the offsets (1000 voxels 64 -> 64 15.0 us, 17.7 with a loop inside it)
-          for (int k0 = 0; k0 < p.k_vol; k0 += OS_UNROLL) {
+      auto all_stages = [&]() -> bool {
+        for (int tb = t0; tb < t1; tb += gsz, ++grp) {
+          const int per_k = min(gsz, t1 - tb) * kch;
+          if (per_k == 1) {
+            // a single stage per offset: one loop over the offsets (1000 voxels 64 -> 64 15.0 us, 17.7 with a loop inside it)
+            for (int k0 = 0; k0 < p.k_vol; k0 += OS_UNROLL) {
 #pragma unroll
-            for (int u = 0; u < OS_UNROLL; ++u) {
-              if (k0 + u >= p.k_vol) break;
-              take_weights();
-              if (!stage(k0 + u == 0, k0 + u + 1 == p.k_vol)) goto done;
+              for (int u = 0; u < OS_UNROLL; ++u) {
+                if (k0 + u >= p.k_vol) break;
+                if (!take_weights()) return false;
+                if (!stage(k0 + u == 0, k0 + u + 1 == p.k_vol)) return false;
+                free_weights();
+              }
+            }
+          } else {
+            for (int k = 0; k < p.k_vol; ++k) {
+              if (!take_weights()) return false;
+              for (int r0 = 0; r0 < per_k; r0 += OS_UNROLL) {
+#pragma unroll
+                for (int u = 0; u < OS_UNROLL; ++u) {
+                  if (r0 + u >= per_k) break;
+                  if (!stage(k == 0, k + 1 == p.k_vol)) return false;
+                }
+              }
               free_weights();
             }
           }
-        } else {
-          for (int k = 0; k < p.k_vol; ++k) {
-            take_weights();
-            for (int r0 = 0; r0 < per_k; r0 += OS_UNROLL) {
-#pragma unroll
-              for (int u = 0; u < OS_UNROLL; ++u) {
-                if (r0 + u >= per_k) break;
-                if (!stage(k == 0, k + 1 == p.k_vol)) goto done;
-              }
-            }
-            free_weights();
-          }
         }
-      }
-    done:
+        return true;
+      };
+      ok = all_stages();
       mma_drain(smem_u32(&sh->drained));
     }
     __syncwarp();
