@@ -22,6 +22,7 @@
 #include "umma_gms3.cuh"
 #include "umma_wgrad3.cuh"
 #include "rows_wgrad.cuh"
+#include "rows_wgrad16.cuh"
 #include "peer_exchange.cuh"
 #include "umma_osfwd.cuh"
 
@@ -342,7 +343,7 @@ int fgms_b200_wgrad(const void* in_feats, const void* out_grad, void* kernel_gra
   bool launched = false;
   if (umma) {
     const bool f16 = dtype == FGMS_DTYPE_F16;
-    int rc = fgms::launch_rows_wgrad(p, f16, st, di.sms, di.max_smem_optin);
+    int rc = f16 ? fgms::launch_rows_wgrad16(p, st, di.sms, di.max_smem_optin) : fgms::launch_rows_wgrad(p, st, di.sms, di.max_smem_optin);
     if (rc == 1) rc = fgms::launch_umma_wgrad3(p, f16, st, di.sms, di.max_smem_optin);
     if (rc == 0) {
       if (int rc2 = check_launch("weight-gradient kernel")) return rc2;

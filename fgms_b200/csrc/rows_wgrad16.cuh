@@ -1,0 +1,275 @@
+// Weight gradient for short fp16 rows: every warp gathers tiles of 16 pairs into a ring of its own in shared memory.
+//
+//   dw[k] (c_in x c_out, fp32 sums) += sum over the pairs j of offset k of feats[in_map[j]]^T (x) out_grad[out_map[j]]
+//
+// The pair index is the contraction index of the product.  A tile's rows lie in shared memory as they are in memory, pair by
+// pair, and ldmatrix.trans hands both operands of mma.sync out of them, so nothing is exchanged between registers.  Copies
+// (16-byte cp.async), map entries (4-byte cp.async, a ring's length ahead of the rows) and products of a warp overlap
+// without registers to hold them: the form that gathered straight into registers (rows_wgrad.cuh, which tf32 keeps) had
+// two tiles a warp in flight, waited for its entries' registers and spent 220 instructions a tile.  In a row of launches,
+// that form / this one: 9.1 M pairs 32 -> 32 198 / 99.5 us (two gathers of these rows from L2 at 17 TB/s: 69), 0.93 M
+// pairs 64 -> 64 43.7 / 31.7, 48 -> 48 41.1 / 29.3, 16 -> 16 16.7 / 12.1, 0.14 M 64 -> 64 13.3 / 11.1, 84 k 32 -> 32 7.5 / 6.5.
+//
+// What bounds it now: with 8 warps at 64 -> 64 (two a scheduler; 128 of a lane's registers are sums) the matrix
+// instructions' fixed issue latency (3.3 of 6.7 cycles an instruction, tensor pipe 45 % busy); with 16 warps at 32 -> 32
+// the same (2.7) and the entries' and rows' latency (1.4); on few pairs the sum of the warps' results at the end of an
+// offset, about 2 us each time.  Two warps that share a tile and split a side of dW between them (twice the warps at
+// 64 -> 64) were slower, 34 and 39 us.  The ring's length does not matter from three tiles on (four here; 8.1 M pairs in
+// spread order want the fourth: 113 us with three).
+//
+// One block per SM takes a share of the pairs, its warps take the share's tiles of 16 in turn, and the block adds up its
+// warps' fp32 sums when the offset changes.  Where those sums go straight into an fp16 gradient every block's is rounded,
+// and the pairs are shared out in units of 256 of one offset, the stages of the tcgen05 form, so that an offset of up to
+// 256 pairs is rounded once.  Shares cut by single tiles split such an offset among up to six blocks: relative error of
+// the gradient (32 -> 32, 27 offsets) 4.3e-4 against 2.1e-4 in units for 80 pairs each, 4.7e-4 against 3.6e-4 for 1300.
+#pragma once
+#include "common.cuh"
+#include "rows_gms.cuh"  // rw_mma, rw_max_regs
+#include "umma.cuh"
+
+namespace fgms {
+
+constexpr int WH_UNIT = 4;       // log2 of a unit's tiles where block sums are rounded to fp16; single tiles elsewhere
+constexpr int WH_MAX_DEPTH = 4;  // tiles of a ring
+
+// One operand's rows of a tile in shared memory: U units of 16 channels (two 16-byte chunks) a row.  The chunks of the
+// eight rows that an ldmatrix reads together lie in different banks: rows of 1, 2 or 4 units exchange their chunks by row
+// number, rows of 3 units are an odd number of chunks apart.
+template <int U>
+struct WhRows {
+  static constexpr int CHUNKS = 2 * U;
+  static constexpr uint32_t BYTES = U * 32;                    // of a row in global memory
+  static constexpr uint32_t LD = U == 3 ? BYTES + 16 : BYTES;  // of a row in shared memory
+  static constexpr uint32_t TILE = 16 * LD;
+  static constexpr int LANES = U == 3 ? 8 : CHUNKS;            // lanes that copy a row, a chunk each
+  static constexpr int ROUNDS = 16 * LANES / 32;               // warp-wide copies of a tile
+  __device__ static __forceinline__ uint32_t at(int row, int chunk) {
+    const int x = U == 4 ? row & 7 : U == 2 ? (row >> 1) & 3 : U == 1 ? (row >> 2) & 1 : 0;
+    return (uint32_t)row * LD + (uint32_t)((chunk ^ x) << 4);
+  }
+  // chunk 2 u further on than the one at `addr`; rows without padding are aligned to their length
+  __device__ static __forceinline__ uint32_t unit(uint32_t addr, int u) { return U == 3 ? addr + 32 * u : addr ^ (32 * u); }
+  // this lane's chunk of a row, from src + lane's chunk; `on` says what rows there are, the others become zeros
+  template <bool WHOLE>
+  __device__ static __forceinline__ void copy(uint32_t slot, const uint8_t* src, int e, int first, unsigned on, int lane) {
+    const int r0 = lane / LANES, c = lane % LANES;
+#pragma unroll
+    for (int i = 0; i < ROUNDS; ++i) {
+      const int row = r0 + i * (32 / LANES), idx = __shfl_sync(0xffffffffu, e, first + row);
+      if (LANES > CHUNKS && c >= CHUNKS) continue;
+      if (WHOLE) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot + at(row, c)), "l"(src + (size_t)(unsigned)idx * BYTES) : "memory");
+      else umma::cp_async16(slot + at(row, c), src + ((on >> row) & 1 ? (size_t)(unsigned)idx * BYTES : 0), (on >> row) & 1);
+    }
+  }
+};
+
+__device__ __forceinline__ void wh_ldmatrix(uint32_t addr, uint32_t (&v)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
+}
+
+template <int MU, int NU, int WARPS, int DEPTH>
+__global__ void __maxnreg__(rw_max_regs(WARPS * 32, true)) rows_wgrad16_kernel(WgradParams p, bool spread) {
+  static_assert(WARPS <= 1 << WH_UNIT, "a full unit has a tile for every warp");
+  static_assert(DEPTH >= 2, "a tile is filled while another is used");
+  using A = WhRows<MU>;
+  using B = WhRows<NU>;
+  constexpr uint32_t STAGE = A::TILE + B::TILE, ENTRIES = 128;
+  constexpr int NT = 2 * NU, SUMS = MU * 4 * NT;  // n-tiles of 8 columns; accumulators per lane
+  constexpr uint32_t RINGS = WARPS * (DEPTH * STAGE + (DEPTH - 1) * ENTRIES), ALL_SUMS = WARPS * SUMS * 128;
+  extern __shared__ __align__(128) uint8_t wh_smem[];  // the warps' rings, later [WARPS][SUMS][32] sums; then the tile table
+  int* tile_start = reinterpret_cast<int*>(wh_smem + (RINGS > ALL_SUMS ? RINGS : ALL_SUMS));
+  int* kpos_s = tile_start + p.k_vol + 2;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int n_seg = p.k_vol + 1;
+
+  umma::griddep_wait();
+  umma::griddep_launch_dependents();
+  const int unit = p.dw_f16 != nullptr ? WH_UNIT : 0;
+  build_tile_table(16 << unit, p.kpos, p.pairs, p.k_vol, 0, kpos_s, tile_start);
+  // Units by turns; spread (see Turns) when the rows exceed what L2 holds.
+  const int total = tile_start[n_seg], share = (total + gridDim.x - 1) / gridDim.x;
+  int t0 = min(total, (int)blockIdx.x * share);
+  const int t1 = min(total, t0 + share);
+
+  const uint32_t ring = umma::smem_u32(wh_smem) + warp * DEPTH * STAGE;
+  const uint32_t entries = umma::smem_u32(wh_smem) + WARPS * DEPTH * STAGE + warp * (DEPTH - 1) * ENTRIES + lane * 4;
+  const uint8_t* feats = static_cast<const uint8_t*>(p.feats) + lane % A::LANES * 16;
+  const uint8_t* og = static_cast<const uint8_t*>(p.out_grad) + lane % B::LANES * 16;
+  // ldmatrix: lanes 0-7, 8-15, 16-23, 24-31 name the rows of the four 8 x 8 matrices
+  const uint32_t a_off = A::at((lane & 7) + ((lane >> 4) << 3), (lane >> 3) & 1);
+  const uint32_t b_off = B::at((lane & 7) + (((lane >> 3) & 1) << 3), lane >> 4);
+  const int32_t* __restrict__ map = lane < 16 ? p.in_map : p.out_map;
+  const unsigned n_rows = lane < 16 ? p.n_in : p.n_out;
+
+  while (t0 < t1) {
+    // this block's turns inside one offset; warp w takes tiles w, w + WARPS, ... of their units
+    const int seg = find_segment(tile_start, n_seg, t0);
+    const int units = min(t1, tile_start[seg + 1]) - t0;
+    const Turns turns(tile_start[seg], tile_start[seg + 1], share, (int)blockIdx.x, t0, spread);
+    const int j_begin = kpos_s[seg], j_end = kpos_s[seg + 1];
+    // a single unit may be the offset's last, partly filled one; of several at least one is full
+    const int run = units > 1 ? units << unit : min(1 << unit, (j_end - j_begin + 15) / 16 - (turns.tile(0) << unit));
+    t0 += units;
+    float acc[MU][NT][4];
+#pragma unroll
+    for (int u = 0; u < MU; ++u)
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[u][j][e] = 0.f;
+
+    // position of this lane's map entry of tile n: lanes 0-15 the input rows of its pairs, lanes 16-31 the output rows
+    auto entry_at = [&](int n) {
+      return (n < run ? j_begin + 16 * ((turns.tile(n >> unit) << unit) + (n & ((1 << unit) - 1))) : j_end) + (lane & 15);
+    };
+    auto fetch_entry = [&](int n, uint32_t slot) {
+      const int j = entry_at(n);
+      if (j < j_end) umma::cp_async4(slot, map + j);
+      else umma::st_shared_i32(slot, -1);
+    };
+    auto start = [&](int e, uint32_t slot) {  // the rows of a tile's entries on their way
+      const unsigned in = __ballot_sync(0xffffffffu, (unsigned)e < n_rows), ok = in & (in >> 16) & 0xffffu;
+      if (ok == 0xffffu) {
+        A::template copy<true>(slot, feats, e, 0, ok, lane);
+        B::template copy<true>(slot + A::TILE, og, e, 16, ok, lane);
+      } else {  // the offset's last tile, or entries outside the tensors
+        const unsigned there = __ballot_sync(0xffffffffu, e != -1), bad = ((there | there >> 16) & ~ok) & 0xffffu;
+        if ((bad >> lane) & 1) report_problem();  // pair skipped, counted once
+        A::template copy<false>(slot, feats, e, 0, ok, lane);
+        B::template copy<false>(slot + A::TILE, og, e, 16, ok, lane);
+      }
+    };
+    if (warp < run) {
+      // group d of a warp's copies: the rows of its tile d and the entries of its tile d + DEPTH - 1
+      int e[DEPTH - 1];
+#pragma unroll
+      for (int d = 0; d < DEPTH - 1; ++d) {
+        const int j = entry_at(warp + d * WARPS);
+        e[d] = j < j_end ? __ldg(map + j) : -1;
+      }
+#pragma unroll
+      for (int d = 0; d < DEPTH - 1; ++d) {
+        if (warp + d * WARPS < run) start(e[d], ring + d * STAGE);
+        fetch_entry(warp + (d + DEPTH - 1) * WARPS, entries + d * ENTRIES);
+        umma::cp_async_commit();
+      }
+      uint32_t put = (DEPTH - 1) * STAGE, get = 0, ent = 0;
+#pragma unroll 1
+      for (int n = warp; n < run; n += WARPS) {
+        umma::cp_async_wait<DEPTH - 2>();
+        __syncwarp();  // the tile has landed for every lane, and every lane is done with the slot that is filled next
+        // operands first: the next tile's copies are prepared while they come
+        uint32_t a[MU][4], b[NU][4];
+        const uint32_t sa = ring + get + a_off, sb = ring + get + A::TILE + b_off;
+#pragma unroll
+        for (int v = 0; v < NU; ++v) wh_ldmatrix(B::unit(sb, v), b[v]);
+#pragma unroll
+        for (int u = 0; u < MU; ++u) wh_ldmatrix(A::unit(sa, u), a[u]);
+        if (n + (DEPTH - 1) * WARPS < run) {
+          start(umma::ld_shared_i32(entries + ent), ring + put);
+          fetch_entry(n + 2 * (DEPTH - 1) * WARPS, entries + ent);
+          ent = ent == (DEPTH - 2) * ENTRIES ? 0 : ent + ENTRIES;
+          put = put == (DEPTH - 1) * STAGE ? 0 : put + STAGE;
+        }
+        umma::cp_async_commit();
+#pragma unroll
+        for (int u = 0; u < MU; ++u)
+#pragma unroll
+          for (int j = 0; j < NT; ++j) rw_mma(acc[u][j], a[u], b[j / 2][2 * (j & 1)], b[j / 2][2 * (j & 1) + 1], false);
+        get = get == (DEPTH - 1) * STAGE ? 0 : get + STAGE;
+      }
+    }
+    umma::cp_async_wait_all();
+    __syncthreads();  // every warp is done with its ring
+    if (warp < run) {
+      float* mine = reinterpret_cast<float*>(wh_smem) + warp * SUMS * 32 + lane;
+#pragma unroll
+      for (int u = 0; u < MU; ++u)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) mine[((u * 4 + e) * NT + j) * 32] = acc[u][j][e];
+    }
+    const int used = min(run, WARPS);
+    __syncthreads();
+    // element e = 2 h + c of n-tile j in lane (g, t): gradient row 16 u + 8 h + g, column 8 j + 2 t + c.  Four lanes' two
+    // elements are eight consecutive columns.
+    for (int item = threadIdx.x; item < MU * 2 * NT * 8; item += WARPS * 32) {
+      const int g = item & 7, j = (item >> 3) % NT, uh = (item >> 3) / NT;
+      const float* from = reinterpret_cast<const float*>(wh_smem) + (uh * 2 * NT + j) * 32 + 4 * g;
+      float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      for (int w = 0; w < used; ++w) {
+        const float4 x = *reinterpret_cast<const float4*>(from + w * SUMS * 32);
+        const float4 y = *reinterpret_cast<const float4*>(from + w * SUMS * 32 + NT * 32);
+        s[0] += x.x; s[1] += y.x; s[2] += x.y; s[3] += y.y; s[4] += x.z; s[5] += y.z; s[6] += x.w; s[7] += y.w;
+      }
+      const size_t at = ((size_t)seg * (MU * 16) + 8 * uh + g) * (NU * 16) + 8 * j;
+      if (p.dw_f16 != nullptr) {
+        red_add_h8(p.dw_f16 + at, pack_half2(s[0], s[1]), pack_half2(s[2], s[3]), pack_half2(s[4], s[5]), pack_half2(s[6], s[7]));
+      } else {
+        red_add_v4(p.dw + at, s[0], s[1], s[2], s[3]);
+        red_add_v4(p.dw + at + 4, s[4], s[5], s[6], s[7]);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------------------
+// Warps of the block: as many as the registers allow (sums, operands, about fifty for the rest), 16 at most; the ring as
+// long as shared memory allows, with room for a block of the exchange beside it.
+constexpr int wh_warps(int mu, int nu) {
+  const int regs = 8 * mu * nu + 4 * (mu + nu) + 48, fit = 61440 / (32 * ((regs + 7) / 8 * 8)) / 4 * 4;
+  return fit > 16 ? 16 : fit;
+}
+constexpr int wh_depth(int mu, int nu) {
+  const int stage = 512 * (mu + nu) + (mu == 3 ? 256 : 0) + (nu == 3 ? 256 : 0), fit = 200 * 1024 / (wh_warps(mu, nu) * (stage + 128));
+  return fit > WH_MAX_DEPTH ? WH_MAX_DEPTH : fit;
+}
+// Shapes this kernel takes: multiples of 16 up to 64 channels on both sides.
+inline bool wh_supported(int c_in, int c_out) { return c_in % 16 == 0 && c_out % 16 == 0 && c_in >= 16 && c_out >= 16 && c_in <= 64 && c_out <= 64; }
+
+template <int MU, int NU>
+inline int wh_launch_as(const WgradParams& p, cudaStream_t st, int sms, int max_smem) {
+  constexpr int WARPS = wh_warps(MU, NU), DEPTH = wh_depth(MU, NU);
+  auto kernel = rows_wgrad16_kernel<MU, NU, WARPS, DEPTH>;
+  constexpr size_t rings = (size_t)WARPS * (DEPTH * (WhRows<MU>::TILE + WhRows<NU>::TILE) + (DEPTH - 1) * 128);
+  constexpr size_t sums = (size_t)WARPS * MU * 8 * NU * 128;
+  const size_t smem = (rings > sums ? rings : sums) + (size_t)(2 * p.k_vol + 3) * sizeof(int);
+  if (smem > (size_t)max_smem) return 1;
+  static std::atomic<int> granted[64];
+  if (int rc = ensure_smem(kernel, max_smem, granted)) return rc;
+  const long long units = (long long)p.pairs / (p.dw_f16 != nullptr ? 16 << WH_UNIT : 16) + p.k_vol + 1;
+  const bool spread = spread_tiles((size_t)p.n_in * WhRows<MU>::BYTES + (size_t)p.n_out * WhRows<NU>::BYTES);
+  return launch_pdl(kernel, (int)(units < sms ? units : sms), WARPS * 32, smem, st, p, spread) == cudaSuccess ? 0 : -1;
+}
+template <int MU>
+inline int wh_launch_n(const WgradParams& p, cudaStream_t st, int sms, int max_smem) {
+  switch (p.c_out / 16) {
+    case 1: return wh_launch_as<MU, 1>(p, st, sms, max_smem);
+    case 2: return wh_launch_as<MU, 2>(p, st, sms, max_smem);
+    case 3: return wh_launch_as<MU, 3>(p, st, sms, max_smem);
+    case 4: return wh_launch_as<MU, 4>(p, st, sms, max_smem);
+  }
+  return 1;
+}
+
+// 0 launched, 1 not a shape of this kernel or a pointer is not 16-byte aligned, < 0 CUDA error
+inline int launch_rows_wgrad16(const WgradParams& p, cudaStream_t st, int sms, int max_smem) {
+  if (!wh_supported(p.c_in, p.c_out)) return 1;
+  if ((long long)p.pairs > 0x7fffffffll - 65536) return 1;  // positions a few turns past the end stay in an int
+  if ((reinterpret_cast<uintptr_t>(p.feats) | reinterpret_cast<uintptr_t>(p.out_grad) | reinterpret_cast<uintptr_t>(p.dw) |
+       reinterpret_cast<uintptr_t>(p.dw_f16)) & 15) return 1;
+  switch (p.c_in / 16) {
+    case 1: return wh_launch_n<1>(p, st, sms, max_smem);
+    case 2: return wh_launch_n<2>(p, st, sms, max_smem);
+    case 3: return wh_launch_n<3>(p, st, sms, max_smem);
+    case 4: return wh_launch_n<4>(p, st, sms, max_smem);
+  }
+  return 1;
+}
+
+}  // namespace fgms
