@@ -12,16 +12,27 @@
 // while consecutive stages belong to the same offset and is flushed with 16-byte vector reds to the
 // fp32 gradient when the offset changes (split-K across CTAs).
 //
-//   producers (8 warps)  warp w owns rows [w pb/8, (w+1) pb/8) of every stage: it fetches those rows' map
-//                        entries from global memory four stages ahead and gathers both operands with
-//                        16-byte cp.async;
+//   producers (2 teams   the teams take the stages in turn; warp w of a team owns rows [w pb/4, (w+1) pb/4) of its team's
+//   of 4 warps)          stages: it fetches those rows' map entries two of them ahead into a ring of its own and gathers both
+//                        operands with 16-byte cp.async;
 //   MMA warp             one lane issues tcgen05.mma per stage and commits the stage back to the producers;
 //                        on a change of offset it commits the accumulator to the epilogue;
 //   epilogue (4 warps)   tcgen05.ld -> private 4 KB patch -> reds with consecutive lanes on consecutive
 //                        addresses of one gradient row.
 // All waits are bounded; a wait that runs out sets the CTA's abort flag and every role leaves its loop; in-flight copies and MMAs
 // are awaited before tensor memory is freed.
+//
+// What bounded it were the producers' instructions: with every copy left out it took as long.  Eight warps went through all
+// stages together, tested for each of eight possible pieces of a row whether the row has it, and waited in every stage for
+// the map entries they had just asked for.  Straight code for the usual numbers of pieces: 128 -> 128 on 303 k pairs 26.9 -> 20.2
+// us in a row of launches; two teams of four that are in different phases of a stage (one copies while the other is at its
+// entries and barriers) 18.4, two teams of eight with fewer registers 20.8; the MMA lane's loops 18.0.  Also 96 -> 160
+// on 358 k pairs 43.6 -> 27.7, tf32 64 -> 64 on 296 k 25.6 -> 17.2, tf32 48 -> 64 on 591 k 53.2 -> 28.3, 64 -> 128 stride 2 on 50 k 9.5 ->
+// 8.7; 256 -> 256, where every stage is 32 pairs and the sums' reds are the larger part, 15.0 -> 15.2 (27 k pairs).
+// Now a stage of 128 pairs at 128 -> 128 is about 1500 cycles, of which shared memory needs 1024 (64 KB written, read by the MMAs).
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 #include "umma.cuh"
 #include "umma_gms3.cuh"  // G3Walk, g3_wait
@@ -31,14 +42,16 @@ namespace fgms {
 constexpr int W3_EPI_WARPS = 4;
 constexpr int W3_MMA_WARP = 4;
 constexpr int W3_PROD_WARP0 = 5;
-constexpr int W3_PROD_WARPS = 8;
+constexpr int W3_PROD_WARPS = 4;  // of a team: they share a stage
+constexpr int W3_PROD_TEAMS = 2;  // take the stages in turn
 constexpr int W3_PROD_THREADS = W3_PROD_WARPS * 32;
-constexpr int W3_THREADS = (W3_PROD_WARP0 + W3_PROD_WARPS) * 32;
-__device__ __forceinline__ int w3_producer_index(int warp) { return warp - W3_PROD_WARP0; }  // < 0: no producer
+constexpr int W3_THREADS = (W3_PROD_WARP0 + W3_PROD_TEAMS * W3_PROD_WARPS) * 32;
 constexpr int W3_MAX_STAGES = 12;
-constexpr int W3_MAX_PB = 256;
+constexpr int W3_MAX_PB = 128;
 constexpr int W3_PATCH_BYTES = W3_EPI_WARPS * 4096;
-constexpr int W3_PREFETCH = 4;  // map entries are fetched this many stages ahead
+constexpr int W3_PREFETCH = 2;  // map entries are fetched this many of the team's stages ahead
+// the producers' rings of map entries: W3_PREFETCH + 1 slots of both entries of every pair of a stage
+__host__ __device__ constexpr int w3_ring_bytes(int pb) { return W3_PROD_TEAMS * (W3_PREFETCH + 1) * 2 * 4 * pb; }
 
 struct W3Shared {
   uint64_t full[W3_MAX_STAGES];
@@ -52,7 +65,7 @@ struct W3Shared {
 constexpr int W3_SHARED_BYTES = (sizeof(W3Shared) + 15) & ~15;
 
 struct W3Config {
-  int pb;         // pairs per stage: 32, 64, 128 or 256
+  int pb;         // pairs per stage: 32, 64 or 128
   int pack;       // pairs that share one staged row (their rows side by side): 1, 2 or 4
   int slot_a, slot_b;  // packed stages: bytes a pair's row takes in the staged row of A / of B
   int n_mtile;    // 1 or 2 accumulator row tiles: all of 128 rows but possibly the last
@@ -92,7 +105,8 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
   const uint32_t stage_bytes = (uint32_t)kr * 128u * (cfg.pa + cfg.pbp);
   uint8_t* sStage = smem;
   uint8_t* sPatch = sStage + (size_t)n_stage * stage_bytes;
-  W3Shared* sh = reinterpret_cast<W3Shared*>(sPatch + W3_PATCH_BYTES);
+  uint8_t* sRing = sPatch + W3_PATCH_BYTES;
+  W3Shared* sh = reinterpret_cast<W3Shared*>(sRing + w3_ring_bytes(pb));
   int* tile_start = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(sh) + W3_SHARED_BYTES);  // [k_vol + 2]
   int* kpos_s = tile_start + p.k_vol + 2;                                                        // [k_vol + 1]
 
@@ -137,10 +151,10 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
 
   if (t0 >= t1) {
     // nothing for this CTA
-  } else if (w3_producer_index(warp) >= 0) {
+  } else if (warp >= W3_PROD_WARP0) {
     // ------------------------------------------------------------------ producers
-    const int pw = w3_producer_index(warp);
-    const int rpw = pb / W3_PROD_WARPS;  // rows of a stage owned by this warp: 4, 8, 16 or 32
+    const int team = (warp - W3_PROD_WARP0) / W3_PROD_WARPS, pw = (warp - W3_PROD_WARP0) % W3_PROD_WARPS;
+    const int rpw = pb / W3_PROD_WARPS;  // rows of a stage owned by this warp: 8, 16 or 32
     const uint8_t* feats = static_cast<const uint8_t*>(p.feats);
     const uint8_t* og = static_cast<const uint8_t*>(p.out_grad);
     const uint32_t a_row_bytes = (uint32_t)p.c_in * ES, b_row_bytes = (uint32_t)p.c_out * ES;
@@ -157,99 +171,134 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
     // rs, rs + rpp, ... of the warp's block: one shuffle and one address per row, then one cp.async per
     // piece at a fixed distance (128 bytes in global memory, `lbo` in shared memory).
     const int rs = lane / lpr, cc = lane % lpr;
-    // 128-byte pieces of a row this lane's 16-byte chunk exists in (the last piece of a row that is no whole
-    // number of pieces is filled in part): 0 .. 8
-    const int nha = FULL ? (int)a_row_bytes / 128 : ((int)a_row_bytes - cc * 16 + 127) / 128;
-    const int nhb = FULL ? (int)b_row_bytes / 128 : ((int)b_row_bytes - cc * 16 + 127) / 128;
-    // piece 0 of row rs + rpp u, relative to the operand's start in the stage: rows 8 apart are 1024 bytes apart in
-    // both layouts, so with 4 rows per round two offsets (u even / odd) and a multiple of 1024 give all of them,
-    // with 8 or 16 rows per round one offset and a multiple of 1024 or 2048
-    uint32_t dst_rel[2];
+    const int np_a = ((int)a_row_bytes + 127) / 128, np_b = ((int)b_row_bytes + 127) / 128;  // pieces of a row
+    // this lane's chunk exists in the last piece, which a row that is no whole number of pieces fills in part
+    const bool tail_a = FULL || (np_a - 1) * 128 + cc * 16 < (int)a_row_bytes;
+    const bool tail_b = FULL || (np_b - 1) * 128 + cc * 16 < (int)b_row_bytes;
+    // Where the chunk of round u = 0 .. 3 lies in the operand's stage.  Packed stages: pair j sits in staged row j / pack,
+    // its rows at byte (j % pack) * slot_a of A and (j % pack) * slot_b of B (a position beyond 128 bytes is a further
+    // piece).  Rows 8 apart are 1024 bytes apart in both layouts, so four more rounds are a fixed distance further on.
     const int pack = PACKED ? cfg.pack : 1;
+    const uint32_t row0 = (uint32_t)(pw * rpw + rs) / (uint32_t)pack, row_step = (uint32_t)(rpp / pack);
+    const uint32_t slot = (uint32_t)((pw * rpw + rs) % pack);
+    const uint32_t byte_a = (PACKED ? slot * (uint32_t)cfg.slot_a : 0u) + (uint32_t)cc * 16u;
+    const uint32_t byte_b = (PACKED ? slot * (uint32_t)cfg.slot_b : 0u) + (uint32_t)cc * 16u;
+    uint32_t rel_a[4], rel_b[4];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const uint32_t row = (uint32_t)(pw * rpw + rs + 4 * u);
-      dst_rel[u] = TF32 ? mnmajor32_offset(row, (uint32_t)cc * 16u, lbo, 512u) : mnmajor_offset(row, (uint32_t)cc * 16u, lbo, 1024u);
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t row = row0 + (uint32_t)u * row_step;
+      rel_a[u] = TF32 ? mnmajor32_offset(row, byte_a, lbo, 512u) : mnmajor_offset(row, byte_a, lbo, 1024u);
+      rel_b[u] = TF32 ? mnmajor32_offset(row, byte_b, lbo, 512u) : mnmajor_offset(row, byte_b, lbo, 1024u);
     }
-    const bool four = rpp == 4;
-    const uint32_t u_step = four ? 1024u : (uint32_t)(rpp >> 3) * 1024u;
-    // Packed stages: pair j of the stage sits in staged row j / pack, its rows at byte (j % pack) * slot_a of A and
-    // (j % pack) * slot_b of B (a position beyond 128 bytes is a further piece).  Round u covers the staged row
-    // row0 + u * rpp / pack; the offsets are worked out per round.
-    const uint32_t pk_row0 = (uint32_t)(pw * rpw + rs) / (uint32_t)pack, pk_step = (uint32_t)(rpp / pack);
-    const uint32_t pk_byte_a = (uint32_t)((pw * rpw + rs) % pack) * (uint32_t)cfg.slot_a + (uint32_t)cc * 16u;
-    const uint32_t pk_byte_b = (uint32_t)((pw * rpw + rs) % pack) * (uint32_t)cfg.slot_b + (uint32_t)cc * 16u;
+    const uint32_t four_rounds = row_step * 512u;
     const uint8_t* feats_c = feats + cc * 16;
     const uint8_t* og_c = og + cc * 16;
-    // lane r < rpw fetches both map entries of the warp's row r (-1 beyond the stage)
-    auto load_entry = [&](const G3Walk& w, int* ea, int* eb) {
+    // The pieces of R rows of one operand.  What this role spends its time on are instructions (with the copies left out
+    // the kernel took as long: tests of every one of eight possible pieces and address arithmetic, 400 instructions a
+    // warp and stage), so the usual numbers of pieces have their own straight code.
+    // The pieces of R rows of one operand; the usual numbers of pieces have their own straight code.
+    auto copy_pieces = [&](auto rounds, auto pieces, const uint8_t* const (&from)[4], const uint32_t (&rel)[4], uint32_t to, const uint32_t (&n)[4],
+                           int np, bool tail) {
+      constexpr int R = decltype(rounds)::value, NP = decltype(pieces)::value;
+      if constexpr (NP > 0) {
+#pragma unroll
+        for (int h = 0; h < NP; ++h)
+#pragma unroll
+          for (int u = 0; u < R; ++u)
+            if (FULL || h + 1 < NP || tail) cp_async16_n(to + (uint32_t)h * lbo + rel[u], from[u] + h * 128, n[u]);
+      } else {
+#pragma unroll 1
+        for (int h = 0; h < np; ++h)
+#pragma unroll
+          for (int u = 0; u < R; ++u)
+            if (FULL || h + 1 < np || tail) cp_async16_n(to + (uint32_t)h * lbo + rel[u], from[u] + h * 128, n[u]);
+      }
+    };
+    // rows rs + rpp u of rounds u0 .. u0 + R - 1 of one operand; their entries are in lanes rs + rpp u of `cur`, -1 zero-fills
+    auto copy_rows = [&](auto rounds, int u0, int cur, const uint8_t* base, uint32_t row_bytes, const uint32_t (&rel)[4], uint32_t to, int np, bool tail) {
+      constexpr int R = decltype(rounds)::value;
+      const uint8_t* from[4];
+      uint32_t n[4];
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        const int i = __shfl_sync(0xffffffffu, cur, rs + rpp * (u0 + u));
+        n[u] = i >= 0 ? 16u : 0u;  // 0 bytes read: the chunk is zero-filled
+        from[u] = base + (size_t)max(i, 0) * row_bytes;
+      }
+      if (np == 2) copy_pieces(rounds, std::integral_constant<int, 2>(), from, rel, to, n, np, tail);
+      else if (np == 1) copy_pieces(rounds, std::integral_constant<int, 1>(), from, rel, to, n, np, tail);
+      else if (np == 3) copy_pieces(rounds, std::integral_constant<int, 3>(), from, rel, to, n, np, tail);
+      else if (np == 4) copy_pieces(rounds, std::integral_constant<int, 4>(), from, rel, to, n, np, tail);
+      else copy_pieces(rounds, std::integral_constant<int, 0>(), from, rel, to, n, np, tail);
+    };
+    auto copy_rounds = [&](auto rounds, int u0, int cur_a, int cur_b, uint32_t sa, uint32_t sb) {
+      copy_rows(rounds, u0, cur_a, feats_c, a_row_bytes, rel_a, sa, np_a, tail_a);
+      copy_rows(rounds, u0, cur_b, og_c, b_row_bytes, rel_b, sb, np_b, tail_b);
+    };
+    // lane r < rpw fetches both map entries of the warp's row r (-1 beyond the stage) into its words of a ring slot: copied
+    // there, they are waited for when they are used, where entries handed on through registers were waited for a stage after
+    // they had been asked for
+    const uint32_t ring = smem_u32(sRing) + (uint32_t)(team * (W3_PREFETCH + 1) * pb + pw * rpw + min(lane, rpw - 1)) * 8u;
+    const uint32_t ring_step = (uint32_t)pb * 8u;
+    auto fetch_entry = [&](const G3Walk& w, uint32_t slot) {
       int base, cnt;
       w3_stage(w, pb, kpos_s, &base, &cnt);
       const int row = pw * rpw + lane;
-      *ea = *eb = -1;
-      if (lane < rpw && row < cnt) {
-        *ea = __ldg(p.in_map + base + row);
-        *eb = __ldg(p.out_map + base + row);
+      if (lane >= rpw) return;
+      if (row < cnt) {
+        cp_async4(slot, p.in_map + base + row);
+        cp_async4(slot + 4, p.out_map + base + row);
+      } else {
+        st_shared_i32(slot, -1);
+        st_shared_i32(slot + 4, -1);
       }
     };
     G3Walk pf;
-    pf.init(tile_start, n_seg, t0);
-    int ea[W3_PREFETCH], eb[W3_PREFETCH];
+    if (t0 + team < t1) pf.init(tile_start, n_seg, t0 + team);
+    else pf.t = t1;
+    uint32_t put = 0, get = 0;  // slots, in bytes from the ring's start
+    auto fetch_next = [&]() {
+      if (pf.t < t1) fetch_entry(pf, ring + put);
+      cp_async_commit();  // also closes the group of the stage before
 #pragma unroll
-    for (int d = 0; d < W3_PREFETCH; ++d) {
-      ea[d] = eb[d] = -1;
-      if (pf.t < t1) load_entry(pf, &ea[d], &eb[d]);
-      pf.next(tile_start, n_seg);
-    }
-    int s = 0, sg = 0;  // stage, and its position in its group
+      for (int i = 0; i < W3_PROD_TEAMS; ++i)
+        if (pf.t < t1) pf.next(tile_start, n_seg);
+      put = put == W3_PREFETCH * ring_step ? 0 : put + ring_step;
+    };
+    for (int d = 0; d < W3_PREFETCH; ++d) fetch_next();
+    // Ring slot, its position in its group, the slot's phase.  Waiting by parity is safe with two teams: a team's stage before,
+    // two back, was let in after the one a ring before that had been consumed, and stages are consumed in order, so the barrier
+    // is at most one phase behind the one waited for (a ring has at least two slots, or three groups).
+    int s = team, sg = team % cfg.group;
     uint32_t ph = 0;
-    for (int t = t0; t < t1 && ok; ++t) {
-      int cur_a = ea[0], cur_b = eb[0];
-#pragma unroll
-      for (int d = 0; d + 1 < W3_PREFETCH; ++d) { ea[d] = ea[d + 1]; eb[d] = eb[d + 1]; }
-      ea[W3_PREFETCH - 1] = eb[W3_PREFETCH - 1] = -1;
-      if (pf.t < t1) load_entry(pf, &ea[W3_PREFETCH - 1], &eb[W3_PREFETCH - 1]);
-      pf.next(tile_start, n_seg);
+    for (int t = t0 + team; t < t1 && ok; t += W3_PROD_TEAMS) {
+      fetch_next();
+      cp_async_wait<W3_PREFETCH>();  // this stage's entries have landed
+      int cur_a = -1, cur_b = -1;
+      if (lane < rpw) { cur_a = ld_shared_i32(ring + get); cur_b = ld_shared_i32(ring + get + 4); }
+      get = get == W3_PREFETCH * ring_step ? 0 : get + ring_step;
       // a pair is used only if both its entries are inside the tensors
       if (!((unsigned)cur_a < (unsigned)p.n_in && (unsigned)cur_b < (unsigned)p.n_out)) {
         if (cur_a != -1 || cur_b != -1) report_problem();  // counted once per skipped pair
         cur_a = cur_b = -1;
       }
-      if (sg == 0) {
-        ok = g3_wait(&sh->empty[s], ph ^ 1u, abort_flag);
-        if (!ok) break;
-      }
+      ok = g3_wait(&sh->empty[s - sg], ph ^ 1u, abort_flag);
+      if (!ok) break;
       const uint32_t sa = smem_u32(sStage + (size_t)s * stage_bytes);
       const uint32_t sb = sa + a_bytes;
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (u < n_pass) {
-          const int ia = __shfl_sync(0xffffffffu, cur_a, rs + rpp * u);
-          const int ib = __shfl_sync(0xffffffffu, cur_b, rs + rpp * u);
-          const uint32_t na = ia >= 0 ? 16u : 0u, nb = ib >= 0 ? 16u : 0u;  // 0 bytes read: the chunk is zero-filled
-          const uint8_t* pa = feats_c + (size_t)max(ia, 0) * a_row_bytes;
-          const uint8_t* pb_ = og_c + (size_t)max(ib, 0) * b_row_bytes;
-          uint32_t rel_a, rel_b;
-          if (!PACKED) {
-            rel_a = rel_b = four ? dst_rel[u & 1] + (uint32_t)(u >> 1) * 1024u : dst_rel[0] + (uint32_t)u * u_step;
-          } else {
-            const uint32_t row = pk_row0 + (uint32_t)u * pk_step;
-            rel_a = TF32 ? mnmajor32_offset(row, pk_byte_a, lbo, 512u) : mnmajor_offset(row, pk_byte_a, lbo, 1024u);
-            rel_b = TF32 ? mnmajor32_offset(row, pk_byte_b, lbo, 512u) : mnmajor_offset(row, pk_byte_b, lbo, 1024u);
-          }
-          const uint32_t da = sa + rel_a, db = sb + rel_b;
-#pragma unroll
-          for (int h = 0; h < 8; ++h)
-            if (h < nha) cp_async16_n(da + (uint32_t)h * lbo, pa + h * 128, na);
-#pragma unroll
-          for (int h = 0; h < 8; ++h)
-            if (h < nhb) cp_async16_n(db + (uint32_t)h * lbo, pb_ + h * 128, nb);
-        }
+      if (n_pass >= 4) {
+        for (int u0 = 0; u0 < n_pass; u0 += 4) copy_rounds(std::integral_constant<int, 4>(), u0, cur_a, cur_b, sa + (uint32_t)(u0 >> 2) * four_rounds, sb + (uint32_t)(u0 >> 2) * four_rounds);
+      } else if (n_pass == 2) {
+        copy_rounds(std::integral_constant<int, 2>(), 0, cur_a, cur_b, sa, sb);
+      } else {
+        copy_rounds(std::integral_constant<int, 1>(), 0, cur_a, cur_b, sa, sb);
       }
       // the stage's barrier hears from this thread when everything it has issued so far has landed
       cp_async_arrive_noinc(smem_u32(&sh->full[s]));
-      if (++sg == cfg.group) sg = 0;
-      if (++s == n_stage) { s = 0; ph ^= 1u; }
+      s += W3_PROD_TEAMS;
+      if (s >= n_stage) { s -= n_stage; ph ^= 1u; }
+      sg += W3_PROD_TEAMS;
+      while (sg >= cfg.group) sg -= cfg.group;
     }
   } else if (warp == W3_MMA_WARP) {
     // ------------------------------------------------------------------ MMA issuer
@@ -266,52 +315,56 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
       a_desc0[mt] = make_sdesc(stage0 + (uint32_t)mt * mtile_stride, mt + 1 == cfg.n_mtile ? last_lbo : lbo, sbo, ltype);
+    const int n_ks = kr / UK;  // 2, 4, 8 or 16
     const uint32_t ks_step = (uint32_t)UK * 8u;  // UK contraction rows of 128 bytes, in 16-byte units
-    G3Walk cur;
-    cur.init(tile_start, n_seg, t0);
-    int s = 0, sg = 0, run_i = 0, cur_seg = -1;
-    uint32_t ph = 0;
-    bool first = true;
     // One lane, named by elect.sync (see elect_one), runs the whole loop — waits, issue, commits — so that no warp-wide
-    // hand-shake sits between a stage landing and its MMAs; the other lanes wait at the end.
-    if (elect_one()) {
-    for (int t = t0; t < t1 && ok; ++t) {
-      if (cur.seg != cur_seg) {
-        if (cur_seg >= 0) {
-          mma_commit(smem_u32(&sh->tmem_full[run_i & (cfg.n_buf - 1)]));
-          ++run_i;
-        }
-        cur_seg = cur.seg;
-        first = true;
-        const uint32_t use = (uint32_t)run_i >> cfg.buf_shift;
-        ok = mbar_wait(smem_u32(&sh->tmem_empty[run_i & (cfg.n_buf - 1)]), (use & 1u) ^ 1u, abort_flag);
-        if (!ok) break;
+    // hand-shake sits between a stage landing and its MMAs; the other lanes wait at the end.  A loop over the CTA's offsets
+    // around one over an offset's stages, whose body has its row tiles and (eight, four or two at a time) its steps written
+    // out: tests and branches are what this lane spends its time on.
+    auto issue = [&](auto row_tiles, auto steps) -> bool {
+      constexpr int MT = decltype(row_tiles)::value, N = decltype(steps)::value;
+      const uint32_t idesc0 = MT == 1 ? idesc_last : idesc_full;
+      int s = 0, sg = 0, buf = 0;
+      uint32_t ph = 0, buf_ph = 1;
+      int t = t0, seg = find_segment(tile_start, n_seg, t0);
+      while (t < t1) {
+        while (t >= tile_start[seg + 1]) ++seg;
+        const int run_end = min(t1, tile_start[seg + 1]);
+        if (!mbar_wait(smem_u32(&sh->tmem_empty[buf]), buf_ph, abort_flag)) return false;
         tc_fence_after();
-      }
-      const int buf = run_i & (cfg.n_buf - 1);
-      ok = mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag);
-      if (!ok) break;
-      {
-        fence_proxy_async();  // the stage was written through cp.async; the MMA reads it through the async proxy
-        tc_fence_after();
-        const uint64_t s_off = (uint64_t)((uint32_t)s * (stage_bytes >> 4));
         const uint32_t d0 = tmem_base + (uint32_t)buf * buf_cols;
-        for (int ks = 0; ks < kr / UK; ++ks) {
-          const uint64_t off = s_off + (uint64_t)((uint32_t)ks * ks_step);
-          mma_ss<TF32>(d0, a_desc0[0] + off, b_desc0 + off, cfg.n_mtile == 1 ? idesc_last : idesc_full, !(first && ks == 0));
-          if (cfg.n_mtile == 2)
-            mma_ss<TF32>(d0 + (uint32_t)cfg.n_acc, a_desc0[1] + off, b_desc0 + off, idesc_last, !(first && ks == 0));
+        bool more = false;  // the accumulator holds something
+        for (; t < run_end; ++t) {
+          if (!mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag)) return false;
+          fence_proxy_async();  // the stage was written through cp.async; the MMA reads it through the async proxy
+          tc_fence_after();
+          uint64_t off = (uint64_t)((uint32_t)s * (stage_bytes >> 4));
+          for (int ks = 0; ks < n_ks; ks += N) {
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+              mma_ss<TF32>(d0, a_desc0[0] + off, b_desc0 + off, idesc0, more || i > 0);
+              if (MT == 2) mma_ss<TF32>(d0 + (uint32_t)cfg.n_acc, a_desc0[1] + off, b_desc0 + off, idesc_last, more || i > 0);
+              off += ks_step;
+            }
+            more = true;
+          }
+          // one commit per group of stages (and one for the CTA's last stage, which nobody waits for)
+          if (sg == cfg.group - 1 || t + 1 == t1) mma_commit(smem_u32(&sh->empty[s - sg]));
+          sg = sg == cfg.group - 1 ? 0 : sg + 1;
+          if (++s == n_stage) { s = 0; ph ^= 1u; }
         }
-        // one commit per group of stages (and one for the CTA's last stage, which nobody waits for)
-        if (sg == cfg.group - 1 || t + 1 == t1) mma_commit(smem_u32(&sh->empty[s - sg]));
+        mma_commit(smem_u32(&sh->tmem_full[buf]));
+        if (++buf == cfg.n_buf) { buf = 0; buf_ph ^= 1u; }
       }
-      first = false;
-      if (++sg == cfg.group) sg = 0;
-      if (++s == n_stage) { s = 0; ph ^= 1u; }
-      cur.next(tile_start, n_seg);
-    }
-    if (ok && cur_seg >= 0) mma_commit(smem_u32(&sh->tmem_full[run_i & (cfg.n_buf - 1)]));
-    mma_drain(smem_u32(&sh->drained));
+      return true;
+    };
+    if (elect_one()) {
+      using One = std::integral_constant<int, 1>;
+      using Two = std::integral_constant<int, 2>;
+      if (n_ks >= 8) ok = cfg.n_mtile == 1 ? issue(One(), std::integral_constant<int, 8>()) : issue(Two(), std::integral_constant<int, 8>());
+      else if (n_ks == 4) ok = cfg.n_mtile == 1 ? issue(One(), std::integral_constant<int, 4>()) : issue(Two(), std::integral_constant<int, 4>());
+      else ok = cfg.n_mtile == 1 ? issue(One(), Two()) : issue(Two(), Two());
+      mma_drain(smem_u32(&sh->drained));
     }
     __syncwarp();
     ok = __all_sync(0xffffffffu, ok) != 0;
@@ -461,13 +514,13 @@ inline bool w3_plan(int c_in, int c_out, int es, int k_vol, int max_smem, W3Conf
   if (buf_cols > 512) { if (cfg->pack > 1) continue; return false; }
   cfg->n_buf = 4 * buf_cols <= 512 ? 4 : (2 * buf_cols <= 512 ? 2 : 1);
   cfg->buf_shift = cfg->n_buf == 4 ? 2 : (cfg->n_buf == 2 ? 1 : 0);
-  // pairs per stage: 4, 8, 16 or 32 rows per producer warp (packed stages: always 32, the stage is small)
+  // pairs per stage: 8, 16 or 32 rows per producer warp (packed stages: always 32, the stage is small)
   int pb = W3_MAX_PB;
   const int fixed = 1024 + W3_PATCH_BYTES + W3_SHARED_BYTES + (((2 * k_vol + 3) * 4 + 15) & ~15);
   const int row_bytes = 128 * (cfg->pa + cfg->pbp) / cfg->pack;  // staged bytes per pair
   // keep at least three stages in flight; a packed stage keeps the producers' round a whole number of staged rows
-  while (pb > (cfg->pack > 1 ? 128 : 32) && (max_smem - fixed) / (pb * row_bytes) < 3) pb >>= 1;
-  int n_stage = (max_smem - fixed) / (pb * row_bytes);
+  while (pb > (cfg->pack > 1 ? 128 : 32) && (max_smem - fixed - w3_ring_bytes(pb)) / (pb * row_bytes) < 3) pb >>= 1;
+  int n_stage = (max_smem - fixed - w3_ring_bytes(pb)) / (pb * row_bytes);
   if (n_stage > W3_MAX_STAGES) n_stage = W3_MAX_STAGES;
   if (cfg->pack > 1 && n_stage < 3) continue;  // too large packed: plan it unpacked
   if (n_stage < 2) return false;
@@ -477,7 +530,7 @@ inline bool w3_plan(int c_in, int c_out, int es, int k_vol, int max_smem, W3Conf
     if ((n_stage - n_stage % g) / g >= 3) { cfg->group = g; n_stage -= n_stage % g; break; }
   cfg->pb = pb;
   cfg->n_stage = n_stage;
-  cfg->smem = fixed + n_stage * pb * row_bytes;
+  cfg->smem = fixed + w3_ring_bytes(pb) + n_stage * pb * row_bytes;
   return true;
   }
   return false;
