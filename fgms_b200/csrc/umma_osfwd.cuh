@@ -18,10 +18,17 @@
 // matter (the accumulators are cleared by the epilogue before the first MMA).
 //
 // Roles (20 warps): 12 producers, each filling whole stages (16-byte cp.async gathers into the K-major 128-byte-swizzled
-// ring), one MMA warp, one warp that loads weights by TMA, 4 epilogue warps.  All waits are bounded; all but the MMA lane's
-// are parked (85 -> 79 us on the layer below).  64 -> 64 on a full block of 48^3 (2.9 M pairs, 27 stages for each of 864 tiles):
-// 141 us with eight warps that each filled 16 rows of every stage and copied zeros, 56 us now: 650 cycles a stage, of which
-// 400-580 are the stage's 32 warp-wide copies; 128 -> 128 246 -> 93 us, 1000 voxels 64 -> 64 32 -> 15 us.
+// ring), up to three MMA warps, one warp that loads weights by TMA, 4 epilogue warps.  All waits are bounded; all but the MMA
+// lanes' are parked (85 -> 79 us on the layer below).
+//
+// An MMA lane's stage is some 130 instructions one after the other, 540-650 cycles, of which it waits for rows during 95; its four
+// MMAs of 128 x 64 x 16 are 192.  So the work is dealt to up to three pipelines, each an MMA lane with ring slots and
+// producers of its own: tiles of a group, or, where a CTA has fewer than three tiles, offsets, whose partial accumulators the
+// epilogue adds in the pipelines' order.  Against one pipeline: 64 -> 64 on a full block of 48^3 (2.9 M pairs, 27 stages for each of
+// 864 tiles) 55.9 -> 40.7 us, 400 cycles a stage, of which shared memory needs 320 (rows written, rows and weights read by the
+// MMAs); 32 -> 32 52.4 -> 35.1; 64 -> 64 on a surface of 100 k voxels 54.7 -> 39.1, on 30^3 26.5 -> 20.4, on 1000 voxels 14.8 -> 12.6 (by
+// offsets); 128 -> 128 on 48^3 95 -> 92; 256 -> 256 on 512 voxels, which has slots for one pipeline only, 72.5 -> 73.4.
+// (With eight warps that each filled 16 rows of every stage and copied zeros the block took 141 us.)
 #pragma once
 #include "common.cuh"
 #include "umma.cuh"
@@ -30,7 +37,10 @@
 namespace fgms {
 
 constexpr int OS_EPI_WARPS = 4;
-constexpr int OS_MMA_WARP = 4;
+constexpr int OS_MMA_WARP = 4;   // and 12 and 16: one per pipeline, all on one scheduler
+constexpr int OS_MAX_PIPES = 3;
+// pipeline of an MMA warp (< 0: none)
+__device__ __forceinline__ int os_mma_pipe(int warp) { return warp == 4 ? 0 : warp == 12 ? 1 : warp == 16 ? 2 : -1; }
 constexpr int OS_W_WARP = 8;
 constexpr int OS_PROD_WARPS = 12;
 constexpr int OS_THREADS = 640;
@@ -43,7 +53,10 @@ constexpr int OS_MAX_GROUP = 8;  // tiles walked together, an accumulator each
 
 struct OsConfig {
   int n_stage, n_wbuf, w_bytes;
-  int n_prod;  // producer warps that work: no more than there are stages (see the producers)
+  int n_pipe;  // pipelines: each an MMA warp with producers and n_stage / n_pipe ring slots of its own
+  int by_offset;  // 0: the tiles of a group are dealt to the pipelines; 1: the offsets are, every pipeline has an accumulator of
+                  // its own for each of the CTA's tiles (which are one group), and the epilogue adds them up
+  int n_prod;  // producer warps of a pipeline that work: no more than it has slots (see the producers)
   int kch;     // 128-byte chunks of an input row (= stages of a tile and offset)
   int n_acc;   // tensor-memory columns of an accumulator: whole 128-byte blocks of the output row
   int group;   // tiles walked together
@@ -69,10 +82,10 @@ struct OsShared {
   uint64_t empty[OS_MAX_STAGES];  // stage consumed (tcgen05.commit)
   uint64_t tmem_full[OS_MAX_GROUP];
   uint64_t tmem_empty[OS_MAX_GROUP];  // accumulator read and cleared (one arrival per epilogue warp)
-  uint64_t w_full[2];
-  uint64_t w_free[2];
+  uint64_t w_full[2 * OS_MAX_PIPES];
+  uint64_t w_free[2 * OS_MAX_PIPES];
   uint4 on[OS_MAX_STAGES];  // rows a stage holds, a bit each
-  uint64_t drained;  // every MMA has finished
+  uint64_t drained[OS_MAX_PIPES];  // every MMA of the pipeline has finished
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -102,7 +115,8 @@ __global__ void os_fill_nbr_kernel(const int32_t* __restrict__ kpos, const int32
   }
 }
 
-template <bool TF32>
+// BY_OFFSET: cfg.by_offset, known at compile time (asked at run time it cost every stage of the other form 2-6 %)
+template <bool TF32, bool BY_OFFSET = false>
 __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, OsConfig cfg, const __grid_constant__ CUtensorMap w_map) {
   using namespace umma;
   constexpr int ES = TF32 ? 4 : 2;
@@ -115,12 +129,14 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
   OsShared* sh = reinterpret_cast<OsShared*>(sPatch + OS_EPI_WARPS * 4096);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int kch = cfg.kch, n_stage = cfg.n_stage, gsz = cfg.group;
+  const int kch = cfg.kch, n_pipe = cfg.n_pipe, n_slot = cfg.n_stage / n_pipe, gsz = cfg.group;  // ring slots of a pipeline
+  constexpr bool by_offset = BY_OFFSET;
+  const int n_part = by_offset ? n_pipe : 1;  // accumulators of a tile
   const int k_bytes = p.c_in * ES;
   volatile int* abort_flag = &sh->abort_flag;
 
   if (tid == 0) {
-    for (int s = 0; s < n_stage; ++s) {
+    for (int s = 0; s < cfg.n_stage; ++s) {
       mbar_init(smem_u32(&sh->full[s]), 33);
       mbar_init(smem_u32(&sh->empty[s]), 1);
     }
@@ -128,16 +144,16 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
       mbar_init(smem_u32(&sh->tmem_full[b]), 1);
       mbar_init(smem_u32(&sh->tmem_empty[b]), OS_EPI_WARPS);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < 2 * OS_MAX_PIPES; ++b) {
       mbar_init(smem_u32(&sh->w_full[b]), 1);
-      mbar_init(smem_u32(&sh->w_free[b]), 1);
+      mbar_init(smem_u32(&sh->w_free[b]), by_offset ? 1 : n_pipe);
     }
-    mbar_init(smem_u32(&sh->drained), 1);
+    for (int b = 0; b < OS_MAX_PIPES; ++b) mbar_init(smem_u32(&sh->drained[b]), 1);
     sh->abort_flag = 0;
     mbar_fence_init();
   }
   uint32_t tmem_cols = 32;
-  while (tmem_cols < (uint32_t)(gsz * cfg.n_acc)) tmem_cols <<= 1;
+  while (tmem_cols < (uint32_t)(gsz * n_part * cfg.n_acc)) tmem_cols <<= 1;
   if (warp == OS_MMA_WARP) {
     tmem_alloc(smem_u32(&sh->tmem_base), tmem_cols);
     tmem_relinquish();
@@ -153,19 +169,23 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
   int t0, t1;
   cta_tile_range(p.n_tiles, &t0, &t1);
   bool ok = true;
+  // Pipeline m has tiles m, m + n_pipe, ... of a group, or offsets m, m + n_pipe, ...; its stages come offset by offset, tile by tile,
+  // chunk by chunk.
+  auto tiles_of = [&](int tb, int pipe) { return by_offset ? min(gsz, t1 - tb) : (min(gsz, t1 - tb) - pipe + n_pipe - 1) / n_pipe; };
+  auto offsets_of = [&](int pipe) { return by_offset ? (p.k_vol - pipe + n_pipe - 1) / n_pipe : p.k_vol; };
 
   if (t0 >= t1) {
     // nothing for this CTA
-  } else if (os_producer(warp) >= cfg.n_prod) {
-    // more warps than stages
+  } else if (os_producer(warp) >= n_pipe * cfg.n_prod || os_mma_pipe(warp) >= n_pipe) {
+    // more warps than slots, or than pipelines
   } else if (os_producer(warp) >= 0) {
     // ------------------------------------------------------------------ producers
-    // Warp w fills stages w, w + nw, ...  With nw <= n_stage a wait for a ring slot by parity is safe: the warp's stage
-    // before, q - nw, was let in after stage q - nw - n_stage had been consumed, stages are consumed in order, and so the slot's
+    // Warp w of a pipeline fills its stages w, w + nw, ...  With nw <= n_slot a wait for a ring slot by parity is safe: the warp's stage
+    // before, q - nw, was let in after stage q - nw - n_slot had been consumed, stages are consumed in order, and so the slot's
     // barrier is at most one phase behind the one that stage q waits for.  (With more warps than slots it may be two behind,
     // which looks the same, and two warps fill one slot.)  Lane l holds the neighbour entries of the tile's rows l, l + 32,
     // l + 64, l + 96, and copies 16-byte chunk l % 8 of the rows l / 8, l / 8 + 4, ...
-    const int w = os_producer(warp), nw = cfg.n_prod;
+    const int pipe = os_producer(warp) % n_pipe, w = os_producer(warp) / n_pipe, nw = cfg.n_prod;
     const int rs = lane >> 3, pc = lane & 7;
     const uint8_t* src = static_cast<const uint8_t*>(p.src) + pc * 16;
     uint32_t a_dst[2];  // rows rs, rs + 4 of a group of eight
@@ -178,14 +198,16 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
     int s = w, base = 0;  // the warp's next ring slot, stages of the groups before
     uint32_t ph = 0;
     for (int tb = t0; tb < t1 && ok; tb += gsz) {
-      // the group's stages: offset k, then r = tile of the group * kch + chunk
-      const int per_k = min(gsz, t1 - tb) * kch, n = per_k * p.k_vol;
+      // the pipeline's stages of the group: offset k, then r = tile of the pipeline * kch + chunk
+      const int per_k = tiles_of(tb, pipe) * kch, n = per_k * offsets_of(pipe);
+      if (n == 0) continue;
       const int first = (w + nw - base % nw) % nw;
       const int step_k = nw / per_k, step_r = nw % per_k;
       int k = first / per_k, r = first % per_k;
       auto load_entries = [&](int (&e)[4]) {
         const int g = (int)((uint32_t)r * kch_recip >> 16);
-        const int32_t* at = p.nbr + (long long)k * p.nbr_stride + (long long)(tb + g) * OS_TILE + lane;
+        const int tile = tb + (by_offset ? g : pipe + n_pipe * g), offset = by_offset ? pipe + n_pipe * k : k;
+        const int32_t* at = p.nbr + (long long)offset * p.nbr_stride + (long long)tile * OS_TILE + lane;
 #pragma unroll
         for (int x = 0; x < 4; ++x) e[x] = __ldg(at + 32 * x);
       };
@@ -193,7 +215,8 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
       if (first < n) load_entries(e);
       for (int i = first; i < n; i += nw) {
         const int kc = r - (int)((uint32_t)r * kch_recip >> 16) * kch;
-        ok = g3_wait(&sh->empty[s], ph ^ 1u, abort_flag);
+        const int slot = pipe * n_slot + s;
+        ok = g3_wait(&sh->empty[slot], ph ^ 1u, abort_flag);
         if (!ok) break;
         int ent[4];
         uint32_t on[4];
@@ -207,7 +230,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
         k += step_k; r += step_r;
         if (r >= per_k) { r -= per_k; ++k; }
         if (i + nw < n) load_entries(e);
-        const uint32_t st = smem_u32(sStage) + (uint32_t)s * G3_STAGE_BYTES;
+        const uint32_t st = smem_u32(sStage) + (uint32_t)slot * G3_STAGE_BYTES;
         const uint8_t* from = src + kc * 128;
         // a place whose row has no neighbour keeps what it held: the MMA leaves that accumulator row alone
         const bool pc_ok = kc * 128 + pc * 16 < k_bytes;
@@ -217,12 +240,12 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
           if (g >= 0 && pc_ok) cp_async16(st + a_dst[x & 1] + (uint32_t)(x >> 1) * 1024u, from + (size_t)(unsigned)g * (uint32_t)k_bytes, true);
         }
         if (lane == 0) {
-          sh->on[s] = make_uint4(on[0], on[1], on[2], on[3]);
-          mbar_arrive(smem_u32(&sh->full[s]));
+          sh->on[slot] = make_uint4(on[0], on[1], on[2], on[3]);
+          mbar_arrive(smem_u32(&sh->full[slot]));
         }
-        cp_async_arrive_noinc(smem_u32(&sh->full[s]));
+        cp_async_arrive_noinc(smem_u32(&sh->full[slot]));
         s += nw;
-        if (s >= n_stage) { s -= n_stage; ph ^= 1u; }
+        if (s >= n_slot) { s -= n_slot; ph ^= 1u; }
       }
       base += n;
     }
@@ -230,27 +253,31 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
     // ------------------------------------------------------------------ weights: W_k, once per group and offset, a TMA box per
     // 128-byte column block (by one warp with cp.async it bounded wide layers: 128 -> 128 on a full block of 48^3 270 us)
     if (elect_one()) {
-      int n_load = 0;
+      int wb = 0, loads = 0;
+      uint32_t w_ph = 0;
       for (int tb = t0; tb < t1 && ok; tb += gsz)
-        for (int k = 0; k < p.k_vol; ++k, ++n_load) {
-          const int wb = cfg.n_wbuf == 2 ? n_load & 1 : 0;
-          const uint32_t use = (uint32_t)(cfg.n_wbuf == 2 ? n_load >> 1 : n_load);
-          ok = mbar_parked_wait(smem_u32(&sh->w_free[wb]), (use & 1u) ^ 1u, abort_flag);
+        for (int k = 0; k < p.k_vol; ++k) {
+          ok = mbar_parked_wait(smem_u32(&sh->w_free[wb]), w_ph ^ 1u, abort_flag);
           if (!ok) break;
           const uint32_t bar = smem_u32(&sh->w_full[wb]), sw = smem_u32(sW + (size_t)wb * cfg.w_bytes);
           mbar_expect_tx(bar, (uint32_t)cfg.w_bytes);
           for (int b = 0; b * EPR < cfg.n_acc; ++b) tma_load_2d(sw + (uint32_t)(b * p.c_in) * 128u, &w_map, bar, b * EPR, k * p.c_in);
+          if (loads < cfg.n_wbuf) ++loads;
+          if (++wb == cfg.n_wbuf) { wb = 0; w_ph ^= 1u; }
         }
-      // the CTA's shared memory outlives its copies, also after a wait that ran out
-      for (int i = max(0, n_load - cfg.n_wbuf); i < n_load; ++i)
-        mbar_parked_wait(smem_u32(&sh->w_full[cfg.n_wbuf == 2 ? i & 1 : 0]), (uint32_t)(cfg.n_wbuf == 2 ? i >> 1 : i) & 1u, nullptr);
+      // the CTA's shared memory outlives its copies, also after a wait that ran out: the last load of every buffer
+      for (; loads > 0; --loads) {
+        if (--wb < 0) { wb = cfg.n_wbuf - 1; w_ph ^= 1u; }
+        mbar_parked_wait(smem_u32(&sh->w_full[wb]), w_ph, nullptr);
+      }
     }
     __syncwarp();
     ok = __all_sync(0xffffffffu, ok) != 0;
-  } else if (warp == OS_MMA_WARP) {
-    // ------------------------------------------------------------------ MMA issuer
+  } else if (os_mma_pipe(warp) >= 0) {
+    // ------------------------------------------------------------------ MMA issuers
     const uint32_t idesc = make_idesc(TF32, false, true, OS_TILE, cfg.n_acc);
-    const uint64_t a_desc0 = make_sdesc(smem_u32(sStage), 16u, 1024u);
+    const int pipe = os_mma_pipe(warp);
+    const uint64_t a_desc0 = make_sdesc(smem_u32(sStage) + (uint32_t)(pipe * n_slot) * G3_STAGE_BYTES, 16u, 1024u);
     const uint64_t b_desc0 = make_sdesc(smem_u32(sW), (uint32_t)p.c_in * 128u, TF32 ? 512u : 1024u, TF32 ? 1u : 2u);
     constexpr uint32_t B_KC = (uint32_t)EPR * 8u, B_KS = (32u / ES) * 8u;  // one 128-byte K chunk / 32-byte MMA step further, in 16-byte units
     // One lane, named by elect.sync (see elect_one), runs the whole loop (waits, issue, commits); the other lanes wait at the
@@ -259,19 +286,24 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
     // accumulator whose rows or weights did not land reaches the epilogue, none that it may still be reading is written, and no
     // stage or buffer is handed back that is still being filled (one test of all waits behind a stage's last: 57.5 us).
     if (elect_one()) {
-      int s = 0, wb = 0, grp = 0, g = 0, kc = 0;  // ring slot, weight buffer, group; tile of the group, chunk of its row
+      // accumulators: the tiles' of the pipeline, or every tile's part of it
+      const int g_step = n_pipe, w_step = by_offset ? n_pipe : 1;  // (weight buffers are a multiple of the pipelines then)
+      int s = 0, wb = by_offset ? pipe : 0, grp = 0, g = pipe, kc = 0;  // ring slot, weight buffer, group; accumulator, chunk of the row
+      const uint32_t full = smem_u32(sh->full + pipe * n_slot), empty = smem_u32(sh->empty + pipe * n_slot);
+      const uint4* const rows_on = sh->on + pipe * n_slot;
       uint32_t ph = 0, w_ph = 0;
       auto take_weights = [&]() { return mbar_wait(smem_u32(&sh->w_full[wb]), w_ph, abort_flag, cfg.w_limit); };
       auto free_weights = [&]() {
         mma_commit(smem_u32(&sh->w_free[wb]));
-        if (++wb == cfg.n_wbuf) { wb = 0; w_ph ^= 1u; }
-        g = 0;
+        wb += w_step;
+        if (wb >= cfg.n_wbuf) { wb -= cfg.n_wbuf; w_ph ^= 1u; }
+        g = pipe;
       };
       auto stage = [&](bool first_k, bool last_k) -> bool {
         // first offset of the group: the accumulator must have been read and cleared
         if (first_k && kc == 0 && !mbar_wait(smem_u32(&sh->tmem_empty[g]), (uint32_t)grp & 1u, abort_flag)) return false;
-        if (!mbar_wait(smem_u32(&sh->full[s]), ph, abort_flag)) return false;
-        const uint4 on = sh->on[s];
+        if (!mbar_wait(full + 8u * (uint32_t)s, ph, abort_flag)) return false;
+        const uint4 on = rows_on[s];
         fence_proxy_async();  // the stage was written through cp.async; the MMA reads it through the async proxy
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(g * cfg.n_acc);
@@ -282,36 +314,36 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
         for (int ks = 0; ks < 4; ++ks)
           if (ks < n_ks)
             mma_ss_masked<TF32>(d_tmem, a_desc + (uint64_t)(ks * 2), b_desc + (uint64_t)((uint32_t)ks * B_KS), idesc, ~on.x, ~on.y, ~on.z, ~on.w);
-        mma_commit(smem_u32(&sh->empty[s]));
-        if (++s == n_stage) { s = 0; ph ^= 1u; }
+        mma_commit(empty + 8u * (uint32_t)s);
+        if (++s == n_slot) { s = 0; ph ^= 1u; }
         if (++kc == kch) {
           if (last_k) mma_commit(smem_u32(&sh->tmem_full[g]));
-          kc = 0; ++g;
+          kc = 0; g += g_step;
         }
         return true;
       };
       auto all_stages = [&]() -> bool {
         for (int tb = t0; tb < t1; tb += gsz, ++grp) {
-          const int per_k = min(gsz, t1 - tb) * kch;
+          const int per_k = tiles_of(tb, pipe) * kch, n_k = offsets_of(pipe);
           if (per_k == 1) {
             // a single stage per offset: one loop over the offsets (1000 voxels 64 -> 64 15.0 us, 17.7 with a loop inside it)
-            for (int k0 = 0; k0 < p.k_vol; k0 += OS_UNROLL) {
+            for (int k0 = 0; k0 < n_k; k0 += OS_UNROLL) {
 #pragma unroll
               for (int u = 0; u < OS_UNROLL; ++u) {
-                if (k0 + u >= p.k_vol) break;
+                if (k0 + u >= n_k) break;
                 if (!take_weights()) return false;
-                if (!stage(k0 + u == 0, k0 + u + 1 == p.k_vol)) return false;
+                if (!stage(k0 + u == 0, k0 + u + 1 == n_k)) return false;
                 free_weights();
               }
             }
           } else {
-            for (int k = 0; k < p.k_vol; ++k) {
+            for (int k = 0; k < n_k; ++k) {
               if (!take_weights()) return false;
               for (int r0 = 0; r0 < per_k; r0 += OS_UNROLL) {
 #pragma unroll
                 for (int u = 0; u < OS_UNROLL; ++u) {
                   if (r0 + u >= per_k) break;
-                  if (!stage(k == 0, k + 1 == p.k_vol)) return false;
+                  if (!stage(k == 0, k + 1 == n_k)) return false;
                 }
               }
               free_weights();
@@ -321,7 +353,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
         return true;
       };
       ok = all_stages();
-      mma_drain(smem_u32(&sh->drained));
+      mma_drain(smem_u32(&sh->drained[pipe]));
     }
     __syncwarp();
     ok = __all_sync(0xffffffffu, ok) != 0;
@@ -336,7 +368,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
     uint8_t* patch = sPatch + warp * 4096;
     const uint32_t sw7 = (uint32_t)(lane & 7);
     const uint32_t ch = (uint32_t)(lane & 7), rsub = (uint32_t)(lane >> 3);
-    for (int g = 0; g < min(gsz, t1 - t0); ++g)
+    for (int g = 0; g < min(gsz, t1 - t0) * n_part; ++g)
       for (int c = 0; c < cfg.n_acc; c += 16) tmem_zero16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(g * cfg.n_acc + c));
     tmem_st_wait();
     tc_fence_before();
@@ -346,11 +378,11 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
     for (int tb = t0; tb < t1 && ok; tb += gsz, ++grp_i) {
       const int gv = min(gsz, t1 - tb);
       for (int g = 0; g < gv && ok; ++g) {
-        ok = g3_wait(&sh->tmem_full[g], (uint32_t)grp_i & 1u, abort_flag);
+        for (int q = 0; q < n_part && ok; ++q) ok = g3_wait(&sh->tmem_full[g * n_part + q], (uint32_t)grp_i & 1u, abort_flag);
         if (!ok) break;
         tc_fence_after();
         const int row0 = (tb + g) * OS_TILE + 32 * warp;  // output row of this warp's lane 0
-        const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(g * cfg.n_acc);
+        const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(g * n_part * cfg.n_acc);
         for (uint32_t cb = 0; cb < row_bytes; cb += 128) {
           const uint32_t vb = min(128u, row_bytes - cb);  // bytes of this block that belong to the row
           const uint32_t col0 = cb / ES;
@@ -364,6 +396,12 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
             float f[16];
 #pragma unroll
             for (int k = 0; k < 16; ++k) f[k] = __uint_as_float(v[k]);
+            for (int q = 1; q < n_part; ++q) {  // (one group: these accumulators are not used again)
+              tmem_ld16(taddr + (uint32_t)(q * cfg.n_acc) + col0 + c0, v);
+              tmem_ld_wait();
+#pragma unroll
+              for (int k = 0; k < 16; ++k) f[k] += __uint_as_float(v[k]);
+            }
             if (p.bias != nullptr) {
               if (TF32) {
                 const float4* b4 = reinterpret_cast<const float4*>(static_cast<const float*>(p.bias) + col0 + c0);
@@ -451,10 +489,47 @@ inline bool os_plan(int c_in, int c_out, int es, int max_smem, OsConfig* cfg) {
   cfg->n_stage = (max_smem - fixed - cfg->n_wbuf * cfg->w_bytes) / G3_STAGE_BYTES;
   if (cfg->n_stage > OS_MAX_STAGES) cfg->n_stage = OS_MAX_STAGES;
   if (cfg->n_stage < 2) return false;
+  cfg->n_pipe = 1;
+  cfg->by_offset = 0;
   cfg->n_prod = cfg->n_stage < OS_PROD_WARPS ? cfg->n_stage : OS_PROD_WARPS;
   cfg->smem = fixed + cfg->n_wbuf * cfg->w_bytes + cfg->n_stage * G3_STAGE_BYTES;
   cfg->w_limit = umma::WAIT_LIMIT_CYCLES;
   return true;
+}
+
+// Pipelines for CTAs of up to `tiles` tiles.  Where a CTA has too few tiles to deal out, the offsets are dealt out, if their
+// accumulators fit tensor memory and a weight buffer or two for every pipeline leave each two ring slots.
+inline void os_split(OsConfig* cfg, int tiles, int k_vol, int max_smem) {
+  int n = OS_MAX_PIPES;
+  while (n > 1 && (tiles < n || cfg->group < n || cfg->n_stage < 3 * n)) --n;
+  const int other = cfg->smem - cfg->n_wbuf * cfg->w_bytes - cfg->n_stage * G3_STAGE_BYTES;
+  for (int m = OS_MAX_PIPES; m > n && tiles < OS_MAX_PIPES; --m) {
+    if (m > k_vol || tiles * m > OS_MAX_GROUP || tiles * m * cfg->n_acc > 512) continue;
+    for (int wbufs = 2 * m; wbufs >= m; wbufs -= m) {
+      const int stages = (max_smem - other - wbufs * cfg->w_bytes) / G3_STAGE_BYTES;
+      if (max_smem - other < wbufs * cfg->w_bytes || stages < (wbufs > m ? 3 : 2) * m) continue;
+      cfg->by_offset = 1;
+      cfg->n_pipe = m;
+      cfg->n_wbuf = wbufs;
+      cfg->n_stage = stages < OS_MAX_STAGES ? stages : OS_MAX_STAGES;
+      cfg->group = tiles;
+      cfg->smem = other + cfg->n_wbuf * cfg->w_bytes + cfg->n_stage * G3_STAGE_BYTES;
+      const int most = OS_PROD_WARPS / m, slots = cfg->n_stage / m;
+      cfg->n_prod = slots < most ? slots : most;
+      return;
+    }
+  }
+  cfg->n_pipe = n;
+  cfg->group = cfg->group / n * n;
+  const int most = OS_PROD_WARPS / n, slots = cfg->n_stage / n;
+  cfg->n_prod = slots < most ? slots : most;
+}
+
+template <bool TF32, bool BY_OFFSET>
+inline int os_launch_as(const OsParams& p, const OsConfig& cfg, const CUtensorMap& w_map, int grid, cudaStream_t st, int max_smem) {
+  static std::atomic<int> granted[64];
+  if (int rc = ensure_smem(umma_osfwd_kernel<TF32, BY_OFFSET>, max_smem, granted)) return rc;
+  return launch_pdl(umma_osfwd_kernel<TF32, BY_OFFSET>, grid, OS_THREADS, (size_t)cfg.smem, st, p, cfg, w_map) == cudaSuccess ? 0 : -1;
 }
 
 // 0 launched, 1 the shape has no plan or a pointer is not 16-byte aligned (there is no CUDA-core form of this
@@ -468,16 +543,11 @@ inline int launch_umma_osfwd(const OsParams& p, bool f16, cudaStream_t st, int s
   if (!g3_plan(p.c_in, p.c_out, f16 ? 2 : 4, p.k_vol, max_smem, false, &scatter) || !os_plan(p.c_in, p.c_out, f16 ? 2 : 4, max_smem, &cfg)) return 1;
   const int grid = p.n_tiles < sms ? p.n_tiles : sms;
   if (grid <= 0) return 0;
+  os_split(&cfg, (p.n_tiles + grid - 1) / grid, p.k_vol, max_smem);
   CUtensorMap w_map;
   if (int rc = weight_tensor_map(&w_map, p.weights, p.k_vol, p.c_in, p.c_out, f16, true)) return rc;
-  if (f16) {
-    static std::atomic<int> granted[64];
-    if (int rc = ensure_smem(umma_osfwd_kernel<false>, max_smem, granted)) return rc;
-    return launch_pdl(umma_osfwd_kernel<false>, grid, OS_THREADS, (size_t)cfg.smem, st, p, cfg, w_map) == cudaSuccess ? 0 : -1;
-  }
-  static std::atomic<int> granted[64];
-  if (int rc = ensure_smem(umma_osfwd_kernel<true>, max_smem, granted)) return rc;
-  return launch_pdl(umma_osfwd_kernel<true>, grid, OS_THREADS, (size_t)cfg.smem, st, p, cfg, w_map) == cudaSuccess ? 0 : -1;
+  if (f16) return cfg.by_offset ? os_launch_as<false, true>(p, cfg, w_map, grid, st, max_smem) : os_launch_as<false, false>(p, cfg, w_map, grid, st, max_smem);
+  return cfg.by_offset ? os_launch_as<true, true>(p, cfg, w_map, grid, st, max_smem) : os_launch_as<true, false>(p, cfg, w_map, grid, st, max_smem);
 }
 
 }  // namespace fgms
