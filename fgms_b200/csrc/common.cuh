@@ -31,6 +31,7 @@ struct GmsParams {
   int k_vol;
   int dense_rows;              // > 0: one more segment of `dense_rows` identity pairs ...
   int dense_weight;            // ... that uses this weight index (the "separate mid" term)
+  int beside = 0;              // the kernel ahead in the stream is the weight gradient of the same backward: run beside it (griddep_begin)
 };
 
 struct WgradParams {

@@ -107,12 +107,15 @@ __global__ void __launch_bounds__(FF_THREADS, ff_gms_blocks(PT)) ffma_gms_kernel
   float* dst = static_cast<float*>(p.dst);
   const int n_seg = p.k_vol + 1;
 
-  umma::griddep_wait();
+  umma::griddep_begin(p.beside);
   umma::griddep_launch_dependents();
   build_tile_table(tile_pairs, p.kpos, p.pairs, p.k_vol, p.dense_rows, kpos_s, tile_start);
   int t, t1;
   cta_tile_range(tile_start[n_seg], &t, &t1);
-  if (t >= t1) return;
+  if (t >= t1) {
+    umma::griddep_end(p.beside);
+    return;
+  }
 
   const int kp = (p.k_dim + 3) / 4 * 4;
   const bool vec_in = VEC || (p.k_dim % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0);
@@ -237,6 +240,7 @@ __global__ void __launch_bounds__(FF_THREADS, ff_gms_blocks(PT)) ffma_gms_kernel
     }
     t = t_end;
   }
+  umma::griddep_end(p.beside);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------

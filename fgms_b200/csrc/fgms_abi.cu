@@ -128,11 +128,17 @@ int launch_simt_gms(const fgms::GmsParams& p, cudaStream_t st, int sms) {
   return check_launch("simt_gms_kernel");
 }
 
+// How a pass of a backward shares the chip with the other one.
+struct Beside {
+  bool on = false;  // run beside the kernel ahead in the stream, the weight gradient, instead of behind it
+  int sms = 0;      // > 0: the SMs the pass is to have
+};
+
 // One gather-GEMM-scatter pass (forward when !trans, dgrad when trans).
 int run_gms(bool trans, const void* src, const void* kernel, void* dst, const int32_t* kpos,
             const int32_t* gather_map, const int32_t* scatter_map, int64_t map_len, int n_gather, int n_scatter,
             int c_in, int c_out, int k_vol, int dtype, int math, int dense_rows, int dense_weight,
-            cudaStream_t st) {
+            cudaStream_t st, Beside beside = Beside()) {
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
   fgms::GmsParams p;
@@ -144,6 +150,9 @@ int run_gms(bool trans, const void* src, const void* kernel, void* dst, const in
   p.n_dim = trans ? c_in : c_out;
   p.c_in = c_in; p.c_out = c_out; p.k_vol = k_vol;
   p.dense_rows = dense_rows; p.dense_weight = dense_weight;
+  p.beside = beside.on ? 1 : 0;
+  const int all_sms = di.sms;
+  if (beside.sms > 0) di.sms = beside.sms;
   if (plan_gms(trans, c_in, c_out, k_vol, dtype, math, di.max_smem_optin)) {
     // Several small blocks to an SM are spread over all SMs however few there are, so with SMs to leave free the
     // short-row kernel stands back for the one with one block per SM.
@@ -156,11 +165,11 @@ int run_gms(bool trans, const void* src, const void* kernel, void* dst, const in
     g_fallbacks.fetch_add(1, std::memory_order_relaxed);  // pointers not 16-byte aligned: CUDA-core path, counted
   }
   if (dtype == FGMS_DTYPE_F16)
-    return trans ? launch_simt_gms<__half, true>(p, st, di.sms) : launch_simt_gms<__half, false>(p, st, di.sms);
-  const int rc = fgms::launch_ffma_gms(p, trans, st, di.sms);
+    return trans ? launch_simt_gms<__half, true>(p, st, all_sms) : launch_simt_gms<__half, false>(p, st, all_sms);
+  const int rc = fgms::launch_ffma_gms(p, trans, st, all_sms);
   if (rc == 0) return check_launch("ffma_gms_kernel");
   if (rc < 0) return fail(FGMS_ERR_CUDA, "ffma_gms_kernel setup failed (%d)", rc);
-  return trans ? launch_simt_gms<float, true>(p, st, di.sms) : launch_simt_gms<float, false>(p, st, di.sms);
+  return trans ? launch_simt_gms<float, true>(p, st, all_sms) : launch_simt_gms<float, false>(p, st, all_sms);
 }
 
 int mid_offset(int k_vol) { return (k_vol % 2 == 1) ? k_vol / 2 : 0; }
@@ -201,112 +210,82 @@ struct TraceRange {
   TraceRange& operator=(const TraceRange&) = delete;
 };
 
-}  // namespace
-
-extern "C" {
-
-int fgms_b200_fusion_fwd(const void* in_feats, const void* kernel, void* out_feats,
-                         const int32_t* kpos, const int32_t* qkpos, const int32_t* in_map,
-                         const int32_t* out_map, int64_t map_len, int n_in, int n_out, int c_in,
-                         int kernel_c_in, int c_out, int k_vol, int64_t sum_nnz, int dtype, int math,
-                         int separate_mid, void* stream) {
-  TraceRange trace_range("fgms_b200_fusion_fwd");
-  (void)qkpos;
-  if (int rc = check_fwd_args(in_feats, kernel, out_feats, kpos, in_map, out_map, map_len, n_in, n_out, c_in,
-                              kernel_c_in, c_out, k_vol, sum_nnz, dtype, math, separate_mid))
-    return rc;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (separate_mid && n_out > 0) {
-    // the reference's centre GEMM runs first with beta = 0: previous contents are discarded
-    cudaError_t e = cudaMemsetAsync(out_feats, 0, (size_t)n_out * c_out * elem_size(dtype), st);
-    if (e != cudaSuccess) return fail(FGMS_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
+struct Range {
+  const void* p;
+  size_t bytes;
+  bool overlaps(const Range& o) const {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(o.p);
+    return a < b + o.bytes && b < a + bytes;
   }
-  return run_gms(false, in_feats, kernel, out_feats, kpos, in_map, out_map, map_len, n_in, n_out, c_in, c_out,
-                 k_vol, dtype, math, separate_mid ? n_in : 0, mid_offset(k_vol), st);
+};
+
+// SMs of the weight gradient where the two passes of a backward share the chip; 0: each has all of it.
+//
+// Side by side the passes overlap each other's fixed parts (launch, tile table, first rows; the sums' way out) and what they are
+// bound by, reds of rows in the input gradient, instructions of the gathers in the weight gradient.  The weight gradient goes
+// first, with one block per SM on its share; the input gradient's blocks find room on the others only.  Either pass takes about
+// c + u * (128-pair units) / SMs microseconds, the constants below fitted to the passes by themselves; the share is the
+// one at which the later one ends first.  Behind one another / side by side, in a row of launches: fp16 64 -> 64 0.93 M pairs 66.7 /
+// 61.4 us, 137 k 19.0 / 14.9, 32 -> 32 9.1 M 250 / 234, 84 k 10.2 / 8.1; 128 -> 128 303 k 44.1 / 38.3, 98 k 21.6 / 16.7, 256 -> 256 28 k
+// 25.7 / 19.3, stride 2 64 -> 128 9 k 12.7 / 7.4; tf32 32 -> 64 stride 2 200 k 28.8 / 26.9.  A share a sixth off gives the gain
+// away (64 -> 64 0.93 M pairs at 0.36 / 0.48 / 0.60 of the SMs 77.9 / 61.4 / 78.1).
+int split_backward(int64_t pairs, int c_in, int c_out, int k_vol, int dtype, int math, const DeviceInfo& di) {
+  fgms::G3Config g;
+  fgms::W3Config w;
+  const bool f16 = dtype == FGMS_DTYPE_F16;
+  const int es = f16 ? 2 : 4;
+  // (the CUDA-core kernels have several small blocks on every SM and overlap as they are)
+  if (math == FGMS_MATH_FP32 || !fgms::g3_plan(c_in, c_out, es, k_vol, di.max_smem_optin, true, &g) ||
+      !fgms::w3_plan(c_in, c_out, es, k_vol, di.max_smem_optin, &w) || di.sms < 16)
+    return 0;
+  const double both = c_in + c_out, area = (double)c_in * c_out, units = (double)pairs / 128 + k_vol;
+  double c_d = 4, u_d = 0.1 + 0.1 * g.kch + 0.43 * ((c_in * es + 127) / 128);
+  double c_w = 5.5 + area / 8192, u_w = 0.36 * (128.0 / w.pb) + 0.09 * (w.pa + w.pbp) / w.pack;
+  if (fgms::rw_supported(c_out, c_in, f16)) c_d = 3.5, u_d = both * (f16 ? 0.0046 : 0.01);
+  if (f16 && fgms::wh_supported(c_in, c_out))
+    c_w = 5 + area / 2048, u_w = 0.094 + 0.026 * area / 256 + 0.075 * ((c_in == 48) + (c_out == 48));
+  if (!f16 && fgms::rw_wgrad_supported(c_in, c_out)) c_w = 5 + area / 2048, u_w = 0.0115 * both;
+  int best = 0;
+  // behind one another, where the input gradient on all SMs meets L2's rate of reds
+  double least = 0.97 * (c_d + c_w - 2 + (1.07 * u_d + u_w) * units / di.sms);
+  for (int s = di.sms / 4; s <= di.sms - di.sms / 4; s += 2) {
+    const double d = c_d + u_d * units / (di.sms - s), v = c_w + u_w * units / s, end = d > v ? d : v;
+    if (end < least) { least = end; best = s; }
+  }
+  return best;
 }
 
-int fgms_b200_seq_fwd(const void* in_feats, const void* kernel, void* out_feats,
-                      const int32_t* kernel_nnz_host, const int32_t* kpos, const int32_t* in_map,
-                      const int32_t* out_map, int64_t map_len, int n_in, int n_out, int c_in,
-                      int kernel_c_in, int c_out, int k_vol, int64_t sum_nnz, int dtype, int math,
-                      int separate_mid, void* stream) {
-  TraceRange trace_range("fgms_b200_seq_fwd");
-  if (int rc = check_fwd_args(in_feats, kernel, out_feats, kpos, in_map, out_map, map_len, n_in, n_out, c_in,
-                              kernel_c_in, c_out, k_vol, sum_nnz, dtype, math, separate_mid))
-    return rc;
-  if (!kernel_nnz_host) return fail(FGMS_ERR_INVALID_ARG, "kernel_nnz (host) must not be null");
-  long long total = 0;
-  for (int k = 0; k < k_vol; ++k) {
-    if (kernel_nnz_host[k] < 0) return fail(FGMS_ERR_INVALID_ARG, "kernel_nnz[%d] is negative", k);
-    total += kernel_nnz_host[k];
-  }
-  if (total != sum_nnz)
-    return fail(FGMS_ERR_INVALID_ARG, "kernel_nnz sums to %lld but sum_nnz is %lld", total, (long long)sum_nnz);
-  if (total > map_len)
-    return fail(FGMS_ERR_INVALID_ARG, "kernel_nnz sums to %lld but the maps hold %lld entries", total, (long long)map_len);
-  return run_gms(false, in_feats, kernel, out_feats, kpos, in_map, out_map, map_len, n_in, n_out, c_in, c_out,
-                 k_vol, dtype, math, separate_mid ? n_in : 0, mid_offset(k_vol),
-                 static_cast<cudaStream_t>(stream));
-}
-
-int fgms_b200_dgrad(const void* out_grad, const void* kernel, void* in_grad, const int32_t* kpos,
-                    const int32_t* in_map, const int32_t* out_map, int64_t map_len, int n_in, int n_out,
-                    int c_in, int c_out, int k_vol, int dtype, int math, void* stream) {
-  TraceRange trace_range("fgms_b200_dgrad");
+int check_dgrad_args(const void* out_grad, const void* kernel, const void* in_grad, const int32_t* kpos, const int32_t* in_map,
+                     const int32_t* out_map, int64_t map_len, int n_in, int n_out, int c_in, int c_out, int k_vol, int dtype, int math) {
   if (int rc = check_dims(n_in, n_out, c_in, c_out, k_vol)) return rc;
   if (int rc = check_math(dtype, math)) return rc;
   if (!kernel || !kpos) return fail(FGMS_ERR_INVALID_ARG, "kernel / kpos must not be null");
   if ((n_out > 0 && !out_grad) || (n_in > 0 && !in_grad)) return fail(FGMS_ERR_INVALID_ARG, "gradient pointer is null");
-  if (int rc = check_maps(in_map, out_map, map_len)) return rc;
+  return check_maps(in_map, out_map, map_len);
+}
+
+int run_dgrad(const void* out_grad, const void* kernel, void* in_grad, const int32_t* kpos, const int32_t* in_map,
+              const int32_t* out_map, int64_t map_len, int n_in, int n_out, int c_in, int c_out, int k_vol, int dtype, int math,
+              cudaStream_t st, Beside beside) {
+  TraceRange trace_range("fgms_b200_dgrad");
+  if (int rc = check_dgrad_args(out_grad, kernel, in_grad, kpos, in_map, out_map, map_len, n_in, n_out, c_in, c_out, k_vol, dtype, math)) return rc;
   return run_gms(true, out_grad, kernel, in_grad, kpos, out_map, in_map, map_len, n_out, n_in, c_in, c_out, k_vol,
-                 dtype, math, 0, 0, static_cast<cudaStream_t>(stream));
+                 dtype, math, 0, 0, st, beside);
 }
 
-int fgms_b200_zero2(void* a, size_t a_bytes, void* b, size_t b_bytes, void* stream) {
-  TraceRange trace_range("fgms_b200_zero2");
-  if ((a_bytes > 0 && !a) || (b_bytes > 0 && !b)) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
-  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) return fail(FGMS_ERR_INVALID_ARG, "buffers must be 16-byte aligned");
-  if (a_bytes + b_bytes == 0) return FGMS_OK;
-  DeviceInfo di;
-  if (int rc = device_info(&di)) return rc;
-  // four 16-byte stores per thread, at most eight blocks of 256 threads per SM
-  const size_t want = (a_bytes + b_bytes) / (256 * 64) + 1, most = (size_t)di.sms * 8;
-  if (fgms::launch_pdl(fgms::zero2_kernel, (int)(want < most ? want : most), 256, 0, static_cast<cudaStream_t>(stream),
-                       static_cast<uint8_t*>(a), a_bytes, static_cast<uint8_t*>(b), b_bytes) != cudaSuccess)
-    return fail(FGMS_ERR_CUDA, "zero2_kernel launch failed");
-  return check_launch("zero2_kernel");
-}
-
-size_t fgms_b200_wgrad_workspace_bytes(int c_in, int c_out, int k_vol, int dtype) {
-  if (dtype != FGMS_DTYPE_F16 || c_in < 1 || c_out < 1 || k_vol < 1) return 0;
-  return (size_t)k_vol * c_in * c_out * sizeof(float);
-}
-
-int fgms_b200_wgrad_finalize(void* kernel_grad_f16, const void* workspace_f32, int64_t count, void* stream) {
-  TraceRange trace_range("fgms_b200_wgrad_finalize");
-  if (count < 0) return fail(FGMS_ERR_INVALID_ARG, "negative count");
-  if (count == 0) return FGMS_OK;
-  if (!kernel_grad_f16 || !workspace_f32) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
-  int blocks = (int)((count + 255) / 256);
-  if (blocks > 1184) blocks = 1184;
-  fgms::wgrad_finalize_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__half*>(kernel_grad_f16), static_cast<const float*>(workspace_f32), (long long)count);
-  return check_launch("wgrad_finalize_kernel");
-}
-
-int fgms_b200_wgrad(const void* in_feats, const void* out_grad, void* kernel_grad,
-                    const int32_t* kpos, const int32_t* in_map, const int32_t* out_map, int64_t map_len,
-                    int n_in, int n_out, int c_in, int c_out, int k_vol, int dtype, int math,
-                    void* workspace, size_t workspace_bytes, int accumulate_into_kernel_grad, void* stream) {
+int run_wgrad(const void* in_feats, const void* out_grad, void* kernel_grad, const int32_t* kpos, const int32_t* in_map,
+              const int32_t* out_map, int64_t map_len, int n_in, int n_out, int c_in, int c_out, int k_vol, int dtype, int math,
+              void* workspace, size_t workspace_bytes, int accumulate_into_kernel_grad, cudaStream_t st, int sms) {
   TraceRange trace_range("fgms_b200_wgrad");
   if (int rc = check_dims(n_in, n_out, c_in, c_out, k_vol)) return rc;
   if (int rc = check_math(dtype, math)) return rc;
   if (!kpos) return fail(FGMS_ERR_INVALID_ARG, "kpos must not be null");
   if (int rc = check_maps(in_map, out_map, map_len)) return rc;
   if ((n_in > 0 && !in_feats) || (n_out > 0 && !out_grad)) return fail(FGMS_ERR_INVALID_ARG, "feature pointer is null");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
+  const int all_sms = di.sms;
+  if (sms > 0) di.sms = sms;
   const size_t count = (size_t)k_vol * c_in * c_out;
 
   float* acc = nullptr;
@@ -359,17 +338,112 @@ int fgms_b200_wgrad(const void* in_feats, const void* out_grad, void* kernel_gra
   if (!launched) {
     if (dtype == FGMS_DTYPE_F16) {
       const size_t dyn = (size_t)(2 * k_vol + 3) * sizeof(int);
-      const int grid = simt_grid(map_len, 0, k_vol, fgms::SIMT_WG_TILE, di.sms);
+      const int grid = simt_grid(map_len, 0, k_vol, fgms::SIMT_WG_TILE, all_sms);
       if (c_in <= 16 && c_out <= 16) fgms::simt_wgrad_kernel<__half, 1><<<grid, fgms::SIMT_THREADS, dyn, st>>>(p);
       else fgms::simt_wgrad_kernel<__half, 4><<<grid, fgms::SIMT_THREADS, dyn, st>>>(p);
-    } else if (fgms::launch_ffma_wgrad(p, st, di.sms) != 0) {
+    } else if (fgms::launch_ffma_wgrad(p, st, all_sms) != 0) {
       return fail(FGMS_ERR_CUDA, "ffma_wgrad_kernel setup failed");
     }
     if (int rc = check_launch("CUDA-core weight-gradient kernel")) return rc;
   }
   if (dtype == FGMS_DTYPE_F16 && accumulate_into_kernel_grad && !direct_f16)
-    return fgms_b200_wgrad_finalize(kernel_grad, workspace, (int64_t)count, stream);
+    return fgms_b200_wgrad_finalize(kernel_grad, workspace, (int64_t)count, st);
   return FGMS_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int fgms_b200_fusion_fwd(const void* in_feats, const void* kernel, void* out_feats,
+                         const int32_t* kpos, const int32_t* qkpos, const int32_t* in_map,
+                         const int32_t* out_map, int64_t map_len, int n_in, int n_out, int c_in,
+                         int kernel_c_in, int c_out, int k_vol, int64_t sum_nnz, int dtype, int math,
+                         int separate_mid, void* stream) {
+  TraceRange trace_range("fgms_b200_fusion_fwd");
+  (void)qkpos;
+  if (int rc = check_fwd_args(in_feats, kernel, out_feats, kpos, in_map, out_map, map_len, n_in, n_out, c_in,
+                              kernel_c_in, c_out, k_vol, sum_nnz, dtype, math, separate_mid))
+    return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (separate_mid && n_out > 0) {
+    // the reference's centre GEMM runs first with beta = 0: previous contents are discarded
+    cudaError_t e = cudaMemsetAsync(out_feats, 0, (size_t)n_out * c_out * elem_size(dtype), st);
+    if (e != cudaSuccess) return fail(FGMS_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
+  }
+  return run_gms(false, in_feats, kernel, out_feats, kpos, in_map, out_map, map_len, n_in, n_out, c_in, c_out,
+                 k_vol, dtype, math, separate_mid ? n_in : 0, mid_offset(k_vol), st);
+}
+
+int fgms_b200_seq_fwd(const void* in_feats, const void* kernel, void* out_feats,
+                      const int32_t* kernel_nnz_host, const int32_t* kpos, const int32_t* in_map,
+                      const int32_t* out_map, int64_t map_len, int n_in, int n_out, int c_in,
+                      int kernel_c_in, int c_out, int k_vol, int64_t sum_nnz, int dtype, int math,
+                      int separate_mid, void* stream) {
+  TraceRange trace_range("fgms_b200_seq_fwd");
+  if (int rc = check_fwd_args(in_feats, kernel, out_feats, kpos, in_map, out_map, map_len, n_in, n_out, c_in,
+                              kernel_c_in, c_out, k_vol, sum_nnz, dtype, math, separate_mid))
+    return rc;
+  if (!kernel_nnz_host) return fail(FGMS_ERR_INVALID_ARG, "kernel_nnz (host) must not be null");
+  long long total = 0;
+  for (int k = 0; k < k_vol; ++k) {
+    if (kernel_nnz_host[k] < 0) return fail(FGMS_ERR_INVALID_ARG, "kernel_nnz[%d] is negative", k);
+    total += kernel_nnz_host[k];
+  }
+  if (total != sum_nnz)
+    return fail(FGMS_ERR_INVALID_ARG, "kernel_nnz sums to %lld but sum_nnz is %lld", total, (long long)sum_nnz);
+  if (total > map_len)
+    return fail(FGMS_ERR_INVALID_ARG, "kernel_nnz sums to %lld but the maps hold %lld entries", total, (long long)map_len);
+  return run_gms(false, in_feats, kernel, out_feats, kpos, in_map, out_map, map_len, n_in, n_out, c_in, c_out,
+                 k_vol, dtype, math, separate_mid ? n_in : 0, mid_offset(k_vol),
+                 static_cast<cudaStream_t>(stream));
+}
+
+int fgms_b200_dgrad(const void* out_grad, const void* kernel, void* in_grad, const int32_t* kpos,
+                    const int32_t* in_map, const int32_t* out_map, int64_t map_len, int n_in, int n_out,
+                    int c_in, int c_out, int k_vol, int dtype, int math, void* stream) {
+  return run_dgrad(out_grad, kernel, in_grad, kpos, in_map, out_map, map_len, n_in, n_out, c_in, c_out, k_vol, dtype, math,
+                   static_cast<cudaStream_t>(stream), Beside());
+}
+
+int fgms_b200_zero2(void* a, size_t a_bytes, void* b, size_t b_bytes, void* stream) {
+  TraceRange trace_range("fgms_b200_zero2");
+  if ((a_bytes > 0 && !a) || (b_bytes > 0 && !b)) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
+  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) return fail(FGMS_ERR_INVALID_ARG, "buffers must be 16-byte aligned");
+  if (a_bytes + b_bytes == 0) return FGMS_OK;
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  // four 16-byte stores per thread, at most eight blocks of 256 threads per SM
+  const size_t want = (a_bytes + b_bytes) / (256 * 64) + 1, most = (size_t)di.sms * 8;
+  if (fgms::launch_pdl(fgms::zero2_kernel, (int)(want < most ? want : most), 256, 0, static_cast<cudaStream_t>(stream),
+                       static_cast<uint8_t*>(a), a_bytes, static_cast<uint8_t*>(b), b_bytes) != cudaSuccess)
+    return fail(FGMS_ERR_CUDA, "zero2_kernel launch failed");
+  return check_launch("zero2_kernel");
+}
+
+size_t fgms_b200_wgrad_workspace_bytes(int c_in, int c_out, int k_vol, int dtype) {
+  if (dtype != FGMS_DTYPE_F16 || c_in < 1 || c_out < 1 || k_vol < 1) return 0;
+  return (size_t)k_vol * c_in * c_out * sizeof(float);
+}
+
+int fgms_b200_wgrad_finalize(void* kernel_grad_f16, const void* workspace_f32, int64_t count, void* stream) {
+  TraceRange trace_range("fgms_b200_wgrad_finalize");
+  if (count < 0) return fail(FGMS_ERR_INVALID_ARG, "negative count");
+  if (count == 0) return FGMS_OK;
+  if (!kernel_grad_f16 || !workspace_f32) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
+  int blocks = (int)((count + 255) / 256);
+  if (blocks > 1184) blocks = 1184;
+  fgms::wgrad_finalize_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<__half*>(kernel_grad_f16), static_cast<const float*>(workspace_f32), (long long)count);
+  return check_launch("wgrad_finalize_kernel");
+}
+
+int fgms_b200_wgrad(const void* in_feats, const void* out_grad, void* kernel_grad,
+                    const int32_t* kpos, const int32_t* in_map, const int32_t* out_map, int64_t map_len,
+                    int n_in, int n_out, int c_in, int c_out, int k_vol, int dtype, int math,
+                    void* workspace, size_t workspace_bytes, int accumulate_into_kernel_grad, void* stream) {
+  return run_wgrad(in_feats, out_grad, kernel_grad, kpos, in_map, out_map, map_len, n_in, n_out, c_in, c_out, k_vol, dtype, math,
+                   workspace, workspace_bytes, accumulate_into_kernel_grad, static_cast<cudaStream_t>(stream), 0);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -427,11 +501,33 @@ int fgms_b200_bwd(const void* out_grad, const void* in_feats, const void* kernel
   if (c_in != kernel_c_in)
     return fail(FGMS_ERR_CHANNEL_MISMATCH, "Input feature size and kernel size mismatch");
   if (sum_nnz < 0) return fail(FGMS_ERR_INVALID_ARG, "sum_nnz is negative");
-  if (int rc = fgms_b200_dgrad(out_grad, kernel, in_grad, kpos, in_map, out_map, map_len, n_in, n_out, c_in,
-                               c_out, k_vol, dtype, math, stream))
-    return rc;
-  return fgms_b200_wgrad(in_feats, out_grad, kernel_grad, kpos, in_map, out_map, map_len, n_in, n_out, c_in,
-                         c_out, k_vol, dtype, math, workspace, workspace_bytes, 1, stream);
+  if (int rc = check_dgrad_args(out_grad, kernel, in_grad, kpos, in_map, out_map, map_len, n_in, n_out, c_in, c_out, k_vol, dtype, math)) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  auto dgrad = [&](Beside beside) {
+    return run_dgrad(out_grad, kernel, in_grad, kpos, in_map, out_map, map_len, n_in, n_out, c_in, c_out, k_vol, dtype, math, st, beside);
+  };
+  auto wgrad = [&](int sms) {
+    return run_wgrad(in_feats, out_grad, kernel_grad, kpos, in_map, out_map, map_len, n_in, n_out, c_in, c_out, k_vol, dtype, math,
+                     workspace, workspace_bytes, 1, st, sms);
+  };
+  // The two passes run side by side where the weight gradient is one kernel and their buffers do not overlap (what each writes
+  // then is neither read nor written by the other); otherwise one behind the other, the input gradient first.
+  const size_t es = elem_size(dtype), maps = (size_t)map_len * sizeof(int32_t);
+  const Range in{in_feats, (size_t)n_in * c_in * es}, og{out_grad, (size_t)n_out * c_out * es}, w{kernel, (size_t)k_vol * c_in * c_out * es};
+  const Range dx{in_grad, in.bytes}, dw{kernel_grad, w.bytes}, kp{kpos, (size_t)(k_vol + 1) * sizeof(int32_t)}, im{in_map, maps}, om{out_map, maps};
+  bool apart = (dtype != FGMS_DTYPE_F16 || !workspace) && !dx.overlaps(dw);
+  for (const Range& r : {in, og, w, kp, im, om}) apart = apart && !r.overlaps(dx) && !r.overlaps(dw);
+  DeviceInfo di;
+  if (!apart || n_in == 0 || n_out == 0 || map_len == 0 || device_info(&di) != FGMS_OK) {
+    if (int rc = dgrad(Beside())) return rc;
+    return wgrad(0);
+  }
+  Beside beside;
+  beside.on = true;
+  const int wgrad_sms = di.reserved > 0 ? 0 : split_backward(map_len, c_in, c_out, k_vol, dtype, math, di);
+  if (wgrad_sms > 0) beside.sms = di.sms - wgrad_sms;
+  if (int rc = wgrad(wgrad_sms)) return rc;
+  return dgrad(beside);
 }
 
 int fgms_b200_kernel_family(int pass, int c_in, int c_out, int k_vol, int dtype, int math) {

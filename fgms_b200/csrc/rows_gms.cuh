@@ -151,7 +151,7 @@ __global__ void __maxnreg__(rw_max_regs(RW_THREADS * MIN_BLOCKS, TRANS)) rows_gm
   const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int n_seg = p.k_vol + 1;
 
-  umma::griddep_wait();
+  umma::griddep_begin(p.beside);
   umma::griddep_launch_dependents();
   build_tile_table(TILE, p.kpos, p.pairs, p.k_vol, p.dense_rows, kpos_s, tile_start);
 
@@ -160,7 +160,10 @@ __global__ void __maxnreg__(rw_max_regs(RW_THREADS * MIN_BLOCKS, TRANS)) rows_gm
   const int me = (int)blockIdx.x * RW_WARPS + (int)(threadIdx.x >> 5);
   int tile = min((long long)total, (long long)me * share);
   const int tile_end = min(total, tile + share);
-  if (tile >= tile_end) return;
+  if (tile >= tile_end) {
+    umma::griddep_end(p.beside);
+    return;
+  }
   int seg = find_segment(tile_start, n_seg, tile);
 
   const uint8_t* src = static_cast<const uint8_t*>(p.src) + t4 * 16;
@@ -271,6 +274,7 @@ __global__ void __maxnreg__(rw_max_regs(RW_THREADS * MIN_BLOCKS, TRANS)) rows_gm
       r1 = r2;
     }
   }
+  umma::griddep_end(p.beside);
 }
 
 // ---------------------------------------------------------------------------------------------

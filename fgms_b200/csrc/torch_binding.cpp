@@ -180,10 +180,15 @@ struct SparseConv : torch::autograd::Function<SparseConv> {
     const int n_in = (int)feats.size(0), n_out = (int)grad_out.size(0), c_in = (int)weight.size(1), c_out = (int)weight.size(2);
     check_status(fgms_b200_zero2(need_in ? ptr(in_grad) : nullptr, need_in ? bytes_of(in_grad) : 0, need_w ? ptr(w_grad) : nullptr,
                                  need_w ? bytes_of(w_grad) : 0, st));
-    if (need_in)
+    if (need_in && need_w) {  // in one call, which lets them run side by side
+      const Tensor ws = wgrad_workspace(w_grad, a, g_fp32_sums.load(std::memory_order_relaxed));
+      check_status(fgms_b200_bwd(ptr(grad_out), ptr(feats), ptr(weight), ptr(in_grad), ptr(w_grad), iptr(kpos), nullptr, iptr(imap),
+                                 iptr(omap), imap.numel(), n_in, n_out, c_in, c_in, c_out, k_vol, 0, a.dtype, a.math, 0,
+                                 ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? (size_t)ws.numel() * 4 : 0, st));
+    } else if (need_in) {
       check_status(fgms_b200_dgrad(ptr(grad_out), ptr(weight), ptr(in_grad), iptr(kpos), iptr(imap), iptr(omap), imap.numel(), n_in,
                                    n_out, c_in, c_out, k_vol, a.dtype, a.math, st));
-    if (need_w) {
+    } else if (need_w) {
       const Tensor ws = wgrad_workspace(w_grad, a, g_fp32_sums.load(std::memory_order_relaxed));
       check_status(fgms_b200_wgrad(ptr(feats), ptr(grad_out), ptr(w_grad), iptr(kpos), iptr(imap), iptr(omap), imap.numel(), n_in,
                                    n_out, c_in, c_out, k_vol, a.dtype, a.math, ws.defined() ? ws.data_ptr() : nullptr,

@@ -102,6 +102,17 @@ __device__ __forceinline__ bool mbar_parked_wait(uint32_t bar, uint32_t parity, 
 // before the call.  griddep_launch_dependents() lets the next such kernel in the stream start its own
 // preamble as soon as this grid's CTAs make room.  Both do nothing in a kernel launched the plain way.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A kernel that neither reads nor overwrites what the kernel ahead of it in the stream writes or reads may run beside it: instead of
+// waiting at its start it waits before it ends.  The one ahead lets it go (griddep_launch_dependents) behind its own wait in every
+// CTA, so all that came earlier has finished; the fence keeps this SM from answering out of what it held before that.
+// Whoever waits for this kernel thereby waits for both.  All threads call both.
+__device__ __forceinline__ void griddep_begin(bool beside) {
+  if (beside) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  else griddep_wait();
+}
+__device__ __forceinline__ void griddep_end(bool beside) {
+  if (beside) griddep_wait();
+}
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ------------------------------------------------------------------ cp.async (16-byte, zero fill)

@@ -293,7 +293,7 @@ class UNetStep:
         # a small fp32 workspace for layers whose weight gradient has no single-launch fp16 form (single rank only)
         self._ws = None
         p = lambda t: t.data_ptr() if t.numel() > 0 else None
-        self._fwd, self._bwd = [], []
+        self._fwd, self._bwd, self._both = [], [], {}
         for i, l in enumerate(self.spec):
             km = umaps.of(l)
             pairs = int(km.pairs)
@@ -317,6 +317,10 @@ class UNetStep:
                 dgrad = (p(g_dst), p(self.weights[i]), p(self.grad[l.src]), p(km.kpos), p(km.imap), p(km.omap), pairs,
                          km.n_in, km.n_out, l.c_in, l.c_out, l.k_vol, dtype, math_)
             self._bwd.append((l, wgrad, dgrad))
+            # one rank: both gradients in one call, which lets them run side by side
+            if dgrad is not None and not self.multi and ws is None:
+                self._both[i] = (dgrad[0], p(src), dgrad[1], dgrad[2], p(self.w_grads[i]), p(km.kpos), None, p(km.imap), p(km.omap), pairs,
+                                 km.n_in, km.n_out, l.c_in, l.c_in, l.c_out, l.k_vol, 0, dtype, math_, 0, None, 0)
         for _, wgrad, _ in self._bwd:
             if wgrad[14] == "ws":
                 wgrad[14], wgrad[15] = self._ws.data_ptr(), self._ws.numel() * 4
@@ -362,6 +366,9 @@ class UNetStep:
                 # the skip source's gradient starts as this layer's output gradient; the encoder layer that
                 # reads the skip source adds its input gradient later in this loop
                 self.grad[l.skip].copy_(self.grad[l.dst])
+            if i in self._both:
+                check(L.fgms_b200_bwd(*self._both[i], st))
+                continue
             check(L.fgms_b200_wgrad(*wgrad, st))
             if self._collective and i in self._bucket_end:
                 lo, hi = self._bucket_end[i]
