@@ -606,8 +606,8 @@ def run_ours(args):
             which.backward()
         else:
             layer.forward(p.feats, p.weights, out)
-            backend.fgms_dgrad_cuda(p.grad_out, p.weights, in_grad, p.kpos, p.imap, p.omap, p.arch80)
-            wgrad_kernel_only()
+            backend.fgms_bwd_cuda(p.grad_out, p.feats, p.weights, p.qsum, in_grad, w_grad, p.kpos, p.qkpos, p.imap, p.omap, False,
+                                  p.arch80)
         if record: e[1].record()
         return e
 

@@ -308,6 +308,10 @@ class BoundSceneLayer:
         target = self.part if (self.part is not None and not self.fp16) else w_grad
         self._wgrad_args = (p(feats), p(grad_out), p(target), p(kpos), p(imap), p(omap), pairs, n_in, n_out, c_in, c_out,
                             k_vol, dtype, math, ws_ptr, ws_bytes, accumulate)
+        # one rank: both gradients in one call, which lets them run side by side
+        self._bwd_args = None if self.multi or ws_ptr is not None else (
+            p(grad_out), p(feats), p(weights), p(in_grad), p(w_grad), p(kpos), None, p(imap), p(omap), pairs, n_in, n_out, c_in, c_in,
+            c_out, k_vol, 0, dtype, math, 0, None, 0)
 
     def _stream(self):
         import torch
@@ -319,11 +323,15 @@ class BoundSceneLayer:
             self._check(self._L.fgms_b200_fusion_fwd(*self._fwd_args, self._stream()))
 
     def backward(self):
-        """wgrad first, its all-reduce beside dgrad, then the sums are added to ``w_grad``."""
+        """On one rank both gradients by one call; on several wgrad first, its all-reduce beside dgrad, then the sums are added
+        to ``w_grad``."""
         import torch
         import torch.distributed as dist
         with torch.cuda.device(self.device):  # the library launches on the current device
             st = self._stream()
+            if self._bwd_args is not None:
+                self._check(self._L.fgms_b200_bwd(*self._bwd_args, st))
+                return
             if self.part is not None and not self.fp16:
                 self.part.zero_()
             self._check(self._L.fgms_b200_wgrad(*self._wgrad_args, st))
