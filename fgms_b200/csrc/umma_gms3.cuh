@@ -16,8 +16,8 @@
 //                        vector reds with consecutive lanes on consecutive addresses of one row.  The map
 //                        entries of its 32 rows come from global memory two tiles ahead as well.
 //
-// What bounds it: at many tiles a CTA what L2 gives, 5.4 TB/s of reds beside 12 TB/s of gathers (128 -> 128 on 303 k pairs
-// 23.0 us, 77 MB each way); at few the chain from kpos to the last red.  Weights by the producers' own cp.async, a nested MMA
+// What bounds it: at many tiles a CTA what L2 gives, 5.4 TB/s of reds beside 17 TB/s of gathers (128 -> 128 on 303 k pairs
+// 23.0 us, 77 MB each way; without its reds 18.3, without its epilogue 14.7); at few the chain from kpos to the last red.  Weights by the producers' own cp.async, a nested MMA
 // loop, waits that keep issuing and one red per patch read took 24.5 us there, 256 -> 256 on 3000 / 600 voxels 14.6 / 8.9 us
 // (now 12.9 / 7.6), 96 -> 256 on 50 k pairs 12.2 (10.5), 96 -> 160 on 358 k pairs 35.4 (32.5).
 //

@@ -148,7 +148,9 @@ int fgms_b200_wgrad_f16_noalloc(const void* in_feats, const void* out_grad, void
                                 int math, void* stream);
 
 /* Both gradients.  Replaces ConvolutionBackward (backend/spconv.cu:414-571; Python name
- * fgms_bwd_cuda).  separate_mid is accepted and ignored, as in the reference. */
+ * fgms_bwd_cuda).  separate_mid is accepted and ignored, as in the reference.  The two kernels run side by
+ * side on `stream`, each on a share of the SMs where that is faster; whatever is enqueued next waits for both.
+ * With a workspace for fp16 sums, or buffers that overlap, one runs behind the other, the input gradient first. */
 int fgms_b200_bwd(const void* out_grad, const void* in_feats, const void* kernel, void* in_grad,
                   void* kernel_grad, const int32_t* kpos, const int32_t* qkpos,
                   const int32_t* in_map, const int32_t* out_map, int64_t map_len, int n_in, int n_out,
