@@ -22,7 +22,6 @@
 #include "umma_gms3.cuh"
 #include "umma_wgrad3.cuh"
 #include "rows_wgrad.cuh"
-#include "rows_wgrad16.cuh"
 #include "peer_exchange.cuh"
 #include "umma_osfwd.cuh"
 
@@ -242,9 +241,9 @@ int split_backward(int64_t pairs, int c_in, int c_out, int k_vol, int dtype, int
   double c_d = 4, u_d = 0.1 + 0.1 * g.kch + 0.43 * ((c_in * es + 127) / 128);
   double c_w = 5.5 + area / 8192, u_w = 0.36 * (128.0 / w.pb) + 0.09 * (w.pa + w.pbp) / w.pack;
   if (fgms::rw_supported(c_out, c_in, f16)) c_d = 3.5, u_d = both * (f16 ? 0.0046 : 0.01);
-  if (f16 && fgms::wh_supported(c_in, c_out))
+  if (f16 && fgms::wh_supported(c_in, c_out, true))
     c_w = 5 + area / 2048, u_w = 0.094 + 0.026 * area / 256 + 0.075 * ((c_in == 48) + (c_out == 48));
-  if (!f16 && fgms::rw_wgrad_supported(c_in, c_out)) c_w = 5 + area / 2048, u_w = 0.0115 * both;
+  if (!f16 && fgms::wh_supported(c_in, c_out, false)) c_w = 5 + area / 2048, u_w = 0.1 + 0.003 * both + 0.035 * area / 256 + 0.1 * ((c_in == 48) + (c_out == 48));
   int best = 0;
   // behind one another, where the input gradient on all SMs meets L2's rate of reds
   double least = 0.97 * (c_d + c_w - 2 + (1.07 * u_d + u_w) * units / di.sms);
@@ -322,7 +321,7 @@ int run_wgrad(const void* in_feats, const void* out_grad, void* kernel_grad, con
   bool launched = false;
   if (umma) {
     const bool f16 = dtype == FGMS_DTYPE_F16;
-    int rc = f16 ? fgms::launch_rows_wgrad16(p, st, di.sms, di.max_smem_optin) : fgms::launch_rows_wgrad(p, st, di.sms, di.max_smem_optin);
+    int rc = fgms::launch_rows_wgrad(p, f16, st, di.sms, di.max_smem_optin);
     if (rc == 1) rc = fgms::launch_umma_wgrad3(p, f16, st, di.sms, di.max_smem_optin);
     if (rc == 0) {
       if (int rc2 = check_launch("weight-gradient kernel")) return rc2;
