@@ -32,6 +32,7 @@ struct GmsParams {
   int dense_rows;              // > 0: one more segment of `dense_rows` identity pairs ...
   int dense_weight;            // ... that uses this weight index (the "separate mid" term)
   int beside = 0;              // the kernel ahead in the stream is the weight gradient of the same backward: run beside it (griddep_begin)
+  int alone = 0;               // SMs are to stay free: the kernel behind this one in the stream is not let go before this one ends
 };
 
 struct WgradParams {
@@ -46,6 +47,7 @@ struct WgradParams {
   // fp16 storage, tensor-core kernel only: add every CTA's fp32 partial sums, rounded to fp16, straight
   // into the fp16 gradient (dw is then unused)
   __half* dw_f16 = nullptr;
+  int alone = 0;  // see GmsParams
 };
 
 // ---------------------------------------------------------------------------------------------

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(FF_THREADS, ff_gms_blocks(PT)) ffma_gms_kernel
   const int n_seg = p.k_vol + 1;
 
   umma::griddep_begin(p.beside);
-  umma::griddep_launch_dependents();
+  if (!p.alone) umma::griddep_launch_dependents();
   build_tile_table(tile_pairs, p.kpos, p.pairs, p.k_vol, p.dense_rows, kpos_s, tile_start);
   int t, t1;
   cta_tile_range(tile_start[n_seg], &t, &t1);
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(FF_THREADS, FF_WGRAD_BLOCKS) ffma_wgrad_kernel
   const int tid = threadIdx.x, n_seg = p.k_vol + 1;
 
   umma::griddep_wait();
-  umma::griddep_launch_dependents();
+  if (!p.alone) umma::griddep_launch_dependents();
   build_tile_table(FW_PAIRS, p.kpos, p.pairs, p.k_vol, 0, kpos_s, tile_start);
   int t, t1;
   cta_tile_range(tile_start[n_seg], &t, &t1);

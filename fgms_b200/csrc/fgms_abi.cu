@@ -150,6 +150,7 @@ int run_gms(bool trans, const void* src, const void* kernel, void* dst, const in
   p.c_in = c_in; p.c_out = c_out; p.k_vol = k_vol;
   p.dense_rows = dense_rows; p.dense_weight = dense_weight;
   p.beside = beside.on ? 1 : 0;
+  p.alone = di.reserved > 0;
   const int all_sms = di.sms;
   if (beside.sms > 0) di.sms = beside.sms;
   if (plan_gms(trans, c_in, c_out, k_vol, dtype, math, di.max_smem_optin)) {
@@ -317,6 +318,7 @@ int run_wgrad(const void* in_feats, const void* out_grad, void* kernel_grad, con
   p.pairs = (int)map_len;
   p.n_in = n_in; p.n_out = n_out; p.c_in = c_in; p.c_out = c_out; p.k_vol = k_vol;
   if (direct_f16) p.dw_f16 = static_cast<__half*>(kernel_grad);
+  p.alone = di.reserved > 0;
 
   bool launched = false;
   if (umma) {
@@ -510,20 +512,21 @@ int fgms_b200_bwd(const void* out_grad, const void* in_feats, const void* kernel
                      workspace, workspace_bytes, 1, st, sms);
   };
   // The two passes run side by side where the weight gradient is one kernel and their buffers do not overlap (what each writes
-  // then is neither read nor written by the other); otherwise one behind the other, the input gradient first.
+  // then is neither read nor written by the other); otherwise one behind the other, the input gradient first.  So they are where SMs
+  // are to stay free: the blocks of the one let go early would take just those that the other leaves.
   const size_t es = elem_size(dtype), maps = (size_t)map_len * sizeof(int32_t);
   const Range in{in_feats, (size_t)n_in * c_in * es}, og{out_grad, (size_t)n_out * c_out * es}, w{kernel, (size_t)k_vol * c_in * c_out * es};
   const Range dx{in_grad, in.bytes}, dw{kernel_grad, w.bytes}, kp{kpos, (size_t)(k_vol + 1) * sizeof(int32_t)}, im{in_map, maps}, om{out_map, maps};
   bool apart = (dtype != FGMS_DTYPE_F16 || !workspace) && !dx.overlaps(dw);
   for (const Range& r : {in, og, w, kp, im, om}) apart = apart && !r.overlaps(dx) && !r.overlaps(dw);
   DeviceInfo di;
-  if (!apart || n_in == 0 || n_out == 0 || map_len == 0 || device_info(&di) != FGMS_OK) {
+  if (!apart || n_in == 0 || n_out == 0 || map_len == 0 || device_info(&di) != FGMS_OK || di.reserved > 0) {
     if (int rc = dgrad(Beside())) return rc;
     return wgrad(0);
   }
   Beside beside;
   beside.on = true;
-  const int wgrad_sms = di.reserved > 0 ? 0 : split_backward(map_len, c_in, c_out, k_vol, dtype, math, di);
+  const int wgrad_sms = split_backward(map_len, c_in, c_out, k_vol, dtype, math, di);
   if (wgrad_sms > 0) beside.sms = di.sms - wgrad_sms;
   if (int rc = wgrad(wgrad_sms)) return rc;
   return dgrad(beside);
@@ -833,6 +836,7 @@ int fgms_b200_fwd_output_stationary(const void* in_feats, const void* kernel, vo
   p.nbr_stride = (long long)p.n_tiles * fgms::OS_TILE;
   p.n_in = n_in; p.n_out = n_out; p.c_in = c_in; p.c_out = c_out; p.k_vol = k_vol;
   p.relu = relu ? 1 : 0; p.accumulate = accumulate ? 1 : 0;
+  p.alone = di.reserved > 0;
   const int rc = fgms::launch_umma_osfwd(p, dtype == FGMS_DTYPE_F16, static_cast<cudaStream_t>(stream), di.sms, di.max_smem_optin);
   if (rc == 0) return check_launch("umma_osfwd_kernel");
   if (rc < 0) return fail(FGMS_ERR_CUDA, "umma_osfwd_kernel setup failed (%d)", rc);

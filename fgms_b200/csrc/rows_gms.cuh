@@ -152,7 +152,7 @@ __global__ void __maxnreg__(rw_max_regs(RW_THREADS * MIN_BLOCKS, TRANS)) rows_gm
   const int n_seg = p.k_vol + 1;
 
   umma::griddep_begin(p.beside);
-  umma::griddep_launch_dependents();
+  if (!p.alone) umma::griddep_launch_dependents();
   build_tile_table(TILE, p.kpos, p.pairs, p.k_vol, p.dense_rows, kpos_s, tile_start);
 
   // warp `me` has the turns [me F, me F + F) of all tiles' turns

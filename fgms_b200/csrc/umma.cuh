@@ -100,7 +100,8 @@ __device__ __forceinline__ bool mbar_parked_wait(uint32_t bar, uint32_t parity, 
 // it in the stream is still running.  griddep_wait() returns once that kernel has finished and its writes
 // are visible: nothing it may have written (or may still read and this kernel overwrites) is touched
 // before the call.  griddep_launch_dependents() lets the next such kernel in the stream start its own
-// preamble as soon as this grid's CTAs make room.  Both do nothing in a kernel launched the plain way.
+// preamble as soon as this grid's CTAs make room, also on SMs that this grid has left free: where those are meant for a kernel
+// of another stream it is left out (`alone`).  Both do nothing in a kernel launched the plain way.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // A kernel that neither reads nor overwrites what the kernel ahead of it in the stream writes or reads may run beside it: instead of
 // waiting at its start it waits before it ends.  The one ahead lets it go (griddep_launch_dependents) behind its own wait in every

@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
   }
   // everything above touches no global memory; from here on the previous kernel's results may be needed
   griddep_begin(p.beside);
-  griddep_launch_dependents();
+  if (!p.alone) griddep_launch_dependents();
   build_tile_table(G3_TILE_M, p.kpos, p.pairs, p.k_vol, p.dense_rows, kpos_s, tile_start);  // syncs the CTA
   tc_fence_before();
   __syncthreads();

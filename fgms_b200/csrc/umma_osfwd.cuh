@@ -75,6 +75,7 @@ struct OsParams {
   int c_in, c_out, k_vol;
   int relu;        // 1: max(x, 0) after the bias
   int accumulate;  // 1: out += result (what the reference's forward does); 0: out = result
+  int alone = 0;   // see GmsParams
 };
 
 struct OsShared {
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
     tmem_relinquish();
   }
   griddep_wait();
-  griddep_launch_dependents();
+  if (!p.alone) griddep_launch_dependents();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

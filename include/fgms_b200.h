@@ -150,7 +150,8 @@ int fgms_b200_wgrad_f16_noalloc(const void* in_feats, const void* out_grad, void
 /* Both gradients.  Replaces ConvolutionBackward (backend/spconv.cu:414-571; Python name
  * fgms_bwd_cuda).  separate_mid is accepted and ignored, as in the reference.  The two kernels run side by
  * side on `stream`, each on a share of the SMs where that is faster; whatever is enqueued next waits for both.
- * With a workspace for fp16 sums, or buffers that overlap, one runs behind the other, the input gradient first. */
+ * With a workspace for fp16 sums, buffers that overlap or SMs to leave free (fgms_b200_set_reserved_sms), one runs behind the
+ * other, the input gradient first. */
 int fgms_b200_bwd(const void* out_grad, const void* in_feats, const void* kernel, void* in_grad,
                   void* kernel_grad, const int32_t* kpos, const int32_t* qkpos,
                   const int32_t* in_map, const int32_t* out_map, int64_t map_len, int n_in, int n_out,
@@ -272,7 +273,8 @@ int fgms_b200_peer_exchange(const float* const* sums, float* const* reduced, uin
  * library to launch on `n` fewer SMs; the setting is process-wide and applies to the launches that follow
  * (set it around the one call it is meant for).  While it is not 0, forward and input gradient of layers of up to 64
  * channels run on the tcgen05 kernel, which has one CTA per SM, instead of the faster one for short rows.  The
- * CUDA-core kernels follow the number only roughly.  0 restores the full grid.  No counterpart in the reference,
+ * CUDA-core kernels follow the number only roughly.  What is enqueued behind such a launch starts when it has ended
+ * (otherwise its blocks would take the free SMs early).  0 restores the full grid.  No counterpart in the reference,
  * whose grids follow the problem size (backend/spconv.cu:111-245). */
 int fgms_b200_set_reserved_sms(int n);
 

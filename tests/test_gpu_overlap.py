@@ -30,6 +30,10 @@ class _Layer:
     def dgrad(self):
         backend.fgms_dgrad_cuda(self.grad_out, self.weight, self.in_grad, self.kpos, self.imap, self.omap, True)
 
+    def bwd(self):
+        backend.fgms_bwd_cuda(self.grad_out, self.feats, self.weight, 0, self.in_grad, torch.zeros_like(self.weight), self.kpos, None,
+                              self.imap, self.omap, False, True)
+
 
 def _side_and_main_ms(call, side, beside):
     """Times from the start of ``call()`` to the end of ``beside()`` on ``side`` and of the call itself."""
@@ -77,3 +81,19 @@ def test_reserved_sms_are_free_for_another_stream(c_in, c_out):
     finally:
         _lib.lib.fgms_b200_set_reserved_sms(0)
     assert best[0] < 0.75 * best[1], f"the other kernel ended after {best[0]:.3f} ms, the input gradient after {best[1]:.3f} ms"
+
+
+@pytest.mark.parametrize("c_in,c_out", [(32, 32), (64, 64), (128, 128)])
+def test_reserved_sms_are_free_throughout_a_backward(c_in, c_out):
+    """The same kernel beside both gradients of one call, let go while the first of them runs."""
+    layer = _Layer(c_in, c_out, torch.float16)
+    side = torch.cuda.Stream(priority=-1)
+    x = torch.randn((8, 16384), device="cuda")
+    torch.softmax(x, 1)
+    try:
+        assert _lib.lib.fgms_b200_set_reserved_sms(16) == 0
+        layer.bwd()
+        best = min((_side_and_main_ms(layer.bwd, side, lambda: torch.softmax(x, 1)) for _ in range(5)), key=lambda t: t[0] / t[1])
+    finally:
+        _lib.lib.fgms_b200_set_reserved_sms(0)
+    assert best[0] < 0.4 * best[1], f"the other kernel ended after {best[0]:.3f} ms, the backward after {best[1]:.3f} ms"
