@@ -196,6 +196,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
     // ------------------------------------------------------------------ weights: a TMA box per 128-byte column block, as soon as
     // the buffer is free (load number n goes to buffer n % n_wbuf)
     if (elect_one()) {
+      if (p.beside) fence_proxy_async_global();
       int wb = 0, loads = 0, cur_w = -1;
       uint32_t ph = 0;
       for (int seg = find_segment(tile_start, n_seg, t0); seg < n_seg && tile_start[seg] < t1; ++seg) {

@@ -50,6 +50,26 @@ def test_both_gradients_between_kernels_of_others(mode, c_in, c_out, counts):
         assert torch.equal(got[0].double(), want[0]) and torch.equal(got[1].double(), want[1])
 
 
+@pytest.mark.parametrize("mode,c_in,c_out", SHAPES)
+def test_weights_written_by_the_kernel_just_ahead(mode, c_in, c_out):
+    """What the input gradient reads without waiting for the weight gradient: weights (by TMA in the wide layers), map, gradient."""
+    p, draw = _problem(mode, c_in, c_out, [1800, 0, 1500])
+    p.feats = draw(p.feats)
+    dx, dw = torch.zeros_like(p.feats), torch.zeros_like(p.weights)
+    for _ in range(6):
+        weights, grad, big = draw(p.weights), draw(p.grad_out), torch.zeros(1 << 24, device="cuda")
+        turn = torch.randperm(1500, device="cuda").int()
+        imap, omap = p.imap.clone(), p.omap.clone()
+        imap[1800:], omap[1800:] = imap[1800:][turn.long()], omap[1800:][turn.long()]
+        dx.zero_(); dw.zero_()
+        big.add_(1)
+        p.grad_out.copy_(grad); p.imap.copy_(imap); p.omap.copy_(omap); p.weights.copy_(weights)
+        _bwd(p, dx, dw)
+        got = dx + 0, dw + 0
+        want = _want(p)
+        assert torch.equal(got[0].double(), want[0]) and torch.equal(got[1].double(), want[1])
+
+
 @pytest.mark.parametrize("mode,c,pairs", [("fp16", 64, 400_000), ("fp16", 128, 200_000), ("tf32", 64, 100_000)])
 def test_shares_of_large_layers(mode, c, pairs):
     p, draw = _problem(mode, c, c, [pairs // 4] * 4)
