@@ -116,8 +116,10 @@ __global__ void os_fill_nbr_kernel(const int32_t* __restrict__ kpos, const int32
   }
 }
 
-// BY_OFFSET: cfg.by_offset, known at compile time (asked at run time it cost every stage of the other form 2-6 %)
-template <bool TF32, bool BY_OFFSET = false>
+// What is dealt out to the pipelines, known at compile time: by_offset asked at run time cost every stage of the other forms 2-6 %, the
+// number of pipelines asked where there is one 2-4 %.
+enum { OS_ONE_PIPE, OS_DEAL_TILES, OS_DEAL_OFFSETS };
+template <bool TF32, int DEAL = OS_ONE_PIPE>
 __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, OsConfig cfg, const __grid_constant__ CUtensorMap w_map) {
   using namespace umma;
   constexpr int ES = TF32 ? 4 : 2;
@@ -130,8 +132,8 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
   OsShared* sh = reinterpret_cast<OsShared*>(sPatch + OS_EPI_WARPS * 4096);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int kch = cfg.kch, n_pipe = cfg.n_pipe, n_slot = cfg.n_stage / n_pipe, gsz = cfg.group;  // ring slots of a pipeline
-  constexpr bool by_offset = BY_OFFSET;
+  const int kch = cfg.kch, n_pipe = DEAL == OS_ONE_PIPE ? 1 : cfg.n_pipe, n_slot = cfg.n_stage / n_pipe, gsz = cfg.group;  // ring slots of a pipeline
+  constexpr bool by_offset = DEAL == OS_DEAL_OFFSETS;
   const int n_part = by_offset ? n_pipe : 1;  // accumulators of a tile
   const int k_bytes = p.c_in * ES;
   volatile int* abort_flag = &sh->abort_flag;
@@ -186,7 +188,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
     // barrier is at most one phase behind the one that stage q waits for.  (With more warps than slots it may be two behind,
     // which looks the same, and two warps fill one slot.)  Lane l holds the neighbour entries of the tile's rows l, l + 32,
     // l + 64, l + 96, and copies 16-byte chunk l % 8 of the rows l / 8, l / 8 + 4, ...
-    const int pipe = os_producer(warp) % n_pipe, w = os_producer(warp) / n_pipe, nw = cfg.n_prod;
+    const int pipe = DEAL == OS_ONE_PIPE ? 0 : os_producer(warp) % n_pipe, w = os_producer(warp) / n_pipe, nw = cfg.n_prod;
     const int rs = lane >> 3, pc = lane & 7;
     const uint8_t* src = static_cast<const uint8_t*>(p.src) + pc * 16;
     uint32_t a_dst[2];  // rows rs, rs + 4 of a group of eight
@@ -230,7 +232,6 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
         }
         k += step_k; r += step_r;
         if (r >= per_k) { r -= per_k; ++k; }
-        if (i + nw < n) load_entries(e);
         const uint32_t st = smem_u32(sStage) + (uint32_t)slot * G3_STAGE_BYTES;
         const uint8_t* from = src + kc * 128;
         // a place whose row has no neighbour keeps what it held: the MMA leaves that accumulator row alone
@@ -245,6 +246,9 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
           mbar_arrive(smem_u32(&sh->full[slot]));
         }
         cp_async_arrive_noinc(smem_u32(&sh->full[slot]));
+        // behind the copies: asked for ahead of them, the entries were waited for in front of the copies (10-18 % where rows or entries
+        // come from memory: tf32 160 -> 96 on 110 k voxels 273 -> 225 us, fp16 192 -> 192 217 -> 195; 64 -> 64 on 30 k 20.0 -> 19.5)
+        if (i + nw < n) load_entries(e);
         s += nw;
         if (s >= n_slot) { s -= n_slot; ph ^= 1u; }
       }
@@ -277,7 +281,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
   } else if (os_mma_pipe(warp) >= 0) {
     // ------------------------------------------------------------------ MMA issuers
     const uint32_t idesc = make_idesc(TF32, false, true, OS_TILE, cfg.n_acc);
-    const int pipe = os_mma_pipe(warp);
+    const int pipe = DEAL == OS_ONE_PIPE ? 0 : os_mma_pipe(warp);
     const uint64_t a_desc0 = make_sdesc(smem_u32(sStage) + (uint32_t)(pipe * n_slot) * G3_STAGE_BYTES, 16u, 1024u);
     const uint64_t b_desc0 = make_sdesc(smem_u32(sW), (uint32_t)p.c_in * 128u, TF32 ? 512u : 1024u, TF32 ? 1u : 2u);
     constexpr uint32_t B_KC = (uint32_t)EPR * 8u, B_KS = (32u / ES) * 8u;  // one 128-byte K chunk / 32-byte MMA step further, in 16-byte units
@@ -290,21 +294,24 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
       // accumulators: the tiles' of the pipeline, or every tile's part of it
       const int g_step = n_pipe, w_step = by_offset ? n_pipe : 1;  // (weight buffers are a multiple of the pipelines then)
       int s = 0, wb = by_offset ? pipe : 0, grp = 0, g = pipe, kc = 0;  // ring slot, weight buffer, group; accumulator, chunk of the row
-      const uint32_t full = smem_u32(sh->full + pipe * n_slot), empty = smem_u32(sh->empty + pipe * n_slot);
-      const uint4* const rows_on = sh->on + pipe * n_slot;
+      const int off = pipe * n_slot;
       uint32_t ph = 0, w_ph = 0;
       auto take_weights = [&]() { return mbar_wait(smem_u32(&sh->w_full[wb]), w_ph, abort_flag, cfg.w_limit); };
       auto free_weights = [&]() {
         mma_commit(smem_u32(&sh->w_free[wb]));
-        wb += w_step;
-        if (wb >= cfg.n_wbuf) { wb -= cfg.n_wbuf; w_ph ^= 1u; }
+        if (by_offset) {
+          wb += w_step;
+          if (wb >= cfg.n_wbuf) { wb -= cfg.n_wbuf; w_ph ^= 1u; }
+        } else if (++wb == cfg.n_wbuf) {
+          wb = 0; w_ph ^= 1u;
+        }
         g = pipe;
       };
       auto stage = [&](bool first_k, bool last_k) -> bool {
         // first offset of the group: the accumulator must have been read and cleared
         if (first_k && kc == 0 && !mbar_wait(smem_u32(&sh->tmem_empty[g]), (uint32_t)grp & 1u, abort_flag)) return false;
-        if (!mbar_wait(full + 8u * (uint32_t)s, ph, abort_flag)) return false;
-        const uint4 on = rows_on[s];
+        if (!mbar_wait(smem_u32(&sh->full[off + s]), ph, abort_flag)) return false;
+        const uint4 on = sh->on[off + s];
         fence_proxy_async();  // the stage was written through cp.async; the MMA reads it through the async proxy
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(g * cfg.n_acc);
@@ -315,7 +322,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
         for (int ks = 0; ks < 4; ++ks)
           if (ks < n_ks)
             mma_ss_masked<TF32>(d_tmem, a_desc + (uint64_t)(ks * 2), b_desc + (uint64_t)((uint32_t)ks * B_KS), idesc, ~on.x, ~on.y, ~on.z, ~on.w);
-        mma_commit(empty + 8u * (uint32_t)s);
+        mma_commit(smem_u32(&sh->empty[off + s]));
         if (++s == n_slot) { s = 0; ph ^= 1u; }
         if (++kc == kch) {
           if (last_k) mma_commit(smem_u32(&sh->tmem_full[g]));
@@ -526,11 +533,18 @@ inline void os_split(OsConfig* cfg, int tiles, int k_vol, int max_smem) {
   cfg->n_prod = slots < most ? slots : most;
 }
 
-template <bool TF32, bool BY_OFFSET>
+template <bool TF32, int DEAL>
 inline int os_launch_as(const OsParams& p, const OsConfig& cfg, const CUtensorMap& w_map, int grid, cudaStream_t st, int max_smem) {
   static std::atomic<int> granted[64];
-  if (int rc = ensure_smem(umma_osfwd_kernel<TF32, BY_OFFSET>, max_smem, granted)) return rc;
-  return launch_pdl(umma_osfwd_kernel<TF32, BY_OFFSET>, grid, OS_THREADS, (size_t)cfg.smem, st, p, cfg, w_map) == cudaSuccess ? 0 : -1;
+  if (int rc = ensure_smem(umma_osfwd_kernel<TF32, DEAL>, max_smem, granted)) return rc;
+  return launch_pdl(umma_osfwd_kernel<TF32, DEAL>, grid, OS_THREADS, (size_t)cfg.smem, st, p, cfg, w_map) == cudaSuccess ? 0 : -1;
+}
+
+template <bool TF32>
+inline int os_launch(const OsParams& p, const OsConfig& cfg, const CUtensorMap& w_map, int grid, cudaStream_t st, int max_smem) {
+  if (cfg.by_offset) return os_launch_as<TF32, OS_DEAL_OFFSETS>(p, cfg, w_map, grid, st, max_smem);
+  if (cfg.n_pipe > 1) return os_launch_as<TF32, OS_DEAL_TILES>(p, cfg, w_map, grid, st, max_smem);
+  return os_launch_as<TF32, OS_ONE_PIPE>(p, cfg, w_map, grid, st, max_smem);
 }
 
 // 0 launched, 1 the shape has no plan or a pointer is not 16-byte aligned (there is no CUDA-core form of this
@@ -547,8 +561,7 @@ inline int launch_umma_osfwd(const OsParams& p, bool f16, cudaStream_t st, int s
   os_split(&cfg, (p.n_tiles + grid - 1) / grid, p.k_vol, max_smem);
   CUtensorMap w_map;
   if (int rc = weight_tensor_map(&w_map, p.weights, p.k_vol, p.c_in, p.c_out, f16, true)) return rc;
-  if (f16) return cfg.by_offset ? os_launch_as<false, true>(p, cfg, w_map, grid, st, max_smem) : os_launch_as<false, false>(p, cfg, w_map, grid, st, max_smem);
-  return cfg.by_offset ? os_launch_as<true, true>(p, cfg, w_map, grid, st, max_smem) : os_launch_as<true, false>(p, cfg, w_map, grid, st, max_smem);
+  return f16 ? os_launch<false>(p, cfg, w_map, grid, st, max_smem) : os_launch<true>(p, cfg, w_map, grid, st, max_smem);
 }
 
 }  // namespace fgms
