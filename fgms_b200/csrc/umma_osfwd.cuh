@@ -505,32 +505,59 @@ inline bool os_plan(int c_in, int c_out, int es, int max_smem, OsConfig* cfg) {
   return true;
 }
 
-// Pipelines for CTAs of up to `tiles` tiles.  Where a CTA has too few tiles to deal out, the offsets are dealt out, if their
-// accumulators fit tensor memory and a weight buffer or two for every pipeline leave each two ring slots.
+// Cycles between two stages of a CTA's pipelines: what an MMA lane's stage takes, what it takes from asking for a stage's rows to its
+// slot being free again (more where a row is long), shared out over the slots of a ring, and what shared memory takes for a stage of every
+// pipeline.
+inline int os_stage_cycles(int pipes, int n_stage, int kch) {
+  const int rows = (kch > 3 ? 3300 : 3100) / (n_stage / pipes), shared = 360 * pipes, lane = 550;
+  return rows > shared ? (rows > lane ? rows : lane) : (shared > lane ? shared : lane);
+}
+
+// Pipelines for CTAs of up to `tiles` tiles.
+//
+// A CTA of one tile has its offsets dealt out to three pipelines, if their accumulators fit tensor memory, each has a weight
+// buffer, and the rings together hold three rows of the input.  (fp16 128 -> 128 on 1000 voxels 22.8 -> 21.2 us, 160 -> 48 25.2 -> 20.7, tf32 64 -> 64
+// 22.0 -> 17.5.  With smaller rings or two pipelines a pipeline waits for its one buffer of weights, or for rows: 160 -> 160 30.6 -> 44.8, 256 ->
+// 128 33.4 -> 44.1, 208 -> 64 28.6 -> 30.1, tf32 80 -> 80 26.2 -> 29.9; 16 -> 208 with two pipelines 18.5 -> 19.0.)  Two weight buffers each, where the rings
+// then hold six rows: 64 -> 128 16.0 -> 14.8, but tf32 48 -> 48 17.6 -> 18.3; then a CTA of two tiles has its offsets dealt out as well
+// (16 -> 16 on 30 k voxels 15.5, by tiles 16.3; 128 -> 64 30.6 / 28.6).
+//
+// Otherwise tiles are dealt out so that the most loaded pipeline ends first; equally good, three for rows of one 128-byte chunk (fp16
+// 16 -> 16 on 100 k voxels, six tiles, with one / two / three 48.5 / 35.2 / 31.6 us), fewer for longer ones (96 -> 96 88.3 / 72.5 / 78.1).  With three
+// slots and an odd number of tiles two pipelines lose what they gain: 144 -> 144 on 52 k voxels, three tiles, 75.2 / 83.4, on 100 k 145 / 135; 224 -> 112
+// 80.3 / 101.4, on 30 k (two tiles) 56.6 / 58.2; with two slots always (160 -> 160 on 100 k 166 / 190).
 inline void os_split(OsConfig* cfg, int tiles, int k_vol, int max_smem) {
-  int n = OS_MAX_PIPES;
-  while (n > 1 && (tiles < n || cfg->group < n || cfg->n_stage < 3 * n)) --n;
   const int other = cfg->smem - cfg->n_wbuf * cfg->w_bytes - cfg->n_stage * G3_STAGE_BYTES;
-  for (int m = OS_MAX_PIPES; m > n && tiles < OS_MAX_PIPES; --m) {
-    if (m > k_vol || tiles * m > OS_MAX_GROUP || tiles * m * cfg->n_acc > 512) continue;
-    for (int wbufs = 2 * m; wbufs >= m; wbufs -= m) {
-      const int stages = (max_smem - other - wbufs * cfg->w_bytes) / G3_STAGE_BYTES;
-      if (max_smem - other < wbufs * cfg->w_bytes || stages < (wbufs > m ? 3 : 2) * m) continue;
+  constexpr int M = OS_MAX_PIPES;
+  auto set = [&](int pipes) {
+    const int most = OS_PROD_WARPS / pipes, slots = cfg->n_stage / pipes;
+    cfg->n_pipe = pipes;
+    cfg->n_prod = slots < most ? slots : most;
+  };
+  if (tiles < M && M <= k_vol && tiles * M <= OS_MAX_GROUP && tiles * M * cfg->n_acc <= 512) {
+    for (int each = 2; each >= (tiles == 1 ? 1 : 2); --each) {
+      const int room = max_smem - other - each * M * cfg->w_bytes;
+      if (room < 2 * M * G3_STAGE_BYTES) continue;
+      const int fit = room / G3_STAGE_BYTES, stages = fit < OS_MAX_STAGES ? fit : OS_MAX_STAGES;
+      if (stages / M * M < 3 * each * cfg->kch) continue;
       cfg->by_offset = 1;
-      cfg->n_pipe = m;
-      cfg->n_wbuf = wbufs;
-      cfg->n_stage = stages < OS_MAX_STAGES ? stages : OS_MAX_STAGES;
+      cfg->n_wbuf = each * M;
+      cfg->n_stage = stages;
       cfg->group = tiles;
       cfg->smem = other + cfg->n_wbuf * cfg->w_bytes + cfg->n_stage * G3_STAGE_BYTES;
-      const int most = OS_PROD_WARPS / m, slots = cfg->n_stage / m;
-      cfg->n_prod = slots < most ? slots : most;
+      set(M);
       return;
     }
   }
-  cfg->n_pipe = n;
-  cfg->group = cfg->group / n * n;
-  const int most = OS_PROD_WARPS / n, slots = cfg->n_stage / n;
-  cfg->n_prod = slots < most ? slots : most;
+  int pipes = 1;
+  long long least = 0;
+  for (int n = 1; n <= M && n <= tiles && n <= cfg->group && cfg->n_stage >= 2 * n; ++n) {
+    const int group = cfg->group / n * n, last = tiles % group;
+    const long long turns = (long long)(tiles / group) * (group / n) + (last + n - 1) / n, cycles = turns * os_stage_cycles(n, cfg->n_stage, cfg->kch);
+    if (n == 1 || cycles < least || (cycles == least && cfg->kch == 1)) pipes = n, least = cycles;
+  }
+  cfg->group = cfg->group / pipes * pipes;
+  set(pipes);
 }
 
 template <bool TF32, int DEAL>
