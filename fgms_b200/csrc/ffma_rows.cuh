@@ -107,13 +107,12 @@ __global__ void __launch_bounds__(FF_THREADS, ff_gms_blocks(PT)) ffma_gms_kernel
   float* dst = static_cast<float*>(p.dst);
   const int n_seg = p.k_vol + 1;
 
-  umma::griddep_begin(p.beside);
-  if (!p.alone) umma::griddep_launch_dependents();
+  umma::griddep_begin(TRANS && p.beside, p.alone);
   build_tile_table(tile_pairs, p.kpos, p.pairs, p.k_vol, p.dense_rows, kpos_s, tile_start);
   int t, t1;
   cta_tile_range(tile_start[n_seg], &t, &t1);
   if (t >= t1) {
-    umma::griddep_end(p.beside);
+    umma::griddep_end(TRANS && p.beside);
     return;
   }
 
@@ -240,7 +239,7 @@ __global__ void __launch_bounds__(FF_THREADS, ff_gms_blocks(PT)) ffma_gms_kernel
     }
     t = t_end;
   }
-  umma::griddep_end(p.beside);
+  umma::griddep_end(TRANS && p.beside);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -267,8 +266,7 @@ __global__ void __launch_bounds__(FF_THREADS, FF_WGRAD_BLOCKS) ffma_wgrad_kernel
   const float* __restrict__ og = static_cast<const float*>(p.out_grad);
   const int tid = threadIdx.x, n_seg = p.k_vol + 1;
 
-  umma::griddep_wait();
-  if (!p.alone) umma::griddep_launch_dependents();
+  umma::griddep_begin(0, p.alone);
   build_tile_table(FW_PAIRS, p.kpos, p.pairs, p.k_vol, 0, kpos_s, tile_start);
   int t, t1;
   cta_tile_range(tile_start[n_seg], &t, &t1);

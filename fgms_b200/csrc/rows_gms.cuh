@@ -151,8 +151,7 @@ __global__ void __maxnreg__(rw_max_regs(RW_THREADS * MIN_BLOCKS, TRANS)) rows_gm
   const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int n_seg = p.k_vol + 1;
 
-  umma::griddep_begin(p.beside);
-  if (!p.alone) umma::griddep_launch_dependents();
+  umma::griddep_begin(TRANS && p.beside, p.alone);
   build_tile_table(TILE, p.kpos, p.pairs, p.k_vol, p.dense_rows, kpos_s, tile_start);
 
   // warp `me` has the turns [me F, me F + F) of all tiles' turns
@@ -161,7 +160,7 @@ __global__ void __maxnreg__(rw_max_regs(RW_THREADS * MIN_BLOCKS, TRANS)) rows_gm
   int tile = min((long long)total, (long long)me * share);
   const int tile_end = min(total, tile + share);
   if (tile >= tile_end) {
-    umma::griddep_end(p.beside);
+    umma::griddep_end(TRANS && p.beside);
     return;
   }
   int seg = find_segment(tile_start, n_seg, tile);
@@ -274,7 +273,7 @@ __global__ void __maxnreg__(rw_max_regs(RW_THREADS * MIN_BLOCKS, TRANS)) rows_gm
       r1 = r2;
     }
   }
-  umma::griddep_end(p.beside);
+  umma::griddep_end(TRANS && p.beside);
 }
 
 // ---------------------------------------------------------------------------------------------

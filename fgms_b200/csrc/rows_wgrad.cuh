@@ -101,8 +101,7 @@ __global__ void __maxnreg__(rw_max_regs(WARPS * 32, true)) rows_wgrad_kernel(Wgr
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int n_seg = p.k_vol + 1;
 
-  umma::griddep_wait();
-  if (!p.alone) umma::griddep_launch_dependents();
+  umma::griddep_begin(0, p.alone);
   const int unit = !TF32 && p.dw_f16 != nullptr ? WH_UNIT : 0;
   build_tile_table(16 << unit, p.kpos, p.pairs, p.k_vol, 0, kpos_s, tile_start);
   // Units by turns; spread (see Turns) when the rows exceed what L2 holds.

@@ -176,8 +176,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
     tmem_relinquish();
   }
   // everything above touches no global memory; from here on the previous kernel's results may be needed
-  griddep_begin(p.beside);
-  if (!p.alone) griddep_launch_dependents();
+  griddep_begin(TRANS_W && p.beside, p.alone);
   build_tile_table(G3_TILE_M, p.kpos, p.pairs, p.k_vol, p.dense_rows, kpos_s, tile_start);  // syncs the CTA
   tc_fence_before();
   __syncthreads();
@@ -196,7 +195,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
     // ------------------------------------------------------------------ weights: a TMA box per 128-byte column block, as soon as
     // the buffer is free (load number n goes to buffer n % n_wbuf)
     if (elect_one()) {
-      if (p.beside) fence_proxy_async_global();
+      if (TRANS_W && p.beside) fence_proxy_async_global();
       int wb = 0, loads = 0, cur_w = -1;
       uint32_t ph = 0;
       for (int seg = find_segment(tile_start, n_seg, t0); seg < n_seg && tile_start[seg] < t1; ++seg) {
@@ -482,7 +481,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
   tc_fence_before();
   __syncthreads();
   if (warp == G3_MMA_WARP) tmem_dealloc(tmem_base, tmem_cols);
-  griddep_end(p.beside);
+  griddep_end(TRANS_W && p.beside);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -161,8 +161,7 @@ __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, O
     tmem_alloc(smem_u32(&sh->tmem_base), tmem_cols);
     tmem_relinquish();
   }
-  griddep_wait();
-  if (!p.alone) griddep_launch_dependents();
+  griddep_begin(0, p.alone);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

@@ -137,8 +137,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
     tmem_relinquish();
   }
   // everything above touches no global memory; from here on the previous kernel's results may be needed
-  griddep_wait();
-  if (!p.alone) griddep_launch_dependents();
+  griddep_begin(0, p.alone);
   build_tile_table(pb, p.kpos, p.pairs, p.k_vol, 0, kpos_s, tile_start);  // syncs the CTA
   tc_fence_before();
   __syncthreads();
