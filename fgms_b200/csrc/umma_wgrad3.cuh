@@ -12,8 +12,8 @@
 // while consecutive stages belong to the same offset and is flushed with 16-byte vector reds to the
 // fp32 gradient when the offset changes (split-K across CTAs).
 //
-//   producers (2 teams   the teams take the stages in turn; warp w of a team owns rows [w pb/4, (w+1) pb/4) of its team's
-//   of 4 warps)          stages: it fetches those rows' map entries two of them ahead into a ring of its own and gathers both
+//   producers (2 teams   the teams take the stages in turn; warp w of a team of four owns rows [w pb/4, (w+1) pb/4) of its team's
+//   of 4 warps, or 8)    stages: it fetches those rows' map entries two of them ahead into a ring of its own and gathers both
 //                        operands with 16-byte cp.async;
 //   MMA warp             one lane issues tcgen05.mma per stage and commits the stage back to the producers;
 //                        on a change of offset it commits the accumulator to the epilogue;
@@ -42,9 +42,13 @@ namespace fgms {
 constexpr int W3_EPI_WARPS = 4;
 constexpr int W3_MMA_WARP = 4;
 constexpr int W3_PROD_WARP0 = 5;
-constexpr int W3_PROD_WARPS = 4;  // of a team: they share a stage
-constexpr int W3_PROD_TEAMS = 2;  // take the stages in turn
-constexpr int W3_PROD_THREADS = W3_PROD_WARPS * 32;
+constexpr int W3_PROD_WARPS = 4;  // of a team where there are as many as can be: they share a stage
+constexpr int W3_PROD_TEAMS = 2;  // at most; they take the stages in turn
+// CTAs of up to this many stages have one team of all producers: there the first stage's copies are part of the time.  Two teams /
+// one: 256 -> 208 on 12 k pairs, one or two stages a CTA, 14.8 / 14.1 us, 128 -> 128 on 12 k 6.3 / 5.8, tf32 208 -> 144 on 2.9 k 10.0 / 9.6, 224 -> 208 on 6.8 k
+// 19.4 / 19.1; two or three: 128 -> 128 on 39 k 8.5 / 8.6, tf32 160 -> 160 on 11 k 14.6 / 14.8, 256 -> 256 on 28 k 15.3 / 15.2; six: 256 -> 256 on 55 k 17.9 / 18.0;
+// more: 128 -> 128 on 303 k 18.1 / 21.0.
+constexpr int W3_ONE_TEAM_STAGES = 2;
 constexpr int W3_THREADS = (W3_PROD_WARP0 + W3_PROD_TEAMS * W3_PROD_WARPS) * 32;
 constexpr int W3_MAX_STAGES = 12;
 constexpr int W3_MAX_PB = 128;
@@ -92,9 +96,11 @@ __device__ __forceinline__ void w3_stage(const G3Walk& w, int pb, const int* kpo
 
 // FULL: both row lengths are whole 128-byte pieces; the producers' copy loops then carry no per-chunk test.
 // PACKED: several pairs share a staged row (cfg.pack > 1); the unpacked instantiations carry none of its arithmetic.
-template <bool TF32, bool FULL, bool PACKED>
+// TEAMS: of producers.
+template <bool TF32, bool FULL, bool PACKED, int TEAMS>
 __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams p, W3Config cfg) {
   using namespace umma;
+  constexpr int TEAM_WARPS = W3_PROD_TEAMS * W3_PROD_WARPS / TEAMS;
   constexpr int ES = TF32 ? 4 : 2;
   constexpr int UK = 32 / ES;  // contraction length of one MMA
   extern __shared__ uint8_t smem_raw[];
@@ -118,7 +124,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
 
   if (tid == 0) {
     for (int s = 0; s < n_stage; ++s) {
-      mbar_init(smem_u32(&sh->full[s]), W3_PROD_THREADS);  // one hardware arrival per producer thread
+      mbar_init(smem_u32(&sh->full[s]), TEAM_WARPS * 32);  // one hardware arrival per producer thread
       mbar_init(smem_u32(&sh->empty[s]), 1);
     }
     for (int b = 0; b < 4; ++b) {
@@ -152,8 +158,8 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
     // nothing for this CTA
   } else if (warp >= W3_PROD_WARP0) {
     // ------------------------------------------------------------------ producers
-    const int team = (warp - W3_PROD_WARP0) / W3_PROD_WARPS, pw = (warp - W3_PROD_WARP0) % W3_PROD_WARPS;
-    const int rpw = pb / W3_PROD_WARPS;  // rows of a stage owned by this warp: 8, 16 or 32
+    const int team = (warp - W3_PROD_WARP0) / TEAM_WARPS, pw = (warp - W3_PROD_WARP0) % TEAM_WARPS;
+    const int rpw = pb / TEAM_WARPS;  // rows of a stage owned by this warp: 4, 8, 16 or 32
     const uint8_t* feats = static_cast<const uint8_t*>(p.feats);
     const uint8_t* og = static_cast<const uint8_t*>(p.out_grad);
     const uint32_t a_row_bytes = (uint32_t)p.c_in * ES, b_row_bytes = (uint32_t)p.c_out * ES;
@@ -260,7 +266,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
       if (pf.t < t1) fetch_entry(pf, ring + put);
       cp_async_commit();  // also closes the group of the stage before
 #pragma unroll
-      for (int i = 0; i < W3_PROD_TEAMS; ++i)
+      for (int i = 0; i < TEAMS; ++i)
         if (pf.t < t1) pf.next(tile_start, n_seg);
       put = put == W3_PREFETCH * ring_step ? 0 : put + ring_step;
     };
@@ -270,7 +276,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
     // is at most one phase behind the one waited for (a ring has at least two slots, or three groups).
     int s = team, sg = team % cfg.group;
     uint32_t ph = 0;
-    for (int t = t0 + team; t < t1 && ok; t += W3_PROD_TEAMS) {
+    for (int t = t0 + team; t < t1 && ok; t += TEAMS) {
       fetch_next();
       cp_async_wait<W3_PREFETCH>();  // this stage's entries have landed
       int cur_a = -1, cur_b = -1;
@@ -294,9 +300,9 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
       }
       // the stage's barrier hears from this thread when everything it has issued so far has landed
       cp_async_arrive_noinc(smem_u32(&sh->full[s]));
-      s += W3_PROD_TEAMS;
+      s += TEAMS;
       if (s >= n_stage) { s -= n_stage; ph ^= 1u; }
-      sg += W3_PROD_TEAMS;
+      sg += TEAMS;
       while (sg >= cfg.group) sg -= cfg.group;
     }
   } else if (warp == W3_MMA_WARP) {
@@ -535,19 +541,25 @@ inline bool w3_plan(int c_in, int c_out, int es, int k_vol, int max_smem, W3Conf
   return false;
 }
 
-template <bool TF32, bool FULL, bool PACKED>
+template <bool TF32, bool FULL, bool PACKED, int TEAMS>
 inline int w3_launch_as(const WgradParams& p, const W3Config& cfg, cudaStream_t st, int sms, int max_smem) {
   static std::atomic<int> granted[64];
-  if (int rc = ensure_smem(umma_wgrad3_kernel<TF32, FULL, PACKED>, max_smem, granted)) return rc;
-  return launch_pdl(umma_wgrad3_kernel<TF32, FULL, PACKED>, sms, W3_THREADS, (size_t)cfg.smem, st, p, cfg) == cudaSuccess ? 0 : -1;
+  if (int rc = ensure_smem(umma_wgrad3_kernel<TF32, FULL, PACKED, TEAMS>, max_smem, granted)) return rc;
+  return launch_pdl(umma_wgrad3_kernel<TF32, FULL, PACKED, TEAMS>, sms, W3_THREADS, (size_t)cfg.smem, st, p, cfg) == cudaSuccess ? 0 : -1;
+}
+template <bool TF32, bool FULL, bool PACKED>
+inline int w3_launch_teams(const WgradParams& p, const W3Config& cfg, cudaStream_t st, int sms, int max_smem) {
+  const bool few = p.pairs / cfg.pb + p.k_vol / 2 <= W3_ONE_TEAM_STAGES * sms;  // (an offset's last stage is half empty on average)
+  return few ? w3_launch_as<TF32, FULL, PACKED, 1>(p, cfg, st, sms, max_smem)
+             : w3_launch_as<TF32, FULL, PACKED, W3_PROD_TEAMS>(p, cfg, st, sms, max_smem);
 }
 template <bool TF32>
 inline int w3_launch(const WgradParams& p, const W3Config& cfg, cudaStream_t st, int sms, int max_smem) {
   const int es = TF32 ? 4 : 2;
   const bool full = (p.c_in * es) % 128 == 0 && (p.c_out * es) % 128 == 0;
   if (cfg.pack > 1)
-    return full ? w3_launch_as<TF32, true, true>(p, cfg, st, sms, max_smem) : w3_launch_as<TF32, false, true>(p, cfg, st, sms, max_smem);
-  return full ? w3_launch_as<TF32, true, false>(p, cfg, st, sms, max_smem) : w3_launch_as<TF32, false, false>(p, cfg, st, sms, max_smem);
+    return full ? w3_launch_teams<TF32, true, true>(p, cfg, st, sms, max_smem) : w3_launch_teams<TF32, false, true>(p, cfg, st, sms, max_smem);
+  return full ? w3_launch_teams<TF32, true, false>(p, cfg, st, sms, max_smem) : w3_launch_teams<TF32, false, false>(p, cfg, st, sms, max_smem);
 }
 
 // 0 launched, 1 the pointers are not 16-byte aligned or the shape has no plan (the caller takes the CUDA-core

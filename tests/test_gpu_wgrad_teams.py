@@ -1,6 +1,7 @@
 """The producer teams of the tcgen05 weight gradient (``csrc/umma_wgrad3.cuh``): every number of 128-byte pieces a row may have,
-packed stages, shares of one stage, of as many as the ring has slots, and of several rounds, offsets that end inside a share,
-and entries outside the tensors.  Whole numbers of at most 3 keep every sum below 2^24, so fp32 sums have to be exact."""
+packed stages, one team and two, shares of one stage (of 32 pairs, or up to four times that), of as many as the ring has slots (three
+to five), and of several rounds (48 of 32 pairs: sixteen stages of 128), offsets that end inside a share, and entries
+outside the tensors.  Whole numbers of at most 3 keep every sum below 2^24, so fp32 sums have to be exact."""
 import pytest
 import torch
 
@@ -13,7 +14,7 @@ WIDTHS = [("fp16", 128, 128), ("fp16", 96, 160), ("fp16", 256, 256), ("fp16", 16
           ("tf32", 96, 32), ("tf32", 160, 192), ("tf32", 256, 224), ("tf32", 16, 128)]
 
 
-@pytest.mark.parametrize("stages", [0, 1, 2, 3, 4, 5, 9])
+@pytest.mark.parametrize("stages", [0, 1, 2, 3, 4, 5, 9, 48])
 @pytest.mark.parametrize("mode,c_in,c_out", WIDTHS)
 def test_sums_are_exact_whatever_a_share_holds(mode, c_in, c_out, stages):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
