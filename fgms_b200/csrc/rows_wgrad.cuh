@@ -10,7 +10,7 @@
 // flight, waited for its entries' registers and spent 220 instructions a tile.  In a row of launches, that form / this one:
 // fp16 9.1 M pairs 32 -> 32 198 / 99.5 us (two gathers of these rows from L2 at 17 TB/s: 69), 0.93 M pairs 64 -> 64 43.7 / 31.7,
 // 48 -> 48 41.1 / 29.3, 16 -> 16 16.7 / 12.1, 0.14 M 64 -> 64 13.3 / 11.1, 84 k 32 -> 32 7.5 / 6.5; tf32 4.6 M pairs 32 -> 32 189 / 104,
-// 0.59 M 28.1 / 18.3, 0.2 M 32 -> 64 17.7 / 14.0, 55 k 32 -> 32 7.6 / 6.7, 0.42 M 48 -> 48 (twelve chunks in sixteen lanes) 25.9 / 26.5.
+// 0.59 M 28.1 / 18.3, 0.2 M 32 -> 64 17.7 / 14.0, 55 k 32 -> 32 7.6 / 6.7, 0.37 M 48 -> 48 23.9 / 22.6.
 //
 // What bounds it now: with 8 warps at fp16 64 -> 64 (two a scheduler; 128 of a lane's registers are sums) the matrix
 // instructions' fixed issue latency (3.3 of 6.7 cycles an instruction, tensor pipe 45 % busy); with 16 warps at 32 -> 32
@@ -45,8 +45,10 @@ struct WhRows {
   // rows that are read together lie 8 (24) banks apart.
   static constexpr uint32_t LD = TF32 ? BYTES + 32 : U == 3 ? BYTES + 16 : BYTES;
   static constexpr uint32_t TILE = 16 * LD;
-  static constexpr int LANES = CHUNKS == 6 ? 8 : CHUNKS == 12 ? 16 : CHUNKS;  // lanes that copy a row, a chunk each
-  static constexpr int ROUNDS = 16 * LANES / 32;                              // warp-wide copies of a tile
+  // Lanes that copy a row, a chunk each; three rounds of four for twelve chunks (in sixteen lanes of which four do nothing
+  // 0.37 M pairs tf32 48 -> 48 24.3 us, 22.6 this way, 0.59 M 33.8 / 30.1; but six chunks in rounds of two 23.0 us, 18.5 in eight lanes).
+  static constexpr int LANES = CHUNKS == 6 ? 8 : CHUNKS == 12 ? 4 : CHUNKS, PARTS = CHUNKS > LANES ? CHUNKS / LANES : 1;
+  static constexpr int ROUNDS = 16 * LANES / 32;  // turns through a tile's rows
   __device__ static __forceinline__ uint32_t at(int row, int chunk) {
     const int x = TF32 ? 0 : U == 4 ? row & 7 : U == 2 ? (row >> 1) & 3 : U == 1 ? (row >> 2) & 1 : 0;
     return (uint32_t)row * LD + (uint32_t)((chunk ^ x) << 4);
@@ -75,8 +77,13 @@ struct WhRows {
     for (int i = 0; i < ROUNDS; ++i) {
       const int row = r0 + i * (32 / LANES), idx = __shfl_sync(0xffffffffu, e, first + row);
       if (LANES > CHUNKS && c >= CHUNKS) continue;
-      if (WHOLE) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot + at(row, c)), "l"(src + (size_t)(unsigned)idx * BYTES) : "memory");
-      else umma::cp_async16(slot + at(row, c), src + ((on >> row) & 1 ? (size_t)(unsigned)idx * BYTES : 0), (on >> row) & 1);
+      const uint8_t* from = src + (WHOLE || ((on >> row) & 1) ? (size_t)(unsigned)idx * BYTES : 0);
+#pragma unroll
+      for (int k = 0; k < PARTS; ++k) {
+        const uint32_t to = slot + at(row, c + k * LANES);
+        if (WHOLE) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from + k * LANES * 16) : "memory");
+        else umma::cp_async16(to, from + k * LANES * 16, (on >> row) & 1);
+      }
     }
   }
 };
