@@ -26,9 +26,10 @@
 // stages together, tested for each of eight possible pieces of a row whether the row has it, and waited in every stage for
 // the map entries they had just asked for.  Straight code for the usual numbers of pieces: 128 -> 128 on 303 k pairs 26.9 -> 20.2
 // us in a row of launches; two teams of four that are in different phases of a stage (one copies while the other is at its
-// entries and barriers) 18.4, two teams of eight with fewer registers 20.8; the MMA lane's loops 18.0.  Also 96 -> 160
-// on 358 k pairs 43.6 -> 27.7, tf32 64 -> 64 on 296 k 25.6 -> 17.2, tf32 48 -> 64 on 591 k 53.2 -> 28.3, 64 -> 128 stride 2 on 50 k 9.5 ->
-// 8.7; 256 -> 256, where every stage is 32 pairs and the sums' reds are the larger part, 15.0 -> 15.2 (27 k pairs).
+// entries and barriers) 18.4, two teams of eight with fewer registers 20.8; the MMA lane's loops 18.0; a commit for every stage
+// instead of groups of stages that no shape had more than one in 17.7.  Also 96 -> 160
+// on 358 k pairs 43.6 -> 27.7, tf32 64 -> 64 on 296 k 25.6 -> 17.2, tf32 48 -> 64 on 208 k 23.0 -> 13.6, 160 -> 160 on 296 k 40.3 -> 28.5, 64 -> 128 stride 2
+// on 9 k 6.9 -> 6.4; 256 -> 256, where a stage is 64 pairs, a CTA has three and the sums' reds are the larger part, 15.1 -> 15.1 (28 k pairs).
 // Now a stage of 128 pairs at 128 -> 128 is about 1500 cycles, of which shared memory needs 1024 (64 KB written, read by the MMAs).
 #pragma once
 #include <type_traits>
@@ -50,7 +51,7 @@ constexpr int W3_PROD_TEAMS = 2;  // at most; they take the stages in turn
 // more: 128 -> 128 on 303 k 18.1 / 21.0.
 constexpr int W3_ONE_TEAM_STAGES = 2;
 constexpr int W3_THREADS = (W3_PROD_WARP0 + W3_PROD_TEAMS * W3_PROD_WARPS) * 32;
-constexpr int W3_MAX_STAGES = 12;
+constexpr int W3_MAX_STAGES = 8;
 constexpr int W3_MAX_PB = 128;
 constexpr int W3_PATCH_BYTES = W3_EPI_WARPS * 4096;
 constexpr int W3_PREFETCH = 2;  // map entries are fetched this many of the team's stages ahead
@@ -59,7 +60,7 @@ __host__ __device__ constexpr int w3_ring_bytes(int pb) { return W3_PROD_TEAMS *
 
 struct W3Shared {
   uint64_t full[W3_MAX_STAGES];
-  uint64_t empty[W3_MAX_STAGES];  // used at the first stage of every group: the group's stages have been consumed
+  uint64_t empty[W3_MAX_STAGES];
   uint64_t tmem_full[4];
   uint64_t tmem_empty[4];
   uint64_t drained;  // every MMA has finished
@@ -70,7 +71,7 @@ constexpr int W3_SHARED_BYTES = (sizeof(W3Shared) + 15) & ~15;
 
 struct W3Config {
   int pb;         // pairs per stage: 32, 64 or 128
-  int pack;       // pairs that share one staged row (their rows side by side): 1, 2 or 4
+  int pack;       // pairs that share one staged row (their rows side by side): 1 or 2
   int slot_a, slot_b;  // packed stages: bytes a pair's row takes in the staged row of A / of B
   int n_mtile;    // 1 or 2 accumulator row tiles: all of 128 rows but possibly the last
   int last_m;     // rows of the last tile's MMA: 128, or 64 when at most 64 rows remain
@@ -82,8 +83,7 @@ struct W3Config {
   int smem;       // dynamic shared memory of the launch
   int n_buf;      // TMEM accumulator sets: 1, 2 or 4
   int buf_shift;  // log2(n_buf)
-  int n_stage;    // a multiple of `group`
-  int group;      // stages handed back to the producers by one tcgen05.commit (a commit drains the MMA pipe)
+  int n_stage;
 };
 
 // stage t of the table: first pair and number of pairs
@@ -163,19 +163,12 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
     const uint8_t* feats = static_cast<const uint8_t*>(p.feats);
     const uint8_t* og = static_cast<const uint8_t*>(p.out_grad);
     const uint32_t a_row_bytes = (uint32_t)p.c_in * ES, b_row_bytes = (uint32_t)p.c_out * ES;
-    // `lpr` lanes share a row, one 16-byte chunk each: 8 when the longer of the two rows exceeds 64 bytes, 4 / 2
-    // for rows of at most 64 / 32 bytes, so that a warp-wide copy of short rows still carries 32 chunks (8 / 16
-    // rows instead of 4).  The time of a stage's copies goes with the number of warp-wide copy rounds, not with
-    // the bytes they carry.
-    const uint32_t max_row = a_row_bytes > b_row_bytes ? a_row_bytes : b_row_bytes;
-    int lpr = (FULL || max_row > 64) ? 8 : (max_row > 32 ? 4 : 2);
-    if (32 / lpr > rpw) lpr = 8;         // fewer rows per warp than such a round would cover
-    const int rpp = 32 / lpr;            // rows per round: 4, 8 or 16
-    const int n_pass = rpw / rpp;        // rounds per stage: 1 .. 8
-    // Lane (rs, c) = (lane / lpr, lane % lpr) copies 16-byte chunk c of every 128-byte piece of the rows
-    // rs, rs + rpp, ... of the warp's block: one shuffle and one address per row, then one cp.async per
-    // piece at a fixed distance (128 bytes in global memory, `lbo` in shared memory).
-    const int rs = lane / lpr, cc = lane % lpr;
+    // Lane (rs, cc) = (lane / 8, lane % 8) copies 16-byte chunk cc of every 128-byte piece of the rows rs, rs + 4, ... of the warp's
+    // block: one shuffle and one address per row, then one cp.async per piece at a fixed distance (128 bytes in global memory,
+    // `lbo` in shared memory).
+    constexpr int rpp = 4;         // rows per round
+    const int n_pass = rpw / rpp;  // rounds per stage: 1 .. 8
+    const int rs = lane >> 3, cc = lane & 7;
     const int np_a = ((int)a_row_bytes + 127) / 128, np_b = ((int)b_row_bytes + 127) / 128;  // pieces of a row
     // this lane's chunk exists in the last piece, which a row that is no whole number of pieces fills in part
     const bool tail_a = FULL || (np_a - 1) * 128 + cc * 16 < (int)a_row_bytes;
@@ -201,7 +194,6 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
     // The pieces of R rows of one operand.  What this role spends its time on are instructions (with the copies left out
     // the kernel took as long: tests of every one of eight possible pieces and address arithmetic, 400 instructions a
     // warp and stage), so the usual numbers of pieces have their own straight code.
-    // The pieces of R rows of one operand; the usual numbers of pieces have their own straight code.
     auto copy_pieces = [&](auto rounds, auto pieces, const uint8_t* const (&from)[4], const uint32_t (&rel)[4], uint32_t to, const uint32_t (&n)[4],
                            int np, bool tail) {
       constexpr int R = decltype(rounds)::value, NP = decltype(pieces)::value;
@@ -271,10 +263,10 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
       put = put == W3_PREFETCH * ring_step ? 0 : put + ring_step;
     };
     for (int d = 0; d < W3_PREFETCH; ++d) fetch_next();
-    // Ring slot, its position in its group, the slot's phase.  Waiting by parity is safe with two teams: a team's stage before,
-    // two back, was let in after the one a ring before that had been consumed, and stages are consumed in order, so the barrier
-    // is at most one phase behind the one waited for (a ring has at least two slots, or three groups).
-    int s = team, sg = team % cfg.group;
+    // Ring slot and its phase.  Waiting by parity is safe with two teams: a team's stage before, two back, was let in after the one a
+    // ring before that had been consumed, and stages are consumed in order, so the barrier is at most one phase behind the one
+    // waited for (a ring has at least two slots).
+    int s = team;
     uint32_t ph = 0;
     for (int t = t0 + team; t < t1 && ok; t += TEAMS) {
       fetch_next();
@@ -287,7 +279,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
         if (cur_a != -1 || cur_b != -1) report_problem();  // counted once per skipped pair
         cur_a = cur_b = -1;
       }
-      ok = g3_wait(&sh->empty[s - sg], ph ^ 1u, abort_flag);
+      ok = g3_wait(&sh->empty[s], ph ^ 1u, abort_flag);
       if (!ok) break;
       const uint32_t sa = smem_u32(sStage + (size_t)s * stage_bytes);
       const uint32_t sb = sa + a_bytes;
@@ -302,8 +294,6 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
       cp_async_arrive_noinc(smem_u32(&sh->full[s]));
       s += TEAMS;
       if (s >= n_stage) { s -= n_stage; ph ^= 1u; }
-      sg += TEAMS;
-      while (sg >= cfg.group) sg -= cfg.group;
     }
   } else if (warp == W3_MMA_WARP) {
     // ------------------------------------------------------------------ MMA issuer
@@ -329,7 +319,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
     auto issue = [&](auto row_tiles, auto steps) -> bool {
       constexpr int MT = decltype(row_tiles)::value, N = decltype(steps)::value;
       const uint32_t idesc0 = MT == 1 ? idesc_last : idesc_full;
-      int s = 0, sg = 0, buf = 0;
+      int s = 0, buf = 0;
       uint32_t ph = 0, buf_ph = 1;
       int t = t0, seg = find_segment(tile_start, n_seg, t0);
       while (t < t1) {
@@ -353,9 +343,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
             }
             more = true;
           }
-          // one commit per group of stages (and one for the CTA's last stage, which nobody waits for)
-          if (sg == cfg.group - 1 || t + 1 == t1) mma_commit(smem_u32(&sh->empty[s - sg]));
-          sg = sg == cfg.group - 1 ? 0 : sg + 1;
+          mma_commit(smem_u32(&sh->empty[s]));
           if (++s == n_stage) { s = 0; ph ^= 1u; }
         }
         mma_commit(smem_u32(&sh->tmem_full[buf]));
@@ -487,22 +475,19 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
 inline bool w3_plan(int c_in, int c_out, int es, int k_vol, int max_smem, W3Config* cfg) {
   if (!umma_supported(c_in, c_out, es)) return false;
   const int epr = 128 / es;  // elements per 128-byte piece
-  // Packed stages: `pack` pairs share a staged row, their rows side by side in A and in B, so one MMA contracts
-  // pack times as many pairs — an MMA of 64 x 64 x 16 costs what one of 128 x 128 x 16 does, and with rows of up to
-  // 128 bytes the issue loop is what bounds the kernel.  The accumulator then holds pack x pack blocks; the epilogue
-  // keeps the diagonal.  Rows of at most 32 / 64 bytes: 4 pairs in slots of 32 / 64 bytes (a 64 x 64 accumulator,
-  // or 128 x 128 for the 64-byte slots of fp16: one MMA per 64 pairs).  Longer rows whose
-  // lengths are powers of two: 2 pairs, each row its own slot, while both fit one 128-row, 256-column accumulator
-  // (twice, so that two accumulators alternate) and three packed stages of 128 pairs fit shared memory — else the
-  // shape is planned unpacked (second pass of the loop).
+  // Packed stages: two pairs share a staged row, their rows side by side in A and in B, so one MMA contracts
+  // twice as many pairs — an MMA of 64 x 64 x 16 costs what one of 128 x 128 x 16 does, and with rows of up to
+  // 256 bytes the issue loop is what bounds the kernel.  The accumulator then holds 2 x 2 blocks; the epilogue
+  // keeps the diagonal.  For rows of more than 64 bytes whose lengths are powers of two, each its own slot, while both fit one
+  // 128-row, 256-column accumulator (twice, so that two accumulators alternate) and three packed stages of 128 pairs fit shared
+  // memory — else the shape is planned unpacked (second pass of the loop).  (Shorter rows come here only with more pairs
+  // than the short-row kernel's positions hold.)
   const int a_row = c_in * es, b_row = c_out * es, max_row = a_row > b_row ? a_row : b_row;
   const bool pow2 = (a_row & (a_row - 1)) == 0 && (b_row & (b_row - 1)) == 0;
   for (int attempt = 0; attempt < 2; ++attempt) {
   cfg->pack = 1; cfg->slot_a = cfg->slot_b = 0;
   if (attempt == 0) {
-    if (max_row <= 32) { cfg->pack = 4; cfg->slot_a = cfg->slot_b = 32; }
-    else if (max_row <= 64) { cfg->pack = 4; cfg->slot_a = cfg->slot_b = 64; }
-    else if (pow2 && 2 * c_in <= 128 && 2 * c_out <= 256) { cfg->pack = 2; cfg->slot_a = a_row; cfg->slot_b = b_row; }
+    if (max_row > 64 && pow2 && 2 * c_in <= 128 && 2 * c_out <= 256) { cfg->pack = 2; cfg->slot_a = a_row; cfg->slot_b = b_row; }
     else continue;
   }
   // rows and columns of the accumulator
@@ -529,10 +514,6 @@ inline bool w3_plan(int c_in, int c_out, int es, int k_vol, int max_smem, W3Conf
   if (n_stage > W3_MAX_STAGES) n_stage = W3_MAX_STAGES;
   if (cfg->pack > 1 && n_stage < 3) continue;  // too large packed: plan it unpacked
   if (n_stage < 2) return false;
-  // stages per commit: as many as leave three groups in flight
-  cfg->group = 1;
-  for (int g = 4; g >= 2; --g)
-    if ((n_stage - n_stage % g) / g >= 3) { cfg->group = g; n_stage -= n_stage % g; break; }
   cfg->pb = pb;
   cfg->n_stage = n_stage;
   cfg->smem = fixed + w3_ring_bytes(pb) + n_stage * pb * row_bytes;

@@ -37,7 +37,7 @@ int main() {
           if (!w3_plan(ci, co, es, kv, max_smem, &w)) { fail("w3_plan refused", es, ci, co, kv); continue; }
           if (w.smem > max_smem) fail("w3 smem over the limit", es, ci, co, kv);
           if (w.n_stage < 3 && w.pb > 32) fail("w3 fewer than three stages", es, ci, co, kv);
-          if (w.n_stage % w.group) fail("w3 stages no multiple of the group", es, ci, co, kv);
+          if (w.n_stage < 2 || w.n_stage > W3_MAX_STAGES) fail("w3 stage count", es, ci, co, kv);
           if (w.n_buf * w.n_mtile * w.n_acc > 512) fail("w3 accumulators", es, ci, co, kv);
           if (w.pb % W3_PROD_WARPS || w.pb / W3_PROD_WARPS < 4 || w.pb > W3_MAX_PB) fail("w3 pairs per stage", es, ci, co, kv);
           if (w.pack > 1) {
