@@ -356,10 +356,12 @@ def run_cfg5(args, dev, rank, world, flush):
         for r in rows:
             l, run_l = by_name[r["layer"]]  # as specified (flops and bytes count the real channels) and as run
             pairs = int(umaps.of(l).pairs)
-            b = workloads.layer_bytes(pairs, l.c_in, l.c_out, l.k_vol, 2, r["pass"])
-            fl = 2.0 * pairs * l.c_in * l.c_out
+            passes = ("wgrad", "dgrad") if r["pass"] == "bwd" else (r["pass"],)  # "bwd": both gradients by one call
+            b = sum(workloads.layer_bytes(pairs, l.c_in, l.c_out, l.k_vol, 2, q) for q in passes)
+            fl = len(passes) * 2.0 * pairs * l.c_in * l.c_out
             t_roof = max(b / (hbm * 1e9), fl / (f16_peak * 1e12)) * 1e3
-            fam = FAMILY[backend.kernel_family(r["pass"], run_l.c_in, run_l.c_out, torch.float16, True, l.k_vol)]
+            fam = " / ".join(dict.fromkeys(FAMILY[backend.kernel_family(q, run_l.c_in, run_l.c_out, torch.float16, True, l.k_vol)]
+                                           for q in passes))
             row = {"layer": l.name, "pass": r["pass"], "shape": f"{l.c_in}->{l.c_out} k{l.k_vol}", "pairs": pairs,
                    "ms": round(r["ms"], 5), "frac": round(t_roof / r["ms"], 4), "family": fam}
             table.append(row)

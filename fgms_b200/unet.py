@@ -396,10 +396,12 @@ class UNetStep:
             self.forward()
             self.backward()
 
-    def profile(self, reps: int = 5, flush=None):
+    def profile(self, reps: int = 5, flush=None, apart: bool = False):
         """Per-call device times of the step (mean over ``reps`` steps, CUDA events around every operator call):
-        a list of ``{layer, pass, ms}`` in execution order.  ``flush`` (a callable) runs before every step,
-        untimed.  Single rank only; meant for reports, not for the timed benchmark."""
+        a list of ``{layer, pass, ms}`` in execution order.  A layer's two gradients that the step computes by one call, side by
+        side, are one row, ``"bwd"``; with ``apart`` they are two calls, each with the whole chip, which the step does not
+        make.  ``flush`` (a callable) runs before every step, untimed.  Single rank only; meant for reports, not for the
+        timed benchmark."""
         import torch
         if self.multi:
             raise ValueError("profile() times the kernels of one rank: build the step with exchange=False")
@@ -425,6 +427,11 @@ class UNetStep:
                     l, wgrad, dgrad = self._bwd[i]
                     if l.skip is not None:
                         self.grad[l.skip].copy_(self.grad[l.dst])
+                    if i in self._both and not apart:
+                        a, b = ev(), ev()
+                        a.record(); check(L.fgms_b200_bwd(*self._both[i], st)); b.record()
+                        marks.append((l.name, "bwd", a, b))
+                        continue
                     a, b = ev(), ev()
                     a.record(); check(L.fgms_b200_wgrad(*wgrad, st)); b.record()
                     marks.append((l.name, "wgrad", a, b))

@@ -120,3 +120,18 @@ def test_bound_step_equals_the_autograd_module():
     for i, layer in enumerate(net.layers):
         ref = step.w_grads[i].float()
         assert float((layer.weight.grad.float() - ref).abs().max()) <= 2e-2 * float(ref.abs().max()), spec[i].name
+
+
+def test_profile_times_the_calls_that_the_step_makes():
+    """Both gradients of a layer are one call in the step, and one row; apart they are two.  Either way the step's results stand."""
+    wl, spec, host, dev, weights = _setup(8_000, 96, 1)
+    step = unet.UNetStep(spec, dev, weights, torch.from_numpy(wl.feats).cuda(), torch.from_numpy(wl.grad_out).cuda())
+    step.run()
+    want = [g.clone() for g in step.w_grads]
+    rows = step.profile(reps=1)
+    back = [(l.name, "bwd" if i > 0 else "wgrad") for i, l in reversed(list(enumerate(step.run_spec)))]
+    assert [(r["layer"], r["pass"]) for r in rows] == [(l.name, "fwd") for l in step.run_spec] + back
+    for got, ref in zip(step.w_grads, want):
+        assert float((got.float() - ref.float()).abs().max()) <= 1e-2 * float(ref.float().abs().max())
+    apart = step.profile(reps=1, apart=True)
+    assert len(apart) == 3 * len(spec) - 1 and {r["pass"] for r in apart} == {"fwd", "wgrad", "dgrad"}
