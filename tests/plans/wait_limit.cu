@@ -106,9 +106,46 @@ static int forms(int c_in, int c_out, int sms, int max_smem) {
   return bad;
 }
 
+// several pipelines: CTAs of up to `tiles` tiles and three offsets, the deal that the launcher makes
+template <bool F16, int DEAL>
+static int pipelines(int c_in, int c_out, int tiles, int sms, int max_smem) {
+  const int es = F16 ? 2 : 4, k_vol = 3, n_tiles = sms * (tiles - 1) + sms / 2, n = n_tiles * 128 - 91;
+  std::vector<int> table((size_t)k_vol * n_tiles * 128, -1);
+  for (int k = 0; k < k_vol; ++k)
+    for (int i = 0; i < n; ++i) table[(size_t)k * n_tiles * 128 + i] = (i + 1000 * k) % n;
+  std::vector<unsigned char> v((size_t)n * (c_in > c_out ? c_in : c_out) * es);
+  for (size_t i = 0; i < v.size(); i += es) {
+    if (F16) { const unsigned short h = 0x3400; std::memcpy(&v[i], &h, 2); }
+    else { const float f = 0.25f; std::memcpy(&v[i], &f, 4); }
+  }
+  const size_t w_bytes = (size_t)k_vol * c_in * c_out * es;
+  if (w_bytes > v.size()) return 1;
+  int* nbr;
+  void *weights, *src, *dst;
+  CHECK(cudaMalloc(&nbr, table.size() * 4)); CHECK(cudaMalloc(&weights, w_bytes)); CHECK(cudaMalloc(&src, v.size())); CHECK(cudaMalloc(&dst, v.size()));
+  CHECK(cudaMemcpy(nbr, table.data(), table.size() * 4, cudaMemcpyHostToDevice));
+  CHECK(cudaMemcpy(weights, v.data(), w_bytes, cudaMemcpyHostToDevice));
+  CHECK(cudaMemcpy(src, v.data(), v.size(), cudaMemcpyHostToDevice));
+  OsParams p = {};
+  p.weights = weights; p.src = src; p.dst = dst; p.nbr = nbr; p.nbr_stride = (long long)n_tiles * 128;
+  p.n_in = p.n_out = n; p.n_tiles = n_tiles; p.c_in = c_in; p.c_out = c_out; p.k_vol = k_vol;
+  OsConfig cfg;
+  if (!os_plan(c_in, c_out, es, max_smem, &cfg)) return 1;
+  os_split(&cfg, tiles, k_vol, max_smem);
+  char name[96];
+  std::snprintf(name, sizeof(name), "output-stationary %s %d -> %d, %d pipelines by %s", F16 ? "fp16" : "tf32", c_in, c_out, cfg.n_pipe, cfg.by_offset ? "offset" : "tile");
+  int bad = cfg.n_pipe < 2 || cfg.by_offset != (DEAL == OS_DEAL_OFFSETS);
+  if (bad) std::printf("%s: not the deal that is to be checked\n", name);
+  else bad = check(name, umma_osfwd_kernel<!F16, DEAL>, p, cfg, sms, OS_THREADS, max_smem, F16, true, (size_t)n * c_out * es);
+  CHECK(cudaFree(nbr)); CHECK(cudaFree(weights)); CHECK(cudaFree(src)); CHECK(cudaFree(dst));
+  return bad;
+}
+
 int main() {
   cudaDeviceProp prop;
   CHECK(cudaGetDeviceProperties(&prop, 0));
   const int sms = prop.multiProcessorCount, max_smem = (int)prop.sharedMemPerBlockOptin;
-  return forms<true>(128, 128, sms, max_smem) | forms<false>(48, 80, sms, max_smem);
+  return forms<true>(128, 128, sms, max_smem) | forms<false>(48, 80, sms, max_smem) | pipelines<true, OS_DEAL_TILES>(64, 64, 6, sms, max_smem) |
+         pipelines<false, OS_DEAL_TILES>(48, 48, 3, sms, max_smem) | pipelines<true, OS_DEAL_OFFSETS>(128, 128, 1, sms, max_smem) |
+         pipelines<false, OS_DEAL_OFFSETS>(48, 48, 1, sms, max_smem);
 }
