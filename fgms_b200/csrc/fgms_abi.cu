@@ -225,10 +225,16 @@ struct Range {
 // bound by, reds of rows in the input gradient, instructions of the gathers in the weight gradient.  The weight gradient goes
 // first, with one block per SM on its share; the input gradient's blocks find room on the others only.  Either pass takes about
 // c + u * (128-pair units) / SMs microseconds, the constants below fitted to the passes by themselves; the share is the
-// one at which the later one ends first.  Behind one another / side by side, in a row of launches: fp16 64 -> 64 0.93 M pairs 66.7 /
-// 61.4 us, 137 k 19.0 / 14.9, 32 -> 32 9.1 M 250 / 234, 84 k 10.2 / 8.1; 128 -> 128 303 k 44.1 / 38.3, 98 k 21.6 / 16.7, 256 -> 256 28 k
-// 25.7 / 19.3, stride 2 64 -> 128 9 k 12.7 / 7.4; tf32 32 -> 64 stride 2 200 k 28.8 / 26.9.  A share a sixth off gives the gain
-// away (64 -> 64 0.93 M pairs at 0.36 / 0.48 / 0.60 of the SMs 77.9 / 61.4 / 78.1).
+// one at which the later one ends first.  Behind one another / started together but with all SMs each / with the share, in a row of
+// launches: fp16 64 -> 64 0.93 M pairs 69.0 / 66.0 / 61.9 us, 137 k 19.8 / 18.9 / 15.2, 32 -> 32 9.1 M 254 / 252 / 237, 84 k 12.1 / 10.3 / 7.9; 128 -> 128 303 k
+// 44.5 / 44.2 / 38.8, 256 -> 256 28 k 25.9 / 25.7 / 22.1, stride 2 64 -> 128 9 k 12.1 / 12.2 / 7.5; tf32 32 -> 64 stride 2 200 k 25.9 / 24.1 / 22.2.  A share a
+// sixth off gives the gain away (64 -> 64 0.93 M pairs at 0.36 / 0.48 / 0.60 of the SMs 77.9 / 61.4 / 78.1).
+//
+// How good the model is: against every fourth share, over 36 shapes of 16 to 256 channels and 4 k to 9 M pairs, it was within 3 % of the best
+// one in 17, within 10 % in 29, and 0.62 to 0.99 of one behind the other in all.  It is off where both passes are short (256 -> 256 28 k
+// 22.1 where 88 of the SMs take 17.5, 4 k 12.1 / 9.6; 128 -> 128 12 k 10.3 / 8.2; stride 2 128 -> 256 20 k 14.1 / 11.1) and on LiDAR maps of two pairs a
+// row (32 -> 32 173 k pairs 13.9 / 12.7, 12.8 with all SMs each; 43 k 7.7 / 6.3).  0.97 and 1.07, the margins of "behind one another", and the terms for
+// 48 channels, whose rows are copied with idle lanes, are fitted like the others.
 int split_backward(int64_t pairs, int c_in, int c_out, int k_vol, int dtype, int math, const DeviceInfo& di) {
   fgms::G3Config g;
   fgms::W3Config w;

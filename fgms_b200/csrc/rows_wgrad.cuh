@@ -22,7 +22,7 @@
 //
 // One block per SM takes a share of the pairs, its warps take the share's tiles of 16 in turn, and the block adds up its
 // warps' fp32 sums when the offset changes.  Where those sums go straight into an fp16 gradient every block's is rounded,
-// and the pairs are shared out in units of 256 of one offset, the stages of the tcgen05 form, so that an offset of up to
+// and the pairs are shared out in units of 256 of one offset, a tile for every warp, so that an offset of up to
 // 256 pairs is rounded once.  Shares cut by single tiles split such an offset among up to six blocks: relative error of
 // the gradient (32 -> 32, 27 offsets) 4.3e-4 against 2.1e-4 in units for 80 pairs each, 4.7e-4 against 3.6e-4 for 1300.
 #pragma once

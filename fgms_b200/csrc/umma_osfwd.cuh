@@ -22,12 +22,12 @@
 // lanes' are parked (85 -> 79 us on the layer below).
 //
 // An MMA lane's stage is some 130 instructions one after the other, 540-650 cycles, of which it waits for rows during 95; its four
-// MMAs of 128 x 64 x 16 are 192.  So the work is dealt to up to three pipelines, each an MMA lane with ring slots and
-// producers of its own: tiles of a group, or, where a CTA has fewer than three tiles, offsets, whose partial accumulators the
-// epilogue adds in the pipelines' order.  Against one pipeline: 64 -> 64 on a full block of 48^3 (2.9 M pairs, 27 stages for each of
-// 864 tiles) 55.9 -> 40.7 us, 400 cycles a stage, of which shared memory needs 320 (rows written, rows and weights read by the
-// MMAs); 32 -> 32 52.4 -> 35.1; 64 -> 64 on a surface of 100 k voxels 54.7 -> 39.1, on 30^3 26.5 -> 20.4, on 1000 voxels 14.8 -> 12.6 (by
-// offsets); 128 -> 128 on 48^3 95 -> 92; 256 -> 256 on 512 voxels, which has slots for one pipeline only, 72.5 -> 73.4.
+// MMAs of 128 x 64 x 16 are 192.  So where rows are short enough for it (os_split) the work is dealt to up to three pipelines, each an
+// MMA lane with ring slots and producers of its own: tiles of a group, or, where a CTA has fewer than three tiles, offsets, whose
+// partial accumulators the epilogue adds in the pipelines' order.  Against one pipeline: 64 -> 64 on a full block of 48^3 (2.9 M
+// pairs, 27 stages for each of 864 tiles) 55.8 -> 39.9 us, 390 cycles a stage, of which shared memory needs 320 (rows written, rows
+// and weights read by the MMAs); 32 -> 32 52.5 -> 35.1; 64 -> 64 on a surface of 100 k voxels 54.4 -> 38.3, on 30^3 26.5 -> 20.0, on 1000
+// voxels 15.0 -> 12.6 (by offsets); 128 -> 128 on 48^3 95 -> 92; 256 -> 256 on 512 voxels, which has one pipeline, 72.2 -> 72.2.
 // (With eight warps that each filled 16 rows of every stage and copied zeros the block took 141 us.)
 #pragma once
 #include "common.cuh"
@@ -117,7 +117,8 @@ __global__ void os_fill_nbr_kernel(const int32_t* __restrict__ kpos, const int32
 }
 
 // What is dealt out to the pipelines, known at compile time: by_offset asked at run time cost every stage of the other forms 2-6 %, the
-// number of pipelines asked where there is one 2-4 %.
+// number of pipelines asked where there is one 2-4 %.  (The offsets' form spills 24 bytes in fp16 and 48 in tf32 at the 96 registers that
+// 640 threads leave, the other two none; it is the faster one where it is chosen all the same, see os_split.)
 enum { OS_ONE_PIPE, OS_DEAL_TILES, OS_DEAL_OFFSETS };
 template <bool TF32, int DEAL = OS_ONE_PIPE>
 __global__ void __launch_bounds__(OS_THREADS, 1) umma_osfwd_kernel(OsParams p, OsConfig cfg, const __grid_constant__ CUtensorMap w_map) {

@@ -142,7 +142,8 @@ class PeerExchange:
         self.count = (int(count) + 3) // 4 * 4
         self.group = group
         # CTAs of 128 threads and 32 registers, one per 512 values of the buffer (a 16-byte piece a thread: beside the
-        # weight gradient of a 32 -> 32 layer 18.4 us, 22.5 with a CTA per 2048): between 16 and 128 (at most one per
+        # weight gradient of a 32 -> 32 layer 18.4 us, 22.5 with a CTA per 2048; measured with one rank only, several ranks'
+        # CTAs each poll all their flags and have not been timed): between 16 and 128 (at most one per
         # SM, resident all at once beside a persistent kernel) for buffers of up to 4 MB; up to 512 for larger ones,
         # which are bound by the bytes in flight over the link (a few of these CTAs fit an SM beside a persistent one)
         self.ctas = int(ctas) if ctas else max(16, min(128, self.count // 512) if self.count <= (1 << 20) else min(512, self.count // 2048))
