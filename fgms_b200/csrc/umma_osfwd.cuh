@@ -516,11 +516,13 @@ inline int os_stage_cycles(int pipes, int n_stage, int kch) {
 // Pipelines for CTAs of up to `tiles` tiles.
 //
 // A CTA of one tile has its offsets dealt out to three pipelines, if their accumulators fit tensor memory, each has a weight
-// buffer, and the rings together hold three rows of the input.  (fp16 128 -> 128 on 1000 voxels 22.8 -> 21.2 us, 160 -> 48 25.2 -> 20.7, tf32 64 -> 64
-// 22.0 -> 17.5.  With smaller rings or two pipelines a pipeline waits for its one buffer of weights, or for rows: 160 -> 160 30.6 -> 44.8, 256 ->
-// 128 33.4 -> 44.1, 208 -> 64 28.6 -> 30.1, tf32 80 -> 80 26.2 -> 29.9; 16 -> 208 with two pipelines 18.5 -> 19.0.)  Two weight buffers each, where the rings
-// then hold six rows: 64 -> 128 16.0 -> 14.8, but tf32 48 -> 48 17.6 -> 18.3; then a CTA of two tiles has its offsets dealt out as well
-// (16 -> 16 on 30 k voxels 15.5, by tiles 16.3; 128 -> 64 30.6 / 28.6).
+// buffer, and the rings together hold three rows of the input or nine stages.  (fp16 128 -> 128 on 1000 voxels 22.8 -> 21.2 us, 160 -> 48 25.2 ->
+// 20.7, tf32 64 -> 64 22.0 -> 17.5, 128 -> 16 29.0 -> 25.5.  With smaller rings a pipeline waits for its one buffer of weights, or for
+// rows: 160 -> 160 30.6 -> 44.8, 256 -> 128 33.4 -> 44.1, 208 -> 64 28.6 -> 30.1, tf32 80 -> 80 26.2 -> 29.9.)  Two weight buffers each, where that takes no slots
+// (80 -> 64 16.3 -> 15.0) or the rings then hold six rows: 64 -> 128 16.0 -> 14.8, but tf32 48 -> 48 17.6 -> 18.3; with six rows a CTA of two tiles
+// has its offsets dealt out as well (16 -> 16 on 30 k voxels 15.5, by tiles 16.3; 128 -> 64 30.6 / 28.6).  Where the accumulators of two fit, two
+// with two buffers each, if rings hold three rows and weights are what it waits for: 48 -> 240 22.0 -> 19.6, 64 -> 208 23.2 -> 21.5, 32 -> 208 (16 KB of
+// weights) 19.6 -> 18.9, but 16 -> 208 (8 KB) 18.5 -> 19.0 and with one buffer each 64 -> 208 26.4.
 //
 // Otherwise tiles are dealt out so that the most loaded pipeline ends first; equally good, three for rows of one 128-byte chunk (fp16
 // 16 -> 16 on 100 k voxels, six tiles, with one / two / three 48.5 / 35.2 / 31.6 us), fewer for longer ones (96 -> 96 88.3 / 72.5 / 78.1).  With three
@@ -528,30 +530,37 @@ inline int os_stage_cycles(int pipes, int n_stage, int kch) {
 // 80.3 / 101.4, on 30 k (two tiles) 56.6 / 58.2; with two slots always (160 -> 160 on 100 k 166 / 190).
 inline void os_split(OsConfig* cfg, int tiles, int k_vol, int max_smem) {
   const int other = cfg->smem - cfg->n_wbuf * cfg->w_bytes - cfg->n_stage * G3_STAGE_BYTES;
-  constexpr int M = OS_MAX_PIPES;
   auto set = [&](int pipes) {
     const int most = OS_PROD_WARPS / pipes, slots = cfg->n_stage / pipes;
     cfg->n_pipe = pipes;
     cfg->n_prod = slots < most ? slots : most;
   };
-  if (tiles < M && M <= k_vol && tiles * M <= OS_MAX_GROUP && tiles * M * cfg->n_acc <= 512) {
-    for (int each = 2; each >= (tiles == 1 ? 1 : 2); --each) {
-      const int room = max_smem - other - each * M * cfg->w_bytes;
-      if (room < 2 * M * G3_STAGE_BYTES) continue;
-      const int fit = room / G3_STAGE_BYTES, stages = fit < OS_MAX_STAGES ? fit : OS_MAX_STAGES;
-      if (stages / M * M < 3 * each * cfg->kch) continue;
-      cfg->by_offset = 1;
-      cfg->n_wbuf = each * M;
-      cfg->n_stage = stages;
-      cfg->group = tiles;
-      cfg->smem = other + cfg->n_wbuf * cfg->w_bytes + cfg->n_stage * G3_STAGE_BYTES;
-      set(M);
-      return;
-    }
+  auto stages = [&](int wbufs) {  // that fit beside so many weight buffers
+    const int fit = (max_smem - other - wbufs * cfg->w_bytes) / G3_STAGE_BYTES;
+    return max_smem - other < wbufs * cfg->w_bytes ? 0 : fit < OS_MAX_STAGES ? fit : OS_MAX_STAGES;
+  };
+  auto fits = [&](int pipes) { return pipes <= k_vol && tiles * pipes <= OS_MAX_GROUP && tiles * pipes * cfg->n_acc <= 512; };
+  int m = 0, each = 0;  // pipelines that offsets are dealt out to, weight buffers of each
+  if (tiles < 3 && fits(3)) {
+    const int one = stages(3) / 3 * 3, two = stages(6) / 3 * 3;
+    if (two >= 6 && two >= 6 * cfg->kch) m = 3, each = 2;
+    else if (tiles == 1 && one >= 6 && (one >= 9 || one >= 3 * cfg->kch)) m = 3, each = two == one ? 2 : 1;
+  } else if (tiles == 1 && fits(2)) {
+    const int two = stages(4) / 2 * 2;
+    if (two >= 4 && two >= 3 * cfg->kch && cfg->w_bytes >= 16384) m = 2, each = 2;
+  }
+  if (m > 0) {
+    cfg->by_offset = 1;
+    cfg->n_wbuf = each * m;
+    cfg->n_stage = stages(cfg->n_wbuf);
+    cfg->group = tiles;
+    cfg->smem = other + cfg->n_wbuf * cfg->w_bytes + cfg->n_stage * G3_STAGE_BYTES;
+    set(m);
+    return;
   }
   int pipes = 1;
   long long least = 0;
-  for (int n = 1; n <= M && n <= tiles && n <= cfg->group && cfg->n_stage >= 2 * n; ++n) {
+  for (int n = 1; n <= OS_MAX_PIPES && n <= tiles && n <= cfg->group && cfg->n_stage >= 2 * n; ++n) {
     const int group = cfg->group / n * n, last = tiles % group;
     const long long turns = (long long)(tiles / group) * (group / n) + (last + n - 1) / n, cycles = turns * os_stage_cycles(n, cfg->n_stage, cfg->kch);
     if (n == 1 || cycles < least || (cycles == least && cfg->kch == 1)) pipes = n, least = cycles;

@@ -1,7 +1,7 @@
 // Host-side check of the deal of the output-stationary forward (os_split) over every channel pair, CTAs of one to forty tiles and
 // kernel volumes from 1 to 4096: what is launched fits shared and tensor memory and starts on the boundaries its copies need; no more
 // producer warps than ring slots, weight buffers a multiple of the pipelines where offsets are dealt out; a pipeline of an offset
-// deal has a weight buffer and the rings hold three rows; a deal of tiles is not slower than one pipeline by the cycles the
+// deal has a weight buffer and the rings hold three rows or nine stages; a deal of tiles is not slower than one pipeline by the cycles the
 // rule goes by.  Prints one line per violation; exit status 1 if there are any.
 #include <cstdio>
 #include <initializer_list>
@@ -29,7 +29,7 @@ int main() {
                       c.group * parts * c.n_acc <= 512 && c.group * c.kch <= 64 && c.w_bytes % 1024 == 0 && c.smem <= max_smem &&
                       c.smem == 1024 + OS_EPI_WARPS * 4096 + OS_SHARED_BYTES + c.n_wbuf * c.w_bytes + c.n_stage * G3_STAGE_BYTES;
             if (c.by_offset) {
-              ok = ok && n <= kv && tiles <= c.group && c.n_wbuf % n == 0 && slots * n >= 3 * c.kch;
+              ok = ok && n <= kv && tiles <= c.group && c.n_wbuf % n == 0 && (slots * n >= 9 || slots * n >= 3 * c.kch);
             } else {
               ok = ok && c.group % n == 0;
               int turns = 0;
