@@ -193,23 +193,16 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
     const uint8_t* og_c = og + cc * 16;
     // The pieces of R rows of one operand.  What this role spends its time on are instructions (with the copies left out
     // the kernel took as long: tests of every one of eight possible pieces and address arithmetic, 400 instructions a
-    // warp and stage), so the usual numbers of pieces have their own straight code.
+    // warp and stage), so the usual numbers of pieces have their own straight code.  (tf32 rows of 5 to 8 pieces with eight tests / in a loop /
+    // so: 240 -> 240 on 268 k pairs 65 / 69 / 57 us, 160 -> 208 on 754 k 138 / 133 / 103, 80 -> 224 stride 2 on 5.8 k 8.5 / 8.9 / 8.4.)
     auto copy_pieces = [&](auto rounds, auto pieces, const uint8_t* const (&from)[4], const uint32_t (&rel)[4], uint32_t to, const uint32_t (&n)[4],
-                           int np, bool tail) {
+                           bool tail) {
       constexpr int R = decltype(rounds)::value, NP = decltype(pieces)::value;
-      if constexpr (NP > 0) {
 #pragma unroll
-        for (int h = 0; h < NP; ++h)
+      for (int h = 0; h < NP; ++h)
 #pragma unroll
-          for (int u = 0; u < R; ++u)
-            if (FULL || h + 1 < NP || tail) cp_async16_n(to + (uint32_t)h * lbo + rel[u], from[u] + h * 128, n[u]);
-      } else {
-#pragma unroll 1
-        for (int h = 0; h < np; ++h)
-#pragma unroll
-          for (int u = 0; u < R; ++u)
-            if (FULL || h + 1 < np || tail) cp_async16_n(to + (uint32_t)h * lbo + rel[u], from[u] + h * 128, n[u]);
-      }
+        for (int u = 0; u < R; ++u)
+          if (FULL || h + 1 < NP || tail) cp_async16_n(to + (uint32_t)h * lbo + rel[u], from[u] + h * 128, n[u]);
     };
     // rows rs + rpp u of rounds u0 .. u0 + R - 1 of one operand; their entries are in lanes rs + rpp u of `cur`, -1 zero-fills
     auto copy_rows = [&](auto rounds, int u0, int cur, const uint8_t* base, uint32_t row_bytes, const uint32_t (&rel)[4], uint32_t to, int np, bool tail) {
@@ -222,14 +215,24 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
         n[u] = i >= 0 ? 16u : 0u;  // 0 bytes read: the chunk is zero-filled
         from[u] = base + (size_t)max(i, 0) * row_bytes;
       }
-      // (tf32 rows of 8 pieces: 240 -> 240 on 268 k pairs 64.7 us with eight tests, 68.7 in a loop, 56.7 this way; 5 to 7 stay in the loop,
-      // 160 -> 160 on 131 k 32.3 / 27.8, 192 -> 192 34.3 / 30.6)
-      if (np == 2) copy_pieces(rounds, std::integral_constant<int, 2>(), from, rel, to, n, np, tail);
-      else if (np == 1) copy_pieces(rounds, std::integral_constant<int, 1>(), from, rel, to, n, np, tail);
-      else if (np == 3) copy_pieces(rounds, std::integral_constant<int, 3>(), from, rel, to, n, np, tail);
-      else if (np == 4) copy_pieces(rounds, std::integral_constant<int, 4>(), from, rel, to, n, np, tail);
-      else if (TF32 && np == 8) copy_pieces(rounds, std::integral_constant<int, TF32 ? 8 : 0>(), from, rel, to, n, np, tail);
-      else copy_pieces(rounds, std::integral_constant<int, 0>(), from, rel, to, n, np, tail);
+      if (np == 2) copy_pieces(rounds, std::integral_constant<int, 2>(), from, rel, to, n, tail);
+      else if (np == 1) copy_pieces(rounds, std::integral_constant<int, 1>(), from, rel, to, n, tail);
+      else if (np == 3) copy_pieces(rounds, std::integral_constant<int, 3>(), from, rel, to, n, tail);
+      else if (np == 4) copy_pieces(rounds, std::integral_constant<int, 4>(), from, rel, to, n, tail);
+      else if constexpr (TF32) {
+        if (np == 8) copy_pieces(rounds, std::integral_constant<int, 8>(), from, rel, to, n, tail);
+        else if (np == 7) copy_pieces(rounds, std::integral_constant<int, 7>(), from, rel, to, n, tail);
+        else if (np == 6) copy_pieces(rounds, std::integral_constant<int, 6>(), from, rel, to, n, tail);
+        else copy_pieces(rounds, std::integral_constant<int, 5>(), from, rel, to, n, tail);
+      } else {
+        // any other number (no fp16 row has one); with nothing here the compiler lays the others out worse: 128 -> 64 on 591 k 23.9 -> 26.9 us,
+        // 128 -> 128 on 303 k 17.7 -> 18.7
+#pragma unroll 1
+        for (int h = 0; h < np; ++h)
+#pragma unroll
+          for (int u = 0; u < R; ++u)
+            if (FULL || h + 1 < np || tail) cp_async16_n(to + (uint32_t)h * lbo + rel[u], from[u] + h * 128, n[u]);
+      }
     };
     auto copy_rounds = [&](auto rounds, int u0, int cur_a, int cur_b, uint32_t sa, uint32_t sb) {
       copy_rows(rounds, u0, cur_a, feats_c, a_row_bytes, rel_a, sa, np_a, tail_a);

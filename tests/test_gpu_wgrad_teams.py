@@ -11,7 +11,7 @@ from tests.util import Problem
 
 pytestmark = pytest.mark.gpu
 WIDTHS = [("fp16", 128, 128), ("fp16", 96, 160), ("fp16", 256, 256), ("fp16", 16, 208), ("tf32", 64, 64), ("tf32", 48, 64),
-          ("tf32", 96, 32), ("tf32", 160, 192), ("tf32", 256, 224), ("tf32", 16, 128)]
+          ("tf32", 96, 32), ("tf32", 160, 192), ("tf32", 256, 224), ("tf32", 16, 128), ("tf32", 144, 240)]
 
 
 @pytest.mark.parametrize("stages", [0, 1, 2, 3, 4, 5, 9, 48])
