@@ -3,19 +3,27 @@
 //
 // The products of a ragged layer (20 -> 36 channels, 390 k pairs) are 7.5 us of FMA a pass, moving its rows 11-15 us;
 // the tiles of simt_kernels.cuh, 64 x 64 whatever the width, read shared memory a word at a time and keep no row in
-// flight, and take 61 / 100 / 124 us (forward, dgrad, weight gradient); here 34 / 33 / 38 us, 64 -> 64 on 591 k pairs
-// 205 / 204 / 186 -> 165 / 161 / 169 us, 3 -> 64 69 / 86 / 199 -> 36 / 41 / 47 us.  Bound by shared memory (twelve 16-byte
-// reads of four cycles for 64 packed FMAs) and, with short rows, by the instructions of a tile's gather and reds.
+// flight, and take 61 / 100 / 124 us (forward, dgrad, weight gradient); here 33 / 32 / 38 us, 64 -> 64 on 591 k pairs
+// 205 / 204 / 186 -> 157 / 156 / 152 us, 3 -> 64 69 / 86 / 199 -> 35 / 41 / 43 us.  Bound by the FMA pipe and what waits for it: a packed
+// FMA takes 2.4 cycles a scheduler (3.1 where no operand is the last one's), and multiplications of addresses and copies of registers go through
+// the same pipe (forward 64 -> 64: 38 of 54 M instructions there are the products, it is busy for 62 % of the time, 2.4 warps a scheduler
+// wait for it or for shared memory); with short rows the instructions of a tile's gather and reds.
 //
 //   * the work of a pass is cut to the layer's width: four (forward) or eight by four (weight gradient) channels per
 //     thread, as many threads side by side as the width needs, the others take further pairs;
 //   * operands come from shared memory 16 bytes at a time, rows laid an odd number of 16-byte units apart so that the
 //     lanes of a quarter warp meet different banks;
 //   * rows are copied with cp.async a tile ahead, their map entries another tile ahead;
-//   * the forward sums even and odd contraction channels side by side (fma.rn.f32x2 on two halves of a 16-byte word):
-//     half the instructions, and nothing to duplicate.
+//   * products are packed FMAs, half the instructions: the forward sums even and odd contraction channels side by side (fma.rn.f32x2
+//     on two halves of a 16-byte word: nothing to duplicate), the weight gradient two input channels, with the output channel in both halves.
+//     Fewer instructions leave the two passes of a backward, which share the SMs, more of each other's: 64 -> 64 on 591 k pairs 365 -> 293 us,
+//     20 -> 36 on 390 k 72.3 -> 67.7, 40 -> 33 on 208 k 91 -> 84.
+//
+// Weights kept in registers, a lane's share of the contraction each (16 to 24 channels by four), were slower: forward 20 -> 36 48.8 us, dgrad
+// 64 -> 64 212.
 #pragma once
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "umma.cuh"  // launch_pdl, griddep_*
@@ -25,12 +33,23 @@ namespace fgms {
 constexpr int FF_WARPS = 4;
 constexpr int FF_THREADS = FF_WARPS * 32;
 constexpr int FF_MAX_K = 128;
-constexpr int FF_WGRAD_BLOCKS = 6;  // per SM, by registers
 constexpr int ff_gms_blocks(int pt) { return pt == 8 ? 3 : 4; }  // 64 accumulators, 16 weights and the walk do not fit 128 registers
 
 __device__ __forceinline__ void ff_fma2(uint64_t& c, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
 }
+__device__ __forceinline__ uint64_t ff_mul2(uint64_t a, uint64_t b) {
+  uint64_t c;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(c) : "l"(a), "l"(b));
+  return c;
+}
+__device__ __forceinline__ void ff_add2(uint64_t& c, uint64_t a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(c) : "l"(a)); }
+__device__ __forceinline__ uint64_t ff_two(float lo, float hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float ff_half(uint64_t v, int h) { return __uint_as_float((uint32_t)(v >> (32 * h))); }
 __device__ __forceinline__ void ff_lds2(uint32_t addr, uint64_t& a, uint64_t& b) {
   asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr) : "memory");
 }
@@ -201,26 +220,33 @@ __global__ void __launch_bounds__(FF_THREADS, ff_gms_blocks(PT)) ffma_gms_kernel
         ff_wait<1>();
         __syncwarp();
         uint64_t acc[PT][4];
-#pragma unroll
-        for (int i = 0; i < PT; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
         const uint32_t a0 = a_addr + buf * a_buf;
-#pragma unroll 1
-        for (int k = 0; k < 4 * kp; k += 16) {
+        // four channels of the contraction, `first`: the sums begin
+        auto step = [&](uint32_t k, uint32_t off, auto first) {
           uint64_t b0[4], b1[4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) ff_lds2(b_addr + j * b_step + k, b0[j], b1[j]);
+          for (int j = 0; j < 4; ++j) ff_lds2(b_addr + j * b_step + k + off, b0[j], b1[j]);
 #pragma unroll
           for (int i = 0; i < PT; ++i) {
             uint64_t x0, x1;
-            ff_lds2(a0 + i * a_step + k, x0, x1);
+            ff_lds2(a0 + i * a_step + k + off, x0, x1);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) ff_fma2(acc[i][j], x0, b0[j]);
+            for (int j = 0; j < 4; ++j) {
+              if constexpr (decltype(first)::value) acc[i][j] = ff_mul2(x0, b0[j]);
+              else ff_fma2(acc[i][j], x0, b0[j]);
+            }
 #pragma unroll
             for (int j = 0; j < 4; ++j) ff_fma2(acc[i][j], x1, b1[j]);
           }
+        };
+        step(0u, 0u, std::true_type());
+        uint32_t k = 16;
+#pragma unroll 1
+        for (; k + 16 < 4 * (uint32_t)kp; k += 32) {
+          step(k, 0u, std::false_type());
+          step(k, 16u, std::false_type());
         }
+        if (k < 4 * (uint32_t)kp) step(k, 0u, std::false_type());
         const int n = n0 + 4 * c, valid = min(4, p.n_dim - n);
         if (active && valid > 0) {
 #pragma unroll
@@ -249,15 +275,17 @@ constexpr int FW_PAIRS = 64;    // pairs of a chunk in shared memory, and of a s
 constexpr int FW_BLOCK = 64;    // channels of a block of dW_k on either side
 
 // Block threads: `slices` groups of rg x cg threads, each thread eight input by four output channels; slice s takes pairs
-// s, s + slices, .. of a chunk.  Sums stay in registers over the block's whole run inside one offset; then the slices meet
+// s, s + slices, .. of a chunk.  Sums stay in registers over the block's whole run inside one offset, those of 32 to 64 pairs at a time and
+// the total of these (relative error 64 -> 64 on 591 k pairs 6.5e-7 -> 1.9e-7, 20 -> 36 2.3e-7 -> 1.5e-7; the same time); then the slices meet
 // in shared memory and leave with one red per value.
-__global__ void __launch_bounds__(FF_THREADS, FF_WGRAD_BLOCKS) ffma_wgrad_kernel(WgradParams p) {
+template <int BLOCKS>
+__global__ void __launch_bounds__(FF_THREADS, BLOCKS) ffma_wgrad_kernel(WgradParams p) {
   extern __shared__ __align__(16) int ff_smem_dyn[];
   int* tile_start = ff_smem_dyn;
   int* kpos_s = tile_start + p.k_vol + 2;
   const int bm = min(FW_BLOCK, p.c_in), bn = min(FW_BLOCK, p.c_out);
   const int rg = (bm + 7) / 8, cg = (bn + 3) / 4, ld_a = 8 * rg, ld_g = 4 * cg;
-  const int slices = FF_THREADS / (rg * cg);
+  const int slices = FF_THREADS / (rg * cg), period = max(1, 32 * slices / FW_PAIRS);
   int* rows = ff_smem_dyn + (2 * p.k_vol + 3 + 3) / 4 * 4;                 // [2][in, out][FW_PAIRS]
   float* stage = reinterpret_cast<float*>(rows + 4 * FW_PAIRS);            // [2][FW_PAIRS][ld_a + ld_g]
   const int stage_words = FW_PAIRS * (ld_a + ld_g);
@@ -328,11 +356,13 @@ __global__ void __launch_bounds__(FF_THREADS, FF_WGRAD_BLOCKS) ffma_wgrad_kernel
         __syncthreads();
         start(0);
 
-        float acc[8][4];
+        // input channels 2 i and 2 i + 1, output channel j: the sums of the last few chunks, and of those before
+        uint64_t acc[4][4], total[4][4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+          for (int j = 0; j < 4; ++j) acc[i][j] = total[i][j] = 0ull;
+        int until = period;
         for (int chunk = 0; chunk < chunks; ++chunk) {
           start(chunk + 1);
           ff_wait<1>();
@@ -340,39 +370,56 @@ __global__ void __launch_bounds__(FF_THREADS, FF_WGRAD_BLOCKS) ffma_wgrad_kernel
           store_rows(chunk + 2);  // where this chunk's entries were: every thread has started it
           load_rows(chunk + 3);
           if (slice < slices) {
-            const float* a = stage + (chunk & 1) * stage_words + 8 * r;
+            const uint32_t a = ff_smem(stage + (chunk & 1) * stage_words + 8 * r);
             const float* b = stage + (chunk & 1) * stage_words + FW_PAIRS * ld_a + 4 * c;
-#pragma unroll 4
+#pragma unroll (BLOCKS <= 3 ? 8 : 4)
             for (int j = slice; j < FW_PAIRS; j += slices) {
-              const float4 x0 = *reinterpret_cast<const float4*>(a + j * ld_a), x1 = *reinterpret_cast<const float4*>(a + j * ld_a + 4);
+              uint64_t x[4];
+              ff_lds2(a + 4 * j * ld_a, x[0], x[1]);
+              ff_lds2(a + 4 * j * ld_a + 16, x[2], x[3]);
               const float4 y = *reinterpret_cast<const float4*>(b + j * ld_g);
-              const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+              const uint64_t y2[4] = {ff_two(y.x, y.x), ff_two(y.y, y.y), ff_two(y.z, y.z), ff_two(y.w, y.w)};
 #pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                acc[i][0] = fmaf(x[i], y.x, acc[i][0]);
-                acc[i][1] = fmaf(x[i], y.y, acc[i][1]);
-                acc[i][2] = fmaf(x[i], y.z, acc[i][2]);
-                acc[i][3] = fmaf(x[i], y.w, acc[i][3]);
-              }
+              for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) ff_fma2(acc[i][k], x[i], y2[k]);
             }
+          }
+          if (BLOCKS < 6 && (--until == 0 || chunk + 1 == chunks)) {
+            until = period;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                ff_add2(total[i][j], acc[i][j]);
+                acc[i][j] = 0ull;
+              }
           }
           __syncthreads();  // the chunk's stage is free, the entries of chunk + 2 are visible
         }
         ff_wait<0>();
+        const uint64_t(&sums)[4][4] = BLOCKS < 6 ? total : acc;  // six blocks an SM have a chunk each
         // slices meet: [slices][8 rg][4 cg] words, at most 32 per thread of the block
         if (slice < slices) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
-            *reinterpret_cast<float4*>(stage + (slice * ld_a + 8 * r + i) * ld_g + 4 * c) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+          for (int i = 0; i < 8; ++i) {
+            float4 v;
+            v.x = ff_half(sums[i / 2][0], i & 1); v.y = ff_half(sums[i / 2][1], i & 1); v.z = ff_half(sums[i / 2][2], i & 1); v.w = ff_half(sums[i / 2][3], i & 1);
+            *reinterpret_cast<float4*>(stage + (slice * ld_a + 8 * r + i) * ld_g + 4 * c) = v;
+          }
         }
         __syncthreads();
         for (int e = tid; e < ld_a * cg; e += FF_THREADS) {
           const int m = e / cg, n = 4 * (e - m * cg);
           if (m >= cols_a || n >= cols_g) continue;
           float v[4] = {0.f, 0.f, 0.f, 0.f};
-          for (int s = 0; s < slices; ++s) {
-            const float4 x = *reinterpret_cast<const float4*>(stage + (s * ld_a + m) * ld_g + n);
-            v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+          for (int s = 0; s < slices; s += 4) {  // fours of slices first
+            float4 x[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              x[k] = s + k < slices ? *reinterpret_cast<const float4*>(stage + ((s + k) * ld_a + m) * ld_g + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[0] += (x[0].x + x[1].x) + (x[2].x + x[3].x); v[1] += (x[0].y + x[1].y) + (x[2].y + x[3].y);
+            v[2] += (x[0].z + x[1].z) + (x[2].z + x[3].z); v[3] += (x[0].w + x[1].w) + (x[2].w + x[3].w);
           }
           scatter_add<4>(dwk + (size_t)(m0 + m) * p.c_out + n0 + n, v, min(4, cols_g - n), vec_out);
         }
@@ -413,9 +460,10 @@ inline bool ff_plan(int k_dim, int n_dim, int k_vol, long long pairs, int sms, F
   return found;
 }
 
+inline int ff_by_smem(size_t smem) { return (int)(227 * 1024 / (smem + 1024)); }  // blocks
 // As many blocks as an SM holds by registers (`by_regs`, the launch bound) and by shared memory, not more than tiles.
 inline int ff_grid(long long tiles, size_t smem, int by_regs, int sms) {
-  const long long by_smem = (long long)(227 * 1024 / (smem + 1024)), most = sms * (by_smem < by_regs ? by_smem : by_regs);
+  const long long by_smem = ff_by_smem(smem), most = sms * (by_smem < by_regs ? by_smem : by_regs);
   return (int)(tiles < most ? tiles : most);
 }
 
@@ -447,14 +495,23 @@ inline int launch_ffma_gms(const GmsParams& p, bool trans, cudaStream_t st, int 
   return trans ? ff_launch_pt<true, false>(p, f, st, sms) : ff_launch_pt<false, false>(p, f, st, sms);
 }
 
+template <int BLOCKS>
+inline int ff_launch_wgrad(const WgradParams& p, size_t smem, cudaStream_t st, int sms) {
+  static std::atomic<int> granted[64];
+  if (ensure_smem(ffma_wgrad_kernel<BLOCKS>, (int)smem, granted)) return -1;
+  const int grid = ff_grid((long long)p.pairs / FW_PAIRS + p.k_vol, smem, BLOCKS, sms);
+  return launch_pdl(ffma_wgrad_kernel<BLOCKS>, grid, FF_THREADS, smem, st, p) == cudaSuccess ? 0 : -1;
+}
 inline int launch_ffma_wgrad(const WgradParams& p, cudaStream_t st, int sms) {
   const int rg = ((p.c_in < FW_BLOCK ? p.c_in : FW_BLOCK) + 7) / 8, cg = ((p.c_out < FW_BLOCK ? p.c_out : FW_BLOCK) + 3) / 4;
   const size_t stages = 2 * FW_PAIRS * (size_t)(8 * rg + 4 * cg) * 4, sums = FF_THREADS * 32 * 4;
   const size_t smem = ff_table_bytes(p.k_vol) + 4 * FW_PAIRS * 4 + (stages > sums ? stages : sums);
-  static std::atomic<int> granted[64];
-  if (ensure_smem(ffma_wgrad_kernel, (int)smem, granted)) return -1;
-  const int grid = ff_grid((long long)p.pairs / FW_PAIRS + p.k_vol, smem, FF_WGRAD_BLOCKS, sms);
-  return launch_pdl(ffma_wgrad_kernel, grid, FF_THREADS, smem, st, p) == cudaSuccess ? 0 : -1;
+  // Registers, in which reads of shared memory run ahead of the products, are worth more than warps: four blocks of 128 rather than six
+  // of 80 (24 -> 24 on 296 k pairs 24.2 -> 22.1 us), three of 168 where shared memory holds no more (64 -> 64 on 591 k 161 -> 152).
+  // A call that gives each of six blocks an SM a single chunk has them all the same: 4 -> 16 on 39 k pairs 7.4 us with four, 6.2.
+  const long long tiles = (long long)p.pairs / FW_PAIRS + p.k_vol;
+  if (ff_by_smem(smem) >= 6 && tiles > 4ll * sms && tiles <= 6ll * sms) return ff_launch_wgrad<6>(p, smem, st, sms);
+  return ff_by_smem(smem) > 3 ? ff_launch_wgrad<4>(p, smem, st, sms) : ff_launch_wgrad<3>(p, smem, st, sms);
 }
 
 }  // namespace fgms
