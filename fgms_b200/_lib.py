@@ -23,6 +23,9 @@ SIGNATURES = {
     "fgms_b200_seq_fwd": (c_int, [c_void_p] * 7 + [c_int64] + [c_int] * 6 + [c_int64] + [c_int] * 3 + [c_void_p]),
     "fgms_b200_dgrad": (c_int, [c_void_p] * 6 + [c_int64] + [c_int] * 7 + [c_void_p]),
     "fgms_b200_zero2": (c_int, [c_void_p, c_size_t, c_void_p, c_size_t, c_void_p]),
+    "fgms_b200_zero_list": (c_int, [c_void_p, c_void_p, c_int, c_void_p]),
+    "fgms_b200_add": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_void_p]),
+    "fgms_b200_copy_rows_f16": (c_int, [c_void_p, c_int64, c_int, c_void_p, c_int64, c_int64, c_int, c_void_p]),
     "fgms_b200_wgrad": (c_int, [c_void_p] * 6 + [c_int64] + [c_int] * 7 + [c_void_p, c_size_t, c_int, c_void_p]),
     "fgms_b200_wgrad_finalize": (c_int, [c_void_p, c_void_p, c_int64, c_void_p]),
     "fgms_b200_wgrad_f16_noalloc": (c_int, [c_void_p] * 6 + [c_int64] + [c_int] * 6 + [c_void_p]),

@@ -214,4 +214,67 @@ __global__ void __launch_bounds__(256) zero2_kernel(uint8_t* a, size_t a_bytes, 
   if (i0 < (b_bytes & 15)) b[(b_bytes & ~(size_t)15) + i0] = 0;
 }
 
+// Clears up to ZERO_LIST buffers, 16 bytes per store, each from a 16-byte boundary: the gradients of a whole stack of layers in one
+// launch.  A block clears parts of ZERO_PART bytes of the buffers laid end to end, so that many small ones cost no more than one.
+constexpr int ZERO_LIST = 64;
+constexpr unsigned ZERO_PART = 16384;
+struct ZeroList {
+  uint8_t* at[ZERO_LIST];
+  size_t bytes[ZERO_LIST];
+  unsigned first_part[ZERO_LIST + 1];  // parts before a buffer
+  int n;
+};
+__global__ void __launch_bounds__(256) zero_list_kernel(const __grid_constant__ ZeroList z) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  int i = 0;
+  for (unsigned part = blockIdx.x; part < z.first_part[z.n]; part += gridDim.x) {
+    while (part >= z.first_part[i + 1]) ++i;
+    const size_t from = (size_t)(part - z.first_part[i]) * ZERO_PART, bytes = min((size_t)ZERO_PART, z.bytes[i] - from);
+    uint8_t* at = z.at[i] + from;
+    for (unsigned b = threadIdx.x * 16; b + 16 <= bytes; b += 256 * 16) *reinterpret_cast<uint4*>(at + b) = make_uint4(0, 0, 0, 0);
+    if (threadIdx.x < (bytes & 15)) at[(bytes & ~(size_t)15) + threadIdx.x] = 0;
+  }
+}
+
+// y += x, in fp16 each sum rounded once: the skip connections of a stack and their gradients.  Both start on 16-byte boundaries.
+template <bool F16>
+__global__ void __launch_bounds__(256) add_kernel(uint8_t* y, const uint8_t* x, long long count) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  constexpr int PER = F16 ? 8 : 4;
+  const long long n = count / PER, step = (long long)gridDim.x * blockDim.x, i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  for (long long i = i0; i < n; i += step) {
+    uint4 a = reinterpret_cast<uint4*>(y)[i];
+    const uint4 b = reinterpret_cast<const uint4*>(x)[i];
+    auto sum = [](uint32_t u, uint32_t v) {
+      if (F16) {
+        const __half2 s = __hadd2(*reinterpret_cast<__half2*>(&u), *reinterpret_cast<__half2*>(&v));
+        return *reinterpret_cast<const uint32_t*>(&s);
+      }
+      return __float_as_uint(__uint_as_float(u) + __uint_as_float(v));
+    };
+    a = make_uint4(sum(a.x, b.x), sum(a.y, b.y), sum(a.z, b.z), sum(a.w, b.w));
+    reinterpret_cast<uint4*>(y)[i] = a;
+  }
+  const long long rest = n * PER + i0;
+  if (rest < count) {
+    if (F16) reinterpret_cast<__half*>(y)[rest] = __hadd(reinterpret_cast<__half*>(y)[rest], reinterpret_cast<const __half*>(x)[rest]);
+    else reinterpret_cast<float*>(y)[rest] += reinterpret_cast<const float*>(x)[rest];
+  }
+}
+
+// The first `len` values of `rows` rows from one pitch to another, fp32 rounded to fp16 on the way where the types differ: rows padded
+// to a width that the tensor-core kernels take, and gradients without the padding.
+template <typename From>
+__global__ void __launch_bounds__(256) copy_rows_kernel(const From* src, long long src_pitch, __half* dst, long long dst_pitch, long long rows, int len) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const long long count = rows * len, step = (long long)gridDim.x * blockDim.x;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += step) {
+    const long long r = i / len, c = i - r * len;
+    dst[r * dst_pitch + c] = __float2half_rn((float)src[r * src_pitch + c]);
+  }
+}
+
 }  // namespace fgms

@@ -428,6 +428,74 @@ int fgms_b200_zero2(void* a, size_t a_bytes, void* b, size_t b_bytes, void* stre
   return check_launch("zero2_kernel");
 }
 
+int fgms_b200_zero_list(void* const* buffers, const size_t* bytes, int n, void* stream) {
+  TraceRange trace_range("fgms_b200_zero_list");
+  if (n < 0 || (n > 0 && (!buffers || !bytes))) return fail(FGMS_ERR_INVALID_ARG, "negative count or null pointer");
+  for (int i = 0; i < n; ++i) {
+    if (bytes[i] > 0 && !buffers[i]) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
+    if (reinterpret_cast<uintptr_t>(buffers[i]) & 15) return fail(FGMS_ERR_INVALID_ARG, "buffers must be 16-byte aligned");
+    if (bytes[i] > ((size_t)1 << 42)) return fail(FGMS_ERR_INVALID_ARG, "buffer too large");
+  }
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  for (int i = 0; i < n;) {
+    fgms::ZeroList z = {};
+    for (; i < n && z.n < fgms::ZERO_LIST; ++i) {
+      if (bytes[i] == 0) continue;
+      const size_t parts = (bytes[i] + fgms::ZERO_PART - 1) / fgms::ZERO_PART;
+      if (z.n > 0 && z.first_part[z.n] + parts > (1u << 31)) break;
+      z.at[z.n] = static_cast<uint8_t*>(buffers[i]);
+      z.bytes[z.n] = bytes[i];
+      z.first_part[z.n + 1] = z.first_part[z.n] + (unsigned)parts;
+      ++z.n;
+    }
+    if (z.n == 0) break;
+    const unsigned most = (unsigned)di.sms * 8, grid = z.first_part[z.n] < most ? z.first_part[z.n] : most;
+    if (fgms::launch_pdl(fgms::zero_list_kernel, (int)grid, 256, 0, static_cast<cudaStream_t>(stream), z) != cudaSuccess)
+      return fail(FGMS_ERR_CUDA, "zero_list_kernel launch failed");
+    if (int rc = check_launch("zero_list_kernel")) return rc;
+  }
+  return FGMS_OK;
+}
+
+int fgms_b200_add(void* y, const void* x, int64_t count, int dtype, void* stream) {
+  TraceRange trace_range("fgms_b200_add");
+  if (!dtype_ok(dtype)) return fail(FGMS_ERR_INVALID_ARG, "unknown dtype %d", dtype);
+  if (count < 0 || (count > 0 && (!y || !x))) return fail(FGMS_ERR_INVALID_ARG, "negative count or null pointer");
+  if ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(x)) & 15) return fail(FGMS_ERR_INVALID_ARG, "buffers must be 16-byte aligned");
+  if (count == 0) return FGMS_OK;
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  const bool f16 = dtype == FGMS_DTYPE_F16;
+  const int64_t want = count / (256 * (f16 ? 16 : 8)) + 1, most = (int64_t)di.sms * 8;  // two 16-byte units per thread
+  auto* kernel = f16 ? fgms::add_kernel<true> : fgms::add_kernel<false>;
+  if (fgms::launch_pdl(kernel, (int)(want < most ? want : most), 256, 0, static_cast<cudaStream_t>(stream), static_cast<uint8_t*>(y),
+                       static_cast<const uint8_t*>(x), (long long)count) != cudaSuccess)
+    return fail(FGMS_ERR_CUDA, "add_kernel launch failed");
+  return check_launch("add_kernel");
+}
+
+int fgms_b200_copy_rows_f16(const void* src, int64_t src_pitch, int src_dtype, void* dst, int64_t dst_pitch, int64_t rows, int len, void* stream) {
+  TraceRange trace_range("fgms_b200_copy_rows_f16");
+  if (!dtype_ok(src_dtype)) return fail(FGMS_ERR_INVALID_ARG, "unknown dtype %d", src_dtype);
+  if (rows < 0 || len < 0 || src_pitch < len || dst_pitch < len) return fail(FGMS_ERR_INVALID_ARG, "negative size or a row longer than its pitch");
+  if (rows == 0 || len == 0) return FGMS_OK;
+  if (!src || !dst) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
+  DeviceInfo di;
+  if (int rc = device_info(&di)) return rc;
+  const int64_t want = (rows * len + 255) / 256, most = (int64_t)di.sms * 8;
+  const int grid = (int)(want < most ? want : most);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const cudaError_t e =
+      src_dtype == FGMS_DTYPE_F16
+          ? fgms::launch_pdl(fgms::copy_rows_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(src), (long long)src_pitch,
+                             static_cast<__half*>(dst), (long long)dst_pitch, (long long)rows, len)
+          : fgms::launch_pdl(fgms::copy_rows_kernel<float>, grid, 256, 0, st, static_cast<const float*>(src), (long long)src_pitch,
+                             static_cast<__half*>(dst), (long long)dst_pitch, (long long)rows, len);
+  if (e != cudaSuccess) return fail(FGMS_ERR_CUDA, "copy_rows_kernel launch failed");
+  return check_launch("copy_rows_kernel");
+}
+
 size_t fgms_b200_wgrad_workspace_bytes(int c_in, int c_out, int k_vol, int dtype) {
   if (dtype != FGMS_DTYPE_F16 || c_in < 1 || c_out < 1 || k_vol < 1) return 0;
   return (size_t)k_vol * c_in * c_out * sizeof(float);

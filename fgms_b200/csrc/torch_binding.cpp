@@ -198,6 +198,223 @@ struct SparseConv : torch::autograd::Function<SparseConv> {
   }
 };
 
+// ---------------------------------------------------------------------------------------------
+// a stack of layers as one node
+// ---------------------------------------------------------------------------------------------
+// A node per layer costs 14 us of the engine's host time on top of its launches, and a fill of its own for the output and for the
+// gradients: 1100 us for the 25 layers of an encoder-decoder on 8 k voxels whose kernels run 500 us.  Here the layers' values lie in one
+// allocation, their gradients in another, each cleared by one launch, and the backward is a loop.  The arithmetic is the one of
+// a node per layer: every layer adds into zeros, a skip connection and its gradient are sums rounded once.
+//
+// Value 0 is the input, value l + 1 what layer l produces.
+struct StackLayer { int64_t src, skip /* -1: none */, map, n_in, n_out; };
+using StackPlan = std::vector<int64_t>;  // StackLayer by StackLayer
+constexpr int64_t STACK_FIELDS = 5;
+StackLayer layer_of(const StackPlan& plan, size_t l) {
+  const int64_t* f = plan.data() + l * STACK_FIELDS;
+  return {f[0], f[1], f[2], f[3], f[4]};
+}
+
+// What every layer's own call would accept, and what one node can hold: each value but the last is used, by one layer at most.
+// False: the caller runs layer by layer, and meets its errors there.
+bool stack_suits(const Tensor& feats, at::TensorList weights, at::TensorList maps, const StackPlan& plan, bool arch80) {
+  const size_t n = weights.size();
+  const auto dtype = feats.scalar_type();
+  if (n == 0 || plan.size() != n * STACK_FIELDS || maps.size() % 3 != 0) return false;
+  if (!feats.is_cuda() || feats.dim() != 2 || !feats.is_contiguous() || (dtype != at::kHalf && dtype != at::kFloat)) return false;
+  auto aligned = [](const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; };
+  if (feats.numel() == 0 || !aligned(feats)) return false;
+  for (const Tensor& m : maps)
+    if (m.scalar_type() != at::kInt || m.device() != feats.device() || !m.is_contiguous() || m.requires_grad()) return false;
+  struct Value { int64_t rows, width; int convs, skips; };
+  std::vector<Value> value(1, {feats.size(0), feats.size(1), 0, 0});
+  value.reserve(n + 1);
+  for (size_t l = 0; l < n; ++l) {
+    const StackLayer s = layer_of(plan, l);
+    const Tensor& w = weights[l];
+    const int64_t known = (int64_t)value.size();
+    if (w.scalar_type() != dtype || w.device() != feats.device() || w.dim() != 3 || !w.is_contiguous() || w.numel() == 0 || !aligned(w)) return false;
+    if (s.src < 0 || s.src >= known || s.skip >= known || s.map < 0 || 3 * s.map + 2 >= (int64_t)maps.size() || s.n_out < 1) return false;
+    const Tensor &kpos = maps[3 * s.map], &imap = maps[3 * s.map + 1], &omap = maps[3 * s.map + 2];
+    Value& from = value[s.src];
+    if (from.rows != s.n_in || from.width != w.size(1) || kpos.numel() != w.size(0) + 1 || imap.numel() != omap.numel()) return false;
+    if (from.convs++ > 0) return false;
+    value.push_back({s.n_out, w.size(2), 0, 0});
+    if (s.skip >= 0) {
+      Value& add = value[s.skip];
+      if (add.rows != s.n_out || add.width != w.size(2)) return false;
+      ++add.skips;
+    }
+  }
+  for (size_t v = 1; v < n; ++v)
+    if (value[v].convs + value[v].skips == 0) return false;
+  return true;
+}
+
+struct SparseStack : torch::autograd::Function<SparseStack> {
+  // Where things lie in the buffer of the values, in elements, each from a 256-byte boundary: the values that layers 0 .. n - 2 produce
+  // and, where the input's few fp16 channels are padded to a multiple of 16 (8-byte rows cannot be gathered in 16-byte pieces and
+  // would run on the CUDA cores: 4 -> 32 on 84 k pairs 16 / 42 us forward / weight gradient, padded 4.5 / 5), the padded
+  // input and the weights that go with it.
+  struct Layout {
+    std::vector<int64_t> at;  // of value v, from 1 on
+    int64_t input = 0, weights = 0, end = 0;
+    int64_t pad = 0;          // channels of the padded input, 0: as it is
+    template <typename Kept>
+    Layout(const Tensor& feats, at::TensorList kernels, const StackPlan& plan, bool padding, Kept kept) {
+      auto take = [&](int64_t count) { const int64_t from = end; end += (count + 127) / 128 * 128; return from; };
+      const size_t n = kernels.size();
+      at.push_back(0);
+      for (size_t l = 0; l + 1 < n; ++l) at.push_back(kept(l + 1) ? take(layer_of(plan, l).n_out * kernels[l].size(2)) : 0);
+      at.push_back(0);
+      if (!padding || feats.scalar_type() != at::kHalf || feats.size(1) % 16 == 0 || feats.size(1) > 256) return;
+      const Tensor* reader = nullptr;  // the layer of the input
+      for (size_t l = 0; l < n; ++l) {
+        if (layer_of(plan, l).skip == 0) return;
+        if (layer_of(plan, l).src == 0) reader = &kernels[l];
+      }
+      if (!reader || reader->size(2) % 16 != 0 || reader->size(2) > 256) return;
+      pad = (feats.size(1) + 15) / 16 * 16;
+      input = take(feats.size(0) * pad);
+      weights = take(reader->size(0) * pad * reader->size(2));
+    }
+  };
+  static uint8_t* element(const Tensor& t, int64_t i) { return static_cast<uint8_t*>(t.data_ptr()) + i * t.element_size(); }
+
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& feats, at::TensorList weights, at::TensorList maps,
+                        const StackPlan& plan, bool arch80) {
+    const size_t n = weights.size();
+    c10::cuda::CUDAGuard guard(feats.device());
+    void* st = stream_of(feats);
+    const Arith a = arith(feats, arch80);
+    const Layout in(feats, weights, plan, true, [](size_t) { return true; });
+    const auto options = feats.options().requires_grad(false);
+    const Tensor values = at::empty({in.end}, options);
+    Tensor out = at::empty({layer_of(plan, n - 1).n_out, weights[n - 1].size(2)}, options);
+    check_status(fgms_b200_zero2(ptr(values), bytes_of(values), ptr(out), bytes_of(out), st));
+    auto value = [&](int64_t v) -> void* {
+      if (v == 0) return in.pad ? element(values, in.input) : feats.data_ptr();
+      return v == (int64_t)n ? out.data_ptr() : element(values, in.at[v]);
+    };
+    if (in.pad) check_status(fgms_b200_copy_rows_f16(ptr(feats), feats.size(1), a.dtype, value(0), in.pad, feats.size(0), (int)feats.size(1), st));
+    for (size_t l = 0; l < n; ++l) {
+      const StackLayer s = layer_of(plan, l);
+      const Tensor &w = weights[l], &imap = maps[3 * s.map + 1];
+      const void* kernel = ptr(w);
+      int c_in = (int)w.size(1);
+      if (s.src == 0 && in.pad) {
+        kernel = element(values, in.weights);
+        check_status(fgms_b200_copy_rows_f16(ptr(w), c_in * w.size(2), a.dtype, element(values, in.weights), in.pad * w.size(2), w.size(0), c_in * (int)w.size(2), st));
+        c_in = (int)in.pad;
+      }
+      check_status(fgms_b200_fusion_fwd(value(s.src), kernel, value(l + 1), iptr(maps[3 * s.map]), nullptr, iptr(imap), iptr(maps[3 * s.map + 2]),
+                                        imap.numel(), (int)s.n_in, (int)s.n_out, c_in, c_in, (int)w.size(2), (int)w.size(0), 0, a.dtype, a.math, 0, st));
+      if (s.skip >= 0) check_status(fgms_b200_add(value(l + 1), value(s.skip), s.n_out * w.size(2), a.dtype, st));
+    }
+    torch::autograd::variable_list saved;
+    saved.reserve(2 + n + maps.size());
+    saved.push_back(feats);
+    saved.push_back(values);
+    saved.insert(saved.end(), weights.begin(), weights.end());
+    saved.insert(saved.end(), maps.begin(), maps.end());
+    ctx->save_for_backward(std::move(saved));
+    ctx->saved_data["plan"] = plan;
+    ctx->saved_data["arch80"] = arch80;
+    return out;
+  }
+
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const StackPlan plan = ctx->saved_data["plan"].toIntVector();
+    const bool arch80 = ctx->saved_data["arch80"].toBool();
+    const size_t n = plan.size() / STACK_FIELDS;
+    const Tensor &feats = saved[0], &values = saved[1];
+    const at::TensorList weights(saved.data() + 2, n), maps(saved.data() + 2 + n, saved.size() - 2 - n);
+    TORCH_CHECK_VALUE(stack_suits(feats, weights, maps, plan, arch80), "saved tensors of the stack are not the ones it was run with");
+    Tensor grad_out = grads[0].contiguous();
+    check_feat("out_feats_grad", grad_out, 2, feats);
+    if (reinterpret_cast<uintptr_t>(grad_out.data_ptr()) & 15) grad_out = grad_out.clone();
+    c10::cuda::CUDAGuard guard(feats.device());
+    void* st = stream_of(feats);
+    const Arith a = arith(feats, arch80);
+    TORCH_CHECK_VALUE(grad_out.size(0) == layer_of(plan, n - 1).n_out && grad_out.size(1) == weights[n - 1].size(2),
+                      "out_feats_grad has another shape than the output");
+    const Layout in(feats, weights, plan, true, [](size_t) { return true; });
+    TORCH_CHECK_VALUE(values.scalar_type() == feats.scalar_type() && values.device() == feats.device() && values.is_contiguous() && values.numel() == in.end &&
+                      (reinterpret_cast<uintptr_t>(values.data_ptr()) & 15) == 0, "saved values of the stack are not the ones it was run with");
+    // gradients that something needs: a value's, if a weight before it or the input needs one
+    std::vector<char> need(n + 1, 0), need_w(n);
+    need[0] = ctx->needs_input_grad(0);
+    for (size_t l = 0; l < n; ++l) {
+      const StackLayer s = layer_of(plan, l);
+      need_w[l] = ctx->needs_input_grad(1 + l);
+      need[l + 1] = need_w[l] || need[s.src] || (s.skip >= 0 && need[s.skip]);
+    }
+    const Layout out(feats, weights, plan, false, [&](size_t v) { return need[v] != 0; });
+    torch::autograd::variable_list result(1 + n + maps.size() + 2);
+    const Tensor g_values = at::empty({out.end}, feats.options().requires_grad(false));
+    std::vector<void*> clear;
+    std::vector<size_t> bytes;
+    auto cleared = [&](const Tensor& t) { clear.push_back(ptr(t)); bytes.push_back(bytes_of(t)); };
+    cleared(g_values);
+    Tensor g_input;
+    if (need[0]) cleared(g_input = at::empty({feats.size(0), in.pad ? in.pad : feats.size(1)}, feats.options().requires_grad(false)));
+    for (size_t l = 0; l < n; ++l)
+      if (need_w[l]) cleared(result[1 + l] = at::empty_like(weights[l]));
+    check_status(fgms_b200_zero_list(clear.data(), bytes.data(), (int)clear.size(), st));
+    auto value = [&](int64_t v) -> void* {
+      if (v == 0) return in.pad ? element(values, in.input) : feats.data_ptr();
+      return element(values, in.at[v]);
+    };
+    auto grad = [&](int64_t v) -> void* {
+      return v == 0 ? g_input.data_ptr() : v == (int64_t)n ? grad_out.data_ptr() : element(g_values, out.at[v]);
+    };
+    std::vector<std::vector<int64_t>> added(n + 1);  // values whose gradient is part of a value's, through a skip connection
+    auto finish = [&](int64_t v, int64_t count) {    // its layer's input gradient is in it
+      for (int64_t from : added[v]) check_status(fgms_b200_add(grad(v), grad(from), count, a.dtype, st));
+    };
+    const bool fp32_sums = g_fp32_sums.load(std::memory_order_relaxed);
+    for (size_t l = n; l-- > 0;) {
+      if (!need[l + 1]) continue;
+      const StackLayer s = layer_of(plan, l);
+      const Tensor &w = weights[l], &imap = maps[3 * s.map + 1];
+      const int32_t *kpos = iptr(maps[3 * s.map]), *im = iptr(imap), *om = iptr(maps[3 * s.map + 2]);
+      const int c_in = (int)w.size(1), c_out = (int)w.size(2), k_vol = (int)w.size(0), n_in = (int)s.n_in, n_out = (int)s.n_out;
+      if (l + 1 < n) finish(l + 1, s.n_out * c_out);
+      if (s.skip >= 0 && need[s.skip]) added[s.skip].push_back(l + 1);
+      if (s.src == 0 && in.pad) {
+        const int pad = (int)in.pad;
+        if (need_w[l]) {  // fp32 sums, of which the rows of the real channels are rounded
+          const Tensor sums = at::empty({(int64_t)k_vol * pad * c_out}, w.options().dtype(at::kFloat).requires_grad(false));
+          check_status(fgms_b200_wgrad(value(0), grad(l + 1), nullptr, kpos, im, om, imap.numel(), n_in, n_out, pad, c_out, k_vol, a.dtype, a.math,
+                                       sums.data_ptr(), bytes_of(sums), 0, st));
+          check_status(fgms_b200_copy_rows_f16(sums.data_ptr(), pad * c_out, FGMS_DTYPE_F32, result[1 + l].data_ptr(), c_in * c_out, k_vol, c_in * c_out, st));
+        }
+        if (need[0])
+          check_status(fgms_b200_dgrad(grad(l + 1), element(values, in.weights), grad(0), kpos, im, om, imap.numel(), n_in, n_out, pad, c_out, k_vol,
+                                       a.dtype, a.math, st));
+        continue;
+      }
+      const Tensor ws = need_w[l] ? wgrad_workspace(result[1 + l], a, fp32_sums) : Tensor();
+      void* ws_ptr = ws.defined() ? ws.data_ptr() : nullptr;
+      const size_t ws_bytes = ws.defined() ? bytes_of(ws) : 0;
+      if (need[s.src] && need_w[l])
+        check_status(fgms_b200_bwd(grad(l + 1), value(s.src), ptr(w), grad(s.src), result[1 + l].data_ptr(), kpos, nullptr, im, om, imap.numel(), n_in,
+                                   n_out, c_in, c_in, c_out, k_vol, 0, a.dtype, a.math, 0, ws_ptr, ws_bytes, st));
+      else if (need[s.src])
+        check_status(fgms_b200_dgrad(grad(l + 1), ptr(w), grad(s.src), kpos, im, om, imap.numel(), n_in, n_out, c_in, c_out, k_vol, a.dtype, a.math, st));
+      else if (need_w[l])
+        check_status(fgms_b200_wgrad(value(s.src), grad(l + 1), result[1 + l].data_ptr(), kpos, im, om, imap.numel(), n_in, n_out, c_in, c_out, k_vol,
+                                     a.dtype, a.math, ws_ptr, ws_bytes, 1, st));
+    }
+    if (need[0]) {
+      finish(0, feats.numel());
+      result[0] = in.pad ? g_input.narrow(1, 0, feats.size(1)).contiguous() : g_input;
+    }
+    return result;
+  }
+};
+
 // output-stationary forward into `out`; nbr is the table fgms_b200_build_neighbor_table fills
 void fwd_os(const Tensor& in_feats, const Tensor& kernel, const Tensor& out, const Tensor& nbr, bool arch80, const Tensor* bias,
             bool relu, bool accumulate) {
@@ -368,6 +585,28 @@ PyObject* py_sparse_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return THPVariable_Wrap(SparseConv::apply(feats, weight, kpos, imap, omap, int_arg(a[5]), bool_arg(a[6])));
   END_HANDLE_TH_ERRORS
 }
+// (in_feats, [kernels], [kpos, in_map, out_map of every map], [src, skip, map, n_in, n_out of every layer], arch80) -> the last layer's
+// output, or None where the layers are to be run one by one
+PyObject* py_sparse_stack(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 5);
+  const Tensor& feats = feat_arg(a[0], "in_feats");
+  auto tensors = [](PyObject* list, const char* name) {
+    TORCH_CHECK_TYPE(PyList_Check(list), name, " must be a list");
+    std::vector<Tensor> out;
+    out.reserve(PyList_GET_SIZE(list));
+    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(list); ++i) out.push_back(feat_arg(PyList_GET_ITEM(list, i), name));
+    return out;
+  };
+  const std::vector<Tensor> weights = tensors(a[1], "kernels"), maps = tensors(a[2], "maps");
+  TORCH_CHECK_TYPE(PyList_Check(a[3]), "plan must be a list");
+  StackPlan plan;
+  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[3]); ++i) plan.push_back(int_arg(PyList_GET_ITEM(a[3], i)));
+  const bool arch80 = bool_arg(a[4]);
+  if (!stack_suits(feats, weights, maps, plan, arch80)) Py_RETURN_NONE;
+  return THPVariable_Wrap(SparseStack::apply(feats, at::TensorList(weights), at::TensorList(maps), plan, arch80));
+  END_HANDLE_TH_ERRORS
+}
 PyObject* py_wgrad_fp32_sums(PyObject*, PyObject* const* a, Py_ssize_t n) {  // () -> the switch; (value) sets it
   HANDLE_TH_ERRORS
   TORCH_CHECK_TYPE(n <= 1, "expected at most 1 argument, got ", n);
@@ -407,6 +646,7 @@ PyObject* py_build_pyramid(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyMethodDef methods[] = {
     FGMS_METHOD("fusion_fwd", py_fusion_fwd), FGMS_METHOD("seq_fwd", py_seq_fwd),         FGMS_METHOD("bwd", py_bwd),
     FGMS_METHOD("fwd_os", py_fwd_os),         FGMS_METHOD("sparse_conv", py_sparse_conv),
+    FGMS_METHOD("sparse_stack", py_sparse_stack),
     FGMS_METHOD("wgrad_fp32_sums", py_wgrad_fp32_sums),
     FGMS_METHOD("build_pyramid", py_build_pyramid), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -65,6 +65,33 @@ class SparseConv3d(torch.nn.Module):
         return sparse_conv(feats, self.weight, kmap, self.arch80)
 
 
+_LAYER_FORWARD = SparseConv3d.forward
+_MODULE = torch.nn.modules.module
+_HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
+
+
+def _one_node(layers) -> bool:
+    """Whether a stack may run as one autograd node: nothing sees the calls of its layers.  Several ranks run layer by layer, because
+    gradients that leave with their layer are exchanged beside the rest of the backward."""
+    if torch._C._get_tracing_state() is not None or torch.compiler.is_compiling() or torch.autograd.forward_ad._current_level >= 0:
+        return False
+    if torch._C._functorch.peek_interpreter_stack() is not None or torch._C._autograd._top_saved_tensors_default_hooks(True) is not None:
+        return False
+    if torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack():
+        return False
+    if torch.distributed.is_available() and torch.distributed.is_initialized():
+        return False
+    if _MODULE._global_forward_hooks or _MODULE._global_forward_pre_hooks or _MODULE._global_backward_hooks or _MODULE._global_backward_pre_hooks:
+        return False
+    if SparseConv3d.forward is not _LAYER_FORWARD or SparseConv3d.__call__ is not torch.nn.Module.__call__:
+        return False
+    for layer in layers:
+        d = layer.__dict__
+        if type(layer) is not SparseConv3d or "forward" in d or d["arch80"] != layers[0].__dict__["arch80"] or any(d[h] for h in _HOOKS):
+            return False
+    return True
+
+
 class SparseUNet(torch.nn.Module):
     """The encoder-decoder stack of :mod:`fgms_b200.unet` as an ``nn.Module`` over the autograd operator: one
     :class:`SparseConv3d` per layer of the specification, decoder skips added to the transposed convolutions'
@@ -81,7 +108,31 @@ class SparseUNet(torch.nn.Module):
             for layer, w in zip(self.layers, weights):
                 layer.weight.copy_(torch.as_tensor(w).to(layer.weight.device, layer.weight.dtype))
 
+    def _forward_as_one(self, feats: torch.Tensor, umaps):
+        """The stack as one autograd node (``csrc/torch_binding.cpp``), or None: see :func:`_one_node`."""
+        layers = list(self.layers)
+        if not layers or len(layers) != len(self.spec) or type(feats) is not torch.Tensor or not _one_node(layers):
+            return None
+        value, seen, weights, maps, plan = {"input": 0}, {}, [], [], []
+        for spec, layer in zip(self.spec, layers):
+            w, km = layer._parameters.get("weight"), umaps.of(spec)
+            if type(w) is not torch.nn.Parameter or spec.src not in value or (spec.skip is not None and spec.skip not in value):
+                return None
+            m = seen.get(id(km))
+            if m is None:
+                m = seen[id(km)] = len(seen)
+                maps += km.kpos, km.imap, km.omap
+            plan += value[spec.src], -1 if spec.skip is None else value[spec.skip], m, km.n_in, km.n_out
+            weights.append(w)
+            value[spec.dst] = len(weights)
+        if not all(type(t) is torch.Tensor for t in maps):
+            return None
+        return _native.sparse_stack(feats, weights, maps, plan, layers[0].arch80)
+
     def forward(self, feats: torch.Tensor, umaps) -> torch.Tensor:
+        out = self._forward_as_one(feats, umaps)
+        if out is not None:
+            return out
         val = {"input": feats}
         for spec, layer in zip(self.spec, self.layers):
             y = layer(val[spec.src], umaps.of(spec))

@@ -99,6 +99,17 @@ int fgms_b200_dgrad(const void* out_grad, const void* kernel, void* in_grad, con
  * its preamble while this one runs. */
 int fgms_b200_zero2(void* a, size_t a_bytes, void* b, size_t b_bytes, void* stream);
 
+/* The same for `n` buffers, whose addresses and sizes are in host memory: one launch for each 64 of them. */
+int fgms_b200_zero_list(void* const* buffers, const size_t* bytes, int n, void* stream);
+
+/* y[i] += x[i] for `count` values of the given dtype, each sum rounded once: a skip connection, or its gradient.  The pointers
+ * must be 16-byte aligned. */
+int fgms_b200_add(void* y, const void* x, int64_t count, int dtype, void* stream);
+
+/* The first `len` values of each of `rows` rows, `src_pitch` and `dst_pitch` values apart, to fp16 storage (values of fp32 storage are
+ * rounded): features and weights padded with channels, gradients freed of them.  What lies behind a row in dst is left alone. */
+int fgms_b200_copy_rows_f16(const void* src, int64_t src_pitch, int src_dtype, void* dst, int64_t dst_pitch, int64_t rows, int len, void* stream);
+
 /* Weight gradient:  kernel_grad[k] += sum over the pairs of offset k of in[in_map[j]]^T (x) out_grad[out_map[j]].
  * Second launch of ConvolutionBackward (backend/spconv.cu:495-548 fp16, 562-569 tf32).
  * Partial sums are accumulated in fp32.  For fp16 storage they live in `workspace`

@@ -1,0 +1,138 @@
+"""``nn.SparseUNet`` as one autograd node against its layers one by one: outputs and gradients, whichever inputs need one; what
+makes it run layer by layer; and the two small kernels behind it, at sizes that fill no vector and no block."""
+import ctypes
+
+import pytest
+import torch
+
+from fgms_b200 import _lib, clouds, nn, unet
+
+pytestmark = pytest.mark.gpu
+
+SPEC = unet.minkunet_spec(4, (16, 32, 48))
+
+
+def _net(spec=SPEC, dtype=torch.float16, n=3000):
+    coords = torch.from_numpy(clouds.uniform_cloud(n, 20, 7)).cuda()
+    umaps = unet.build_unet_maps(coords, (len(spec) - 1) // 6)
+    torch.manual_seed(3)
+    net = nn.SparseUNet(spec, dtype=dtype)
+    with torch.no_grad():
+        for layer in net.layers:
+            layer.weight.mul_(2.0)
+    feats = torch.randn((coords.size(0), spec[0].c_in), device="cuda").to(dtype)
+    grad = torch.randn((coords.size(0), spec[-1].c_out), device="cuda").to(dtype)
+    return net, umaps, feats, grad
+
+
+def _layer_by_layer(net, feats, umaps):
+    val = {"input": feats}
+    for spec, layer in zip(net.spec, net.layers):
+        y = layer(val[spec.src], umaps.of(spec))
+        val[spec.dst] = y if spec.skip is None else y + val[spec.skip]
+    return val[net.spec[-1].dst]
+
+
+def _close(a, b, dtype):
+    # the same sums in another order: at most 27 (forward, input gradient) or a few hundred partial sums, through 13 layers
+    tol = 2e-2 if dtype == torch.float16 else 1e-2
+    assert float((a.double() - b.double()).norm()) <= tol * float(b.double().norm())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("needs", ["all", "weights", "input", "last", "frozen_middle", "first"])
+def test_one_node_equals_a_node_per_layer(dtype, needs):
+    net, umaps, feats, grad = _net(dtype=dtype)
+    params = list(net.parameters())
+    for i, p in enumerate(params):
+        p.requires_grad_({"all": True, "weights": True, "input": False, "last": i == len(params) - 1,
+                          "frozen_middle": i % 3 != 1, "first": i == 0}[needs])
+    feats.requires_grad_(needs in ("all", "input", "frozen_middle"))
+    wanted = [t for t in [feats] + params if t.requires_grad]
+    got, want = net(feats, umaps), _layer_by_layer(net, feats, umaps)
+    assert got.grad_fn.name() != want.grad_fn.name()
+    _close(got.detach(), want.detach(), dtype)
+    for a, b in zip(torch.autograd.grad(got, wanted, grad, retain_graph=True), torch.autograd.grad(want, wanted, grad)):
+        _close(a, b, dtype)
+    for a, b in zip(torch.autograd.grad(got, wanted[-1:], grad), wanted[-1:]):  # a second backward, of one of them
+        assert a.shape == b.shape
+
+
+def test_no_gradients_and_in_place_changes():
+    net, umaps, feats, grad = _net()
+    with torch.no_grad():
+        assert not net(feats, umaps).requires_grad
+    out = net(feats, umaps)
+    with torch.no_grad():
+        net.layers[2].weight.add_(1)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.backward(grad)
+
+
+def test_what_sees_the_layers_has_them_run_one_by_one():
+    net, umaps, feats, grad = _net()
+    one = net(feats, umaps).grad_fn.name()
+    calls = []
+    handle = net.layers[1].register_forward_hook(lambda *a: calls.append(1))
+    assert net(feats, umaps).grad_fn.name() != one and calls == [1]
+    handle.remove()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t):
+        assert net(feats, umaps).grad_fn.name() != one
+    assert net(feats, umaps).grad_fn.name() == one
+    assert net(feats.t().contiguous().t(), umaps).grad_fn.name() != one  # layer by layer takes any strides
+    with pytest.raises(ValueError):
+        net(feats[:-1].contiguous(), umaps)
+    with pytest.raises(ValueError):
+        net(feats.float(), umaps)
+
+
+def test_a_value_that_two_layers_read_has_a_node_per_layer():
+    spec = [unet.LayerSpec("a", "subm", 16, 16, 0, 0, "input", "x"), unet.LayerSpec("b", "subm", 16, 16, 0, 0, "x", "y"),
+            unet.LayerSpec("c", "subm", 16, 16, 0, 0, "x", "z", skip="y")]
+    coords = torch.from_numpy(clouds.uniform_cloud(500, 12, 7)).cuda()
+    umaps, net = unet.build_unet_maps(coords, 1), nn.SparseUNet(spec)
+    feats = torch.randn((coords.size(0), 16), device="cuda").half()
+    assert net._forward_as_one(feats, umaps) is None
+    net(feats, umaps).sum().backward()
+    assert all(float(p.grad.abs().max()) > 0 for p in net.parameters())
+
+
+@pytest.mark.parametrize("sizes", [[1], [15, 16, 17], [16384, 16385, 0, 3], [7] * 70 + [40000], [1 << 22]])
+def test_zero_list(sizes):
+    buffers = [torch.full((n + 16,), 7, dtype=torch.uint8, device="cuda") for n in sizes]
+    at = (ctypes.c_void_p * len(sizes))(*[b.data_ptr() for b in buffers])
+    _lib.check(_lib.lib.fgms_b200_zero_list(at, (ctypes.c_size_t * len(sizes))(*sizes), len(sizes), torch.cuda.current_stream().cuda_stream))
+    for b, n in zip(buffers, sizes):
+        assert not b[:n].any() and bool((b[n:] == 7).all())
+
+
+@pytest.mark.parametrize("count", [1, 3, 8, 9, 4095, 65537, 3000001])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_add(count, dtype):
+    y, x = torch.randn(count + 8, device="cuda").to(dtype), torch.randn(count + 8, device="cuda").to(dtype)
+    want = torch.cat([y[:count] + x[:count], y[count:]])
+    _lib.check(_lib.lib.fgms_b200_add(y.data_ptr(), x.data_ptr(), count, 1 if dtype == torch.float16 else 0, torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("c_in", [1, 5, 17, 30])
+def test_input_channels_that_are_padded(c_in):
+    net, umaps, feats, grad = _net(unet.minkunet_spec(c_in, (16, 32, 48)))
+    feats.requires_grad_()
+    wanted = [feats] + list(net.parameters())
+    got, want = net(feats, umaps), _layer_by_layer(net, feats, umaps)
+    _close(got.detach(), want.detach(), torch.float16)
+    for a, b in zip(torch.autograd.grad(got, wanted, grad), torch.autograd.grad(want, wanted, grad)):
+        assert a.is_contiguous()
+        _close(a, b, torch.float16)
+
+
+@pytest.mark.parametrize("rows,length,src_pitch,dst_pitch", [(1, 1, 1, 1), (257, 3, 5, 16), (27, 128, 128, 512), (100003, 4, 4, 16)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_copy_rows(rows, length, src_pitch, dst_pitch, dtype):
+    src, dst = torch.randn((rows, src_pitch), device="cuda").to(dtype), torch.full((rows, dst_pitch), 7.0, device="cuda").half()
+    want = dst.clone()
+    want[:, :length] = src[:, :length].half()
+    _lib.check(_lib.lib.fgms_b200_copy_rows_f16(src.data_ptr(), src_pitch, 1 if dtype == torch.float16 else 0, dst.data_ptr(), dst_pitch, rows, length,
+                                                torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(dst, want)
