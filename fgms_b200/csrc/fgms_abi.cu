@@ -791,10 +791,15 @@ int fgms_b200_pyramid_plan(const int32_t* coords, int n, int levels, int what, i
   DeviceInfo di;
   if (int rc = device_info(&di)) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  auto* ws = static_cast<uint8_t*>(workspace);
-  if (!fgms::pyramid::launch_plan(p, a, ws, di.sms, st)) return cuda_fail("pyramid launch");
-  g_launches += 8;
-  if (cudaMemcpyAsync(sizes_host, ws + p.sizes, (size_t)(1 + levels + p.n_jobs) * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+  // page-locked memory is written by the kernel itself, other memory gets a copy
+  cudaPointerAttributes where;
+  int* sizes = nullptr;
+  if (cudaPointerGetAttributes(&where, sizes_host) != cudaSuccess) cudaGetLastError();
+  else if (where.type == cudaMemoryTypeHost) sizes = static_cast<int*>(where.devicePointer);
+  int* target = sizes ? sizes : reinterpret_cast<int*>(static_cast<uint8_t*>(workspace) + p.sizes);
+  if (!fgms::pyramid::launch_plan(a, target, di.sms, st)) return cuda_fail("pyramid launch");
+  g_launches += 1;
+  if ((!sizes && cudaMemcpyAsync(sizes_host, target, (size_t)(1 + levels + p.n_jobs) * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess) ||
       cudaStreamSynchronize(st) != cudaSuccess)
     return cuda_fail("reading the sizes of the maps");
   if (sizes_host[0] != 0) {

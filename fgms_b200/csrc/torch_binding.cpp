@@ -490,20 +490,26 @@ Pyramid try_pyramid(const Tensor& coords, int levels, int what) {
   }
   r.fits = true;
   for (int l = 0; l < levels; ++l) r.voxels.push_back(sizes[1 + l]);
-  std::vector<Tensor> flat;
+  // all maps in one allocation, each on a 256-byte boundary: the device waits for it
+  std::vector<int64_t> at;
+  int64_t end = 0;
+  for (int j = 0; j < n_maps; ++j)
+    for (int side = 0; side < 2; ++side) {
+      at.push_back(end);
+      end += (sizes[1 + levels + j] + 64) / 64 * 64;
+    }
+  const Tensor flat = at::empty({end}, ints);
   std::vector<int32_t*> in_maps, out_maps;
-  for (int j = 0; j < n_maps; ++j) {  // both maps of a layer in one allocation, each on a 256-byte boundary
-    const int64_t pad = (sizes[1 + levels + j] + 64) / 64 * 64;
-    flat.push_back(at::empty({2 * pad}, ints));
-    in_maps.push_back(flat[j].data_ptr<int32_t>());
-    out_maps.push_back(in_maps[j] + pad);
+  for (int j = 0; j < n_maps; ++j) {
+    in_maps.push_back(flat.data_ptr<int32_t>() + at[2 * j]);
+    out_maps.push_back(flat.data_ptr<int32_t>() + at[2 * j + 1]);
   }
   check_status(fgms_b200_pyramid_emit(iptr(coords), n, levels, what, kpos.data_ptr<int32_t>(), coord_ptrs.data(), in_maps.data(),
                                       out_maps.data(), ws.data_ptr(), bytes, st));
   for (int j = 0; j < n_maps; ++j) {
-    const int64_t pairs = sizes[1 + levels + j], pad = flat[j].numel() / 2;
+    const int64_t pairs = sizes[1 + levels + j];
     const bool subm = (what & 1) && j < levels;
-    r.maps.push_back({kpos.narrow(0, j * 28, subm ? 28 : 9), flat[j].narrow(0, 0, pairs), flat[j].narrow(0, pad, pairs)});
+    r.maps.push_back({kpos.narrow(0, j * 28, subm ? 28 : 9), flat.narrow(0, at[2 * j], pairs), flat.narrow(0, at[2 * j + 1], pairs)});
   }
   for (int l = 1; l < levels; ++l) r.out_coords[l - 1] = r.out_coords[l - 1].narrow(0, 0, r.voxels[l]);
   return r;
