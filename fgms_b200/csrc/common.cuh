@@ -76,7 +76,7 @@ __device__ __forceinline__ void build_tile_table(int TILE, const int32_t* __rest
       if (s <= k_vol) {
         const int first = __ldg(kpos + s), next = s < k_vol ? __ldg(kpos + s + 1) : 0;
         const int c = min(max(first, 0), pairs);
-        if (first != c && blockIdx.x == 0) report_problem();
+        if (first != c && blockIdx.x == 0 && blockIdx.y == 0) report_problem();
         kpos_s[s] = c;
         const int cnt = s < k_vol ? min(max(next, 0), pairs) - c : dense_rows;
         v = cnt > 0 ? (cnt + TILE - 1) / TILE : 0;
@@ -104,11 +104,16 @@ __device__ __forceinline__ int find_segment(const int* tile_start, int n_seg, in
   return lo;
 }
 
-// Contiguous share of `total` tiles for this CTA.
+// Contiguous share of `total` tiles for this CTA (of the first row of a grid of two dimensions).
 __device__ __forceinline__ void cta_tile_range(int total, int* t0, int* t1) {
-  long long g = gridDim.x, b = blockIdx.x;
-  *t0 = (int)((long long)total * b / g);
-  *t1 = (int)((long long)total * (b + 1) / g);
+  const unsigned g = gridDim.x, b = blockIdx.x;
+  if (total <= 0x7fffffff / 1024 && g <= 1024) {  // a 64-bit division is a few hundred cycles
+    *t0 = (int)((unsigned)total * b / g);
+    *t1 = (int)((unsigned)total * (b + 1) / g);
+  } else {
+    *t0 = (int)((long long)total * b / g);
+    *t1 = (int)((long long)total * (b + 1) / g);
+  }
 }
 
 // Tiles handed out by turns.  All tiles' turns, offset after offset, are cut into shares of F consecutive ones; worker w

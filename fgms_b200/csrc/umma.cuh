@@ -292,13 +292,12 @@ __host__ __device__ constexpr uint32_t mnmajor32_offset(uint32_t k, uint32_t byt
 
 }  // namespace umma
 
-// Tensor map over weights [k_vol, c_in, c_out] whose box is one 128-byte column block of one matrix: what tma_load_2d writes,
-// block after block c_in * 128 bytes apart, is the 128-byte-swizzled operand: MN-major (forward: rows = contraction index) or
+// Tensor map over weights [k_vol, c_in, c_out] whose box is `box_rows` rows of one 128-byte column block (0: all c_in of a matrix): what tma_load_2d writes, block after block box_rows * 128 bytes apart, is the 128-byte-swizzled operand: MN-major (forward: rows = contraction index) or
 // K-major (input gradient: rows = output index), which differ only for 32-bit elements.  Columns beyond c_out come as zeros.
 // Made for every call (42 ns): nothing is kept by an address.  The encoder wants a context, which a host thread has after its first
 // launch and not after cudaGetDevice: where it finds none, the current device's is made the thread's and the encoder asked again.
 // Returns 0, or -1000 less the driver's status.  An encoder that was not found is looked up again by the next call.
-inline int weight_tensor_map(CUtensorMap* map, const void* weights, int k_vol, int c_in, int c_out, bool f16, bool mn_major) {
+inline int weight_tensor_map(CUtensorMap* map, const void* weights, int k_vol, int c_in, int c_out, bool f16, bool mn_major, int box_rows = 0) {
   using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                               const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
   static std::atomic<Encode> known{nullptr};
@@ -313,7 +312,7 @@ inline int weight_tensor_map(CUtensorMap* map, const void* weights, int k_vol, i
   }
   const int es = f16 ? 2 : 4;
   const cuuint64_t dims[2] = {(cuuint64_t)c_out, (cuuint64_t)k_vol * c_in}, pitch[1] = {(cuuint64_t)c_out * es};
-  const cuuint32_t box[2] = {(cuuint32_t)(128 / es), (cuuint32_t)c_in}, steps[2] = {1, 1};
+  const cuuint32_t box[2] = {(cuuint32_t)(128 / es), (cuuint32_t)(box_rows > 0 ? box_rows : c_in)}, steps[2] = {1, 1};
   auto made = [&] {
     return encode(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(weights), dims, pitch, box, steps,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, f16 || !mn_major ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B,
@@ -329,9 +328,9 @@ inline int weight_tensor_map(CUtensorMap* map, const void* weights, int k_vol, i
 
 // Launch with the programmatic-stream-serialization attribute.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st, Args... args) {
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3((unsigned)grid);
+  lc.gridDim = grid;
   lc.blockDim = dim3((unsigned)block);
   lc.dynamicSmemBytes = smem;
   lc.stream = st;

@@ -81,6 +81,8 @@ struct G3Config {
   int kch;      // 128-byte K chunks (= stages) per tile: ceil(k_dim * elem / 128)
   int n_acc;    // TMEM columns per accumulator: n_dim rounded up to whole 128-byte blocks of the output row
   int n_mma;    // N of the MMA: n_acc for the MN-major weight operand (forward), n_dim for the K-major one (dgrad)
+  int n_split;  // CTAs that share a tile, each with n_cols of the output columns
+  int n_cols;
   int smem;     // dynamic shared memory of the launch
   long long w_limit;  // cycles the MMA lane waits for a weight matrix before it gives up (for anything else: about a second)
 };
@@ -149,6 +151,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
   const int kch = cfg.kch;                   // 128-byte K chunks per gathered row (the last one may be partly filled)
   const int k_bytes = p.k_dim * ES;          // bytes of a gathered row: a multiple of 32
   const int n_stage = cfg.n_stage;
+  const int col0 = (int)blockIdx.y * cfg.n_cols;  // this CTA's first output column
   volatile int* abort_flag = &sh->abort_flag;
 
   if (tid == 0) {
@@ -206,7 +209,9 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
         if (!ok) break;
         const uint32_t bar = smem_u32(&sh->w_full[wb]), sw = smem_u32(sW + (size_t)wb * cfg.w_bytes);
         mbar_expect_tx(bar, (uint32_t)cfg.w_bytes);
-        for (int b = 0; b * p.c_in * 128 < cfg.w_bytes; ++b) tma_load_2d(sw + (uint32_t)(b * p.c_in) * 128u, &w_map, bar, b * EPR, widx * p.c_in);
+        // a box is 128 bytes of columns of W_k: output columns and all rows (forward), contraction columns and the rows of this CTA (dgrad)
+        const int box_rows = TRANS_W ? cfg.n_cols : p.c_in, x0 = TRANS_W ? 0 : col0, y0 = widx * p.c_in + (TRANS_W ? col0 : 0);
+        for (int b = 0; b * box_rows * 128 < cfg.w_bytes; ++b) tma_load_2d(sw + (uint32_t)(b * box_rows) * 128u, &w_map, bar, x0 + b * EPR, y0);
         if (loads < cfg.n_wbuf) ++loads;
         if (++wb == cfg.n_wbuf) { wb = 0; ph ^= 1u; }
       }
@@ -267,7 +272,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
       const int other = __shfl_xor_sync(0xffffffffu, e0, 16);
       const int g_own = lane < 16 ? e0 : other, s_own = lane < 16 ? other : e0;
       const bool okp = pair_ok(g_own, s_own);
-      if (!okp && lane < 16 && (g_own != -1 || s_own != -1)) report_problem();  // entry outside the tensors: pair skipped, counted once
+      if (!okp && lane < 16 && col0 == 0 && (g_own != -1 || s_own != -1)) report_problem();  // entry outside the tensors: pair skipped, counted once
       const int ev = okp ? g_own : -1;
       const uint8_t* rsrc[4];
       bool valid[4];
@@ -301,7 +306,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
     const uint64_t a_desc0 = make_sdesc(smem_u32(sStage), 16u, 1024u);
     const uint64_t b_desc0 = TRANS_W ? make_sdesc(smem_u32(sW), 16u, 1024u)
                                      : make_sdesc(smem_u32(sW), (uint32_t)p.k_dim * 128u, TF32 ? 512u : 1024u, TF32 ? 1u : 2u);
-    const uint32_t b_kc_step = TRANS_W ? (uint32_t)p.n_dim * 8u : (uint32_t)EPR * 8u;  // one 128-byte K chunk further, in 16-byte units
+    const uint32_t b_kc_step = TRANS_W ? (uint32_t)cfg.n_cols * 8u : (uint32_t)EPR * 8u;  // one 128-byte K chunk further, in 16-byte units
     const uint32_t b_ks_step = TRANS_W ? 2u : (32u / ES) * 8u;                          // one 32-byte MMA step further
     G3Walk cur;
     cur.init(tile_start, n_seg, t0);
@@ -360,14 +365,14 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
   } else {
     // ------------------------------------------------------------------ epilogue (warps 0-7)
     // Two groups of four warps take alternate tiles, so that one group's TMEM reads and conversions run
-    // while the other group's reds drain.  (Blocks of columns instead of tiles: 256 -> 256 on 3000 voxels 12.4 us against
-    // 12.9, but 128 -> 128 on 303 k pairs 25.7 against 23.0.)  Warp q of a group owns TMEM lanes 32 q .. 32 q + 31 (a warp
+    // while the other group's reds drain.  (Blocks of columns instead of tiles throughout: 128 -> 128 on 303 k pairs 25.7 us
+    // against 23.0.)  Warp q of a group owns TMEM lanes 32 q .. 32 q + 31 (a warp
     // may only read the lane quarter given by its index mod 4), i.e. tile rows 32 q .. 32 q + 31, and
     // walks the output row in 128-byte blocks: tcgen05.ld -> convert -> private patch -> reds.
     const int grp = warp >> 2, q4 = warp & 3;
-    const uint32_t row_bytes = (uint32_t)p.n_dim * ES;
+    const uint32_t row_bytes = (uint32_t)cfg.n_cols * ES, row_pitch = (uint32_t)p.n_dim * ES;
     constexpr uint32_t BLK_COLS = 128 / ES;  // accumulator columns per 128-byte block
-    uint8_t* dst = static_cast<uint8_t*>(p.dst);
+    uint8_t* dst = static_cast<uint8_t*>(p.dst) + (size_t)col0 * ES;
     uint8_t* patch = sPatch + warp * 4096;  // 32 rows x 128 bytes, private to the warp
     const uint32_t sw7 = (uint32_t)(lane & 7);
     // map entries of tile row 32 q + lane (-1 beyond the tile)
@@ -385,24 +390,30 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
         st_shared_i32(ds, v);
       }
     };
-    if (t0 + grp < t1) {
+    // With one tile, or two of an even number of column blocks, both groups take every tile and alternate blocks: 256 -> 256 on 600 voxels
+    // 7.9 -> 7.5 us, stride 2 128 -> 256 on 2365 pairs 6.8 -> 6.4.
+    const bool by_cols = row_bytes > 128 && (t1 - t0 == 1 || (t1 - t0 == 2 && row_bytes % 256 == 0));
+    const int tile0 = by_cols ? 0 : grp, d_tile = by_cols ? 1 : 2;
+    const uint32_t cb0 = by_cols ? 128u * grp : 0u, d_cb = by_cols ? 256u : 128u;
+    if (t0 + tile0 < t1) {
       G3Walk pf;
-      pf.init(tile_start, n_seg, t0 + grp);
+      auto skip = [&]() {
+        pf.next(tile_start, n_seg);
+        if (!by_cols) pf.next(tile_start, n_seg);
+      };
+      pf.init(tile_start, n_seg, t0 + tile0);
       fetch_entries(pf, 0);
       cp_async_commit();
-      pf.next(tile_start, n_seg);
-      pf.next(tile_start, n_seg);
+      skip();
       if (pf.t < t1) fetch_entries(pf, 1);
       cp_async_commit();
-      pf.next(tile_start, n_seg);
-      pf.next(tile_start, n_seg);
+      skip();
       int own_i = 0;  // tiles of this group so far
-      for (int t = t0 + grp; t < t1 && ok; t += 2) {
+      for (int t = t0 + tile0; t < t1 && ok; t += d_tile) {
         const int tile_i = t - t0;
         if (pf.t < t1) fetch_entries(pf, (own_i + 2) & (G3_RING_SLOTS - 1));
         cp_async_commit();
-        pf.next(tile_start, n_seg);
-        pf.next(tile_start, n_seg);
+        skip();
         cp_async_wait<2>();  // this tile's entries (fetched two of the group's tiles ago) have landed
         const uint32_t slot = (uint32_t)(own_i & (G3_RING_SLOTS - 1));
         const int g0 = ld_shared_i32(ring + slot * 128u), s0 = ld_shared_i32(ring + (G3_RING_SLOTS + slot) * 128u);
@@ -414,7 +425,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
         if (!ok) break;
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(buf * cfg.n_acc);
-        for (uint32_t cb = 0; cb < row_bytes; cb += 128) {
+        for (uint32_t cb = cb0; cb < row_bytes; cb += d_cb) {
           // bytes of this block that belong to the row; `lpe` lanes share a row in the reds below
           const uint32_t vb = FULL ? 128u : min(128u, row_bytes - cb);
           const uint32_t lpe = (FULL || vb > 64) ? 8u : (vb > 32 ? 4u : 2u), rpe = 32u / lpe;
@@ -439,7 +450,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
               *reinterpret_cast<uint4*>(patch + lane * 128 + (((c0 / 8 + 1) ^ sw7) << 4)) = make_uint4(h[4], h[5], h[6], h[7]);
             }
           }
-          if (cb + 128 >= row_bytes) {
+          if (!by_cols && cb + 128 >= row_bytes) {  // (of two tiles each has an accumulator of its own)
             // accumulator fully read: hand the TMEM buffer back before the last reds go out
             tc_fence_before();
             __syncwarp();
@@ -465,7 +476,7 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
 #pragma unroll
             for (uint32_t u = 0; u < 4; ++u) {
               if (sr[u] < 0 || !ch_ok || (!FULL && u0 + u >= lpe)) continue;
-              uint8_t* o = dcol + (size_t)sr[u] * row_bytes;
+              uint8_t* o = dcol + (size_t)sr[u] * row_pitch;
               if (TF32) red_add_v4(reinterpret_cast<float*>(o), __uint_as_float(v[u].x), __uint_as_float(v[u].y), __uint_as_float(v[u].z), __uint_as_float(v[u].w));
               else red_add_h8(reinterpret_cast<__half*>(o), v[u].x, v[u].y, v[u].z, v[u].w);
             }
@@ -490,10 +501,12 @@ __global__ void __launch_bounds__(G3_THREADS, 1) umma_gms3_kernel(GmsParams p, G
 // Shared-memory plan of a forward (trans = false) or dgrad (trans = true) launch.  Returns false when the
 // shape is outside what the kernel takes or does not fit `max_smem`: the one place that decides it, used by
 // the launcher and by the kernel-family query alike.
-inline bool g3_plan(int c_in, int c_out, int es, int k_vol, int max_smem, bool trans, G3Config* cfg) {
+inline bool g3_plan(int c_in, int c_out, int es, int k_vol, int max_smem, bool trans, G3Config* cfg, int n_split = 1) {
   if (!umma_supported(c_in, c_out, es)) return false;
-  const int k_dim = trans ? c_out : c_in, n_dim = trans ? c_in : c_out;
+  const int k_dim = trans ? c_out : c_in, n_dim = (trans ? c_in : c_out) / n_split;
   const int epr = 128 / es;
+  cfg->n_split = n_split;
+  cfg->n_cols = n_dim;
   cfg->kch = (k_dim * es + 127) / 128;
   cfg->n_acc = (n_dim + epr - 1) / epr * epr;
   cfg->n_mma = trans ? n_dim : cfg->n_acc;
@@ -513,13 +526,24 @@ inline bool g3_plan(int c_in, int c_out, int es, int k_vol, int max_smem, bool t
   return true;
 }
 
+// CTAs that share a tile, each with whole 128-byte blocks of its columns: as many as leave every part a CTA of its own (the tiles are
+// estimated, half of an offset's last one).  A CTA then loads, multiplies and adds that much less behind one another: 256 -> 256 on 41 / 600
+// voxels 7.2 / 7.9 -> 5.4 / 6.1 us, stride 2 128 -> 256 on 2365 pairs 6.8 -> 5.1, tf32 128 -> 128 on 600 voxels 7.2 -> 6.0.  Beyond that line every
+// row is gathered more than once for nothing: 256 -> 256 on 1200 voxels (144 tiles) 8.0 / 8.4, on 9455 20.8 / 21.5, 128 -> 128 on 146 k 23.4 / 31.1.
+inline int g3_split(int n_dim, int es, long long pairs, int segments, int sms) {
+  for (int n = 4; n > 1; --n)
+    if (n_dim * es % (n * 128) == 0 && n * (pairs / 128 + segments / 2) <= sms) return n;
+  return 1;
+}
+
 template <bool TF32, bool TRANS_W, bool FULL>
 inline int g3_launch_as(const GmsParams& p, const G3Config& cfg, cudaStream_t st, int sms, int max_smem) {
   static std::atomic<int> granted[64];
   if (int rc = ensure_smem(umma_gms3_kernel<TF32, TRANS_W, FULL>, max_smem, granted)) return rc;
   CUtensorMap w_map;
-  if (int rc = weight_tensor_map(&w_map, p.weights, p.k_vol, p.c_in, p.c_out, !TF32, !TRANS_W)) return rc;
-  return launch_pdl(umma_gms3_kernel<TF32, TRANS_W, FULL>, sms, G3_THREADS, (size_t)cfg.smem, st, p, cfg, w_map) == cudaSuccess ? 0 : -1;
+  if (int rc = weight_tensor_map(&w_map, p.weights, p.k_vol, p.c_in, p.c_out, !TF32, !TRANS_W, TRANS_W ? cfg.n_cols : p.c_in)) return rc;
+  const dim3 grid((unsigned)(sms / cfg.n_split), (unsigned)cfg.n_split);
+  return launch_pdl(umma_gms3_kernel<TF32, TRANS_W, FULL>, grid, G3_THREADS, (size_t)cfg.smem, st, p, cfg, w_map) == cudaSuccess ? 0 : -1;
 }
 template <bool TF32, bool TRANS_W>
 inline int g3_launch(const GmsParams& p, const G3Config& cfg, cudaStream_t st, int sms, int max_smem) {
@@ -534,6 +558,8 @@ inline int launch_umma_gms3(const GmsParams& p, bool trans, bool f16, cudaStream
   if ((reinterpret_cast<uintptr_t>(p.src) | reinterpret_cast<uintptr_t>(p.weights) | reinterpret_cast<uintptr_t>(p.dst)) & 15) return 1;
   G3Config cfg;
   if (!g3_plan(p.c_in, p.c_out, f16 ? 2 : 4, p.k_vol, max_smem, trans, &cfg)) return 1;
+  const int n_split = g3_split(p.n_dim, f16 ? 2 : 4, (long long)p.pairs + p.dense_rows, p.k_vol + (p.dense_rows > 0), sms);
+  if (n_split > 1) g3_plan(p.c_in, p.c_out, f16 ? 2 : 4, p.k_vol, max_smem, trans, &cfg, n_split);  // it needs less
   if (f16) return trans ? g3_launch<false, true>(p, cfg, st, sms, max_smem) : g3_launch<false, false>(p, cfg, st, sms, max_smem);
   return trans ? g3_launch<true, true>(p, cfg, st, sms, max_smem) : g3_launch<true, false>(p, cfg, st, sms, max_smem);
 }
