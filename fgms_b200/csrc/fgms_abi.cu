@@ -224,18 +224,21 @@ struct Range {
 // Side by side the passes overlap each other's fixed parts (launch, tile table, first rows; the sums' way out) and what they are
 // bound by, reds of rows in the input gradient, instructions of the gathers in the weight gradient.  The weight gradient goes
 // first, with one block per SM on its share; the input gradient's blocks find room on the others only.  Either pass takes about
-// c + u * (128-pair units) / SMs microseconds, the constants below fitted to the passes by themselves; the share is the
-// one at which the later one ends first.  Behind one another / started together but with all SMs each / with the share, in a row of
-// launches: fp16 64 -> 64 0.93 M pairs 69.0 / 66.0 / 61.9 us, 137 k 19.8 / 18.9 / 15.2, 32 -> 32 9.1 M 254 / 252 / 237, 84 k 12.1 / 10.3 / 7.9; 128 -> 128 303 k
-// 44.5 / 44.2 / 38.8, 256 -> 256 28 k 25.9 / 25.7 / 22.1, stride 2 64 -> 128 9 k 12.1 / 12.2 / 7.5; tf32 32 -> 64 stride 2 200 k 25.9 / 24.1 / 22.2.  A share a
-// sixth off gives the gain away (64 -> 64 0.93 M pairs at 0.36 / 0.48 / 0.60 of the SMs 77.9 / 61.4 / 78.1).
+// c + u * (128-pair units) / SMs microseconds; the share is the one at which the later one ends first.  Behind one another / started
+// together but with all SMs each / with the share, in a row of launches: fp16 64 -> 64 0.93 M pairs 69.0 / 66.0 / 61.9 us, 137 k 19.8 / 18.9 / 15.2,
+// 32 -> 32 9.1 M 254 / 252 / 237, 84 k 12.1 / 10.3 / 7.9; 128 -> 128 303 k 44.5 / 44.2 / 37.5.  A share a sixth off gives the gain away (64 -> 64
+// 0.93 M pairs at 0.36 / 0.48 / 0.60 of the SMs 77.9 / 61.4 / 78.1).
 //
-// How good the model is: against every fourth share, over 36 shapes of 16 to 256 channels and 4 k to 9 M pairs, it was within 3 % of the best
-// one in 17, within 10 % in 29, and 0.62 to 0.99 of one behind the other in all.  It is off where both passes are short (256 -> 256 28 k
-// 22.1 where 88 of the SMs take 17.5, 4 k 12.1 / 9.6; 128 -> 128 12 k 10.3 / 8.2; stride 2 128 -> 256 20 k 14.1 / 11.1) and on LiDAR maps of two pairs a
-// row (32 -> 32 173 k pairs 13.9 / 12.7, 12.8 with all SMs each; 43 k 7.7 / 6.3).  0.97 and 1.07, the margins of "behind one another", and the terms for
-// 48 channels, whose rows are copied with idle lanes, are fitted like the others.
-int split_backward(int64_t pairs, int c_in, int c_out, int k_vol, int dtype, int math, const DeviceInfo& di) {
+// With the weight gradient on tcgen05 the constants are fitted to the passes side by side: 151 shapes and sizes (16 to 256 channels, 300 to
+// 0.44 M pairs) times 16 shares.  The share is within 2.6 % of the best of the 16 on average, 19 % at worst; with constants fitted to each pass by
+// itself it was 11.6 % off (256 -> 256 on 39 k pairs 23.6 -> 19.0 us, best 18.8, 128 -> 256 on 98 k 26.3 -> 21.6, stride 2 256 -> 256 on 9 k 14.0 -> 11.3, best
+// 9.5): the input gradient, launched second, takes 1.5 to 5 us longer than by itself.  On maps of few pairs a row
+// (LiDAR and scattered clouds, about two) the rows come from memory rather than from L2, the weight gradient's from both sides: a fifth more for it
+// (passes on new rows each time, 128 -> 128 on 303 k LiDAR pairs 91.6 -> 89.4 us, 96 -> 160 on 110 k 53.8 -> 52.6; stride-2 maps need none).  Slower than
+// with the constants before by up to 2 %: 128 -> 64 on 173 k LiDAR pairs 52.9 -> 53.9.  Rows of up to 64 channels on both sides keep the constants of each pass by itself, within
+// 10 % of the best; 0.97 and 1.07 are the margins of "behind one another", and the terms for 48 channels, whose rows are copied
+// with idle lanes, are fitted like the others.
+int split_backward(int64_t pairs, int rows, int c_in, int c_out, int k_vol, int dtype, int math, const DeviceInfo& di) {
   fgms::G3Config g;
   fgms::W3Config w;
   const bool f16 = dtype == FGMS_DTYPE_F16;
@@ -244,17 +247,36 @@ int split_backward(int64_t pairs, int c_in, int c_out, int k_vol, int dtype, int
   if (math == FGMS_MATH_FP32 || !fgms::g3_plan(c_in, c_out, es, k_vol, di.max_smem_optin, true, &g) ||
       !fgms::w3_plan(c_in, c_out, es, k_vol, di.max_smem_optin, &w) || di.sms < 16)
     return 0;
-  const double both = c_in + c_out, area = (double)c_in * c_out, units = (double)pairs / 128 + k_vol;
-  double c_d = 4, u_d = 0.1 + 0.1 * g.kch + 0.43 * ((c_in * es + 127) / 128);
-  double c_w = 5.5 + area / 8192, u_w = 0.36 * (128.0 / w.pb) + 0.09 * (w.pa + w.pbp) / w.pack;
-  if (fgms::rw_supported(c_out, c_in, f16)) c_d = 3.5, u_d = both * (f16 ? 0.0046 : 0.01);
-  if (f16 && fgms::wh_supported(c_in, c_out, true))
-    c_w = 5 + area / 2048, u_w = 0.094 + 0.026 * area / 256 + 0.075 * ((c_in == 48) + (c_out == 48));
-  if (!f16 && fgms::wh_supported(c_in, c_out, false)) c_w = 5 + area / 2048, u_w = 0.1 + 0.003 * both + 0.035 * area / 256 + 0.1 * ((c_in == 48) + (c_out == 48));
+  const double both = c_in + c_out, area = (double)c_in * c_out;
+  const int blocks = (c_in * es + 127) / 128;  // of an output row of the input gradient
+  const bool short_d = fgms::rw_supported(c_out, c_in, f16), short_w = fgms::wh_supported(c_in, c_out, f16);
+  double c_d, u_d, c_w, u_w, units = (double)pairs / 128 + k_vol;
+  if (short_w) {
+    c_d = 4, u_d = 0.1 + 0.1 * g.kch + 0.43 * blocks;
+    if (short_d) c_d = 3.5, u_d = both * (f16 ? 0.0046 : 0.01);
+    c_w = 5 + area / 2048;
+    u_w = (f16 ? 0.094 + 0.026 * area / 256 + 0.075 * ((c_in == 48) + (c_out == 48))
+               : 0.1 + 0.003 * both + 0.035 * area / 256 + 0.1 * ((c_in == 48) + (c_out == 48)));
+  } else {
+    units = (double)pairs / 128 + 0.5 * k_vol;
+    // 128-byte pieces of the two rows; a last one that is filled in part counts for half of the rest as well
+    const double in = 0.5 * (g.kch + c_out * es / 128.0), out = 0.5 * (blocks + c_in * es / 128.0);
+    c_d = 5.6 + 0.19 * in + 0.2 * out, u_d = 0.05 + 0.182 * in + 0.397 * out;
+    if (short_d) c_d = 5.5, u_d = both * (f16 ? 0.0046 : 0.01);
+    c_w = u_w = 0;  // by its plan, which depends on the share
+  }
+  const bool few = k_vol > 8 && pairs < 4ll * rows;
   int best = 0;
+  double least = 1e30;
   // behind one another, where the input gradient on all SMs meets L2's rate of reds
-  double least = 0.97 * (c_d + c_w - 2 + (1.07 * u_d + u_w) * units / di.sms);
+  if (short_w) least = 0.97 * (c_d + c_w - 2 + (1.07 * u_d + u_w) * units / di.sms);
   for (int s = di.sms / 4; s <= di.sms - di.sms / 4; s += 2) {
+    if (!short_w && (s == di.sms / 4 || !fgms::w3_same_split(c_in, c_out, es, k_vol, pairs, s - 2, s))) {
+      fgms::w3_plan(c_in, c_out, es, k_vol, di.max_smem_optin, &w);
+      fgms::w3_split(c_in, c_out, es, k_vol, pairs, s, di.max_smem_optin, &w);
+      c_w = 5.9 + (w.n_buf == 1 ? 3.01 : 1.02) * w.c_a * w.c_b * es / 32768;
+      u_w = (few ? 1.2 : 1.0) * w.parts_a * w.parts_b * (0.264 + 0.025 * (w.pa + w.pbp) / w.pack + 0.336 * (128.0 / w.pb));
+    }
     const double d = c_d + u_d * units / (di.sms - s), v = c_w + u_w * units / s, end = d > v ? d : v;
     if (end < least) { least = end; best = s; }
   }
@@ -605,7 +627,7 @@ int fgms_b200_bwd(const void* out_grad, const void* in_feats, const void* kernel
                          reinterpret_cast<uintptr_t>(in_grad) | reinterpret_cast<uintptr_t>(kernel_grad)) & 15) == 0;
   Beside beside;
   beside.on = true;
-  const int wgrad_sms = !aligned ? 0 : split_backward(map_len, c_in, c_out, k_vol, dtype, math, di);
+  const int wgrad_sms = !aligned ? 0 : split_backward(map_len, n_in > n_out ? n_in : n_out, c_in, c_out, k_vol, dtype, math, di);
   if (wgrad_sms > 0) beside.sms = di.sms - wgrad_sms;
   if (int rc = wgrad(wgrad_sms)) return rc;
   return dgrad(beside);

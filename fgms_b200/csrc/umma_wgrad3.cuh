@@ -80,6 +80,8 @@ struct W3Config {
                   //    one is real, and the rows it repeats land in accumulator rows that are never written out
   int pa, pbp;    // 128-byte pieces per staged row of A (enough for every row tile) and of B (n_acc columns)
   int n_acc;      // TMEM columns of one row tile: c_out rounded up to a whole piece
+  int parts_a, parts_b;  // blocks of dW_k, one CTA's each: of c_a input by c_b output channels
+  int c_a, c_b;
   int smem;       // dynamic shared memory of the launch
   int n_buf;      // TMEM accumulator sets: 1, 2 or 4
   int buf_shift;  // log2(n_buf)
@@ -119,6 +121,8 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_seg = p.k_vol + 1;
   volatile int* abort_flag = &sh->abort_flag;
+  const int part_a = (int)blockIdx.y % cfg.parts_a;
+  const int a0 = part_a * cfg.c_a, b0 = ((int)blockIdx.y - part_a) / cfg.parts_a * cfg.c_b;  // this CTA's first channels
   const uint32_t lbo = (uint32_t)kr * 128u;  // next 128 bytes of every staged row
   const uint32_t buf_cols = (uint32_t)(cfg.n_mtile * cfg.n_acc);
 
@@ -162,7 +166,8 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
     const int rpw = pb / TEAM_WARPS;  // rows of a stage owned by this warp: 4, 8, 16 or 32
     const uint8_t* feats = static_cast<const uint8_t*>(p.feats);
     const uint8_t* og = static_cast<const uint8_t*>(p.out_grad);
-    const uint32_t a_row_bytes = (uint32_t)p.c_in * ES, b_row_bytes = (uint32_t)p.c_out * ES;
+    const uint32_t a_row_bytes = (uint32_t)cfg.c_a * ES, b_row_bytes = (uint32_t)cfg.c_b * ES;  // of a row's part
+    const uint32_t a_pitch = (uint32_t)p.c_in * ES, b_pitch = (uint32_t)p.c_out * ES;
     // Lane (rs, cc) = (lane / 8, lane % 8) copies 16-byte chunk cc of every 128-byte piece of the rows rs, rs + 4, ... of the warp's
     // block: one shuffle and one address per row, then one cp.async per piece at a fixed distance (128 bytes in global memory,
     // `lbo` in shared memory).
@@ -189,8 +194,8 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
       rel_b[u] = TF32 ? mnmajor32_offset(row, byte_b, lbo, 512u) : mnmajor_offset(row, byte_b, lbo, 1024u);
     }
     const uint32_t four_rounds = row_step * 512u;
-    const uint8_t* feats_c = feats + cc * 16;
-    const uint8_t* og_c = og + cc * 16;
+    const uint8_t* feats_c = feats + a0 * ES + cc * 16;
+    const uint8_t* og_c = og + b0 * ES + cc * 16;
     // The pieces of R rows of one operand.  What this role spends its time on are instructions (with the copies left out
     // the kernel took as long: tests of every one of eight possible pieces and address arithmetic, 400 instructions a
     // warp and stage), so the usual numbers of pieces have their own straight code.  (tf32 rows of 5 to 8 pieces with eight tests / in a loop /
@@ -235,8 +240,8 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
       }
     };
     auto copy_rounds = [&](auto rounds, int u0, int cur_a, int cur_b, uint32_t sa, uint32_t sb) {
-      copy_rows(rounds, u0, cur_a, feats_c, a_row_bytes, rel_a, sa, np_a, tail_a);
-      copy_rows(rounds, u0, cur_b, og_c, b_row_bytes, rel_b, sb, np_b, tail_b);
+      copy_rows(rounds, u0, cur_a, feats_c, a_pitch, rel_a, sa, np_a, tail_a);
+      copy_rows(rounds, u0, cur_b, og_c, b_pitch, rel_b, sb, np_b, tail_b);
     };
     // lane r < rpw fetches both map entries of the warp's row r (-1 beyond the stage) into its words of a ring slot: copied
     // there, they are waited for when they are used, where entries handed on through registers were waited for a stage after
@@ -282,7 +287,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
       get = get == W3_PREFETCH * ring_step ? 0 : get + ring_step;
       // a pair is used only if both its entries are inside the tensors
       if (!((unsigned)cur_a < (unsigned)p.n_in && (unsigned)cur_b < (unsigned)p.n_out)) {
-        if (cur_a != -1 || cur_b != -1) report_problem();  // counted once per skipped pair
+        if (blockIdx.y == 0 && (cur_a != -1 || cur_b != -1)) report_problem();  // counted once per skipped pair
         cur_a = cur_b = -1;
       }
       ok = g3_wait(&sh->empty[s], ph ^ 1u, abort_flag);
@@ -377,7 +382,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
     // Packed stages: staged row k holds `pack` pairs side by side, in A and in B, so the accumulator is pack x pack
     // blocks of slot_m x slot_n elements of which the diagonal ones are sums over pairs (block (s, s): the pairs in
     // position s) and the others mix two pairs' rows and are dropped.  A warp's rows (32 of a 128-row accumulator,
-    // 16 of a 64-row one) lie in one block row; it adds columns [col_base, col_base + c_out) of its rows to gradient
+    // 16 of a 64-row one) lie in one block row; it adds columns [col_base, col_base + c_b) of its rows to gradient
     // rows (row - row_base).  (tf32 with at most 32 staged elements: the 64-row MMA reads them twice, rows 32 .. 63
     // repeat rows 0 .. 31 and are dropped.)
     const int slot_m = PACKED ? cfg.slot_a / ES : 0, slot_n = PACKED ? cfg.slot_b / ES : 0;
@@ -395,14 +400,15 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
       ok = g3_wait(&sh->tmem_full[buf], use & 1u, abort_flag);
       if (!ok) break;
       tc_fence_after();
-      float* dwk = p.dw + (size_t)seg * p.c_in * p.c_out;
+      const size_t first = ((size_t)seg * p.c_in + a0) * p.c_out + b0;
+      float* dwk = p.dw + first;
       if (!TF32 && p.dw_f16 != nullptr) {
         // fp16 destination: 64 columns (128 bytes of fp16) of the warp's 32 rows per round
-        __half* dwk16 = p.dw_f16 + (size_t)seg * p.c_in * p.c_out;
+        __half* dwk16 = p.dw_f16 + first;
         for (int mt = 0; mt < cfg.n_mtile; ++mt) {
           const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)buf * buf_cols + (uint32_t)(mt * cfg.n_acc);
           const bool m128 = mt + 1 < cfg.n_mtile || cfg.last_m == 128;
-          for (int c0 = 0; c0 < p.c_out; c0 += 64) {
+          for (int c0 = 0; c0 < cfg.c_b; c0 += 64) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {  // 16 columns at a time: few registers in flight
               uint32_t v[16], h[8];
@@ -422,7 +428,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
               if (m128) m = blk_ok ? mt * 128 + warp * 32 + (int)r - row_base : -1;
               else m = (r < 16 && blk_ok) ? mt * 128 + warp * 16 + (int)r - row_base : -1;
               const uint4 v = *reinterpret_cast<const uint4*>(patch + r * 128 + ((ch ^ (r & 7)) << 4));
-              if (m >= 0 && m < p.c_in && c0 + (int)(ch << 3) < p.c_out) red_add_h8(dwk16 + (size_t)m * p.c_out + c0 + (ch << 3), v.x, v.y, v.z, v.w);
+              if (m >= 0 && m < cfg.c_a && c0 + (int)(ch << 3) < cfg.c_b) red_add_h8(dwk16 + (size_t)m * p.c_out + c0 + (ch << 3), v.x, v.y, v.z, v.w);
             }
             __syncwarp();
           }
@@ -431,7 +437,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
       for (int mt = 0; mt < cfg.n_mtile; ++mt) {
         const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)buf * buf_cols + (uint32_t)(mt * cfg.n_acc);
         const bool m128 = mt + 1 < cfg.n_mtile || cfg.last_m == 128;
-        for (int c0 = 0; c0 < p.c_out; c0 += 32) {
+        for (int c0 = 0; c0 < cfg.c_b; c0 += 32) {
           uint32_t v0[16], v1[16];
           tmem_ld16(taddr + col_base + c0, v0);
           if (!PACKED || slot_n - c0 > 16) {
@@ -455,7 +461,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
             if (m128) m = blk_ok ? mt * 128 + warp * 32 + (int)r - row_base : -1;
             else m = (r < 16 && blk_ok) ? mt * 128 + warp * 16 + (int)r - row_base : -1;
             const uint4 v = *reinterpret_cast<const uint4*>(patch + r * 128 + ((ch ^ (r & 7)) << 4));
-            if (m >= 0 && m < p.c_in && c0 + (int)(ch << 2) < p.c_out)
+            if (m >= 0 && m < cfg.c_a && c0 + (int)(ch << 2) < cfg.c_b)
               red_add_v4(dwk + (size_t)m * p.c_out + c0 + (ch << 2), __uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
           }
           __syncwarp();
@@ -481,6 +487,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
 inline bool w3_plan(int c_in, int c_out, int es, int k_vol, int max_smem, W3Config* cfg) {
   if (!umma_supported(c_in, c_out, es)) return false;
   const int epr = 128 / es;  // elements per 128-byte piece
+  cfg->parts_a = cfg->parts_b = 1; cfg->c_a = c_in; cfg->c_b = c_out;
   // Packed stages: two pairs share a staged row, their rows side by side in A and in B, so one MMA contracts
   // twice as many pairs — an MMA of 64 x 64 x 16 costs what one of 128 x 128 x 16 does, and with rows of up to
   // 256 bytes the issue loop is what bounds the kernel.  The accumulator then holds 2 x 2 blocks; the epilogue
@@ -528,22 +535,66 @@ inline bool w3_plan(int c_in, int c_out, int es, int k_vol, int max_smem, W3Conf
   return false;
 }
 
+// Sides of dW_k longer than 128 channels are halved, each block a CTA's, where a CTA would have few stages: what such a CTA takes its time
+// for is the way of the sums of 256 x 256 products, 128 KB of reds behind one another (with one set of accumulators, which fills tensor
+// memory, nothing overlaps them), and the halves of rows that are then gathered twice cost less.  Whole / halved, by stages of 128 pairs a CTA
+// (t): both sides, fp16 256 x 256 t = 0.4 / 1 / 1.6 / 3 9.0 / 13.9 / 15.8 / 17.8 -> 7.4 / 9.1 / 11.1 / 14.6 us, 160 x 160 t = 1 11.3 -> 9.4, t = 3 14.1 -> 15.4, one
+// side only 13.3; t = 9 20.8 -> 24.8; 256 x 256 t = 5.3, one side, 21.2 -> 18.9, t = 11 29.5 -> 30.6; tf32 256 x 256 t = 1 / 3 22.3 / 28.0 -> 12.4 / 20.9.
+// One long side: fp16 256 x 64 t = 1 / 3 7.2 / 9.6 -> 6.3 / 9.1, t = 9 15.0 -> 15.9, 128 x 192 (rows of the output side are the longer part of a
+// stage) t = 1 7.9 -> 7.5, t = 3 10.1 -> 10.9; tf32 128 x 256 t = 1 / 3 13.2 / 16.9 -> 10.2 / 14.9.  Shorter sides, fp16, where the halves have a CTA each: 128 x
+// 128 on 65 stages 5.8 -> 5.2, 96 x 96 on 29 5.8 -> 5.2, tf32 128 x 128 on 65 6.8 -> 7.0.
+// The whole plan stays where a half is no multiple of 16 channels.
+struct W3Parts {
+  int a, b;
+  bool operator==(const W3Parts& o) const { return a == o.a && b == o.b; }
+};
+inline W3Parts w3_parts(int c_in, int c_out, int es, int k_vol, long long pairs, int sms) {
+  const double stages = (double)pairs / 128 + 0.5 * k_vol, t = stages / sms;  // (an offset's last stage is half empty on average)
+  int a = 1, b = 1;
+  if (c_in > 128 && c_out > 128) {
+    if (t <= 2.2) a = b = 2;
+    else if (t <= (c_in * c_out >= 224 * 256 ? 5.5 : 3.3)) a = 2;
+  } else if (c_in > 128) {
+    if (t <= 3) a = 2;
+  } else if (c_out > 128) {
+    if (t <= (es == 2 ? 1.2 : 3)) b = 2;
+  } else if (es == 2 && c_in >= 96 && c_out >= 96 && t <= 0.5) {
+    b = 2;
+  }
+  if (c_in % (16 * a)) a = 1;
+  if (c_out % (16 * b)) b = 1;
+  return {a, b};
+}
+inline bool w3_same_split(int c_in, int c_out, int es, int k_vol, long long pairs, int sms, int other) {
+  return w3_parts(c_in, c_out, es, k_vol, pairs, sms) == w3_parts(c_in, c_out, es, k_vol, pairs, other);
+}
+// the plan of such a block in place of the whole one
+inline void w3_split(int c_in, int c_out, int es, int k_vol, long long pairs, int sms, int max_smem, W3Config* cfg) {
+  const W3Parts n = w3_parts(c_in, c_out, es, k_vol, pairs, sms);
+  W3Config part;
+  if (n.a * n.b == 1 || sms < n.a * n.b || !w3_plan(c_in / n.a, c_out / n.b, es, k_vol, max_smem, &part)) return;
+  *cfg = part;
+  cfg->parts_a = n.a;
+  cfg->parts_b = n.b;
+}
+
 template <bool TF32, bool FULL, bool PACKED, int TEAMS>
 inline int w3_launch_as(const WgradParams& p, const W3Config& cfg, cudaStream_t st, int sms, int max_smem) {
   static std::atomic<int> granted[64];
   if (int rc = ensure_smem(umma_wgrad3_kernel<TF32, FULL, PACKED, TEAMS>, max_smem, granted)) return rc;
-  return launch_pdl(umma_wgrad3_kernel<TF32, FULL, PACKED, TEAMS>, sms, W3_THREADS, (size_t)cfg.smem, st, p, cfg) == cudaSuccess ? 0 : -1;
+  const int parts = cfg.parts_a * cfg.parts_b;
+  return launch_pdl(umma_wgrad3_kernel<TF32, FULL, PACKED, TEAMS>, dim3((unsigned)(sms / parts), (unsigned)parts), W3_THREADS, (size_t)cfg.smem, st, p, cfg) == cudaSuccess ? 0 : -1;
 }
 template <bool TF32, bool FULL, bool PACKED>
 inline int w3_launch_teams(const WgradParams& p, const W3Config& cfg, cudaStream_t st, int sms, int max_smem) {
-  const bool few = p.pairs / cfg.pb + p.k_vol / 2 <= W3_ONE_TEAM_STAGES * sms;  // (an offset's last stage is half empty on average)
+  const bool few = p.pairs / cfg.pb + p.k_vol / 2 <= W3_ONE_TEAM_STAGES * (sms / (cfg.parts_a * cfg.parts_b));  // (an offset's last stage is half empty on average)
   return few ? w3_launch_as<TF32, FULL, PACKED, 1>(p, cfg, st, sms, max_smem)
              : w3_launch_as<TF32, FULL, PACKED, W3_PROD_TEAMS>(p, cfg, st, sms, max_smem);
 }
 template <bool TF32>
 inline int w3_launch(const WgradParams& p, const W3Config& cfg, cudaStream_t st, int sms, int max_smem) {
   const int es = TF32 ? 4 : 2;
-  const bool full = (p.c_in * es) % 128 == 0 && (p.c_out * es) % 128 == 0;
+  const bool full = (cfg.c_a * es) % 128 == 0 && (cfg.c_b * es) % 128 == 0;
   if (cfg.pack > 1)
     return full ? w3_launch_teams<TF32, true, true>(p, cfg, st, sms, max_smem) : w3_launch_teams<TF32, false, true>(p, cfg, st, sms, max_smem);
   return full ? w3_launch_teams<TF32, true, false>(p, cfg, st, sms, max_smem) : w3_launch_teams<TF32, false, false>(p, cfg, st, sms, max_smem);
@@ -555,6 +606,7 @@ inline int launch_umma_wgrad3(const WgradParams& p, bool f16, cudaStream_t st, i
   if ((reinterpret_cast<uintptr_t>(p.feats) | reinterpret_cast<uintptr_t>(p.out_grad) | reinterpret_cast<uintptr_t>(p.dw) | reinterpret_cast<uintptr_t>(p.dw_f16)) & 15) return 1;
   W3Config cfg;
   if (!w3_plan(p.c_in, p.c_out, f16 ? 2 : 4, p.k_vol, max_smem, &cfg)) return 1;
+  w3_split(p.c_in, p.c_out, f16 ? 2 : 4, p.k_vol, p.pairs, sms, max_smem, &cfg);
   return f16 ? w3_launch<false>(p, cfg, st, sms, max_smem) : w3_launch<true>(p, cfg, st, sms, max_smem);
 }
 
