@@ -61,10 +61,10 @@ struct WgradParams {
 // `kpos` comes from the caller's device memory and is not trusted: every entry is clamped to
 // [0, pairs] (pairs = length of the maps) on its way into shared memory, so a stale or mismatched
 // kpos can shorten segments but never moves a map read past the end of the maps.  A clamped entry
-// is counted as a problem once per launch.
+// is counted as a problem once per launch (`passes` times by a launch that does several passes' work).
 __device__ __forceinline__ void build_tile_table(int TILE, const int32_t* __restrict__ kpos, int pairs, int k_vol,
                                                  int dense_rows, int* kpos_s /* [k_vol+1] */,
-                                                 int* tile_start /* [k_vol+2] */) {
+                                                 int* tile_start /* [k_vol+2] */, int passes = 1) {
   // The first warp does it alone, 32 segments at a time: both ends of a segment are loaded side by side, so the table
   // costs one trip to memory, one scan by shuffles and one barrier (three barriers and a second pass before).
   if (threadIdx.x < 32) {
@@ -76,7 +76,8 @@ __device__ __forceinline__ void build_tile_table(int TILE, const int32_t* __rest
       if (s <= k_vol) {
         const int first = __ldg(kpos + s), next = s < k_vol ? __ldg(kpos + s + 1) : 0;
         const int c = min(max(first, 0), pairs);
-        if (first != c && blockIdx.x == 0 && blockIdx.y == 0) report_problem();
+        if (first != c && blockIdx.x == 0 && blockIdx.y == 0)
+          for (int r = 0; r < passes; ++r) report_problem();
         kpos_s[s] = c;
         const int cnt = s < k_vol ? min(max(next, 0), pairs) - c : dense_rows;
         v = cnt > 0 ? (cnt + TILE - 1) / TILE : 0;

@@ -523,6 +523,13 @@ size_t fgms_b200_wgrad_workspace_bytes(int c_in, int c_out, int k_vol, int dtype
   return (size_t)k_vol * c_in * c_out * sizeof(float);
 }
 
+size_t fgms_b200_bwd_workspace_bytes(int64_t map_len, int c_in, int c_out, int k_vol, int dtype, int math) {
+  DeviceInfo di;
+  if (dtype != FGMS_DTYPE_F16 || math == FGMS_MATH_FP32 || map_len < fgms::WH_BOTH_PAIRS || !fgms::rows_bwd_supported(c_in, c_out) || k_vol < 1) return 0;
+  if (device_info(&di) != FGMS_OK || di.reserved > 0 || !plan_wgrad(c_in, c_out, k_vol, dtype, math, di.max_smem_optin)) return 0;
+  return fgms_b200_wgrad_workspace_bytes(c_in, c_out, k_vol, dtype);
+}
+
 int fgms_b200_wgrad_finalize(void* kernel_grad_f16, const void* workspace_f32, int64_t count, void* stream) {
   TraceRange trace_range("fgms_b200_wgrad_finalize");
   if (count < 0) return fail(FGMS_ERR_INVALID_ARG, "negative count");
@@ -530,8 +537,9 @@ int fgms_b200_wgrad_finalize(void* kernel_grad_f16, const void* workspace_f32, i
   if (!kernel_grad_f16 || !workspace_f32) return fail(FGMS_ERR_INVALID_ARG, "null pointer");
   int blocks = (int)((count + 255) / 256);
   if (blocks > 1184) blocks = 1184;
-  fgms::wgrad_finalize_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__half*>(kernel_grad_f16), static_cast<const float*>(workspace_f32), (long long)count);
+  if (fgms::launch_pdl(fgms::wgrad_finalize_kernel, blocks, 256, 0, static_cast<cudaStream_t>(stream), static_cast<__half*>(kernel_grad_f16),
+                       static_cast<const float*>(workspace_f32), (long long)count) != cudaSuccess)
+    return fail(FGMS_ERR_CUDA, "wgrad_finalize_kernel launch failed");
   return check_launch("wgrad_finalize_kernel");
 }
 
@@ -613,9 +621,30 @@ int fgms_b200_bwd(const void* out_grad, const void* in_feats, const void* kernel
   const size_t es = elem_size(dtype), maps = (size_t)map_len * sizeof(int32_t);
   const Range in{in_feats, (size_t)n_in * c_in * es}, og{out_grad, (size_t)n_out * c_out * es}, w{kernel, (size_t)k_vol * c_in * c_out * es};
   const Range dx{in_grad, in.bytes}, dw{kernel_grad, w.bytes}, kp{kpos, (size_t)(k_vol + 1) * sizeof(int32_t)}, im{in_map, maps}, om{out_map, maps};
-  bool apart = (dtype != FGMS_DTYPE_F16 || !workspace) && !dx.overlaps(dw);
+  bool apart = !dx.overlaps(dw);
   for (const Range& r : {in, og, w, kp, im, om}) apart = apart && !r.overlaps(dx) && !r.overlaps(dw);
   DeviceInfo di;
+  // With a workspace: one kernel for both, which leaves fp32 sums of the weight gradient there.
+  const size_t need = fgms_b200_bwd_workspace_bytes(map_len, c_in, c_out, k_vol, dtype, math);
+  if (apart && need > 0 && workspace && workspace_bytes >= need && kernel_grad && in_feats && n_in > 0 && n_out > 0) {
+    const Range sums{workspace, need};
+    bool clear = (reinterpret_cast<uintptr_t>(workspace) & 255) == 0 && (reinterpret_cast<uintptr_t>(kernel_grad) & 15) == 0;
+    for (const Range& r : {in, og, w, kp, im, om, dx, dw}) clear = clear && !r.overlaps(sums);
+    if (clear && device_info(&di) == FGMS_OK) {
+      fgms::WgradParams p;
+      p.feats = in_feats; p.out_grad = out_grad; p.dw = static_cast<float*>(workspace); p.kpos = kpos; p.in_map = in_map; p.out_map = out_map;
+      p.pairs = (int)map_len;
+      p.n_in = n_in; p.n_out = n_out; p.c_in = c_in; p.c_out = c_out; p.k_vol = k_vol;
+      const fgms::RowsDgrad dg{kernel, static_cast<__half*>(in_grad)};
+      if (fgms::rows_bwd_takes(p, dg, di.max_smem_optin)) {
+        if (int rc = fgms_b200_zero2(workspace, need, nullptr, 0, stream)) return rc;
+        if (fgms::launch_rows_bwd(p, dg, st, di.sms, di.max_smem_optin) != 0) return fail(FGMS_ERR_CUDA, "rows_wgrad_kernel setup failed");
+        if (int rc = check_launch("rows_wgrad_kernel")) return rc;
+        return fgms_b200_wgrad_finalize(kernel_grad, workspace, (int64_t)k_vol * c_in * c_out, stream);
+      }
+    }
+  }
+  apart = apart && (dtype != FGMS_DTYPE_F16 || !workspace);
   if (!apart || n_in == 0 || n_out == 0 || map_len == 0 || device_info(&di) != FGMS_OK || di.reserved > 0) {
     if (int rc = dgrad(Beside())) return rc;
     return wgrad(0);

@@ -93,15 +93,76 @@ __device__ __forceinline__ void wh_ldmatrix(uint32_t addr, uint32_t (&v)[4]) {
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
 }
 
-template <bool TF32, int MU, int NU, int WARPS, int DEPTH>
-__global__ void __maxnreg__(rw_max_regs(WARPS * 32, true)) rows_wgrad_kernel(WgradParams p, bool spread) {
+// A tile's products with W_k^T, added to the input gradient: what rows_gms_kernel does, with the rows in shared memory.
+template <int MU, int NU>
+__device__ __forceinline__ void wh_dgrad(uint32_t rows, uint32_t to_rows, int lane, const uint32_t (&wt)[NU][2 * MU][2], __half* in_grad) {
+  using S = RowShape<false, NU, MU>;
+  using B = WhRows<false, NU>;
+  const int g = lane >> 2, t4 = lane & 3;
+  int to[2];
+  uint32_t a[2][S::AR];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    to[h] = umma::ld_shared_i32(to_rows + (g + 8 * h) * 4);
+#pragma unroll
+    for (int q = 0; q < S::KFULL; ++q)
+      asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(a[h][4 * q]), "=r"(a[h][4 * q + 1]), "=r"(a[h][4 * q + 2]), "=r"(a[h][4 * q + 3])
+                   : "r"(rows + B::at(g + 8 * h, 4 * q + t4)) : "memory");
+    if constexpr (S::KHALF > 0)
+      asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(a[h][4 * S::KFULL]), "=r"(a[h][4 * S::KFULL + 1])
+                   : "r"(rows + B::at(g + 8 * h, 4 * S::KFULL + (t4 >> 1)) + (t4 & 1) * 8) : "memory");
+  }
+  auto piece = [&](int j_first, auto n_tiles, __half* base) {
+    constexpr int N = decltype(n_tiles)::value;
+    float c[N][4];
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) c[i][k] = 0.f;
+#pragma unroll
+    for (int s = 0; s < S::KSTEPS; ++s) {
+      const uint32_t frag[4] = {a[0][2 * s], a[1][2 * s], a[0][2 * s + 1], a[1][2 * s + 1]};
+#pragma unroll
+      for (int i = 0; i < N; ++i) rw_mma(c[i], frag, wt[s][j_first + i][0], wt[s][j_first + i][1], false);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (to[h] < 0) continue;
+      __half* o = base + (size_t)(unsigned)to[h] * (MU * 16);
+      if (N == 4)
+        red_add_h8(o, pack_half2(c[0][2 * h], c[1][2 * h]), pack_half2(c[N - 2][2 * h], c[N - 1][2 * h]), pack_half2(c[0][2 * h + 1], c[1][2 * h + 1]),
+                   pack_half2(c[N - 2][2 * h + 1], c[N - 1][2 * h + 1]));
+      else red_add_h4(o, pack_half2(c[0][2 * h], c[1][2 * h]), pack_half2(c[0][2 * h + 1], c[1][2 * h + 1]));
+    }
+  };
+#pragma unroll
+  for (int q = 0; q < S::NFULL; ++q) piece(q * S::TPF, std::integral_constant<int, S::TPF>(), in_grad + q * 32 + t4 * 8);
+  if constexpr (S::NHALF > 0) piece(S::NFULL * S::TPF, std::integral_constant<int, 2>(), in_grad + S::NFULL * 32 + t4 * 4);
+}
+
+// The input gradient of the same pairs: in_grad[in_map[j]] += out_grad[out_map[j]] . W_k^T.
+struct RowsDgrad {
+  const void* weights;
+  __half* in_grad;
+};
+
+// DGRAD (fp16): both gradients of a backward.  Side by side, the two passes each gather every pair's row of the output gradient, and
+// the L2 that serves their gathers and reds bounds them; here a tile's rows are copied once, and its products with W_k^T come from the
+// copy in shared memory.  Backwards of 32 -> 32, us, two kernels side by side / this one with the clearing and rounding of its sums:
+// 9.6 M pairs 248 / 208, 1.13 M 32.3 / 31.1; 16 -> 32 on 1.13 M 29.3 / 25.1.  All SMs work on the weight gradient then, and rounded to
+// fp16 by each block, as those of its share were, it would be less exact (error against 64 bits, 1.13 M pairs: 5.0e-4, 4.0e-4 before),
+// so the sums stay fp32 in a workspace (2.1e-4).  Clusters of two blocks that round once were no more than even with the share
+// (4.0e-4; on 9.6 M pairs 4.0e-4 against 3.8e-4).
+template <bool TF32, int MU, int NU, int WARPS, int DEPTH, bool DGRAD>
+__global__ void __maxnreg__(rw_max_regs(WARPS * 32, true)) rows_wgrad_kernel(WgradParams p, bool spread, RowsDgrad dg) {
+  static_assert(!(TF32 && DGRAD), "fp16 only");
   static_assert(WARPS <= 1 << WH_UNIT, "a full unit has a tile for every warp");
   static_assert(DEPTH >= 2, "a tile is filled while another is used");
   using A = WhRows<TF32, MU>;
   using B = WhRows<TF32, NU>;
   constexpr uint32_t STAGE = A::TILE + B::TILE, ENTRIES = 128;
   constexpr int NT = 2 * NU, SUMS = MU * 4 * NT;  // n-tiles of 8 columns; accumulators per lane
-  constexpr uint32_t RINGS = WARPS * (DEPTH * STAGE + (DEPTH - 1) * ENTRIES), ALL_SUMS = WARPS * SUMS * 128;
+  constexpr uint32_t RINGS = WARPS * (DEPTH * STAGE + (DEPTH - 1) * ENTRIES + (DGRAD ? DEPTH * 64 : 0)), ALL_SUMS = WARPS * SUMS * 128;
   extern __shared__ __align__(128) uint8_t wh_smem[];  // the warps' rings, later [WARPS][SUMS][32] sums; then the tile table
   int* tile_start = reinterpret_cast<int*>(wh_smem + (RINGS > ALL_SUMS ? RINGS : ALL_SUMS));
   int* kpos_s = tile_start + p.k_vol + 2;
@@ -110,7 +171,7 @@ __global__ void __maxnreg__(rw_max_regs(WARPS * 32, true)) rows_wgrad_kernel(Wgr
 
   umma::griddep_begin(0, p.alone);
   const int unit = !TF32 && p.dw_f16 != nullptr ? WH_UNIT : 0;
-  build_tile_table(16 << unit, p.kpos, p.pairs, p.k_vol, 0, kpos_s, tile_start);
+  build_tile_table(16 << unit, p.kpos, p.pairs, p.k_vol, 0, kpos_s, tile_start, DGRAD ? 2 : 1);
   // Units by turns; spread (see Turns) when the rows exceed what L2 holds.
   const int total = tile_start[n_seg], share = (total + gridDim.x - 1) / gridDim.x;
   int t0 = min(total, (int)blockIdx.x * share);
@@ -118,6 +179,8 @@ __global__ void __maxnreg__(rw_max_regs(WARPS * 32, true)) rows_wgrad_kernel(Wgr
 
   const uint32_t ring = umma::smem_u32(wh_smem) + warp * DEPTH * STAGE;
   const uint32_t entries = umma::smem_u32(wh_smem) + WARPS * DEPTH * STAGE + warp * (DEPTH - 1) * ENTRIES + lane * 4;
+  // rows of the input gradient of a slot's pairs, -1: none
+  const uint32_t to_rows = umma::smem_u32(wh_smem) + WARPS * (DEPTH * STAGE + (DEPTH - 1) * ENTRIES) + warp * DEPTH * 64;
   const uint8_t* feats = static_cast<const uint8_t*>(p.feats) + lane % A::LANES * 16;
   const uint8_t* og = static_cast<const uint8_t*>(p.out_grad) + lane % B::LANES * 16;
   // ldmatrix: lanes 0-7, 8-15, 16-23, 24-31 name the rows of the four 8 x 8 matrices
@@ -152,18 +215,26 @@ __global__ void __maxnreg__(rw_max_regs(WARPS * 32, true)) rows_wgrad_kernel(Wgr
       if (j < j_end) umma::cp_async4(slot, map + j);
       else umma::st_shared_i32(slot, -1);
     };
-    auto start = [&](int e, uint32_t slot) {  // the rows of a tile's entries on their way
+    auto start = [&](int e, uint32_t at) {  // the rows of a tile's entries on their way
       const unsigned in = __ballot_sync(0xffffffffu, (unsigned)e < n_rows), ok = in & (in >> 16) & 0xffffu;
+      const uint32_t slot = ring + at;
+      if (DGRAD && lane < 16) umma::st_shared_i32(to_rows + at / STAGE * 64 + lane * 4, (ok >> lane) & 1 ? e : -1);
       if (ok == 0xffffu) {
         A::template copy<true>(slot, feats, e, 0, ok, lane);
         B::template copy<true>(slot + A::TILE, og, e, 16, ok, lane);
       } else {  // the offset's last tile, or entries outside the tensors
         const unsigned there = __ballot_sync(0xffffffffu, e != -1), bad = ((there | there >> 16) & ~ok) & 0xffffu;
-        if ((bad >> lane) & 1) report_problem();  // pair skipped, counted once
+        if ((bad >> lane) & 1) {  // pair skipped, counted once in each pass
+          report_problem();
+          if (DGRAD) report_problem();
+        }
         A::template copy<false>(slot, feats, e, 0, ok, lane);
         B::template copy<false>(slot + A::TILE, og, e, 16, ok, lane);
       }
     };
+    uint32_t wt[DGRAD ? NU : 1][2 * MU][2];  // W_k^T as the B operand
+    if constexpr (DGRAD)
+      if (warp < run) rw_load_b<false, true, NU, MU>(static_cast<const uint8_t*>(dg.weights) + (size_t)seg * p.c_in * p.c_out * 2, p.c_out, lane, wt);
     if (warp < run) {
       // group d of a warp's copies: the rows of its tile d and the entries of its tile d + DEPTH - 1
       int e[DEPTH - 1];
@@ -174,7 +245,7 @@ __global__ void __maxnreg__(rw_max_regs(WARPS * 32, true)) rows_wgrad_kernel(Wgr
       }
 #pragma unroll
       for (int d = 0; d < DEPTH - 1; ++d) {
-        if (warp + d * WARPS < run) start(e[d], ring + d * STAGE);
+        if (warp + d * WARPS < run) start(e[d], d * STAGE);
         fetch_entry(warp + (d + DEPTH - 1) * WARPS, entries + d * ENTRIES);
         umma::cp_async_commit();
       }
@@ -185,7 +256,7 @@ __global__ void __maxnreg__(rw_max_regs(WARPS * 32, true)) rows_wgrad_kernel(Wgr
         __syncwarp();  // the tile has landed for every lane, and every lane is done with the slot that is filled next
         auto next_tile = [&]() {
           if (n + (DEPTH - 1) * WARPS < run) {
-            start(umma::ld_shared_i32(entries + ent), ring + put);
+            start(umma::ld_shared_i32(entries + ent), put);
             fetch_entry(n + 2 * (DEPTH - 1) * WARPS, entries + ent);
             ent = ent == (DEPTH - 2) * ENTRIES ? 0 : ent + ENTRIES;
             put = put == (DEPTH - 1) * STAGE ? 0 : put + STAGE;
@@ -224,6 +295,7 @@ __global__ void __maxnreg__(rw_max_regs(WARPS * 32, true)) rows_wgrad_kernel(Wgr
           for (int u = 0; u < MU; ++u)
 #pragma unroll
             for (int j = 0; j < NT; ++j) rw_mma(acc[u][j], a[u], b[j / 2][2 * (j & 1)], b[j / 2][2 * (j & 1) + 1], false);
+          if constexpr (DGRAD) wh_dgrad<MU, NU>(ring + get + A::TILE, to_rows + get / STAGE * 64, lane, wt, dg.in_grad);
         }
         get = get == (DEPTH - 1) * STAGE ? 0 : get + STAGE;
       }
@@ -289,13 +361,13 @@ __global__ void __maxnreg__(rw_max_regs(WARPS * 32, true)) rows_wgrad_kernel(Wgr
 // ---------------------------------------------------------------------------------------------
 // Warps of the block: as many as the registers allow (sums, operands, about fifty for the rest), 16 at most; the ring as
 // long as shared memory allows, with room for a block of the exchange beside it.
-constexpr int wh_warps(bool tf32, int mu, int nu) {
-  const int regs = 8 * mu * nu + 4 * (mu + nu) + (tf32 ? 56 : 48), fit = 61440 / (32 * ((regs + 7) / 8 * 8)) / 4 * 4;
+constexpr int wh_warps(bool tf32, int mu, int nu, bool dgrad = false) {
+  const int regs = 8 * mu * nu + 4 * (mu + nu) + (tf32 ? 56 : 48) + (dgrad ? 4 * mu * nu + 4 * nu + 24 : 0), fit = 61440 / (32 * ((regs + 7) / 8 * 8)) / 4 * 4;
   return fit > 16 ? 16 : fit;
 }
-constexpr int wh_depth(bool tf32, int mu, int nu) {
+constexpr int wh_depth(bool tf32, int mu, int nu, bool dgrad = false) {
   const int stage = tf32 ? 1024 * (mu + nu + 1) : 512 * (mu + nu) + (mu == 3 ? 256 : 0) + (nu == 3 ? 256 : 0);
-  const int fit = 200 * 1024 / (wh_warps(tf32, mu, nu) * (stage + 128));
+  const int fit = 200 * 1024 / (wh_warps(tf32, mu, nu, dgrad) * (stage + (dgrad ? 192 : 128)));
   return fit > WH_MAX_DEPTH ? WH_MAX_DEPTH : fit;
 }
 // Shapes this kernel takes: multiples of 16 up to 64 channels on both sides, in tf32 not 48 -> 64, 64 -> 48 and 64 -> 64.
@@ -304,14 +376,21 @@ inline bool wh_supported(int c_in, int c_out, bool f16) {
   return f16 || c_in + c_out < 112;
 }
 
-template <bool TF32, int MU, int NU>
-inline int wh_launch_as(const WgradParams& p, cudaStream_t st, int sms, int max_smem) {
-  if constexpr (TF32 && MU + NU >= 7) {
+// Shapes of the kernel for both gradients: at most eight pairs of 16-channel units, so that W_k^T fits beside the sums in the
+// registers of eight warps or more (64 -> 48 on 591 k pairs with the four that are left 52.6 us, 42.2 by two kernels; with the weights
+// in shared memory 64 -> 64 67.7 / 61.6).  And the pairs from which clearing and rounding the sums, 2.5 us, are paid for, us by two
+// kernels / this one: 32 -> 64 on 591 k pairs 27.1 / 28.0, on 1.13 M 45.8 / 45.1; 32 -> 32 on 364 k 14.6 / 15.9, on 591 k 19.7 / 20.5.
+constexpr bool wh_both_shape(int mu, int nu) { return mu * nu <= 8; }
+constexpr long long WH_BOTH_PAIRS = 1 << 20;
+
+template <bool TF32, int MU, int NU, bool DGRAD>
+inline int wh_launch_as(const WgradParams& p, const RowsDgrad& dg, cudaStream_t st, int sms, int max_smem) {
+  if constexpr ((TF32 && MU + NU >= 7) || (DGRAD && !wh_both_shape(MU, NU))) {
     return 1;
   } else {
-    constexpr int WARPS = wh_warps(TF32, MU, NU), DEPTH = wh_depth(TF32, MU, NU);
-    auto kernel = rows_wgrad_kernel<TF32, MU, NU, WARPS, DEPTH>;
-    constexpr size_t rings = (size_t)WARPS * (DEPTH * (WhRows<TF32, MU>::TILE + WhRows<TF32, NU>::TILE) + (DEPTH - 1) * 128);
+    constexpr int WARPS = wh_warps(TF32, MU, NU, DGRAD), DEPTH = wh_depth(TF32, MU, NU, DGRAD);
+    auto kernel = rows_wgrad_kernel<TF32, MU, NU, WARPS, DEPTH, DGRAD>;
+    constexpr size_t rings = (size_t)WARPS * (DEPTH * (WhRows<TF32, MU>::TILE + WhRows<TF32, NU>::TILE) + (DEPTH - 1) * 128 + (DGRAD ? DEPTH * 64 : 0));
     constexpr size_t sums = (size_t)WARPS * MU * 8 * NU * 128;
     const size_t smem = (rings > sums ? rings : sums) + (size_t)(2 * p.k_vol + 3) * sizeof(int);
     if (smem > (size_t)max_smem) return 1;
@@ -329,26 +408,26 @@ inline int wh_launch_as(const WgradParams& p, cudaStream_t st, int sms, int max_
     }
     const long long units = (long long)p.pairs / (!TF32 && p.dw_f16 != nullptr ? 16 << WH_UNIT : 16) + p.k_vol + 1;
     const bool spread = spread_tiles((size_t)p.n_in * WhRows<TF32, MU>::BYTES + (size_t)p.n_out * WhRows<TF32, NU>::BYTES);
-    return launch_pdl(kernel, (int)(units < sms ? units : sms), WARPS * 32, smem, st, p, spread) == cudaSuccess ? 0 : -1;
+    return launch_pdl(kernel, (int)(units < sms ? units : sms), WARPS * 32, smem, st, p, spread, dg) == cudaSuccess ? 0 : -1;
   }
 }
-template <bool TF32, int MU>
-inline int wh_launch_n(const WgradParams& p, cudaStream_t st, int sms, int max_smem) {
+template <bool TF32, int MU, bool DGRAD>
+inline int wh_launch_n(const WgradParams& p, const RowsDgrad& dg, cudaStream_t st, int sms, int max_smem) {
   switch (p.c_out / 16) {
-    case 1: return wh_launch_as<TF32, MU, 1>(p, st, sms, max_smem);
-    case 2: return wh_launch_as<TF32, MU, 2>(p, st, sms, max_smem);
-    case 3: return wh_launch_as<TF32, MU, 3>(p, st, sms, max_smem);
-    case 4: return wh_launch_as<TF32, MU, 4>(p, st, sms, max_smem);
+    case 1: return wh_launch_as<TF32, MU, 1, DGRAD>(p, dg, st, sms, max_smem);
+    case 2: return wh_launch_as<TF32, MU, 2, DGRAD>(p, dg, st, sms, max_smem);
+    case 3: return wh_launch_as<TF32, MU, 3, DGRAD>(p, dg, st, sms, max_smem);
+    case 4: return wh_launch_as<TF32, MU, 4, DGRAD>(p, dg, st, sms, max_smem);
   }
   return 1;
 }
-template <bool TF32>
-inline int wh_launch(const WgradParams& p, cudaStream_t st, int sms, int max_smem) {
+template <bool TF32, bool DGRAD = false>
+inline int wh_launch(const WgradParams& p, const RowsDgrad& dg, cudaStream_t st, int sms, int max_smem) {
   switch (p.c_in / 16) {
-    case 1: return wh_launch_n<TF32, 1>(p, st, sms, max_smem);
-    case 2: return wh_launch_n<TF32, 2>(p, st, sms, max_smem);
-    case 3: return wh_launch_n<TF32, 3>(p, st, sms, max_smem);
-    case 4: return wh_launch_n<TF32, 4>(p, st, sms, max_smem);
+    case 1: return wh_launch_n<TF32, 1, DGRAD>(p, dg, st, sms, max_smem);
+    case 2: return wh_launch_n<TF32, 2, DGRAD>(p, dg, st, sms, max_smem);
+    case 3: return wh_launch_n<TF32, 3, DGRAD>(p, dg, st, sms, max_smem);
+    case 4: return wh_launch_n<TF32, 4, DGRAD>(p, dg, st, sms, max_smem);
   }
   return 1;
 }
@@ -359,7 +438,18 @@ inline int launch_rows_wgrad(const WgradParams& p, bool f16, cudaStream_t st, in
   if ((long long)p.pairs > 0x7fffffffll - 65536) return 1;  // positions a few turns past the end stay in an int
   if ((reinterpret_cast<uintptr_t>(p.feats) | reinterpret_cast<uintptr_t>(p.out_grad) | reinterpret_cast<uintptr_t>(p.dw) |
        reinterpret_cast<uintptr_t>(p.dw_f16)) & 15) return 1;
-  return f16 ? wh_launch<false>(p, st, sms, max_smem) : wh_launch<true>(p, st, sms, max_smem);
+  return f16 ? wh_launch<false>(p, RowsDgrad(), st, sms, max_smem) : wh_launch<true>(p, RowsDgrad(), st, sms, max_smem);
+}
+// Whether one kernel takes both gradients of fp16 rows, the weight gradient's sums in fp32; the buffers are distinct.
+inline bool rows_bwd_supported(int c_in, int c_out) { return wh_supported(c_in, c_out, true) && wh_both_shape(c_in / 16, c_out / 16); }
+inline bool rows_bwd_takes(const WgradParams& p, const RowsDgrad& dg, int max_smem) {
+  return rows_bwd_supported(p.c_in, p.c_out) && (long long)p.pairs <= 0x7fffffffll - 65536 &&
+         ((reinterpret_cast<uintptr_t>(p.feats) | reinterpret_cast<uintptr_t>(p.out_grad) | reinterpret_cast<uintptr_t>(p.dw) |
+           reinterpret_cast<uintptr_t>(dg.weights) | reinterpret_cast<uintptr_t>(dg.in_grad)) & 15) == 0 &&
+         216 * 1024 + (size_t)(2 * p.k_vol + 3) * sizeof(int) <= (size_t)max_smem;
+}
+inline int launch_rows_bwd(const WgradParams& p, const RowsDgrad& dg, cudaStream_t st, int sms, int max_smem) {
+  return wh_launch<false, true>(p, dg, st, sms, max_smem);
 }
 
 }  // namespace fgms

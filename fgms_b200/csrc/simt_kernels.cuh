@@ -340,7 +340,9 @@ __global__ void __launch_bounds__(SIMT_THREADS) simt_wgrad_kernel(WgradParams p)
 }
 
 // kernel_grad(fp16) += workspace(fp32)
-__global__ void wgrad_finalize_kernel(__half* __restrict__ kg, const float* __restrict__ ws, long long count) {
+__global__ void wgrad_finalize_kernel(__half* kg, const float* ws, long long count) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the sums are those of the kernel before
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
        i += (long long)gridDim.x * blockDim.x) {
     kg[i] = __float2half_rn(__half2float(kg[i]) + ws[i]);

@@ -136,6 +136,9 @@ int fgms_b200_wgrad_finalize(void* kernel_grad_f16, const void* workspace_f32, i
 
 size_t fgms_b200_wgrad_workspace_bytes(int c_in, int c_out, int k_vol, int dtype);
 
+/* Bytes of a workspace with which fgms_b200_bwd is faster than without one; 0 where it is not, or needs one all the same (above). */
+size_t fgms_b200_bwd_workspace_bytes(int64_t map_len, int c_in, int c_out, int k_vol, int dtype, int math);
+
 /* Weight gradient for fp16 storage that allocates nothing and needs no caller workspace.
  * This entry point has no counterpart in the reference.  It exists for callers that cannot
  * obtain device memory at the time of the call: code running under a memory pool that is already
@@ -161,7 +164,9 @@ int fgms_b200_wgrad_f16_noalloc(const void* in_feats, const void* out_grad, void
 /* Both gradients.  Replaces ConvolutionBackward (backend/spconv.cu:414-571; Python name
  * fgms_bwd_cuda).  separate_mid is accepted and ignored, as in the reference.  The two kernels run side by
  * side on `stream`, each on a share of the SMs where that is faster; whatever is enqueued next waits for both.
- * With a workspace for fp16 sums, buffers that overlap or SMs to leave free (fgms_b200_set_reserved_sms), one runs behind the
+ * Given the workspace that fgms_b200_bwd_workspace_bytes asks for (short fp16 rows, many pairs), one kernel computes both, with fp32
+ * sums of the weight gradient in the workspace that are then added to kernel_grad.
+ * With any other workspace for fp16 sums, buffers that overlap or SMs to leave free (fgms_b200_set_reserved_sms), one runs behind the
  * other, the input gradient first. */
 int fgms_b200_bwd(const void* out_grad, const void* in_feats, const void* kernel, void* in_grad,
                   void* kernel_grad, const int32_t* kpos, const int32_t* qkpos,
