@@ -118,9 +118,8 @@ class SparseUNet(torch.nn.Module):
             w, km = layer._parameters.get("weight"), umaps.of(spec)
             if type(w) is not torch.nn.Parameter or spec.src not in value or (spec.skip is not None and spec.skip not in value):
                 return None
-            m = seen.get(id(km))
-            if m is None:
-                m = seen[id(km)] = len(seen)
+            m, _ = seen.setdefault(id(km), (len(seen), km))  # with the map itself: an id is one object's for as long as it lives
+            if 3 * m == len(maps):
                 maps += km.kpos, km.imap, km.omap
             plan += value[spec.src], -1 if spec.skip is None else value[spec.skip], m, km.n_in, km.n_out
             weights.append(w)
