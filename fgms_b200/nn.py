@@ -70,24 +70,29 @@ _MODULE = torch.nn.modules.module
 _HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
 
 
+def _watched() -> bool:
+    """Whether something beyond the layers themselves sees or transforms their calls.  PyTorch answers most of this under private names
+    only: a release that lacks one counts as watching.  Several ranks count too, because gradients that leave with their layer are
+    exchanged beside the rest of the backward."""
+    try:
+        return (torch._C._get_tracing_state() is not None or torch.compiler.is_compiling() or torch.autograd.forward_ad._current_level >= 0
+                or torch._C._functorch.peek_interpreter_stack() is not None
+                or torch._C._autograd._top_saved_tensors_default_hooks(True) is not None
+                or torch._C._len_torch_dispatch_stack() > 0 or torch._C._len_torch_function_stack() > 0
+                or (torch.distributed.is_available() and torch.distributed.is_initialized())
+                or bool(_MODULE._global_forward_hooks or _MODULE._global_forward_pre_hooks
+                        or _MODULE._global_backward_hooks or _MODULE._global_backward_pre_hooks))
+    except AttributeError:
+        return True
+
+
 def _one_node(layers) -> bool:
-    """Whether a stack may run as one autograd node: nothing sees the calls of its layers.  Several ranks run layer by layer, because
-    gradients that leave with their layer are exchanged beside the rest of the backward."""
-    if torch._C._get_tracing_state() is not None or torch.compiler.is_compiling() or torch.autograd.forward_ad._current_level >= 0:
-        return False
-    if torch._C._functorch.peek_interpreter_stack() is not None or torch._C._autograd._top_saved_tensors_default_hooks(True) is not None:
-        return False
-    if torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack():
-        return False
-    if torch.distributed.is_available() and torch.distributed.is_initialized():
-        return False
-    if _MODULE._global_forward_hooks or _MODULE._global_forward_pre_hooks or _MODULE._global_backward_hooks or _MODULE._global_backward_pre_hooks:
-        return False
-    if SparseConv3d.forward is not _LAYER_FORWARD or SparseConv3d.__call__ is not torch.nn.Module.__call__:
+    """Whether a stack may run as one autograd node: nothing sees the calls of its layers."""
+    if _watched() or SparseConv3d.forward is not _LAYER_FORWARD or SparseConv3d.__call__ is not torch.nn.Module.__call__:
         return False
     for layer in layers:
         d = layer.__dict__
-        if type(layer) is not SparseConv3d or "forward" in d or d["arch80"] != layers[0].__dict__["arch80"] or any(d[h] for h in _HOOKS):
+        if type(layer) is not SparseConv3d or "forward" in d or d["arch80"] != layers[0].__dict__["arch80"] or any(d.get(h, True) for h in _HOOKS):
             return False
     return True
 

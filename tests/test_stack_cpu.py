@@ -34,3 +34,15 @@ def test_every_layer_gets_its_own_map(handed):
     for i, layer in enumerate(SPEC):
         want, (m, n_in, n_out) = maps.of(layer), plan[5 * i + 2: 5 * i + 5]
         assert [int(t) for t in tensors[3 * m: 3 * m + 3]] == [want.n_in] * 3 and (n_in, n_out) == (want.n_in, want.n_out)
+
+
+@pytest.mark.parametrize("owner,name", [(torch._C, "_get_tracing_state"), (torch.autograd.forward_ad, "_current_level"),
+                                        (torch._C._functorch, "peek_interpreter_stack"), (torch._C._autograd, "_top_saved_tensors_default_hooks"),
+                                        (torch._C, "_len_torch_function_stack"), (torch.nn.modules.module, "_global_forward_hooks")])
+def test_a_release_without_a_private_name_runs_layer_by_layer(handed, monkeypatch, owner, name):
+    net, feats = nn.SparseUNet(SPEC, device="cpu"), torch.zeros((2, 4), dtype=torch.float16)
+    with monkeypatch.context() as m:
+        m.delattr(owner, name)
+        one = net._forward_as_one(feats, _MapsPerCall())
+    assert one is None and not handed
+    assert net._forward_as_one(feats, _MapsPerCall()) is feats
