@@ -113,7 +113,7 @@ Tensor wgrad_workspace(const Tensor& kernel_grad, const Arith& a, bool fp32_sums
 }
 
 // The same for both gradients in one call: also where the library is faster with one.  A call whose pointers are not 16-byte aligned
-// gets none, as it has another way without.
+// gets none, nor one for which there is no memory, as it has another way without.
 Tensor bwd_workspace(const void* grad_out, const void* feats, const void* kernel, const void* in_grad, const Tensor& kernel_grad, int64_t pairs,
                      const Arith& a, bool fp32_sums) {
   if (const Tensor ws = wgrad_workspace(kernel_grad, a, fp32_sums); ws.defined() || a.dtype != FGMS_DTYPE_F16) return ws;
@@ -122,7 +122,11 @@ Tensor bwd_workspace(const void* grad_out, const void* feats, const void* kernel
   uintptr_t at = 0;
   for (const void* p : {grad_out, feats, kernel, in_grad, (const void*)kernel_grad.data_ptr()}) at |= reinterpret_cast<uintptr_t>(p);
   if (bytes == 0 || (at & 15) != 0) return {};
-  return at::empty({(int64_t)(bytes / 4)}, kernel_grad.options().dtype(at::kFloat));
+  try {
+    return at::empty({(int64_t)(bytes / 4)}, kernel_grad.options().dtype(at::kFloat));
+  } catch (const c10::OutOfMemoryError&) {
+    return {};
+  }
 }
 
 void bwd(const Tensor& grad_out, const Tensor& in_feats, const Tensor& kernel, int64_t sum_nnz, const Tensor& in_grad,

@@ -63,3 +63,25 @@ def test_weights_off_their_alignment_keep_two_kernels():
     shifted = torch.zeros(p.weights.numel() + 8, dtype=torch.float16, device="cuda")[1: 1 + p.weights.numel()].view_as(p.weights)
     p.weights = shifted.copy_(p.weights)
     _check(p, 2)
+
+
+def test_without_memory_for_the_sums_two_kernels_run():
+    p = _problem(32, 32, LEAST)
+    dx, dw = torch.zeros_like(p.feats), torch.zeros_like(p.weights)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held = []
+    try:  # nothing beyond what is reserved, and of that nothing that 64 KB fit in
+        torch.cuda.set_per_process_memory_fraction(torch.cuda.memory_reserved() / torch.cuda.get_device_properties(0).total_memory)
+        with pytest.raises(torch.OutOfMemoryError):
+            while True:
+                held.append(torch.empty(1 << 16, dtype=torch.uint8, device="cuda"))
+        before = backend.launch_count()
+        backend.fgms_bwd_cuda(p.grad_out, p.feats, p.weights, p.qsum, dx, dw, p.kpos, p.qkpos, p.imap, p.omap, False, p.arch80)
+    finally:
+        held.clear()
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert backend.launch_count() - before == 2
+    want = torch.zeros_like(p.feats)
+    backend.fgms_dgrad_cuda(p.grad_out, p.weights, want, p.kpos, p.imap, p.omap, p.arch80)
+    assert torch.equal(dx, want) and float(dw.abs().max()) > 0
