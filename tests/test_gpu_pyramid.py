@@ -54,3 +54,13 @@ def test_memory_left_behind_by_an_earlier_cloud_does_not_matter():
     for seed in range(4):
         coords = clouds.uniform_cloud(3000 + 700 * seed, 30, seed)
         _check(unet.build_unet_maps(_dev(coords), 2), unet.build_unet_maps_host(coords, 2))
+
+
+def test_every_map_has_memory_of_its_own():
+    """A map that is kept does not keep the others, and an edit of one is no edit of what a backward has saved of another."""
+    m = unet.build_unet_maps(_dev(np.unique(clouds.surface_cloud(5000, 64, 9), axis=0)), 2)
+    maps = m.subm + m.down + m.up
+    assert len({k.imap.untyped_storage().data_ptr() for k in maps}) == len(maps)
+    before = [k.imap._version for k in maps]
+    maps[0].imap[:1] = maps[0].imap[:1].clone()
+    assert [k.imap._version for k in maps[1:]] == before[1:]
