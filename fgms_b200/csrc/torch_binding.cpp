@@ -16,6 +16,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/graph_task.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <pybind11/pybind11.h>
 
@@ -227,10 +228,17 @@ struct SparseConv : torch::autograd::Function<SparseConv> {
 // allocation, their gradients in another, each cleared by one launch, and the backward is a loop.  The arithmetic is the one of
 // a node per layer: every layer adds into zeros, a skip connection and its gradient are sums rounded once.
 //
+// A node per layer needs less memory: it hands back its input and its output's gradient as the backward goes on.  So beyond STACK_BYTES
+// of values, and where there is no memory for one allocation, values and gradients are allocated and cleared one by one and dropped in the
+// same way.  Training steps of the 25 layers, peaks above what is there before: 120 k voxels, 59 MB of values, a node per layer 66 MB, two
+// allocations 123; 240 k voxels, 113 MB, 129 MB a node per layer and one by one, 231 in two allocations.  By then the device is
+// busy for longer than the further allocations and launches take the host: 1970 us a node per layer, 1080-1150 one by one, 965 in two.
+//
 // Value 0 is the input, value l + 1 what layer l produces.
 struct StackLayer { int64_t src, skip /* -1: none */, map, n_in, n_out; };
 using StackPlan = std::vector<int64_t>;  // StackLayer by StackLayer
 constexpr int64_t STACK_FIELDS = 5;
+constexpr int64_t STACK_BYTES = 64 << 20;
 StackLayer layer_of(const StackPlan& plan, size_t l) {
   const int64_t* f = plan.data() + l * STACK_FIELDS;
   return {f[0], f[1], f[2], f[3], f[4]};
@@ -273,34 +281,68 @@ bool stack_suits(const Tensor& feats, at::TensorList weights, at::TensorList map
 }
 
 struct SparseStack : torch::autograd::Function<SparseStack> {
-  // Where things lie in the buffer of the values, in elements, each from a 256-byte boundary: the values that layers 0 .. n - 2 produce
-  // and, where the input's few fp16 channels are padded to a multiple of 16 (8-byte rows cannot be gathered in 16-byte pieces and
-  // would run on the CUDA cores: 4 -> 32 on 84 k pairs 16 / 42 us forward / weight gradient, padded 4.5 / 5), the padded
-  // input and the weights that go with it.
+  // What the node keeps, in elements: the values that layers 0 .. n - 2 produce (slots 1 .. n - 1) and, where the input's few fp16
+  // channels are padded to a multiple of 16 (8-byte rows cannot be gathered in 16-byte pieces and would run on the CUDA cores: 4 -> 32
+  // on 84 k pairs 16 / 42 us forward / weight gradient, padded 4.5 / 5), the padded input (slot 0) and the weights that go with it (slot n).
   struct Layout {
-    std::vector<int64_t> at;  // of value v, from 1 on
-    int64_t input = 0, weights = 0, end = 0;
-    int64_t pad = 0;          // channels of the padded input, 0: as it is
+    std::vector<int64_t> count, at;  // of a slot; its place in a block of all of them, from a 256-byte boundary
+    int64_t end = 0;                 // of that block
+    int64_t pad = 0;                 // channels of the padded input, 0: as it is
     template <typename Kept>
     Layout(const Tensor& feats, at::TensorList kernels, const StackPlan& plan, bool padding, Kept kept) {
-      auto take = [&](int64_t count) { const int64_t from = end; end += (count + 127) / 128 * 128; return from; };
       const size_t n = kernels.size();
-      at.push_back(0);
-      for (size_t l = 0; l + 1 < n; ++l) at.push_back(kept(l + 1) ? take(layer_of(plan, l).n_out * kernels[l].size(2)) : 0);
-      at.push_back(0);
-      if (!padding || feats.scalar_type() != at::kHalf || feats.size(1) % 16 == 0 || feats.size(1) > 256) return;
+      count.resize(n + 1);
+      at.resize(n + 1);
+      for (size_t l = 0; l + 1 < n; ++l)
+        if (kept(l + 1)) count[l + 1] = layer_of(plan, l).n_out * kernels[l].size(2);
       const Tensor* reader = nullptr;  // the layer of the input
-      for (size_t l = 0; l < n; ++l) {
-        if (layer_of(plan, l).skip == 0) return;
+      padding = padding && feats.scalar_type() == at::kHalf && feats.size(1) % 16 != 0 && feats.size(1) <= 256;
+      for (size_t l = 0; padding && l < n; ++l) {
+        padding = layer_of(plan, l).skip != 0;
         if (layer_of(plan, l).src == 0) reader = &kernels[l];
       }
-      if (!reader || reader->size(2) % 16 != 0 || reader->size(2) > 256) return;
-      pad = (feats.size(1) + 15) / 16 * 16;
-      input = take(feats.size(0) * pad);
-      weights = take(reader->size(0) * pad * reader->size(2));
+      if (padding && reader && reader->size(2) % 16 == 0 && reader->size(2) <= 256) {
+        pad = (feats.size(1) + 15) / 16 * 16;
+        count[0] = feats.size(0) * pad;
+        count[n] = reader->size(0) * pad * reader->size(2);
+      }
+      for (size_t i = 0; i <= n; ++i) {
+        at[i] = end;
+        end += (count[i] + 127) / 128 * 128;
+      }
     }
   };
-  static uint8_t* element(const Tensor& t, int64_t i) { return static_cast<uint8_t*>(t.data_ptr()) + i * t.element_size(); }
+  // The slots of a layout: in one block, or by themselves (each until it is dropped).
+  struct Slots {
+    const Layout& layout;
+    at::TensorOptions options;
+    Tensor block;
+    std::vector<Tensor> own;
+    Slots(const Layout& l, const Tensor& like) : layout(l), options(like.options().requires_grad(false)) {}
+    bool apart() const { return !own.empty(); }
+    // a block where there is memory for one and `may` says so
+    void take(bool may) {
+      if (may) {
+        try {
+          block = at::empty({layout.end}, options);
+          return;
+        } catch (const c10::OutOfMemoryError&) {
+        }
+      }
+      own.resize(layout.count.size());
+    }
+    const Tensor& make(size_t i) { return own[i] = at::empty({layout.count[i]}, options); }
+    void drop(size_t i) { if (apart()) own[i].reset(); }
+    void* of(size_t i) const {
+      return apart() ? own[i].data_ptr() : static_cast<uint8_t*>(block.data_ptr()) + layout.at[i] * block.element_size();
+    }
+  };
+  // the input and its layer's weights with further channels of zeros, into cleared slots
+  static void pad_input(const Slots& slots, const Tensor& feats, const Tensor& w, int dtype, void* st) {
+    const int64_t pad = slots.layout.pad, c_in = feats.size(1);
+    check_status(fgms_b200_copy_rows_f16(ptr(feats), c_in, dtype, slots.of(0), pad, feats.size(0), (int)c_in, st));
+    check_status(fgms_b200_copy_rows_f16(ptr(w), c_in * w.size(2), dtype, slots.of(slots.layout.at.size() - 1), pad * w.size(2), w.size(0), (int)(c_in * w.size(2)), st));
+  }
 
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& feats, at::TensorList weights, at::TensorList maps,
                         const StackPlan& plan, bool arch80) {
@@ -309,36 +351,47 @@ struct SparseStack : torch::autograd::Function<SparseStack> {
     void* st = stream_of(feats);
     const Arith a = arith(feats, arch80);
     const Layout in(feats, weights, plan, true, [](size_t) { return true; });
-    const auto options = feats.options().requires_grad(false);
-    const Tensor values = at::empty({in.end}, options);
-    Tensor out = at::empty({layer_of(plan, n - 1).n_out, weights[n - 1].size(2)}, options);
-    check_status(fgms_b200_zero2(ptr(values), bytes_of(values), ptr(out), bytes_of(out), st));
-    auto value = [&](int64_t v) -> void* {
-      if (v == 0) return in.pad ? element(values, in.input) : feats.data_ptr();
-      return v == (int64_t)n ? out.data_ptr() : element(values, in.at[v]);
+    Slots values(in, feats);
+    values.take(in.end * (int64_t)feats.element_size() <= STACK_BYTES);
+    Tensor out = at::empty({layer_of(plan, n - 1).n_out, weights[n - 1].size(2)}, values.options);
+    auto cleared = [&](const Tensor& t) { check_status(fgms_b200_zero2(ptr(t), bytes_of(t), nullptr, 0, st)); };
+    if (values.apart()) cleared(out);
+    else check_status(fgms_b200_zero2(ptr(values.block), bytes_of(values.block), ptr(out), bytes_of(out), st));
+    auto make = [&](size_t i) {
+      if (values.apart()) cleared(values.make(i));
     };
-    if (in.pad) check_status(fgms_b200_copy_rows_f16(ptr(feats), feats.size(1), a.dtype, value(0), in.pad, feats.size(0), (int)feats.size(1), st));
+    auto value = [&](int64_t v) -> void* {
+      if (v == 0) return in.pad ? values.of(0) : feats.data_ptr();
+      return v == (int64_t)n ? out.data_ptr() : values.of(v);
+    };
     for (size_t l = 0; l < n; ++l) {
       const StackLayer s = layer_of(plan, l);
       const Tensor &w = weights[l], &imap = maps[3 * s.map + 1];
-      const void* kernel = ptr(w);
-      int c_in = (int)w.size(1);
-      if (s.src == 0 && in.pad) {
-        kernel = element(values, in.weights);
-        check_status(fgms_b200_copy_rows_f16(ptr(w), c_in * w.size(2), a.dtype, element(values, in.weights), in.pad * w.size(2), w.size(0), c_in * (int)w.size(2), st));
-        c_in = (int)in.pad;
+      const bool padded = s.src == 0 && in.pad;
+      if (padded) {
+        make(0);
+        make(n);
+        pad_input(values, feats, w, a.dtype, st);
       }
-      check_status(fgms_b200_fusion_fwd(value(s.src), kernel, value(l + 1), iptr(maps[3 * s.map]), nullptr, iptr(imap), iptr(maps[3 * s.map + 2]),
-                                        imap.numel(), (int)s.n_in, (int)s.n_out, c_in, c_in, (int)w.size(2), (int)w.size(0), 0, a.dtype, a.math, 0, st));
+      if (l + 1 < n) make(l + 1);
+      const int c_in = padded ? (int)in.pad : (int)w.size(1);
+      check_status(fgms_b200_fusion_fwd(value(s.src), padded ? values.of(n) : ptr(w), value(l + 1), iptr(maps[3 * s.map]), nullptr, iptr(imap),
+                                        iptr(maps[3 * s.map + 2]), imap.numel(), (int)s.n_in, (int)s.n_out, c_in, c_in, (int)w.size(2), (int)w.size(0), 0,
+                                        a.dtype, a.math, 0, st));
       if (s.skip >= 0) check_status(fgms_b200_add(value(l + 1), value(s.skip), s.n_out * w.size(2), a.dtype, st));
+      if (padded) {  // made again for the backward
+        values.drop(0);
+        values.drop(n);
+      }
     }
     torch::autograd::variable_list saved;
     saved.reserve(2 + n + maps.size());
     saved.push_back(feats);
-    saved.push_back(values);
+    saved.push_back(values.block);
     saved.insert(saved.end(), weights.begin(), weights.end());
     saved.insert(saved.end(), maps.begin(), maps.end());
     ctx->save_for_backward(std::move(saved));
+    if (values.apart()) ctx->saved_data["values"] = values.own;
     ctx->saved_data["plan"] = plan;
     ctx->saved_data["arch80"] = arch80;
     return out;
@@ -349,7 +402,7 @@ struct SparseStack : torch::autograd::Function<SparseStack> {
     const StackPlan plan = ctx->saved_data["plan"].toIntVector();
     const bool arch80 = ctx->saved_data["arch80"].toBool();
     const size_t n = plan.size() / STACK_FIELDS;
-    const Tensor &feats = saved[0], &values = saved[1];
+    const Tensor& feats = saved[0];
     const at::TensorList weights(saved.data() + 2, n), maps(saved.data() + 2 + n, saved.size() - 2 - n);
     TORCH_CHECK_VALUE(stack_suits(feats, weights, maps, plan, arch80), "saved tensors of the stack are not the ones it was run with");
     Tensor grad_out = grads[0].contiguous();
@@ -361,8 +414,17 @@ struct SparseStack : torch::autograd::Function<SparseStack> {
     TORCH_CHECK_VALUE(grad_out.size(0) == layer_of(plan, n - 1).n_out && grad_out.size(1) == weights[n - 1].size(2),
                       "out_feats_grad has another shape than the output");
     const Layout in(feats, weights, plan, true, [](size_t) { return true; });
-    TORCH_CHECK_VALUE(values.scalar_type() == feats.scalar_type() && values.device() == feats.device() && values.is_contiguous() && values.numel() == in.end &&
-                      (reinterpret_cast<uintptr_t>(values.data_ptr()) & 15) == 0, "saved values of the stack are not the ones it was run with");
+    Slots values(in, feats);
+    values.block = saved[1];
+    if (const auto kept = ctx->saved_data.find("values"); kept != ctx->saved_data.end()) {
+      // the last backward hands them back on the way
+      values.own = kept->second.toTensorVector();
+      if (!torch::autograd::get_current_graph_task_keep_graph()) ctx->saved_data.erase(kept);
+    } else {
+      const Tensor& block = values.block;
+      TORCH_CHECK_VALUE(block.defined() && block.scalar_type() == feats.scalar_type() && block.device() == feats.device() && block.is_contiguous() &&
+                        block.numel() == in.end && (reinterpret_cast<uintptr_t>(block.data_ptr()) & 15) == 0, "saved values of the stack are not the ones it was run with");
+    }
     // gradients that something needs: a value's, if a weight before it or the input needs one
     std::vector<char> need(n + 1, 0), need_w(n);
     need[0] = ctx->needs_input_grad(0);
@@ -373,38 +435,52 @@ struct SparseStack : torch::autograd::Function<SparseStack> {
     }
     const Layout out(feats, weights, plan, false, [&](size_t v) { return need[v] != 0; });
     torch::autograd::variable_list result(1 + n + maps.size() + 2);
-    const Tensor g_values = at::empty({out.end}, feats.options().requires_grad(false));
-    std::vector<void*> clear;
-    std::vector<size_t> bytes;
-    auto cleared = [&](const Tensor& t) { clear.push_back(ptr(t)); bytes.push_back(bytes_of(t)); };
-    cleared(g_values);
+    Slots g_values(out, feats);
+    g_values.take(!values.apart());
     Tensor g_input;
-    if (need[0]) cleared(g_input = at::empty({feats.size(0), in.pad ? in.pad : feats.size(1)}, feats.options().requires_grad(false)));
-    for (size_t l = 0; l < n; ++l)
-      if (need_w[l]) cleared(result[1 + l] = at::empty_like(weights[l]));
-    check_status(fgms_b200_zero_list(clear.data(), bytes.data(), (int)clear.size(), st));
-    auto value = [&](int64_t v) -> void* {
-      if (v == 0) return in.pad ? element(values, in.input) : feats.data_ptr();
-      return element(values, in.at[v]);
-    };
+    auto make_g_input = [&] { return at::empty({feats.size(0), in.pad ? in.pad : feats.size(1)}, values.options); };
+    if (!g_values.apart()) {  // otherwise each when it is first used
+      std::vector<void*> clear;
+      std::vector<size_t> bytes;
+      auto add = [&](const Tensor& t) { clear.push_back(ptr(t)); bytes.push_back(bytes_of(t)); };
+      add(g_values.block);
+      if (need[0]) add(g_input = make_g_input());
+      for (size_t l = 0; l < n; ++l)
+        if (need_w[l]) add(result[1 + l] = at::empty_like(weights[l]));
+      check_status(fgms_b200_zero_list(clear.data(), bytes.data(), (int)clear.size(), st));
+    }
+    auto cleared = [&](const Tensor& t) { check_status(fgms_b200_zero2(ptr(t), bytes_of(t), nullptr, 0, st)); };
+    auto value = [&](int64_t v) -> void* { return v == 0 && !in.pad ? feats.data_ptr() : values.of(v); };
     auto grad = [&](int64_t v) -> void* {
-      return v == 0 ? g_input.data_ptr() : v == (int64_t)n ? grad_out.data_ptr() : element(g_values, out.at[v]);
+      if (v == (int64_t)n) return grad_out.data_ptr();
+      if (v == 0) {
+        if (!g_input.defined()) cleared(g_input = make_g_input());
+        return g_input.data_ptr();
+      }
+      if (g_values.apart() && !g_values.own[v].defined()) cleared(g_values.make(v));
+      return g_values.of(v);
     };
     std::vector<std::vector<int64_t>> added(n + 1);  // values whose gradient is part of a value's, through a skip connection
     auto finish = [&](int64_t v, int64_t count) {    // its layer's input gradient is in it
-      for (int64_t from : added[v]) check_status(fgms_b200_add(grad(v), grad(from), count, a.dtype, st));
+      for (int64_t from : added[v]) {
+        check_status(fgms_b200_add(grad(v), grad(from), count, a.dtype, st));
+        if (from < (int64_t)n) g_values.drop(from);
+      }
     };
     const bool fp32_sums = g_fp32_sums.load(std::memory_order_relaxed);
-    for (size_t l = n; l-- > 0;) {
-      if (!need[l + 1]) continue;
-      const StackLayer s = layer_of(plan, l);
+    // both gradients of a layer
+    auto layer = [&](size_t l, const StackLayer& s) {
       const Tensor &w = weights[l], &imap = maps[3 * s.map + 1];
       const int32_t *kpos = iptr(maps[3 * s.map]), *im = iptr(imap), *om = iptr(maps[3 * s.map + 2]);
       const int c_in = (int)w.size(1), c_out = (int)w.size(2), k_vol = (int)w.size(0), n_in = (int)s.n_in, n_out = (int)s.n_out;
-      if (l + 1 < n) finish(l + 1, s.n_out * c_out);
-      if (s.skip >= 0 && need[s.skip]) added[s.skip].push_back(l + 1);
+      if (need_w[l] && !result[1 + l].defined()) cleared(result[1 + l] = at::empty_like(w));
       if (s.src == 0 && in.pad) {
         const int pad = (int)in.pad;
+        if (values.apart()) {
+          cleared(values.make(0));
+          cleared(values.make(n));
+          pad_input(values, feats, w, a.dtype, st);
+        }
         if (need_w[l]) {  // fp32 sums, of which the rows of the real channels are rounded
           const Tensor sums = at::empty({(int64_t)k_vol * pad * c_out}, w.options().dtype(at::kFloat).requires_grad(false));
           check_status(fgms_b200_wgrad(value(0), grad(l + 1), nullptr, kpos, im, om, imap.numel(), n_in, n_out, pad, c_out, k_vol, a.dtype, a.math,
@@ -412,9 +488,8 @@ struct SparseStack : torch::autograd::Function<SparseStack> {
           check_status(fgms_b200_copy_rows_f16(sums.data_ptr(), pad * c_out, FGMS_DTYPE_F32, result[1 + l].data_ptr(), c_in * c_out, k_vol, c_in * c_out, st));
         }
         if (need[0])
-          check_status(fgms_b200_dgrad(grad(l + 1), element(values, in.weights), grad(0), kpos, im, om, imap.numel(), n_in, n_out, pad, c_out, k_vol,
-                                       a.dtype, a.math, st));
-        continue;
+          check_status(fgms_b200_dgrad(grad(l + 1), values.of(n), grad(0), kpos, im, om, imap.numel(), n_in, n_out, pad, c_out, k_vol, a.dtype, a.math, st));
+        return;
       }
       const Tensor ws = !need_w[l] ? Tensor()
                         : need[s.src] ? bwd_workspace(grad(l + 1), value(s.src), ptr(w), grad(s.src), result[1 + l], imap.numel(), a, fp32_sums)
@@ -429,9 +504,20 @@ struct SparseStack : torch::autograd::Function<SparseStack> {
       else if (need_w[l])
         check_status(fgms_b200_wgrad(value(s.src), grad(l + 1), result[1 + l].data_ptr(), kpos, im, om, imap.numel(), n_in, n_out, c_in, c_out, k_vol,
                                      a.dtype, a.math, ws_ptr, ws_bytes, 1, st));
+    };
+    for (size_t l = n; l-- > 0;) {
+      const StackLayer s = layer_of(plan, l);
+      if (need[l + 1]) {
+        if (l + 1 < n) finish(l + 1, s.n_out * weights[l].size(2));
+        layer(l, s);
+        if (s.skip >= 0 && need[s.skip]) added[s.skip].push_back(l + 1);
+        else if (l + 1 < n) g_values.drop(l + 1);
+      }
+      values.drop(s.src);  // no other layer reads it
     }
     if (need[0]) {
       finish(0, feats.numel());
+      grad(0);
       result[0] = in.pad ? g_input.narrow(1, 0, feats.size(1)).contiguous() : g_input;
     }
     return result;

@@ -1,5 +1,6 @@
 """``nn.SparseUNet`` as one autograd node against its layers one by one: outputs and gradients, whichever inputs need one; what
 makes it run layer by layer; and the two small kernels behind it, at sizes that fill no vector and no block."""
+import contextlib
 import ctypes
 
 import pytest
@@ -12,8 +13,8 @@ pytestmark = pytest.mark.gpu
 SPEC = unet.minkunet_spec(4, (16, 32, 48))
 
 
-def _net(spec=SPEC, dtype=torch.float16, n=3000):
-    coords = torch.from_numpy(clouds.uniform_cloud(n, 20, 7)).cuda()
+def _net(spec=SPEC, dtype=torch.float16, n=3000, side=20):
+    coords = torch.from_numpy(clouds.uniform_cloud(n, side, 7)).cuda()
     umaps = unet.build_unet_maps(coords, (len(spec) - 1) // 6)
     torch.manual_seed(3)
     net = nn.SparseUNet(spec, dtype=dtype)
@@ -39,11 +40,11 @@ def _close(a, b, dtype):
     assert float((a.double() - b.double()).norm()) <= tol * float(b.double().norm())
 
 
-@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
-@pytest.mark.parametrize("needs", ["all", "weights", "input", "last", "frozen_middle", "first"])
-def test_one_node_equals_a_node_per_layer(dtype, needs):
-    net, umaps, feats, grad = _net(dtype=dtype)
-    params = list(net.parameters())
+NEEDS = ["all", "weights", "input", "last", "frozen_middle", "first"]
+
+
+def _compare(net, umaps, feats, grad, needs):
+    params, dtype = list(net.parameters()), feats.dtype
     for i, p in enumerate(params):
         p.requires_grad_({"all": True, "weights": True, "input": False, "last": i == len(params) - 1,
                           "frozen_middle": i % 3 != 1, "first": i == 0}[needs])
@@ -52,10 +53,96 @@ def test_one_node_equals_a_node_per_layer(dtype, needs):
     got, want = net(feats, umaps), _layer_by_layer(net, feats, umaps)
     assert got.grad_fn.name() != want.grad_fn.name()
     _close(got.detach(), want.detach(), dtype)
-    for a, b in zip(torch.autograd.grad(got, wanted, grad, retain_graph=True), torch.autograd.grad(want, wanted, grad)):
+    first, second = torch.autograd.grad(got, wanted, grad, retain_graph=True), torch.autograd.grad(want, wanted, grad)
+    for a, b in zip(first, second):
         _close(a, b, dtype)
-    for a, b in zip(torch.autograd.grad(got, wanted[-1:], grad), wanted[-1:]):  # a second backward, of one of them
-        assert a.shape == b.shape
+    # further backwards, of some of them: a layer in the middle, the last one, and the first and the last
+    middle = len(wanted) // 2
+    for some in ([middle], [len(wanted) - 1], [0, len(wanted) - 1]):
+        again = torch.autograd.grad(got, [wanted[i] for i in some], grad, retain_graph=some != [0, len(wanted) - 1])
+        for i, a in zip(some, again):
+            _close(a, second[i], dtype)
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(got, wanted[-1:], grad)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("needs", NEEDS)
+def test_one_node_equals_a_node_per_layer(dtype, needs):
+    _compare(*_net(dtype=dtype), needs)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("needs", NEEDS)
+def test_values_and_gradients_one_by_one(dtype, needs):
+    """120 MB of values, 240 in fp32: more than are held in one allocation."""
+    _compare(*_net(dtype=dtype, n=240000, side=160), needs)
+
+
+@contextlib.contextmanager
+def _no_more_than(extra):
+    """Of the memory that is reserved nothing is left that 1 MB fit in, and `extra` bytes can be reserved beyond it."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    limit, held = torch.cuda.get_device_properties(0).total_memory, []
+    try:
+        torch.cuda.set_per_process_memory_fraction(torch.cuda.memory_reserved() / limit)
+        for size in [1 << k for k in range(28, 19, -1)]:
+            with contextlib.suppress(torch.OutOfMemoryError):
+                while True:
+                    held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + extra) / limit)
+        yield
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+def test_a_step_takes_no_more_memory_than_a_node_per_layer():
+    net, umaps, feats, grad = _net(n=240000, side=160)
+    params = list(net.parameters())
+
+    def peak(forward):
+        torch.autograd.grad(forward(), params, grad)
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        torch.autograd.grad(forward(), params, grad)
+        return torch.cuda.max_memory_allocated() - before
+
+    assert peak(lambda: net(feats, umaps)) <= 1.02 * peak(lambda: _layer_by_layer(net, feats, umaps))
+
+
+def test_without_memory_for_all_gradients_at_once():
+    """Of 100 k voxels all values' gradients are 50 MB, those in use at a time 16."""
+    net, umaps, feats, grad = _net(n=100000, side=120)
+    feats.requires_grad_()
+    wanted = [feats] + list(net.parameters())
+    out = net(feats, umaps)
+    want = torch.autograd.grad(out, wanted, grad, retain_graph=True)
+    with _no_more_than(40 << 20):
+        with pytest.raises(torch.OutOfMemoryError):
+            torch.empty(48 << 20, dtype=torch.uint8, device="cuda")
+        got = torch.autograd.grad(out, wanted, grad)
+    for a, b in zip(got, want):
+        _close(a, b, torch.float16)
+
+
+def test_without_memory_for_all_values_at_once():
+    """200 MB are free, but in pieces of 18 MB (beyond them 16 for small tensors)."""
+    net, umaps, feats, grad = _net(n=100000, side=120)
+    params = list(net.parameters())
+    want = torch.autograd.grad(net(feats, umaps), params, grad)
+    with _no_more_than(236 << 20):
+        pieces = [torch.empty(2 << 20, dtype=torch.uint8, device="cuda") for _ in range(110)]
+        kept = pieces[::10]
+        del pieces
+        with pytest.raises(torch.OutOfMemoryError):
+            torch.empty(24 << 20, dtype=torch.uint8, device="cuda")
+        out = net(feats, umaps)
+        assert "Stack" in out.grad_fn.name()
+        got = torch.autograd.grad(out, params, grad)
+    assert len(kept) == 11
+    for a, b in zip(got, want):
+        _close(a, b, torch.float16)
 
 
 def test_no_gradients_and_in_place_changes():
