@@ -98,8 +98,9 @@ __device__ __forceinline__ void w3_stage(const G3Walk& w, int pb, const int* kpo
 
 // FULL: both row lengths are whole 128-byte pieces; the producers' copy loops then carry no per-chunk test.
 // PACKED: several pairs share a staged row (cfg.pack > 1); the unpacked instantiations carry none of its arithmetic.
-// TEAMS: of producers.
-template <bool TF32, bool FULL, bool PACKED, int TEAMS>
+// TEAMS: of producers.  PARTS: several CTAs share dW_k; with one for all of it a row's part is the row, and a kernel that distinguished them all the
+// same was 1.5 to 3 % slower for every whole gradient (417 k pairs 128 -> 128 23.1 / 23.4 us, 128 -> 64 19.8 / 20.4, packed with 72 bytes of spills).
+template <bool TF32, bool FULL, bool PACKED, int TEAMS, bool PARTS>
 __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams p, W3Config cfg) {
   using namespace umma;
   constexpr int TEAM_WARPS = W3_PROD_TEAMS * W3_PROD_WARPS / TEAMS;
@@ -121,8 +122,10 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_seg = p.k_vol + 1;
   volatile int* abort_flag = &sh->abort_flag;
-  const int part_a = (int)blockIdx.y % cfg.parts_a;
-  const int a0 = part_a * cfg.c_a, b0 = ((int)blockIdx.y - part_a) / cfg.parts_a * cfg.c_b;  // this CTA's first channels
+  // this CTA's channels of dW_k, and the first ones
+  const int c_a = PARTS ? cfg.c_a : p.c_in, c_b = PARTS ? cfg.c_b : p.c_out;
+  const int part_a = PARTS ? (int)blockIdx.y % cfg.parts_a : 0;
+  const int a0 = part_a * c_a, b0 = PARTS ? ((int)blockIdx.y - part_a) / cfg.parts_a * c_b : 0;
   const uint32_t lbo = (uint32_t)kr * 128u;  // next 128 bytes of every staged row
   const uint32_t buf_cols = (uint32_t)(cfg.n_mtile * cfg.n_acc);
 
@@ -166,7 +169,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
     const int rpw = pb / TEAM_WARPS;  // rows of a stage owned by this warp: 4, 8, 16 or 32
     const uint8_t* feats = static_cast<const uint8_t*>(p.feats);
     const uint8_t* og = static_cast<const uint8_t*>(p.out_grad);
-    const uint32_t a_row_bytes = (uint32_t)cfg.c_a * ES, b_row_bytes = (uint32_t)cfg.c_b * ES;  // of a row's part
+    const uint32_t a_row_bytes = (uint32_t)c_a * ES, b_row_bytes = (uint32_t)c_b * ES;  // of a row's part
     const uint32_t a_pitch = (uint32_t)p.c_in * ES, b_pitch = (uint32_t)p.c_out * ES;
     // Lane (rs, cc) = (lane / 8, lane % 8) copies 16-byte chunk cc of every 128-byte piece of the rows rs, rs + 4, ... of the warp's
     // block: one shuffle and one address per row, then one cp.async per piece at a fixed distance (128 bytes in global memory,
@@ -287,7 +290,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
       get = get == W3_PREFETCH * ring_step ? 0 : get + ring_step;
       // a pair is used only if both its entries are inside the tensors
       if (!((unsigned)cur_a < (unsigned)p.n_in && (unsigned)cur_b < (unsigned)p.n_out)) {
-        if (blockIdx.y == 0 && (cur_a != -1 || cur_b != -1)) report_problem();  // counted once per skipped pair
+        if ((!PARTS || blockIdx.y == 0) && (cur_a != -1 || cur_b != -1)) report_problem();  // counted once per skipped pair
         cur_a = cur_b = -1;
       }
       ok = g3_wait(&sh->empty[s], ph ^ 1u, abort_flag);
@@ -408,7 +411,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
         for (int mt = 0; mt < cfg.n_mtile; ++mt) {
           const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)buf * buf_cols + (uint32_t)(mt * cfg.n_acc);
           const bool m128 = mt + 1 < cfg.n_mtile || cfg.last_m == 128;
-          for (int c0 = 0; c0 < cfg.c_b; c0 += 64) {
+          for (int c0 = 0; c0 < c_b; c0 += 64) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {  // 16 columns at a time: few registers in flight
               uint32_t v[16], h[8];
@@ -428,7 +431,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
               if (m128) m = blk_ok ? mt * 128 + warp * 32 + (int)r - row_base : -1;
               else m = (r < 16 && blk_ok) ? mt * 128 + warp * 16 + (int)r - row_base : -1;
               const uint4 v = *reinterpret_cast<const uint4*>(patch + r * 128 + ((ch ^ (r & 7)) << 4));
-              if (m >= 0 && m < cfg.c_a && c0 + (int)(ch << 3) < cfg.c_b) red_add_h8(dwk16 + (size_t)m * p.c_out + c0 + (ch << 3), v.x, v.y, v.z, v.w);
+              if (m >= 0 && m < c_a && c0 + (int)(ch << 3) < c_b) red_add_h8(dwk16 + (size_t)m * p.c_out + c0 + (ch << 3), v.x, v.y, v.z, v.w);
             }
             __syncwarp();
           }
@@ -437,7 +440,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
       for (int mt = 0; mt < cfg.n_mtile; ++mt) {
         const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)buf * buf_cols + (uint32_t)(mt * cfg.n_acc);
         const bool m128 = mt + 1 < cfg.n_mtile || cfg.last_m == 128;
-        for (int c0 = 0; c0 < cfg.c_b; c0 += 32) {
+        for (int c0 = 0; c0 < c_b; c0 += 32) {
           uint32_t v0[16], v1[16];
           tmem_ld16(taddr + col_base + c0, v0);
           if (!PACKED || slot_n - c0 > 16) {
@@ -461,7 +464,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) umma_wgrad3_kernel(WgradParams 
             if (m128) m = blk_ok ? mt * 128 + warp * 32 + (int)r - row_base : -1;
             else m = (r < 16 && blk_ok) ? mt * 128 + warp * 16 + (int)r - row_base : -1;
             const uint4 v = *reinterpret_cast<const uint4*>(patch + r * 128 + ((ch ^ (r & 7)) << 4));
-            if (m >= 0 && m < cfg.c_a && c0 + (int)(ch << 2) < cfg.c_b)
+            if (m >= 0 && m < c_a && c0 + (int)(ch << 2) < c_b)
               red_add_v4(dwk + (size_t)m * p.c_out + c0 + (ch << 2), __uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
           }
           __syncwarp();
@@ -578,18 +581,23 @@ inline void w3_split(int c_in, int c_out, int es, int k_vol, long long pairs, in
   cfg->parts_b = n.b;
 }
 
-template <bool TF32, bool FULL, bool PACKED, int TEAMS>
+template <bool TF32, bool FULL, bool PACKED, int TEAMS, bool PARTS>
 inline int w3_launch_as(const WgradParams& p, const W3Config& cfg, cudaStream_t st, int sms, int max_smem) {
   static std::atomic<int> granted[64];
-  if (int rc = ensure_smem(umma_wgrad3_kernel<TF32, FULL, PACKED, TEAMS>, max_smem, granted)) return rc;
+  if (int rc = ensure_smem(umma_wgrad3_kernel<TF32, FULL, PACKED, TEAMS, PARTS>, max_smem, granted)) return rc;
   const int parts = cfg.parts_a * cfg.parts_b;
-  return launch_pdl(umma_wgrad3_kernel<TF32, FULL, PACKED, TEAMS>, dim3((unsigned)(sms / parts), (unsigned)parts), W3_THREADS, (size_t)cfg.smem, st, p, cfg) == cudaSuccess ? 0 : -1;
+  return launch_pdl(umma_wgrad3_kernel<TF32, FULL, PACKED, TEAMS, PARTS>, dim3((unsigned)(sms / parts), (unsigned)parts), W3_THREADS, (size_t)cfg.smem, st, p, cfg) == cudaSuccess ? 0 : -1;
+}
+template <bool TF32, bool FULL, bool PACKED, int TEAMS>
+inline int w3_launch_parts(const WgradParams& p, const W3Config& cfg, cudaStream_t st, int sms, int max_smem) {
+  return cfg.parts_a * cfg.parts_b > 1 ? w3_launch_as<TF32, FULL, PACKED, TEAMS, true>(p, cfg, st, sms, max_smem)
+                                       : w3_launch_as<TF32, FULL, PACKED, TEAMS, false>(p, cfg, st, sms, max_smem);
 }
 template <bool TF32, bool FULL, bool PACKED>
 inline int w3_launch_teams(const WgradParams& p, const W3Config& cfg, cudaStream_t st, int sms, int max_smem) {
   const bool few = p.pairs / cfg.pb + p.k_vol / 2 <= W3_ONE_TEAM_STAGES * (sms / (cfg.parts_a * cfg.parts_b));  // (an offset's last stage is half empty on average)
-  return few ? w3_launch_as<TF32, FULL, PACKED, 1>(p, cfg, st, sms, max_smem)
-             : w3_launch_as<TF32, FULL, PACKED, W3_PROD_TEAMS>(p, cfg, st, sms, max_smem);
+  return few ? w3_launch_parts<TF32, FULL, PACKED, 1>(p, cfg, st, sms, max_smem)
+             : w3_launch_parts<TF32, FULL, PACKED, W3_PROD_TEAMS>(p, cfg, st, sms, max_smem);
 }
 template <bool TF32>
 inline int w3_launch(const WgradParams& p, const W3Config& cfg, cudaStream_t st, int sms, int max_smem) {
