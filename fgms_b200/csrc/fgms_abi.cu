@@ -22,6 +22,7 @@
 #include "umma_gms3.cuh"
 #include "umma_wgrad3.cuh"
 #include "rows_wgrad.cuh"
+#include "backward_share.cuh"
 #include "peer_exchange.cuh"
 #include "umma_osfwd.cuh"
 
@@ -218,70 +219,6 @@ struct Range {
     return a < b + o.bytes && b < a + bytes;
   }
 };
-
-// SMs of the weight gradient where the two passes of a backward share the chip; 0: each has all of it.
-//
-// Side by side the passes overlap each other's fixed parts (launch, tile table, first rows; the sums' way out) and what they are
-// bound by, reds of rows in the input gradient, instructions of the gathers in the weight gradient.  The weight gradient goes
-// first, with one block per SM on its share; the input gradient's blocks find room on the others only.  Either pass takes about
-// c + u * (128-pair units) / SMs microseconds; the share is the one at which the later one ends first.  Behind one another / started
-// together but with all SMs each / with the share, in a row of launches: fp16 64 -> 64 0.93 M pairs 69.0 / 66.0 / 61.9 us, 137 k 19.8 / 18.9 / 15.2,
-// 32 -> 32 9.1 M 254 / 252 / 237, 84 k 12.1 / 10.3 / 7.9; 128 -> 128 303 k 44.5 / 44.2 / 37.5.  A share a sixth off gives the gain away (64 -> 64
-// 0.93 M pairs at 0.36 / 0.48 / 0.60 of the SMs 77.9 / 61.4 / 78.1).
-//
-// With the weight gradient on tcgen05 the constants are fitted to the passes side by side: 151 shapes and sizes (16 to 256 channels, 300 to
-// 0.44 M pairs) times 16 shares.  The share is within 2.6 % of the best of the 16 on average, 19 % at worst; with constants fitted to each pass by
-// itself it was 11.6 % off (256 -> 256 on 39 k pairs 23.6 -> 19.0 us, best 18.8, 128 -> 256 on 98 k 26.3 -> 21.6, stride 2 256 -> 256 on 9 k 14.0 -> 11.3, best
-// 9.5): the input gradient, launched second, takes 1.5 to 5 us longer than by itself.  On maps of few pairs a row
-// (LiDAR and scattered clouds, about two) the rows come from memory rather than from L2, the weight gradient's from both sides: a fifth more for it
-// (passes on new rows each time, 128 -> 128 on 303 k LiDAR pairs 91.6 -> 89.4 us, 96 -> 160 on 110 k 53.8 -> 52.6; stride-2 maps need none).  Slower than
-// with the constants before by up to 2 %: 128 -> 64 on 173 k LiDAR pairs 52.9 -> 53.9.  Rows of up to 64 channels on both sides keep the constants of each pass by itself, within
-// 10 % of the best; 0.97 and 1.07 are the margins of "behind one another", and the terms for 48 channels, whose rows are copied
-// with idle lanes, are fitted like the others.
-int split_backward(int64_t pairs, int rows, int c_in, int c_out, int k_vol, int dtype, int math, const DeviceInfo& di) {
-  fgms::G3Config g;
-  fgms::W3Config w;
-  const bool f16 = dtype == FGMS_DTYPE_F16;
-  const int es = f16 ? 2 : 4;
-  // (the CUDA-core kernels have several small blocks on every SM and overlap as they are)
-  if (math == FGMS_MATH_FP32 || !fgms::g3_plan(c_in, c_out, es, k_vol, di.max_smem_optin, true, &g) ||
-      !fgms::w3_plan(c_in, c_out, es, k_vol, di.max_smem_optin, &w) || di.sms < 16)
-    return 0;
-  const double both = c_in + c_out, area = (double)c_in * c_out;
-  const int blocks = (c_in * es + 127) / 128;  // of an output row of the input gradient
-  const bool short_d = fgms::rw_supported(c_out, c_in, f16), short_w = fgms::wh_supported(c_in, c_out, f16);
-  double c_d, u_d, c_w, u_w, units = (double)pairs / 128 + k_vol;
-  if (short_w) {
-    c_d = 4, u_d = 0.1 + 0.1 * g.kch + 0.43 * blocks;
-    if (short_d) c_d = 3.5, u_d = both * (f16 ? 0.0046 : 0.01);
-    c_w = 5 + area / 2048;
-    u_w = (f16 ? 0.094 + 0.026 * area / 256 + 0.075 * ((c_in == 48) + (c_out == 48))
-               : 0.1 + 0.003 * both + 0.035 * area / 256 + 0.1 * ((c_in == 48) + (c_out == 48)));
-  } else {
-    units = (double)pairs / 128 + 0.5 * k_vol;
-    // 128-byte pieces of the two rows; a last one that is filled in part counts for half of the rest as well
-    const double in = 0.5 * (g.kch + c_out * es / 128.0), out = 0.5 * (blocks + c_in * es / 128.0);
-    c_d = 5.6 + 0.19 * in + 0.2 * out, u_d = 0.05 + 0.182 * in + 0.397 * out;
-    if (short_d) c_d = 5.5, u_d = both * (f16 ? 0.0046 : 0.01);
-    c_w = u_w = 0;  // by its plan, which depends on the share
-  }
-  const bool few = k_vol > 8 && pairs < 4ll * rows;
-  int best = 0;
-  double least = 1e30;
-  // behind one another, where the input gradient on all SMs meets L2's rate of reds
-  if (short_w) least = 0.97 * (c_d + c_w - 2 + (1.07 * u_d + u_w) * units / di.sms);
-  for (int s = di.sms / 4; s <= di.sms - di.sms / 4; s += 2) {
-    if (!short_w && (s == di.sms / 4 || !fgms::w3_same_split(c_in, c_out, es, k_vol, pairs, s - 2, s))) {
-      fgms::w3_plan(c_in, c_out, es, k_vol, di.max_smem_optin, &w);
-      fgms::w3_split(c_in, c_out, es, k_vol, pairs, s, di.max_smem_optin, &w);
-      c_w = 5.9 + (w.n_buf == 1 ? 3.01 : 1.02) * w.c_a * w.c_b * es / 32768;
-      u_w = (few ? 1.2 : 1.0) * w.parts_a * w.parts_b * (0.264 + 0.025 * (w.pa + w.pbp) / w.pack + 0.336 * (128.0 / w.pb));
-    }
-    const double d = c_d + u_d * units / (di.sms - s), v = c_w + u_w * units / s, end = d > v ? d : v;
-    if (end < least) { least = end; best = s; }
-  }
-  return best;
-}
 
 int check_dgrad_args(const void* out_grad, const void* kernel, const void* in_grad, const int32_t* kpos, const int32_t* in_map,
                      const int32_t* out_map, int64_t map_len, int n_in, int n_out, int c_in, int c_out, int k_vol, int dtype, int math) {
@@ -656,7 +593,8 @@ int fgms_b200_bwd(const void* out_grad, const void* in_feats, const void* kernel
                          reinterpret_cast<uintptr_t>(in_grad) | reinterpret_cast<uintptr_t>(kernel_grad)) & 15) == 0;
   Beside beside;
   beside.on = true;
-  const int wgrad_sms = !aligned ? 0 : split_backward(map_len, n_in > n_out ? n_in : n_out, c_in, c_out, k_vol, dtype, math, di);
+  // (the CUDA-core kernels have several small blocks on every SM and overlap as they are)
+  const int wgrad_sms = !aligned || math == FGMS_MATH_FP32 ? 0 : fgms::split_backward(map_len, n_in, n_out, c_in, c_out, k_vol, dtype == FGMS_DTYPE_F16, di.sms, di.max_smem_optin);
   if (wgrad_sms > 0) beside.sms = di.sms - wgrad_sms;
   if (int rc = wgrad(wgrad_sms)) return rc;
   return dgrad(beside);

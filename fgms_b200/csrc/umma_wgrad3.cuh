@@ -568,9 +568,6 @@ inline W3Parts w3_parts(int c_in, int c_out, int es, int k_vol, long long pairs,
   if (c_out % (16 * b)) b = 1;
   return {a, b};
 }
-inline bool w3_same_split(int c_in, int c_out, int es, int k_vol, long long pairs, int sms, int other) {
-  return w3_parts(c_in, c_out, es, k_vol, pairs, sms) == w3_parts(c_in, c_out, es, k_vol, pairs, other);
-}
 // the plan of such a block in place of the whole one
 inline void w3_split(int c_in, int c_out, int es, int k_vol, long long pairs, int sms, int max_smem, W3Config* cfg) {
   const W3Parts n = w3_parts(c_in, c_out, es, k_vol, pairs, sms);
