@@ -34,3 +34,14 @@ def test_a_skipped_pair_is_counted_once():
     backend.device_status(reset=True)
     p.run_fwd()
     assert backend.device_status(reset=True) == 2
+
+
+@pytest.mark.parametrize("rows", [1, 127, 129, lambda s: 128 * (s // 4 - 3) - 1, lambda s: 128 * (s // 2 - 2) + 1])
+@pytest.mark.parametrize("mode,c_in,c_out", [("fp16", 128, 256), ("fp16", 96, 192), ("tf32", 64, 128)])
+def test_parts_of_a_tile_with_a_separate_centre(mode, c_in, c_out, rows):
+    """The centre's rows are a segment of their own, which the line counts too."""
+    n = rows if isinstance(rows, int) else rows(_sms())
+    p = Problem(_map(n, [min(n, c) for c in (40, 1, 0, 130, 7)], 3), c_in, c_out, seed=n, mode=mode)
+    backend.device_status(reset=True)
+    assert err(p.run_fwd(separate_mid=True, fused=False), p.ref_fwd(precompute=True)) <= TOL[mode]
+    assert backend.device_status() == 0

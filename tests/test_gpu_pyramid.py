@@ -1,10 +1,12 @@
 """The pyramid builder (``csrc/map_pyramid.cuh``): every map of every level equals the host builders' bit for bit, for rows
 in any order, boxes around the 32-cell words of its bitmaps, and clouds it has to leave to the hash-table builders."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
-from fgms_b200 import clouds, unet
+from fgms_b200 import _lib, clouds, unet
 from tests.test_gpu_maps import _dev, _same
 
 pytestmark = pytest.mark.gpu
@@ -64,3 +66,33 @@ def test_every_map_has_memory_of_its_own():
     before = [k.imap._version for k in maps]
     maps[0].imap[:1] = maps[0].imap[:1].clone()
     assert [k.imap._version for k in maps[1:]] == before[1:]
+
+
+def test_counts_of_more_blocks_of_rows_than_a_warp_keeps():
+    """A warp keeps the counts of 512 blocks of 256 rows: 131 072 rows.  175 616 are read again, 16 384 at a time."""
+    coords = _block(56, 56, 56)
+    _check(unet.build_unet_maps(_dev(coords), 1), unet.build_unet_maps_host(coords, 1))
+
+
+@pytest.mark.parametrize("levels,what", [(1, 1), (3, 7), (5, 6)])
+def test_sizes_in_memory_that_is_not_page_locked(levels, what):
+    """The kernel writes page-locked sizes itself; others, written by a copy, are the same, and so are kpos and the coordinates."""
+    coords = _dev(np.unique(clouds.surface_cloud(5000, 64, 9), axis=0))
+    n, n_maps = coords.size(0), sum(levels - (kind > 1) for kind in (1, 2, 4) if what & kind)
+    ws = torch.empty(_lib.lib.fgms_b200_pyramid_workspace_bytes(n, levels, what), dtype=torch.uint8, device="cuda")
+
+    def plan(sizes_at):
+        kpos = torch.zeros((n_maps, 28), dtype=torch.int32, device="cuda")
+        coarser = [torch.zeros((n, 3), dtype=torch.int32, device="cuda") for _ in range(levels - 1)]
+        at = (ctypes.c_void_p * max(1, levels - 1))(*[c.data_ptr() for c in coarser])
+        _lib.check(_lib.lib.fgms_b200_pyramid_plan(coords.data_ptr(), n, levels, what, kpos.data_ptr(), at, ws.data_ptr(), ws.numel(), sizes_at,
+                                                   torch.cuda.current_stream().cuda_stream))
+        return [kpos] + coarser
+
+    count = 1 + levels + n_maps
+    locked, pageable = torch.full((count + 1,), 77, dtype=torch.int32, pin_memory=True), (ctypes.c_int32 * (count + 1))(*[77] * (count + 1))
+    a, b = plan(locked.data_ptr()), plan(ctypes.addressof(pageable))
+    assert locked.tolist() == list(pageable) and pageable[0] == 0 and pageable[1] == n and pageable[count] == 77
+    assert all(torch.equal(x, y) for x, y in zip(a, b))
+    for j in range(n_maps):
+        assert pageable[1 + levels + j] == int(a[0][j].max())

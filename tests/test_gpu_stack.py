@@ -2,6 +2,7 @@
 makes it run layer by layer; and the two small kernels behind it, at sizes that fill no vector and no block."""
 import contextlib
 import ctypes
+import gc
 
 import pytest
 import torch
@@ -40,6 +41,25 @@ def _close(a, b, dtype):
     assert float((a.double() - b.double()).norm()) <= tol * float(b.double().norm())
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("needs", ["all", "weights", "input", "last", "frozen_middle", "first"])
+def test_one_node_equals_a_node_per_layer(dtype, needs):
+    net, umaps, feats, grad = _net(dtype=dtype)
+    params = list(net.parameters())
+    for i, p in enumerate(params):
+        p.requires_grad_({"all": True, "weights": True, "input": False, "last": i == len(params) - 1,
+                          "frozen_middle": i % 3 != 1, "first": i == 0}[needs])
+    feats.requires_grad_(needs in ("all", "input", "frozen_middle"))
+    wanted = [t for t in [feats] + params if t.requires_grad]
+    got, want = net(feats, umaps), _layer_by_layer(net, feats, umaps)
+    assert got.grad_fn.name() != want.grad_fn.name()
+    _close(got.detach(), want.detach(), dtype)
+    for a, b in zip(torch.autograd.grad(got, wanted, grad, retain_graph=True), torch.autograd.grad(want, wanted, grad)):
+        _close(a, b, dtype)
+    for a, b in zip(torch.autograd.grad(got, wanted[-1:], grad), wanted[-1:]):  # a second backward, of one of them
+        assert a.shape == b.shape
+
+
 NEEDS = ["all", "weights", "input", "last", "frozen_middle", "first"]
 
 
@@ -68,7 +88,7 @@ def _compare(net, umaps, feats, grad, needs):
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
 @pytest.mark.parametrize("needs", NEEDS)
-def test_one_node_equals_a_node_per_layer(dtype, needs):
+def test_further_backwards_over_a_retained_graph(dtype, needs):
     _compare(*_net(dtype=dtype), needs)
 
 
@@ -82,6 +102,7 @@ def test_values_and_gradients_one_by_one(dtype, needs):
 @contextlib.contextmanager
 def _no_more_than(extra):
     """Of the memory that is reserved nothing is left that 1 MB fit in, and `extra` bytes can be reserved beyond it."""
+    gc.collect()  # what earlier tests left in cycles would otherwise be handed back at any time
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     limit, held = torch.cuda.get_device_properties(0).total_memory, []
@@ -95,6 +116,73 @@ def _no_more_than(extra):
         yield
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+def _in_64_bits(net, umaps, feats, grad, wanted):
+    """The same layers in plain PyTorch, fp64: output and gradients."""
+    twin = {t: t.detach().double().requires_grad_() for t in wanted}
+    val = {"input": twin.get(feats, feats.double())}
+    for spec, layer in zip(net.spec, net.layers):
+        km, x, w = umaps.of(spec), val[spec.src], twin.get(layer.weight, layer.weight.detach().double())
+        at, im, om = km.kpos.tolist(), km.imap.long(), km.omap.long()
+        y = torch.zeros((km.n_out, w.size(2)), dtype=torch.double, device="cuda")
+        for k in range(w.size(0)):
+            y = y.index_add(0, om[at[k]:at[k + 1]], x[im[at[k]:at[k + 1]]] @ w[k])
+        val[spec.dst] = y if spec.skip is None else y + val[spec.skip]
+    out = val[net.spec[-1].dst]
+    return out.detach(), torch.autograd.grad(out, [twin[t] for t in wanted], grad.double())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_against_64_bits(dtype):
+    # a layer rounds its inputs (tf32) or up to ten partial sums of a row (fp16) to 11 bits: 1e-3 relative at most, and 13 layers
+    # there and 13 back in quadrature 5e-3; the bound is _close's
+    net, umaps, feats, grad = _net(dtype=dtype)
+    feats.requires_grad_()
+    wanted = [feats] + list(net.parameters())
+    got = net(feats, umaps)
+    out, grads = _in_64_bits(net, umaps, feats, grad, wanted)
+    _close(got.detach(), out, dtype)
+    for a, b in zip(torch.autograd.grad(got, wanted, grad), grads):
+        _close(a, b, dtype)
+
+
+def test_layers_of_a_million_pairs():
+    """The finest layers take the kernel for both gradients, with a workspace."""
+    net, umaps, feats, grad = _net(n=60000, side=40)
+    assert umaps.subm[0].imap.numel() > 1 << 20
+    feats.requires_grad_()
+    wanted = [feats] + list(net.parameters())
+    got, want = net(feats, umaps), _layer_by_layer(net, feats, umaps)
+    _close(got.detach(), want.detach(), torch.float16)
+    for a, b in zip(torch.autograd.grad(got, wanted, grad), torch.autograd.grad(want, wanted, grad)):
+        _close(a, b, torch.float16)
+
+
+@pytest.mark.parametrize("n,side", [(3000, 20), (240000, 160)])  # two allocations, and one by one
+def test_on_another_stream_and_in_a_captured_graph(n, side):
+    net, umaps, feats, grad = _net(n=n, side=side)
+    params = list(net.parameters())
+
+    def step():
+        out = net(feats, umaps)
+        return (out.detach(), *torch.autograd.grad(out, params, grad))
+
+    want, stream = step(), torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        for a, b in zip(step(), want):
+            _close(a, b, torch.float16)
+    torch.cuda.current_stream().wait_stream(stream)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = step()
+    for t in got:
+        t.fill_(float("nan"))
+    for _ in range(2):
+        graph.replay()
+    for a, b in zip(got, want):
+        _close(a, b, torch.float16)
 
 
 def test_a_step_takes_no_more_memory_than_a_node_per_layer():
