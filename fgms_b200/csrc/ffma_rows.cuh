@@ -275,8 +275,9 @@ constexpr int FW_PAIRS = 64;    // pairs of a chunk in shared memory, and of a s
 constexpr int FW_BLOCK = 64;    // channels of a block of dW_k on either side
 
 // Block threads: `slices` groups of rg x cg threads, each thread eight input by four output channels; slice s takes pairs
-// s, s + slices, .. of a chunk.  Sums stay in registers over the block's whole run inside one offset, those of 32 to 64 pairs at a time and
-// the total of these (relative error 64 -> 64 on 591 k pairs 6.5e-7 -> 1.9e-7, 20 -> 36 2.3e-7 -> 1.5e-7; the same time); then the slices meet
+// s, s + slices, .. of a chunk.  Sums stay in registers over the block's whole run inside one offset, those of 21 to 64 pairs at a time and
+// the total of these (relative error 64 -> 64 on 591 k pairs 6.5e-7 -> 1.9e-7, 20 -> 36 2.3e-7 -> 1.5e-7; the same time, but for three and five
+// slices, of 21 and 26 pairs, 40 -> 32 on 418 k 52.1 -> 53.1 us; of 43 pairs 52.0, and a tenth less exact); then the slices meet
 // in shared memory and leave with one red per value.
 template <int BLOCKS>
 __global__ void __launch_bounds__(FF_THREADS, BLOCKS) ffma_wgrad_kernel(WgradParams p) {

@@ -380,6 +380,10 @@ inline bool wh_supported(int c_in, int c_out, bool f16) {
 // registers of eight warps or more (64 -> 48 on 591 k pairs with the four that are left 52.6 us, 42.2 by two kernels; with the weights
 // in shared memory 64 -> 64 67.7 / 61.6).  And the pairs from which clearing and rounding the sums, 2.5 us, are paid for, us by two
 // kernels / this one: 32 -> 64 on 591 k pairs 27.1 / 28.0, on 1.13 M 45.8 / 45.1; 32 -> 32 on 364 k 14.6 / 15.9, on 591 k 19.7 / 20.5.
+// Above the line 12 shapes on surfaces, scattered and full clouds and strided maps of 1.1 to 4.6 M pairs take 0.71 to 1.03 of two kernels' time, but for
+// two kinds, which stay here because the sums are rounded once (2.1e-4 against 4.0e-4): 32 -> 48 submanifold up to 2.2 M pairs, 1.08 M 47.4 / 50.1; and
+// stride-2 maps with no fewer input than output channels, whose input gradient is one red a row into memory: 32 -> 32 on 1.2 M 48.9 / 50.8, on
+// 3 M 119 / 139, 64 -> 32 on 1.2 M 86.7 / 95.6.  (Transposed 64 -> 32 67.5 / 60.8, stride 2 32 -> 64 58.1 / 53.8.)
 constexpr bool wh_both_shape(int mu, int nu) { return mu * nu <= 8; }
 constexpr long long WH_BOTH_PAIRS = 1 << 20;
 

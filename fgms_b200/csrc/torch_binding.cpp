@@ -283,7 +283,7 @@ bool stack_suits(const Tensor& feats, at::TensorList weights, at::TensorList map
 struct SparseStack : torch::autograd::Function<SparseStack> {
   // What the node keeps, in elements: the values that layers 0 .. n - 2 produce (slots 1 .. n - 1) and, where the input's few fp16
   // channels are padded to a multiple of 16 (8-byte rows cannot be gathered in 16-byte pieces and would run on the CUDA cores: 4 -> 32
-  // on 84 k pairs 16 / 42 us forward / weight gradient, padded 4.5 / 5), the padded input (slot 0) and the weights that go with it (slot n).
+  // on 84 k pairs 16.6 / 45 us forward / weight gradient, padded 4.9 / 6.2), the padded input (slot 0) and the weights that go with it (slot n).
   struct Layout {
     std::vector<int64_t> count, at;  // of a slot; its place in a block of all of them, from a 256-byte boundary
     int64_t end = 0;                 // of that block
